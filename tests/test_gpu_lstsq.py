@@ -115,3 +115,46 @@ def test_rcond_and_wide_rank_deficient(lib, oracle):
     x, res, rk, sv = la.lstsq(W, bw)
     assert rk == 3 and res.size == 0
     np.testing.assert_allclose(x, np.linalg.pinv(W) @ bw, rtol=1e-8, atol=1e-10)
+
+
+@pytest.mark.parametrize("m,n,k", [
+    (63, 31, 1), (64, 31, 1), (64, 32, 9), (65, 33, 2), (127, 63, 1), (128, 64, 20),  # both sides of the reduction's rule
+    (64, 1, 2), (65, 2, 8), (200, 3, 17), (20, 130, 11), (31, 63, 1), (1, 100, 3), (340, 64, 16), (23, 24, 5)])
+def test_reduced_and_direct_sweeps(lib, m, n, k):
+    """Problems at the edges of the reduction to the triangle (max >= 2 min, max >= 64), odd and
+    even column counts, right-hand sides in one group and in several, against numpy's SVD: a
+    backward-stable solution is within a few (m + n) eps cond of it, singular values within a few
+    (m + n) eps of s_max."""
+    rng = np.random.default_rng(m * 131 + n * 7 + k)
+    A = rng.standard_normal((3, m, n))
+    B = rng.standard_normal((3, m, k))
+    X, S, resid = np.zeros((3, n, k)), np.zeros((3, min(m, n))), np.zeros((3, k))
+    rank, has = np.zeros(3, np.int32), np.zeros(3, np.int32)
+    P = _lib.ptr
+    rc = lib.nppb_lstsq_batched(3, m, n, k, P(A), P(B), -1.0, P(X), P(S), P(rank), P(resid), P(has))
+    assert rc == _lib.OK, _lib.last_error()
+    eps = np.finfo(float).eps
+    for i in range(3):
+        s = np.linalg.svd(A[i], compute_uv=False)
+        x = np.linalg.pinv(A[i]) @ B[i]
+        cond = s[0] / s[-1]
+        np.testing.assert_allclose(S[i], s, rtol=0, atol=20 * (m + n) * eps * s[0])
+        assert rank[i] == min(m, n) and has[i] == (m > n)
+        assert np.linalg.norm(X[i] - x) <= 50 * (m + n) * eps * cond ** 2 * max(np.linalg.norm(x), 1.0)
+        if m > n:
+            r = ((A[i] @ x - B[i]) ** 2).sum(axis=0)
+            np.testing.assert_allclose(resid[i], r, rtol=0, atol=100 * (m + n) * eps * (B[i] ** 2).sum(axis=0).max())
+
+
+def test_nan_and_infinity_stay_where_they_are(lib):
+    """A NaN (or an infinity) in one column is that column's singular value; the other values are
+    those of the matrix without it, in tall problems (reduced to the triangle when finite) too."""
+    rng = np.random.default_rng(11)
+    for bad in (np.nan, np.inf):
+        for col in (0, 4, 9):
+            A, b = rng.standard_normal((100, 10)), rng.standard_normal(100)
+            A[17, col] = bad
+            sv = la.lstsq(A, b)[3]
+            assert np.count_nonzero(np.isfinite(sv)) == 9
+            np.testing.assert_allclose(np.sort(sv[np.isfinite(sv)])[::-1],
+                                       np.linalg.svd(np.delete(A, col, 1), compute_uv=False), rtol=1e-12)

@@ -10,6 +10,7 @@
 #include "../../include/numpp_b200.h"
 #include "plan.hpp"
 #include "runtime.hpp"
+#include "sys.hpp"
 
 using namespace nppb;
 
@@ -98,6 +99,31 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
   if ((flags & NPPB_WANT_SLOGDET) && (!dSign || !dLogabs)) return arg_error("slogdet needs Sign and Logabs");
   if ((flags & NPPB_WANT_LU) && nn && (!dLU || !dipiv)) return arg_error("keeping factors needs LU and ipiv");
   if (!device()) return NPPB_E_NODEV;
+  if (n > 32 && n <= kSysMaxN && !(flags & NPPB_WANT_LU)) {
+    // one CTA per system for the whole factorisation, one per strip for the solves
+    DevMem w_m, perm_m, dinv_m, state_m;
+    NPPB_RC(scratch<double>(w_m, (size_t)count * n * sys_ld(n), st));
+    NPPB_RC(scratch<int32_t>(perm_m, (size_t)count * n, st));
+    NPPB_RC(scratch<double>(dinv_m, (size_t)count * sys_dinv(n), st));
+    NPPB_RC(scratch<int32_t>(state_m, (size_t)count, st));
+    SysArgs sa{};
+    sa.A = dA;
+    sa.W = w_m.as<double>();
+    sa.perm = perm_m.as<int32_t>();
+    sa.dinv = dinv_m.as<double>();
+    sa.state = state_m.as<int32_t>();
+    sa.B = dB; sa.X = dX; sa.inv = dInv;
+    sa.det = (flags & NPPB_WANT_DET) ? dDet : nullptr;
+    sa.sign = (flags & NPPB_WANT_SLOGDET) ? dSign : nullptr;
+    sa.logabs = (flags & NPPB_WANT_SLOGDET) ? dLogabs : nullptr;
+    sa.info = dinfo;
+    sa.un = n;
+    sa.unrhs = (flags & NPPB_WANT_SOLVE) ? nrhs : 0;
+    sa.uinv = (flags & NPPB_WANT_INV) ? 1 : 0;
+    NPPB_CUDA(launch_sys_lu(sa, nullptr, (int)count, n, st), "batched LU launch");
+    NPPB_CUDA(launch_sys_solve(sa, nullptr, 0, (int)count, n, st), "batched substitution launch");
+    return NPPB_OK;
+  }
   if (n > 32 && !(flags & NPPB_WANT_LU)) {
     // step-wise kernels in uniform mode: workspace and per-system scratch only
     DevMem lu_m, sc_m;
@@ -176,6 +202,22 @@ int d_getrs(int64_t count, int32_t n, int32_t nrhs, const double* dLU, const int
   if (count == 0 || n == 0 || nrhs == 0) return NPPB_OK;
   if (!dLU || !dipiv || !dB || !dX) return arg_error("getrs needs LU, ipiv, B and X");
   if (!device()) return NPPB_E_NODEV;
+  if (n > 32 && n <= kSysMaxN) {
+    DevMem perm_m, dinv_m;
+    NPPB_RC(scratch<int32_t>(perm_m, (size_t)count * n, st));
+    NPPB_RC(scratch<double>(dinv_m, (size_t)count * sys_dinv(n), st));
+    SysArgs sa{};
+    sa.W = const_cast<double*>(dLU);
+    sa.w_by_position = 1;
+    sa.perm = perm_m.as<int32_t>();
+    sa.dinv = dinv_m.as<double>();
+    sa.B = dB; sa.X = dX;
+    sa.un = n;
+    sa.unrhs = nrhs;
+    NPPB_CUDA(launch_sys_prepare(sa, dipiv, nullptr, (int)count, n, st), "getrs preparation launch");
+    NPPB_CUDA(launch_sys_solve(sa, nullptr, 0, (int)count, n, st), "getrs launch");
+    return NPPB_OK;
+  }
   if (n > 32) {
     int rc = NPPB_OK;
     auto pl = uniform_plan(count, n, nrhs, NPPB_WANT_SOLVE, true, false, &rc);

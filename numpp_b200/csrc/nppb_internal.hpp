@@ -20,6 +20,8 @@ struct SysDesc {
   int64_t b_off;    // B and X (n x nrhs)
   int64_t inv_off;  // inverse output (n x n), < 0 = none
   int64_t piv_off;  // ipiv (n int32)
+  int64_t perm_off; // system-resident path: position -> row (n int32)
+  int64_t dinv_off; //   and the diagonal blocks' inverses (sys_dinv(n) doubles)
 };
 
 // What a launch produces for each system.

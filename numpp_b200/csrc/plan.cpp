@@ -97,7 +97,8 @@ Plan::~Plan() {
   if (done) cudaEventDestroy(done);
   if (cap) cudaStreamDestroy(cap);
   for (void* p : {(void*)d_desc, (void*)d_order, (void*)d_lu, (void*)d_piv, (void*)d_scratch,
-                  (void*)d_step_list, (void*)d_items, (void*)d_back})
+                  (void*)d_step_list, (void*)d_items, (void*)d_back, (void*)d_sys_list, (void*)d_sys_items,
+                  (void*)d_perm, (void*)d_dinv, (void*)d_state})
     if (p) {
       if (alloc_stream) cudaFreeAsync(p, alloc_stream);
       else cudaFree(p);
@@ -131,8 +132,10 @@ int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_
   std::vector<SysDesc> desc(cnt);
   static constexpr int kWarpBounds[3] = {8, 16, 32};
   std::vector<std::vector<int32_t>> warp_members(3);
-  std::vector<int32_t> step_members;
-  int64_t lu = 0, piv = 0;
+  std::vector<int32_t> sys_members, step_members;
+  // orders 33..512 whose factors are not kept: one CTA per system
+  const bool resident = own_lu && !solve_only && !(fl & NPPB_WANT_LU);
+  int64_t lu = 0, piv = 0, perm = 0, dinv = 0;
   for (int64_t i = 0; i < cnt; ++i) {
     const int ni = n[i];
     const int ki = solve ? nrhs[i] : 0;
@@ -149,12 +152,20 @@ int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_
     s.idx = (int32_t)i;
     s.pad_ = -1;
     s.a_off = a_off[i];
+    const bool sys = resident && ni > 32 && ni <= kSysMaxN;
+    if (sys) lu = (lu + 3) & ~int64_t{3};
     s.lu_off = ext_factors ? lu_off_ext[i] : own_lu ? lu : a_off[i];
+    s.perm_off = perm;
+    s.dinv_off = dinv;
     s.b_off = solve ? b_off[i] : 0;
     s.inv_off = (want_inv && inv_off[i] >= 0) ? inv_off[i] : -1;
     s.piv_off = ext_factors ? piv_off_ext[i] : piv;
-    lu += (int64_t)ni * ni;
+    lu += (int64_t)ni * (sys ? sys_ld(ni) : ni);
     piv += ni;
+    if (sys) {
+      perm += ni;
+      dinv += sys_dinv(ni);
+    }
     a_elems = std::max(a_elems, a_off[i] + (int64_t)ni * ni);
     if (solve) b_elems = std::max(b_elems, b_off[i] + (int64_t)ni * ki);
     if (s.inv_off >= 0) inv_elems = std::max(inv_elems, s.inv_off + (int64_t)ni * ni);
@@ -162,6 +173,8 @@ int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_
       int c = 0;
       while (ni > kWarpBounds[c]) ++c;
       warp_members[c].push_back((int32_t)i);
+    } else if (sys) {
+      sys_members.push_back((int32_t)i);
     } else {
       step_members.push_back((int32_t)i);
     }
@@ -188,6 +201,38 @@ int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_
     kind_flops[kKindWarp] += wc.flops;
     warp_classes.push_back(wc);
     order.insert(order.end(), mb.begin(), mb.end());
+  }
+
+  // system-resident set: descending order, slot = rank; a class per number of
+  // 32-row blocks, the strips of each with the most columns first
+  std::stable_sort(sys_members.begin(), sys_members.end(),
+                   [&](int32_t x, int32_t y) { return desc[x].n > desc[y].n; });
+  nsys = (int64_t)sys_members.size();
+  std::vector<SysItem> sys_items;
+  for (int64_t r = 0; r < nsys;) {
+    SysClass sc;
+    sc.first = r;
+    sc.nmax = desc[sys_members[r]].n;
+    sc.item_first = (int64_t)sys_items.size();
+    for (; r < nsys && sys_blocks(desc[sys_members[r]].n) == sys_blocks(sc.nmax); ++r) {
+      SysDesc& s = desc[sys_members[r]];
+      s.pad_ = (int32_t)r;
+      add_cost(s, sys_flops, sys_bytes);
+      const double nd = s.n, cols = (solve ? s.nrhs : 0) + (s.inv_off >= 0 ? nd : 0.0);
+      kind_flops[kKindUpdate] += 2.0 / 3.0 * nd * nd * nd;
+      kind_flops[kKindBack] += 2.0 * nd * nd * cols;
+      auto strips = [&](int16_t inverse, int columns) {
+        for (int c = 0; c < columns; c += 32)
+          sys_items.push_back(SysItem{sys_members[r], inverse, (int16_t)std::min(32, columns - c), c, 0});
+      };
+      if (s.inv_off >= 0) strips(1, s.n);
+      if (solve) strips(0, s.nrhs);
+    }
+    sc.num = r - sc.first;
+    sc.item_count = (int64_t)sys_items.size() - sc.item_first;
+    std::stable_sort(sys_items.begin() + sc.item_first, sys_items.end(),
+                     [](const SysItem& x, const SysItem& y) { return x.width > y.width; });
+    sys_classes.push_back(sc);
   }
 
   // step-wise set: descending order, slot = rank
@@ -299,7 +344,14 @@ int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_
   if (rc == NPPB_OK) rc = upload(&d_step_list, step_members, alloc_stream);
   if (rc == NPPB_OK) rc = upload(&d_items, items, alloc_stream);
   if (rc == NPPB_OK) rc = upload(&d_back, back, alloc_stream);
+  if (rc == NPPB_OK) rc = upload(&d_sys_list, sys_members, alloc_stream);
+  if (rc == NPPB_OK) rc = upload(&d_sys_items, sys_items, alloc_stream);
   if (rc != NPPB_OK) return rc;
+  if (nsys) {
+    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_perm), sizeof(int32_t) * perm, alloc_stream), "plan scratch");
+    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_dinv), sizeof(double) * dinv, alloc_stream), "plan scratch");
+    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_state), sizeof(int32_t) * nsys, alloc_stream), "plan scratch");
+  }
   if (nstep_sys)
     NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_scratch), sizeof(StepScratch) * nstep_sys, alloc_stream),
               "plan scratch");
@@ -363,6 +415,32 @@ StepArgs Plan::step_args(const Ptrs& p) const {
   sa.info = p.info;
   sa.solve_only = solve_only ? 1 : 0;
   return sa;
+}
+
+SysArgs Plan::sys_args(const Ptrs& p) const {
+  SysArgs sa{};
+  sa.desc = d_desc;
+  sa.A = p.A;
+  sa.W = p.LU;
+  sa.perm = d_perm;
+  sa.dinv = d_dinv;
+  sa.B = p.B;
+  sa.X = p.X;
+  sa.inv = p.Inv;
+  sa.det = p.Det;
+  sa.sign = p.Sign;
+  sa.logabs = p.Logabs;
+  sa.info = p.info;
+  sa.state = d_state;
+  return sa;
+}
+
+cudaError_t Plan::launch_sys(const Ptrs& p, int cls, cudaStream_t st) const {
+  const SysClass& c = sys_classes[cls];
+  const SysArgs sa = sys_args(p);
+  const cudaError_t e = launch_sys_lu(sa, d_sys_list + c.first, (int)c.num, c.nmax, st);
+  if (e != cudaSuccess || !c.item_count) return e;
+  return launch_sys_solve(sa, d_sys_items + c.item_first, c.item_count, 0, c.nmax, st);
 }
 
 cudaError_t Plan::launch_warp(const Ptrs& p, int cls, cudaStream_t st) const {
@@ -464,6 +542,12 @@ int Plan::time_kernels(const Ptrs& p, cudaStream_t st, double* ms) const {
     ms[kind] += t;
   };
   for (int c = 0; c < (int)warp_classes.size(); ++c) timed(kKindWarp, [&] { return launch_warp(p, c, st); });
+  for (const SysClass& c : sys_classes) {
+    const SysArgs sa = sys_args(p);
+    timed(kKindUpdate, [&] { return launch_sys_lu(sa, d_sys_list + c.first, (int)c.num, c.nmax, st); });
+    if (c.item_count)
+      timed(kKindBack, [&] { return launch_sys_solve(sa, d_sys_items + c.item_first, c.item_count, 0, c.nmax, st); });
+  }
   const StepArgs sa = step_args(p);
   for (const Chain& ch : chains) {
     if (solve_only) {
@@ -484,6 +568,10 @@ int Plan::time_kernels(const Ptrs& p, cudaStream_t st, double* ms) const {
 }
 
 cudaError_t Plan::launch_steps(const Ptrs& p, cudaStream_t st) const {
+  for (int c = 0; c < (int)sys_classes.size(); ++c) {
+    cudaError_t e = launch_sys(p, c, st);
+    if (e != cudaSuccess) return e;
+  }
   for (int c = 0; c < (int)chains.size(); ++c) {
     cudaError_t e = launch_chain(p, c, st);
     if (e != cudaSuccess) return e;
@@ -506,8 +594,9 @@ int Plan::execute(const Ptrs& p, cudaStream_t st) {
   if (cur != dev) return arg_error("plan used on a different device than it was created on");
   std::lock_guard<std::mutex> lk(mu);
   NPPB_CUDA(ensure_lookahead(), "look-ahead streams");
-  const int nwarp = (int)warp_classes.size();
-  const int branches = nwarp + (int)chains.size();
+  // graph branches: system classes, step chains, warp classes
+  const int ns = (int)sys_classes.size(), nc = (int)chains.size();
+  const int branches = ns + nc + (int)warp_classes.size();
   // executions share the plan's workspace: each one starts after the previous
   if (!done) NPPB_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming), "event");
   else NPPB_CUDA(cudaStreamWaitEvent(st, done, 0), "stream wait");
@@ -534,12 +623,13 @@ int Plan::execute(const Ptrs& p, cudaStream_t st) {
     if (graph) { cudaGraphDestroy(graph); graph = nullptr; }
     NPPB_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), "begin capture");
     cudaError_t err = cudaEventRecord(fork, cap);
-    // the step chains are the long poles: start them first
-    for (int b = 0; b < branches && err == cudaSuccess; ++b) {
-      const int i = (b + nwarp) % branches;
+    // the long poles first: step chains, then system classes from the largest order down
+    for (int i = 0; i < branches && err == cudaSuccess; ++i) {
       err = cudaStreamWaitEvent(side[i], fork, 0);
       if (err == cudaSuccess)
-        err = (i < nwarp) ? launch_warp(p, i, side[i]) : launch_chain(p, i - nwarp, side[i]);
+        err = i < nc        ? launch_chain(p, i, side[i])
+              : i < nc + ns ? launch_sys(p, i - nc, side[i])
+                            : launch_warp(p, i - nc - ns, side[i]);
       if (err == cudaSuccess) err = cudaEventRecord(join[i], side[i]);
       if (err == cudaSuccess) err = cudaStreamWaitEvent(cap, join[i], 0);
     }
@@ -559,7 +649,7 @@ int Plan::execute(const Ptrs& p, cudaStream_t st) {
   return NPPB_OK;
 }
 
-int Plan::num_kernel_groups() const { return (int)warp_classes.size() + (nstep_sys ? 1 : 0); }
+int Plan::num_kernel_groups() const { return (int)warp_classes.size() + (nsys + nstep_sys ? 1 : 0); }
 
 int Plan::launches_per_execute() const {
   // mirrors launch_update (k_rows, plus k_update while rows remain below the
@@ -571,6 +661,7 @@ int Plan::launches_per_execute() const {
   };
   // wide strips: the chain's largest order bounds the passes
   int l = (int)warp_classes.size();
+  for (const SysClass& c : sys_classes) l += 1 + (c.item_count ? 1 : 0);
   for (const Chain& ch : chains) {
     const int nn = (int)ch.narrow_count, nw = (int)(ch.back_count - ch.narrow_count);
     for (int fwd = solve_only ? 1 : 0; fwd >= 0; --fwd) {
@@ -1175,10 +1266,10 @@ int nppb_plan_class_info(const nppb_plan* plan, int c, int* is_warp, int* bound,
     if (bytes) *bytes = w.bytes;
   } else {
     if (is_warp) *is_warp = 0;
-    if (bound) *bound = pl.step_nmax;
-    if (systems) *systems = pl.nstep_sys;
-    if (flops) *flops = pl.step_flops;
-    if (bytes) *bytes = pl.step_bytes;
+    if (bound) *bound = pl.step_nmax ? pl.step_nmax : pl.sys_classes[0].nmax;
+    if (systems) *systems = pl.nsys + pl.nstep_sys;
+    if (flops) *flops = pl.sys_flops + pl.step_flops;
+    if (bytes) *bytes = pl.sys_bytes + pl.step_bytes;
   }
   return NPPB_OK;
 }

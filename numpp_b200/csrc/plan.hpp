@@ -11,6 +11,7 @@
 #include "nppb_internal.hpp"
 #include "nppb_step.hpp"
 #include "runtime.hpp"
+#include "sys.hpp"
 
 namespace nppb {
 
@@ -33,6 +34,13 @@ class Plan {
     int bound;
     int64_t first, num;
     double flops, bytes;
+  };
+  // Systems of 33..512 rows with one number of 32-row blocks: one launch that
+  // factors them (a CTA per system) and one that substitutes (a CTA per strip).
+  struct SysClass {
+    int nmax;
+    int64_t first, num;            // in d_sys_list
+    int64_t item_first, item_count;  // in d_sys_items
   };
   struct PanelRange {
     int64_t first, num;
@@ -72,10 +80,11 @@ class Plan {
   int execute(const Ptrs& p, cudaStream_t st);
   cudaError_t launch_warp(const Ptrs& p, int cls, cudaStream_t st) const;
   cudaError_t launch_chain(const Ptrs& p, int chain, cudaStream_t st) const;
+  cudaError_t launch_sys(const Ptrs& p, int cls, cudaStream_t st) const;
   // Every launch of one execution in order, each between two CUDA events on
   // `st`; ms[kind] accumulates the durations per kernel kind (KernelKind).
   int time_kernels(const Ptrs& p, cudaStream_t st, double* ms) const;
-  cudaError_t launch_steps(const Ptrs& p, cudaStream_t st) const;  // every chain, in order
+  cudaError_t launch_steps(const Ptrs& p, cudaStream_t st) const;  // every system class and chain, in order
   int num_kernel_groups() const;
   // Work each kernel kind does per execution (flops of the arithmetic it runs,
   // triangular parts counted as triangles) and the launches per kind.
@@ -94,11 +103,12 @@ class Plan {
   cudaStream_t alloc_stream = nullptr;  // stream-ordered allocations (freed on it too)
   int64_t a_elems = 0, b_elems = 0, inv_elems = 0, lu_elems = 0, piv_elems = 0;
   std::vector<WarpClass> warp_classes;
+  std::vector<SysClass> sys_classes;  // largest order first
   std::vector<Chain> chains;
   int nchains = 3;
-  int64_t nstep_sys = 0, nback = 0;
+  int64_t nsys = 0, nstep_sys = 0, nback = 0;
   int step_nmax = 0;
-  double step_flops = 0.0, step_bytes = 0.0;
+  double sys_flops = 0.0, sys_bytes = 0.0, step_flops = 0.0, step_bytes = 0.0;
 
   SysDesc* d_desc = nullptr;
   int32_t* d_order = nullptr;
@@ -106,6 +116,11 @@ class Plan {
   StepItem* d_items = nullptr;
   StepItem* d_back = nullptr;
   StepScratch* d_scratch = nullptr;
+  int32_t* d_sys_list = nullptr;
+  SysItem* d_sys_items = nullptr;
+  int32_t* d_perm = nullptr;   // system-resident path: row permutations,
+  double* d_dinv = nullptr;    //   inverses of the diagonal blocks,
+  int32_t* d_state = nullptr;  //   first zero pivots
   double* d_lu = nullptr;
   int32_t* d_piv = nullptr;
 
@@ -121,6 +136,7 @@ class Plan {
   cudaError_t substitute(const StepArgs& sa, const Chain& ch, cudaStream_t st, bool forward) const;
   Batch warp_batch(const Ptrs& p) const;
   StepArgs step_args(const Ptrs& p) const;
+  SysArgs sys_args(const Ptrs& p) const;
 
   std::mutex mu;
   Ptrs key{};

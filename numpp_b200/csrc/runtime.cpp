@@ -1,6 +1,7 @@
 // Host runtime: device probe, errors, per-thread streams, allocations, and the
 // order -> kernel choice for uniform batches. C++20.
 #include "runtime.hpp"
+#include "sys.hpp"
 
 #include <algorithm>
 #include <climits>
@@ -116,6 +117,7 @@ void DevMem::release() {
 
 cudaError_t prepare_kernels() {
   cudaError_t e = step_prepare();
+  if (e == cudaSuccess) e = sys_prepare_kernels();
   return e == cudaSuccess ? mx_prepare() : e;
 }
 

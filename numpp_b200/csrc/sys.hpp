@@ -1,0 +1,62 @@
+// System-resident LU and substitution (orders 33..512): launch interface.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "nppb_internal.hpp"
+
+namespace nppb {
+
+constexpr int kSysMaxN = 512;  // one CTA per system: 16 warps of 32 rows
+
+// Leading dimension of a factor workspace: rows start on 32-byte sectors.
+__host__ __device__ inline int sys_ld(int n) { return (n + 3) & ~3; }
+__host__ __device__ inline int sys_blocks(int n) { return (n + 31) / 32; }
+// Doubles of the diagonal blocks' inverses: per 32-column block L11^-1, then U11^-1.
+__host__ __device__ inline int64_t sys_dinv(int n) { return (int64_t)sys_blocks(n) * 2048; }
+
+// A strip of at most 32 columns of one system's right-hand sides or inverse.
+struct SysItem {
+  int32_t sys;
+  int16_t inverse;  // 1: columns of the inverse
+  int16_t width;
+  int32_t c0;
+  int32_t pad_;
+};
+
+// Systems of one launch. With desc: system list[i] (or i) has its own order and
+// offsets. Without: a uniform batch of order un.
+struct SysArgs {
+  const SysDesc* desc;
+  const double* A;      // input matrices, row-major, leading dimension n
+  double* W;            // factors: row r of A's row order, leading dimension ldw
+  int32_t* perm;        // position -> row of A (and of W, unless w_by_position)
+  double* dinv;         // inverses of the diagonal blocks
+  const double* B;
+  double* X;
+  double* inv;
+  double* det;
+  double* sign;
+  double* logabs;
+  int32_t* info;        // per-system output (may be null)
+  int32_t* state;       // first zero pivot + 1 or 0, by slot (null: every system is solved)
+  int un, unrhs, uinv;  // uniform batch
+  int w_by_position;    // W holds rows in pivoted order with leading dimension n (kept factors)
+};
+
+// LU with partial pivoting of `nsys` systems with (maximum order) nmax <= 512,
+// one CTA of sys_blocks(nmax) warps each.
+cudaError_t launch_sys_lu(const SysArgs& sa, const int32_t* list, int nsys, int nmax, cudaStream_t st);
+// Forward and back substitution of `nitems` strips (items == nullptr: every
+// strip of a uniform batch of nsys systems).
+cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t nitems, int nsys, int nmax,
+                             cudaStream_t st);
+// Permutations and diagonal inverses of kept factors (swap lists ipiv at
+// piv_off): fills sa.perm and sa.dinv.
+cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int32_t* list, int nsys, int nmax,
+                               cudaStream_t st);
+cudaError_t sys_prepare_kernels();
+
+}  // namespace nppb

@@ -34,9 +34,11 @@
 namespace nppb {
 namespace {
 
-constexpr int TS = 36;   // row stride of the 32 x 32 tiles read as mma operands (banks 4g + tq)
-constexpr int US = 40;   // row stride of the transposed U tile (16-byte reads: banks 4g + tq)
-constexpr int PS = 33;   // row stride of the panel staging tiles (one row per thread)
+constexpr int US = 40;   // row stride of the 32 x 32 operand tiles (16-byte reads: banks 4g + t)
+constexpr int BS = 34;   // row stride of the tile read down its columns (banks 4t + g)
+constexpr int TS = 36;   // row stride of the inversions' scratch tile
+constexpr int PS = 34;   // row stride of the panel staging tiles (16-byte reads, one row per thread)
+constexpr int GS = 10;   // row stride of the transposed 8-row U tile of a panel group
 constexpr int kMaxWarps = kSysMaxN / 32;
 constexpr unsigned kAll = 0xffffffffu;
 
@@ -102,19 +104,20 @@ __device__ __forceinline__ void bar_active(int threads) {  // the warps of the p
   asm volatile("bar.sync 1, %0;\n" ::"r"(threads) : "memory");
 }
 
-// A 32 x 32 inverse (row-major in global memory) into a tile of stride TS.
-__device__ __forceinline__ void fetch_inverse(double* tile, const double* g) {
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+// A 32 x 32 inverse (row-major in global memory) into a tile of stride TS, by
+// threads first .. first + nthr - 1.
+__device__ __forceinline__ void fetch_inverse(double* tile, const double* g, int nthr, int first = 0) {
+  for (int i = (int)threadIdx.x - first; i < 512; i += nthr) {
     const int r = i >> 4, c = (i & 15) * 2;
-    cp16(tile + r * TS + c, g + r * 32 + c);
+    cp16(tile + r * US + c, g + r * 32 + c);
   }
   cp_commit();
 }
 
 // The rows of a warp's operand tile: lane 4g + t serves rows g, g+8, g+16, g+24.
 struct Rows {
-  int off[4];  // element offset of the row in W
-  bool ok[4];
+  unsigned off[4];  // byte offset of the row in W
+  int live;         // rows from row g of the tile on: row group i exists when 8i < live
 };
 
 // A warp's operand ring: stages of eight columns of its 32 rows, 2 KB each. A
@@ -125,34 +128,37 @@ struct Rows {
 constexpr int kRing = 4;
 constexpr int kRingDoubles = kRing * 256;  // of one warp
 
-// EDGE: the columns may end inside the block (zeros past them).
+// One row group of a stage: columns col, col + 1 of row 8i + g. EDGE: the columns
+// may end inside the block (zeros past them).
 template <bool VEC, bool EDGE>
-__device__ __forceinline__ void ring_load(double2* ring, int stage, const double* W, const Rows& r, int col, int n,
-                                          bool live) {
-  if (live) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int cols = !r.ok[i] ? 0 : EDGE ? max(0, min(2, n - col)) : 2;
-      const double* p = W + (cols ? r.off[i] + col : 0);
-      const unsigned d =
-          static_cast<unsigned>(__cvta_generic_to_shared(ring + (stage * 4 + i) * 32 + (threadIdx.x & 31)));
-      if constexpr (VEC) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(p), "r"(8 * cols));
-      } else {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(p), "r"(cols > 0 ? 8 : 0));
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d + 8), "l"(cols > 1 ? p + 1 : p),
-                     "r"(cols > 1 ? 8 : 0));
-      }
-    }
+__device__ __forceinline__ void ring_load1(unsigned ring, int stage, int i, const double* W, const Rows& r, int col,
+                                           int n) {
+  const unsigned d = ring + (stage * 4 + i) * 512;
+  int size = 8 * i < r.live ? 16 : 0;
+  if (EDGE) {
+    size = min(size, 8 * max(0, n - col));
+    col = min(col, (n - 1) & ~1);  // the address stays inside the row
   }
-  cp_commit();  // always: the waits count groups
+  const char* p = reinterpret_cast<const char*>(W + col) + r.off[i];
+  if constexpr (VEC) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(p), "r"(size));
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(p), "r"(min(size, 8)));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d + 8), "l"(size > 8 ? p + 8 : p),
+                 "r"(max(size - 8, 0)));
+  }
 }
 
 // The first three stages of block K.
 template <bool VEC, bool EDGE>
-__device__ __forceinline__ void ring_start(double2* ring, const double* W, const Rows& r, int K, int n, bool live) {
+__device__ __forceinline__ void ring_start(unsigned ring, const double* W, const Rows& r, int K, int n, bool live) {
 #pragma unroll
-  for (int q = 0; q < 3; ++q) ring_load<VEC, EDGE>(ring, q, W, r, 32 * K + 8 * q + 2 * (threadIdx.x & 3), n, live);
+  for (int q = 0; q < 3; ++q) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (live) ring_load1<VEC, EDGE>(ring, q, i, W, r, 32 * K + 8 * q + 2 * (threadIdx.x & 3), n);
+    cp_commit();
+  }
 }
 
 // Everything a block step shares. NI: 8-column groups of the strip.
@@ -161,28 +167,52 @@ struct Acc {
   double v[2][NI][4];  // rows 16m + g, 16m + g + 8; columns 8i + 2t, + 1
 };
 
-// acc -= (warp's rows of W, columns 32K..32K+31) * U, with Ut holding -U^T
-// (column c of U at Ut + c * US). The ring holds the first three stages; those
-// of block Knext follow when `more`.
+__device__ __forceinline__ unsigned smem(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ double2 lds2(unsigned p) {  // stays where it is written
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "r"(p));
+  return v;
+}
+
+// acc -= (warp's rows of W, columns 32K..32K+31) * U, with u the lane's place in
+// -U^T (column c of U at c * US; the lane reads column g + 8i, rows 2t, 2t + 1).
+// The ring holds the first three stages; those of block Knext follow when `more`. A tensor instruction holds the pipe for 64 cycles, so every
+// register is reloaded for the next stage right behind its last use and the
+// prefetches are spread between the instructions.
 template <int NI, bool VEC, bool EDGE>
-__device__ __forceinline__ void update(Acc<NI>& acc, double2* ring, const double* W, const Rows& r, const double* Ut,
-                                       int K, int Knext, bool more, int n) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+__device__ __forceinline__ void update(Acc<NI>& acc, unsigned ring, const double* W, const Rows& r,
+                                       unsigned u, int K, int Knext, bool more, int n) {
+  const int t2 = 2 * (threadIdx.x & 3);
+  double2 a[4], b[NI];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) a[i] = lds2(ring + i * 512);
+#pragma unroll
+  for (int i = 0; i < NI; ++i) b[i] = lds2(u + i * (8 * US * 8));
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    if (q == 0) ring_load<VEC, EDGE>(ring, 3, W, r, 32 * K + 24 + 2 * t, n, true);
-    else ring_load<VEC, EDGE>(ring, q - 1, W, r, 32 * Knext + 8 * (q - 1) + 2 * t, n, more);
-    double2 b[NI];
+    const int stage = (q + 3) % 4, col = q == 0 ? 32 * K + 24 + t2 : 32 * Knext + 8 * (q - 1) + t2;
+    const bool live = q == 0 || more;
 #pragma unroll
-    for (int i = 0; i < NI; ++i) b[i] = *reinterpret_cast<const double2*>(Ut + (8 * i + g) * US + 8 * q + 2 * t);
-    cp_wait<3>();  // stage q has landed
-    double2 a[4];
+    for (int i = 0; i < 4; ++i) {
+      if (i < NI) dmma1688(acc.v[0][i], a[0], a[1], b[i]);
+      if (live) ring_load1<VEC, EDGE>(ring, stage, i, W, r, col, n);
+    }
+    cp_commit();
+    cp_wait<2>();  // the next stage has landed
+    const unsigned next = ring + (q + 1) * 2048;
+    if (q < 3) {
+      a[0] = lds2(next);
+      a[1] = lds2(next + 512);
+    }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = ring[(q * 4 + i) * 32 + lane];
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-      for (int i = 0; i < NI; ++i) dmma1688(acc.v[m][i], a[2 * m], a[2 * m + 1], b[i]);
+    for (int i = 0; i < NI; ++i) {
+      dmma1688(acc.v[1][i], a[2], a[3], b[i]);
+      if (q < 3) b[i] = lds2(u + i * (8 * US * 8) + 64 * (q + 1));
+    }
+    if (q < 3) {
+      a[2] = lds2(next + 1024);
+      a[3] = lds2(next + 1536);
+    }
   }
 }
 
@@ -194,41 +224,94 @@ __device__ __forceinline__ void store_tile(double* Tb, const Acc<NI>& acc) {
   for (int m = 0; m < 2; ++m)
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-      *reinterpret_cast<double2*>(Tb + (16 * m + g) * TS + 8 * i + 2 * t) = make_double2(acc.v[m][i][0], acc.v[m][i][1]);
-      *reinterpret_cast<double2*>(Tb + (16 * m + g + 8) * TS + 8 * i + 2 * t) =
-          make_double2(acc.v[m][i][2], acc.v[m][i][3]);
+      double* o = Tb + (16 * m + g) * BS + 8 * i + 2 * t;
+      *reinterpret_cast<double2*>(o) = make_double2(acc.v[m][i][0], acc.v[m][i][1]);
+      *reinterpret_cast<double2*>(o + 8 * BS) = make_double2(acc.v[m][i][2], acc.v[m][i][3]);
     }
 }
 
-// Ut <- -(Li Tb)^T over all warps, an 8 x 8 block of the product at a time;
-// store(row, column, v0, v1) gets the product's column pairs. Li is lower
-// (UPPER: upper) triangular.
-template <int NI, bool UPPER, class Store>
-__device__ __forceinline__ void tile_product(const double* Li, const double* Tb, double* Ut, Store store) {
-  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int u = warp; u < 4 * NI; u += nw) {
-    const int mi = u / NI, ni = u - mi * NI;
-    double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
-    const int k0 = UPPER ? 8 * mi : 0, k1 = UPPER ? 32 : 8 * mi + 8;
-    for (int k = k0; k < k1; k += 8) {
-      dmma884(d0, Li[(8 * mi + g) * TS + k + t], Tb[(k + t) * TS + 8 * ni + g]);
-      dmma884(d1, Li[(8 * mi + g) * TS + k + 4 + t], Tb[(k + 4 + t) * TS + 8 * ni + g]);
+// Ut <- -(Li Tb)^T: the product of a diagonal block's inverse (lower, UPPER: upper
+// triangular: half of the steps for half of its rows) with the block's rows.
+// Warps 0..3, one on each scheduler, take eight columns each (with one group of
+// eight: eight rows each); the others go on to the next barrier.
+template <int NI, bool UPPER>
+__device__ __forceinline__ void tile_product(const double* Li, const double* Tb, double* Ut) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, warp = threadIdx.x >> 5;
+  if (warp >= 4) return;
+  const int step = min(4, (int)(blockDim.x >> 5));
+  auto left = [&](int row, int q) { return *reinterpret_cast<const double2*>(Li + row * US + 8 * q + 2 * t); };
+  auto right = [&](int col, int q) {
+    const double* b = Tb + (8 * q + 2 * t) * BS + col;
+    return make_double2(b[0], b[BS]);
+  };
+  if constexpr (NI > 1) {
+    for (int ni = warp; ni < NI; ni += step) {
+      double d[2][4];
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[m][e] = 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double2 b = right(8 * ni + g, q);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          if (UPPER ? (q < 2 && m == 1) : (q >= 2 && m == 0)) continue;  // zeros of the triangle
+          dmma1688(d[m], left(16 * m + g, q), left(16 * m + 8 + g, q), b);
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          Ut[(8 * ni + 2 * t + (e & 1)) * US + 16 * m + g + 8 * (e >> 1)] = -d[m][e];
     }
-    const double v0 = d0[0] + d1[0], v1 = d0[1] + d1[1];
-    const int row = 8 * mi + g, col = 8 * ni + 2 * t;
-    Ut[col * US + row] = -v0;
-    Ut[(col + 1) * US + row] = -v1;
-    store(row, col, v0, v1);
+  } else {
+    for (int mi = warp; mi < 4; mi += step) {
+      double d[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double2 x = left(8 * mi + g, q), y = right(g, q);
+        dmma884(d[0], x.x, y.x);
+        dmma884(d[1], x.y, y.y);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) Ut[(2 * t + e) * US + 8 * mi + g] = -(d[0][e] + d[1][e]);
+    }
+  }
+}
+
+// The product's rows to memory, by warps first .. first + count - 1 (those that
+// have nothing to update): row(r) is where row r goes, or null; PAIRS: 16 bytes
+// at once, else up to `cols` columns.
+template <int NI, bool PAIRS, class Row>
+__device__ __forceinline__ void product_out(const double* Ut, int cols, int first, int count, Row row) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int mi = (int)(threadIdx.x >> 5) - first; mi < 4; mi += count) {
+    double* o = row(8 * mi + g);
+    if (!o) continue;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int col = 8 * i + 2 * t;
+      const double v0 = -Ut[col * US + 8 * mi + g], v1 = -Ut[(col + 1) * US + 8 * mi + g];
+      if constexpr (PAIRS) {
+        if (col < cols) *reinterpret_cast<double2*>(o + col) = make_double2(v0, v1);
+      } else {
+        if (col < cols) o[col] = v0;
+        if (col + 1 < cols) o[col + 1] = v1;
+      }
+    }
   }
 }
 
 // Inverse of a 32 x 32 triangle by one warp, out (row-major, global memory) in
 // full with its zeros. D (stride PS, shared) holds L below the unit diagonal and
-// U on and above it, kb live rows and columns (identity past them); X is a
-// scratch tile of stride TS. The upper triangle is inverted as the lower
-// triangle U^T. First the four 8 x 8 diagonal blocks, a lane per column, then
-// the blocks below them: X_ij = -X_ii (T_ij X_jj + ... + T_i,i-1 X_i-1,j).
+// U on and above it, kb live rows and columns (identity past them). The upper
+// triangle is inverted as the lower triangle U^T. First the four 8 x 8 diagonal
+// blocks, a lane per column, then the blocks below them:
+// X_ij = -X_ii (T_ij X_jj + ... + T_i,i-1 X_i-1,j). X is a scratch tile of
+// stride TS that two warps share: the lower inverse lives below its diagonal,
+// the upper one (transposed back) on and above it.
 template <bool UPPER>
 __device__ __forceinline__ void tri_inverse(const double* D, double* X, double* __restrict__ out, int kb) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -236,6 +319,8 @@ __device__ __forceinline__ void tri_inverse(const double* D, double* X, double* 
     const bool in = i < kb && k < kb;
     return in ? (UPPER ? D[k * PS + i] : D[i * PS + k]) : (i == k ? 1.0 : 0.0);
   };
+  auto at = [&](int i, int j) -> double& { return UPPER ? X[j * TS + i] : X[i * TS + j]; };
+  auto get = [&](int i, int j) { return i > j || (UPPER && i == j) ? at(i, j) : (i == j ? 1.0 : 0.0); };
   {
     const int b = lane & ~7, c = lane & 7;
     const double rd = UPPER ? 1.0 / T(b + c, b + c) : 1.0;
@@ -249,42 +334,45 @@ __device__ __forceinline__ void tri_inverse(const double* D, double* X, double* 
       x[i] = i >= c ? s : 0.0;
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) X[(b + i) * TS + b + c] = x[i];
+    for (int i = 0; i < 8; ++i)
+      if (i > c || (UPPER && i == c)) at(b + i, b + c) = x[i];
   }
   __syncwarp();
   for (int i = 1; i < 4; ++i)
     for (int j = 0; j < i; ++j) {
       double s[2] = {0.0, 0.0}, x[2] = {0.0, 0.0};
-      for (int k = 8 * j; k < 8 * i; k += 4) dmma884(s, T(8 * i + g, k + t), X[(k + t) * TS + 8 * j + g]);
+      for (int k = 8 * j; k < 8 * i; k += 4) dmma884(s, T(8 * i + g, k + t), get(k + t, 8 * j + g));
       // the sum's place is X_ij's until the product with X_ii replaces it
-      X[(8 * i + g) * TS + 8 * j + 2 * t] = s[0];
-      X[(8 * i + g) * TS + 8 * j + 2 * t + 1] = s[1];
+      at(8 * i + g, 8 * j + 2 * t) = s[0];
+      at(8 * i + g, 8 * j + 2 * t + 1) = s[1];
       __syncwarp();
 #pragma unroll
-      for (int k = 0; k < 8; k += 4)
-        dmma884(x, X[(8 * i + g) * TS + 8 * i + k + t], X[(8 * i + k + t) * TS + 8 * j + g]);
+      for (int k = 0; k < 8; k += 4) dmma884(x, get(8 * i + g, 8 * i + k + t), at(8 * i + k + t, 8 * j + g));
       __syncwarp();
-      X[(8 * i + g) * TS + 8 * j + 2 * t] = -x[0];
-      X[(8 * i + g) * TS + 8 * j + 2 * t + 1] = -x[1];
+      at(8 * i + g, 8 * j + 2 * t) = -x[0];
+      at(8 * i + g, 8 * j + 2 * t + 1) = -x[1];
       __syncwarp();
     }
 #pragma unroll 8
-  for (int r = 0; r < 32; ++r) {
-    const int i = UPPER ? lane : r, j = UPPER ? r : lane;
-    out[r * 32 + lane] = j > i ? 0.0 : X[i * TS + j];
-  }
+  for (int r = 0; r < 32; ++r) out[r * 32 + lane] = UPPER ? (lane >= r ? X[r * TS + lane] : 0.0) : get(r, lane);
 }
 
 // ---------------------------------------------------------------------------
 // Panel: the pivot of each column is the first largest |a| in position order
-// (the reference's rule, linalg.cpp:55-57). One row per thread. Columns go in
-// groups of eight held in a[0..7]: inside a group each pivot step touches the
-// group's columns only (one barrier per column, the warps' candidates through
-// shared memory), then the group's pivot rows are solved for the columns right
-// of it and the eight steps are applied to those at once. The group loop is
-// rolled (the registers rotate by eight), so the code stays in the instruction
-// cache: the form unrolled over 32 columns took 2500 cycles a column, mostly
-// issue of 240 instructions per warp.
+// (the reference's rule, linalg.cpp:55-57). The warps keep their 32 x 32 tiles of
+// the column block in the tensor core's accumulators and take the columns in
+// four groups of eight. A group's columns go through the staging tile to one
+// row per thread; each pivot step then touches the group's columns only (one
+// barrier per column, the warps' candidates through shared memory). After the
+// group its pivot rows are solved for the columns right of it, and the eight
+// steps are applied to those at once by the tensor core.
+//
+// Latency bounds it: a column is two warp reductions, a division and a barrier
+// deep, so everything that can be is started on the likely outcome (the
+// candidate with the largest high word, which is nearly always unique) and
+// repeated exactly otherwise. The group loop is rolled (the accumulators rotate),
+// which keeps the code in the instruction cache.
+// Cycles per column with 1 / 16 warps: PANEL_CYCLES.
 struct __align__(16) Cand {
   unsigned hi, lo;  // |a| as two words; 0, 0: no candidate
   int pos, pad;
@@ -293,158 +381,182 @@ struct __align__(16) Cand {
 struct __align__(16) PanelShared {
   Cand cand[2][kMaxWarps];
   double row[2][kMaxWarps][8];
-  double raw[8][24];  // pivot rows of a group, right of it, before the solve
-  double u[8][24];    // and after
+  double rp[2][kMaxWarps];
+  double raw[8][24];    // pivot rows of a group, right of it, before the solve
   double l8[8][8];
+  double u[24 * GS];    // minus the solved rows, transposed
   int info;
 };
 
 // Whether this lane holds the largest (hi, lo), ties to the smallest pos; `any`:
-// some lane has a candidate. Nearly always one lane has the largest high word.
-__device__ __forceinline__ bool warp_winner(unsigned hi, unsigned lo, int pos, bool& any) {
+// some lane has a candidate.
+__device__ __forceinline__ bool exact_winner(unsigned hi, unsigned lo, int pos, bool& any) {
   const unsigned mh = __reduce_max_sync(kAll, hi);
   bool me = hi == mh;
-  const unsigned top = __ballot_sync(kAll, me);
-  any = true;
-  if ((top & (top - 1)) != 0 || mh == 0) {
-    const unsigned ml = __reduce_max_sync(kAll, me ? lo : 0u);
-    any = (mh | ml) != 0;
-    me = me && lo == ml;
-    const int p = __reduce_min_sync(kAll, me ? pos : INT_MAX);
-    me = me && pos == p && any;
-  }
-  return me;
+  const unsigned ml = __reduce_max_sync(kAll, me ? lo : 0u);
+  any = (mh | ml) != 0;
+  me = any && me && lo == ml;
+  const int first = __reduce_min_sync(kAll, me ? pos : INT_MAX);  // by every lane
+  return me && pos == first;
 }
 
-// 1 / x by Newton's iteration on the mantissa from a single-precision start
-// (error 2^-23, 2^-46, then rounding), without a branch, so that it runs beside
-// the search for the winner. Exponent field of x in 1..2044.
-__device__ __forceinline__ double newton_reciprocal(double x) {
-  const int hi = __double2hiint(x);
-  const double m = __hiloint2double((hi & 0x800fffff) | 0x3ff00000, __double2loint(x));
-  double y = (double)__fdividef(1.0f, (float)m);
-  y = fma(y, fma(-m, y, 1.0), y);
-  y = fma(y, fma(-m, y, 1.0), y);
-  return __hiloint2double(__double2hiint(y) - (((hi >> 20) & 0x7ff) - 1023) * (1 << 20), __double2loint(y));
+constexpr unsigned kInf = 0x7ff00000u;  // high word of infinity
+
+// The rare level-one cases: lanes that share the high word, NaN (no candidate),
+// infinities, or no candidate at all.
+template <class Publish>
+__device__ __forceinline__ void exact_publish(PanelShared& sh, double x, bool live, int par, int aw, int pos,
+                                           Publish publish) {
+  unsigned hi = (unsigned)__double2hiint(x) & 0x7fffffffu, lo = (unsigned)__double2loint(x);
+  if (!live || hi > kInf || (hi == kInf && lo)) hi = lo = 0;
+  bool any;
+  const bool me = exact_winner(hi, lo, pos, any);
+  __syncwarp();
+  if (me) publish(hi, lo, 1.0 / x);
+  else if (!any && (threadIdx.x & 31) == 0) sh.cand[par][aw] = Cand{0u, 0u, INT_MAX, 0};
 }
 
-// a: the thread's row of the column block; pos: its position in the panel (0 =
-// the first row), updated; row: where the finished columns go (32 doubles of
-// the thread's own). Returns 0 or the column of the first zero pivot + 1.
-__device__ __forceinline__ int panel(PanelShared& sh, double (&a)[32], int& pos, bool valid, int kb, int aw, int na,
-                                     double* row, int& nswap) {
-  const int lane = threadIdx.x & 31, nthr = na * 32;
-  bool alive = valid;  // not a pivot row yet
+// acc: the warp's tile of the column block (clobbered); pos: the position in the
+// panel of the thread's row (row `lane` of the tile; 0 = the panel's first row),
+// updated; tile: the warp's staging tile, which ends with the finished columns.
+// Returns 0 or the column of the first zero pivot + 1.
+__device__ __forceinline__ int panel(PanelShared& sh, Acc<4>& acc, int& pos, bool valid, int kb, int aw, int na,
+                                     double* tile, int& nswap) {
+  const int lane = threadIdx.x & 31, nthr = na * 32, g = lane >> 2, t = lane & 3;
+  unsigned live = valid ? 0x7fffffffu : 0u;  // mask of the magnitude's high word; 0: a pivot row already
 #pragma unroll 1
-  for (int sp = 0; sp < 4; ++sp) {
-    const int j0 = 8 * sp;
-    if (j0 < kb) {
+  for (int j0 = 0; j0 < kb; j0 += 8) {
 #pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const int j = j0 + s;
-        if (j < kb) {  // uniform
-          constexpr unsigned kInf = 0x7ff00000u;
-          const int par = s & 1;
-          unsigned hi = (unsigned)__double2hiint(a[s]) & 0x7fffffffu, lo = (unsigned)__double2loint(a[s]);
-          if (!alive || hi > kInf || (hi == kInf && lo)) hi = lo = 0;  // a NaN is no candidate
+    for (int m = 0; m < 2; ++m) {
+      *reinterpret_cast<double2*>(tile + (16 * m + g) * PS + j0 + 2 * t) = make_double2(acc.v[m][0][0], acc.v[m][0][1]);
+      *reinterpret_cast<double2*>(tile + (16 * m + g + 8) * PS + j0 + 2 * t) =
+          make_double2(acc.v[m][0][2], acc.v[m][0][3]);
+    }
+    __syncwarp();
+    double a[8];
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double2 x = *reinterpret_cast<const double2*>(tile + lane * PS + j0 + c);
+      a[c] = x.x;
+      a[c + 1] = x.y;
+    }
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const int j = j0 + s;
+      if (j < kb) {  // uniform
+        const int par = s & 1;
+        const unsigned hi = (unsigned)__double2hiint(a[s]) & live;
+        const unsigned mh = __reduce_max_sync(kAll, hi);
+        const double rp = 1.0 / (hi ? a[s] : 1.0);  // every candidate's, beside the reduction
+        const bool me = hi == mh;
+        const unsigned top = __ballot_sync(kAll, me);
+        auto publish = [&](unsigned h, unsigned l, double r) {
+          sh.cand[par][aw] = Cand{h, l, pos, 0};
+          sh.rp[par][aw] = r;
+#pragma unroll
+          for (int c = s & ~1; c < 8; c += 2)
+            *reinterpret_cast<double2*>(&sh.row[par][aw][c]) = make_double2(a[c], a[c + 1]);
+        };
+        if (me) publish(hi, (unsigned)__double2loint(a[s]), rp);
+        if ((top & (top - 1)) != 0 || mh >= kInf) exact_publish(sh, a[s], live != 0, par, aw, pos, publish);
+        bar_active(nthr);
+        const Cand cd = lane < na ? sh.cand[par][lane] : Cand{0u, 0u, INT_MAX, 0};
+        const unsigned key = lane < na ? (cd.hi & ~15u) | (15u - lane) : 0u;
+        const unsigned mk = __reduce_max_sync(kAll, key);
+        const unsigned amb = __ballot_sync(kAll, lane < na && (key ^ mk) < 16u);
+        int gw = 15 - (int)(mk & 15u);
+        double r = sh.rp[par][gw];
+        int gk = sh.cand[par][gw].pos;
+        if ((amb & (amb - 1)) != 0 || mk < 16u) {
           bool any;
-          if (warp_winner(hi, lo, pos, any)) {
-            sh.cand[par][aw] = Cand{hi, lo, pos, 0};
-#pragma unroll
-            for (int c = s & ~1; c < 8; c += 2)
-              *reinterpret_cast<double2*>(&sh.row[par][aw][c]) = make_double2(a[c], a[c + 1]);
-          }
-          if (!any && lane == 0) sh.cand[par][aw] = Cand{0u, 0u, INT_MAX, 0};
-          bar_active(nthr);
-          const Cand cd = lane < na ? sh.cand[par][lane] : Cand{0u, 0u, INT_MAX, 0};
-          double rp = newton_reciprocal(lane < na ? sh.row[par][lane][s] : 1.0);
-          const bool best = warp_winner(cd.hi, cd.lo, cd.pos, any);
+          const bool best = exact_winner(cd.hi, cd.lo, cd.pos, any);
           if (!any) return j + 1;  // the same in every warp of the panel
-          const int gw = 31 - __clz(__ballot_sync(kAll, best));
-          const int gk = __shfl_sync(kAll, cd.pos, gw);
-          rp = __shfl_sync(kAll, rp, gw);
-          const double* prow = sh.row[par][gw];
-          const unsigned ghi = __shfl_sync(kAll, cd.hi, gw);
-          if (ghi < 0x00100000u || ghi >= 0x7fd00000u) rp = 1.0 / prow[s];  // outside newton_reciprocal's range
-          const bool chosen = pos == gk;
-          if (pos == j) pos = gk;
-          if (chosen) {
-            pos = j;
-            alive = false;
-          }
-          nswap += gk != j;
-          const double f = alive ? a[s] * rp : 0.0;
-          if (alive) a[s] = f;
-#pragma unroll
-          for (int c = s + 1; c < 8; ++c) a[c] = fma(-f, prow[c], a[c]);
+          gw = 31 - __clz(__ballot_sync(kAll, best));
+          r = sh.rp[par][gw];
+          gk = sh.cand[par][gw].pos;
         }
+        const double* prow = sh.row[par][gw];
+        const bool chosen = pos == gk;
+        if (pos == j) pos = gk;
+        if (chosen) {
+          pos = j;
+          live = 0;
+        }
+        nswap += gk != j;
+        const double f = live ? a[s] * r : 0.0;
+        if (live) a[s] = f;
+#pragma unroll
+        for (int c = s + 1; c < 8; ++c) a[c] = fma(-f, prow[c], a[c]);
       }
     }
 #pragma unroll
-    for (int c = 0; c < 8; ++c) row[j0 + c] = a[c];
-    if (j0 + 8 < kb) {
-      const int mine = pos - j0;  // this row's place among the group's pivots
-      if (valid && mine >= 0 && mine < 8) {
+    for (int c = 0; c < 8; c += 2) *reinterpret_cast<double2*>(tile + lane * PS + j0 + c) = make_double2(a[c], a[c + 1]);
+    if (j0 + 8 >= kb) break;
+    // the row's step in the group; 8: still below, -1: done before
+    const bool in_group = valid && pos >= j0 && pos < j0 + 8;
+    const int mine = live ? 8 : in_group ? pos - j0 : -1;
+    if (in_group) {
 #pragma unroll
-        for (int c = 0; c < 24; c += 2) *reinterpret_cast<double2*>(&sh.raw[mine][c]) = make_double2(a[8 + c], a[9 + c]);
+      for (int c = 0; c < 8; c += 2) *reinterpret_cast<double2*>(&sh.l8[pos - j0][c]) = make_double2(a[c], a[c + 1]);
+    }
+    __syncwarp();
+    int lim[4];
 #pragma unroll
-        for (int c = 0; c < 8; c += 2) *reinterpret_cast<double2*>(&sh.l8[mine][c]) = make_double2(a[c], a[c + 1]);
-      }
-      bar_active(nthr);
-      if (aw == 0 && lane < 24) {
-        double x[8];
+    for (int i = 0; i < 4; ++i) {
+      lim[i] = __shfl_sync(kAll, mine, 8 * i + g);
+      if (lim[i] >= 0 && lim[i] < 8) {
 #pragma unroll
-        for (int s = 0; s < 8; ++s) x[s] = sh.raw[s][lane];
-#pragma unroll
-        for (int q = 0; q < 7; ++q)
-#pragma unroll
-          for (int s = q + 1; s < 8; ++s) x[s] = fma(-sh.l8[s][q], x[q], x[s]);
-#pragma unroll
-        for (int s = 0; s < 8; ++s) sh.u[s][lane] = x[s];
-      }
-      const int lim = valid ? min(max(mine, 0), 8) : 0;  // steps this row took part in
-#pragma unroll
-      for (int s = 0; s < 8; ++s) a[s] = s < lim ? a[s] : 0.0;
-      bar_active(nthr);
-#pragma unroll
-      for (int grp = 0; grp < 3; ++grp) {
-        if (j0 + 8 * (grp + 1) < kb) {
-#pragma unroll
-          for (int s = 0; s < 8; ++s) {
-#pragma unroll
-            for (int c = 0; c < 8; c += 2) {
-              const double2 u = *reinterpret_cast<const double2*>(&sh.u[s][8 * grp + c]);
-              a[8 + 8 * grp + c] = fma(-a[s], u.x, a[8 + 8 * grp + c]);
-              a[9 + 8 * grp + c] = fma(-a[s], u.y, a[9 + 8 * grp + c]);
-            }
-          }
-        }
+        for (int ni = 1; ni < 4; ++ni)
+          *reinterpret_cast<double2*>(&sh.raw[lim[i]][8 * (ni - 1) + 2 * t]) =
+              make_double2(acc.v[i >> 1][ni][2 * (i & 1)], acc.v[i >> 1][ni][2 * (i & 1) + 1]);
       }
     }
+    // the multipliers as tensor-core operand; a row takes part in the steps before its own
+    double2 l[4];
 #pragma unroll
-    for (int c = 0; c < 24; ++c) a[c] = a[c + 8];
+    for (int i = 0; i < 4; ++i) {
+      l[i] = *reinterpret_cast<const double2*>(tile + (8 * i + g) * PS + j0 + 2 * t);
+      if (2 * t >= lim[i]) l[i].x = 0.0;
+      if (2 * t + 1 >= lim[i]) l[i].y = 0.0;
+    }
+    bar_active(nthr);
+    if (aw == 0) {
+      const int c = min(lane, 23);
+      double x[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) x[s] = sh.raw[s][c];
+#pragma unroll
+      for (int q = 0; q < 7; ++q) {
+#pragma unroll
+        for (int s = q + 1; s < 8; ++s) x[s] = fma(-sh.l8[s][q], x[q], x[s]);
+      }
+      if (lane < 24) {
+#pragma unroll
+        for (int s = 0; s < 8; s += 2)
+          *reinterpret_cast<double2*>(&sh.u[lane * GS + s]) = make_double2(-x[s], -x[s + 1]);
+      }
+    }
+    bar_active(nthr);
+#pragma unroll
+    for (int ni = 1; ni < 4; ++ni) {
+      const double2 b = *reinterpret_cast<const double2*>(&sh.u[(8 * (ni - 1) + g) * GS + 2 * t]);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        dmma1688(acc.v[m][ni], l[2 * m], l[2 * m + 1], b);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc.v[m][ni - 1][e] = acc.v[m][ni][e];
+      }
+    }
   }
   return 0;
 }
 
-// Shared memory of k_sys_lu, in doubles. The panel's staging tiles take the
-// place of the rings (idle by then); the diagonal block that the inversions
-// read takes U's.
-struct LuLayout {
-  int stage, tb, li, ut, d11, x2, total;
-};
-__host__ __device__ inline LuLayout lu_layout(int warps) {
-  LuLayout l{};
-  l.stage = 0;
-  l.tb = warps * 32 * PS;  // >= the rings' warps * kRingDoubles
-  l.li = l.tb + 32 * TS;
-  l.ut = l.li + 32 * TS;
-  l.d11 = l.ut;
-  l.x2 = l.ut + 32 * US;
-  l.total = l.x2 + 32 * TS;
-  return l;
-}
-static_assert(32 * PS >= kRingDoubles);
+// Shared memory, in doubles: the tiles, then a region per warp that is its operand
+// ring and, in the panel, its staging tile. The diagonal block that the
+// inversions read takes U's place, their scratch tile Tb's.
+constexpr int kTb = 0, kLi = 32 * US, kUt = 64 * US, kWarp = 96 * US, kPerWarp = 32 * PS;
+static_assert(kPerWarp >= kRingDoubles && PS <= US && TS <= US);
+constexpr int sys_smem(int warps) { return 8 * (kWarp + warps * kPerWarp); }
 
 __global__ void __launch_bounds__(kSysMaxN, 1)
 k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
@@ -454,24 +566,25 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
   __shared__ double s_det[3];  // det, log|det|, sign
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const LuLayout lay = lu_layout(nw);
-  double* Tb = sm + lay.tb;
-  double* Li = sm + lay.li;
-  double* Ut = sm + lay.ut;
-  double* D11 = sm + lay.d11;
-  double* X2 = sm + lay.x2;
-  double* stage = sm + lay.stage + warp * 32 * PS;
-  double2* ring = reinterpret_cast<double2*>(sm + warp * kRingDoubles);
-  const View v = view(sa, list ? list[blockIdx.x] : blockIdx.x);
-  const int n = v.n, ldw = v.ldw, nb = sys_blocks(n);
+  double* Tb = sm + kTb;
+  double* Li = sm + kLi;
+  double* Ut = sm + kUt;
+  double* D11 = Ut;
+  double* stage = sm + kWarp + warp * kPerWarp;
+  const unsigned ring = smem(stage) + 16 * lane;
+  const unsigned ulane = smem(Ut + g * US + 2 * t);
+  // what the inner loops do not need stays out of the registers
+  __shared__ View s_v;
+  if (tid == 0) s_v = view(sa, list ? list[blockIdx.x] : blockIdx.x);
+  __syncthreads();
+  double* const W = s_v.W;
+  const int n = s_v.n, nb = sys_blocks(n);
   for (int i = tid; i < n; i += blockDim.x) s_perm[i] = i;
   if (tid == 0) {
     ps.info = 0;
     s_det[0] = s_det[2] = 1.0;
     s_det[1] = 0.0;
   }
-  const bool want_det = sa.det || sa.sign || sa.logabs;
-  const bool avec = n % 2 == 0 && (reinterpret_cast<uintptr_t>(v.A) & 15) == 0;
   __syncthreads();
 
   for (int J = 0; J < nb; ++J) {
@@ -479,18 +592,21 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
     // 1. the warp's rows of the column block
     Acc<4> acc;
     Rows r;
+    const double* A = s_v.A;
+    const bool avec = n % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    r.live = n - 32 * warp - g;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int p = 32 * warp + 8 * i + g;
-      r.ok[i] = p < n;
-      const int row = r.ok[i] ? s_perm[p] : 0;
-      r.off[i] = row * ldw;
-      const double* src = v.A + (int64_t)row * n;
+      const bool ok = p < n;
+      const int row = ok ? s_perm[p] : 0;
+      r.off[i] = (unsigned)row * s_v.ldw * 8;
+      const double* src = A + (int64_t)row * n;
 #pragma unroll
       for (int ni = 0; ni < 4; ++ni) {
         const int col = 32 * J + 8 * ni + 2 * t;
         double x = 0.0, y = 0.0;
-        if (r.ok[i] && col < n) {
+        if (ok && col < n) {
           if (avec) {  // n is even: the pair ends inside the row
             const double2 z = __ldcs(reinterpret_cast<const double2*>(src + col));
             x = z.x;
@@ -508,22 +624,23 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
     if (J > 0) {
       const bool below = warp > 0 && warp < nb;
       if (J == 1) __syncthreads();  // the first block's inverse has been written
-      fetch_inverse(Li, v.dinv);
-      ring_start<true, false>(ring, v.W, r, 0, n, below);
+      fetch_inverse(Li, s_v.dinv, blockDim.x);
+      ring_start<true, false>(ring, W, r, 0, n, below);
+      if (J > 1) __syncthreads();  // Tb is no longer the inversions' scratch tile
       for (int K = 0; K < J; ++K) {
         if (warp == K) store_tile<4>(Tb, acc);
-        cp_wait<3>();  // the inverse; at most three operand stages stay in flight
+        cp_wait<2>();  // the inverse; at most two operand stages stay in flight
         __syncthreads();
-        tile_product<4, false>(Li, Tb, Ut, [&](int row, int col, double v0, double v1) {
-          double* o = v.W + s_perm[32 * K + row] * ldw + 32 * J + col;
-          if (32 * J + col < ldw) *reinterpret_cast<double2*>(o) = make_double2(v0, v1);
-        });
+        tile_product<4, false>(Li, Tb, Ut);
         __syncthreads();
-        if (K + 1 < J) fetch_inverse(Li, v.dinv + (K + 1) * 2048);
-        else cp_commit();
         if (warp > K && warp < nb) {
-          update<4, true, false>(acc, ring, v.W, r, Ut, K, K + 1, K + 1 < J && warp > K + 1, n);
+          update<4, true, false>(acc, ring, W, r, ulane, K, K + 1, K + 1 < J && warp > K + 1, n);
         } else {
+          if (warp <= K) {  // the warps that are done: U out, the next inverse in
+            if (K + 1 < J) fetch_inverse(Li, s_v.dinv + (K + 1) * 2048, 32 * (K + 1));
+            product_out<4, true>(Ut, s_v.ldw - 32 * J, 0, K + 1,
+                                 [&](int row) { return W + s_perm[32 * K + row] * s_v.ldw + 32 * J; });
+          }
 #pragma unroll
           for (int q = 0; q < 4; ++q) cp_commit();  // the waits count groups
         }
@@ -531,41 +648,30 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
       cp_wait<0>();
       __syncthreads();  // the rings become the staging tiles, Ut the diagonal block
     }
-    // 3. the panel: warps J..nb-1, a row per thread
+    // 3. the panel: warps J..nb-1
     if (warp >= J && warp < nb) {
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            stage[(16 * m + g + 8 * (e >> 1)) * PS + 8 * ni + 2 * t + (e & 1)] = acc.v[m][ni][e];
-      __syncwarp();
-      double a[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) a[c] = stage[lane * PS + c];
       const int p = 32 * warp + lane;
       const bool valid = p < n;
       const int phys = valid ? s_perm[p] : 0;
       int pos = p - 32 * J, nswap = 0;
       if (valid && J + 1 < nb) {  // the row's next column block on its way into L2
-        const double* nx = v.A + (int64_t)phys * n + 32 * (J + 1);
+        const double* nx = s_v.A + (int64_t)phys * n + 32 * (J + 1);
         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx));
         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx + min(16, n - 32 * (J + 1) - 1)));
         asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx + min(31, n - 32 * (J + 1) - 1)));
       }
-      const int info = panel(ps, a, pos, valid, kb, warp - J, nb - J, stage + lane * PS, nswap);
+      const int info = panel(ps, acc, pos, valid, kb, warp - J, nb - J, stage, nswap);
       if (info) {
         if (tid == 32 * J) ps.info = 32 * J + info;
       } else {
         if (valid) s_perm[32 * J + pos] = phys;
         __syncwarp();
-        const int off = phys * ldw, at = valid ? pos : n;
+        const int off = phys * s_v.ldw, at = valid ? pos : n;
 #pragma unroll 8
         for (int rr = 0; rr < 32; ++rr) {
           const int o = __shfl_sync(kAll, off, rr), p2 = __shfl_sync(kAll, at, rr);
           const double x = stage[rr * PS + lane];
-          if (p2 < n && lane < kb) v.W[o + 32 * J + lane] = x;
+          if (p2 < n && lane < kb) W[o + 32 * J + lane] = x;
           if (p2 < kb) D11[p2 * PS + lane] = x;
         }
         if (tid == 32 * J && (nswap & 1)) {
@@ -577,20 +683,20 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
     __syncthreads();
     if (ps.info) {
       if (tid == 0) {
-        if (sa.state) sa.state[v.slot] = ps.info;
-        if (sa.det) sa.det[v.idx] = 0.0;
-        if (sa.sign) sa.sign[v.idx] = 0.0;
-        if (sa.logabs) sa.logabs[v.idx] = -INFINITY;
-        if (sa.info) sa.info[v.idx] = ps.info;
+        if (sa.state) sa.state[s_v.slot] = ps.info;
+        if (sa.det) sa.det[s_v.idx] = 0.0;
+        if (sa.sign) sa.sign[s_v.idx] = 0.0;
+        if (sa.logabs) sa.logabs[s_v.idx] = -INFINITY;
+        if (sa.info) sa.info[s_v.idx] = ps.info;
       }
       return;
     }
     // the diagonal block's inverses and the pivots' part of det / slogdet, each by
     // one warp, beside the other warps' loads of the next column block
-    double* di = v.dinv + (int64_t)J * 2048;
+    double* di = s_v.dinv + (int64_t)J * 2048;
     if (warp == 0) tri_inverse<false>(D11, Tb, di, kb);
-    if (warp == 1 % nw) tri_inverse<true>(D11, X2, di + 1024, kb);
-    if (warp == 2 % nw && want_det) {
+    if (warp == 1 % nw) tri_inverse<true>(D11, Tb, di + 1024, kb);
+    if (warp == 2 % nw && (sa.det || sa.sign || sa.logabs)) {
       // folded in the reference's order (linalg.cpp:400-403, 425-431)
       const double pv = lane < kb ? D11[lane * PS + lane] : 1.0;
       const double lg = log(fabs(pv)), sgn = pv / fabs(pv);
@@ -606,17 +712,17 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
         s_det[1] = la;
         s_det[2] = sg;
         if (J + 1 == nb) {
-          if (sa.det) sa.det[v.idx] = det;
-          if (sa.sign) sa.sign[v.idx] = sg;
-          if (sa.logabs) sa.logabs[v.idx] = la;
+          if (sa.det) sa.det[s_v.idx] = det;
+          if (sa.sign) sa.sign[s_v.idx] = sg;
+          if (sa.logabs) sa.logabs[s_v.idx] = la;
         }
       }
     }
   }
-  for (int i = tid; i < n; i += blockDim.x) v.perm[i] = s_perm[i];
+  for (int i = tid; i < n; i += blockDim.x) s_v.perm[i] = s_perm[i];
   if (tid == 0) {
-    if (sa.state) sa.state[v.slot] = 0;
-    if (sa.info) sa.info[v.idx] = 0;
+    if (sa.state) sa.state[s_v.slot] = 0;
+    if (sa.info) sa.info[s_v.idx] = 0;
   }
 }
 
@@ -624,53 +730,58 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
 // Substitution of one strip: C = P B (or P times columns of the identity), then
 // Y_K = L_KK^-1 C_K and C_w -= L_wK Y_K downwards, X_K = U_KK^-1 Y_K and
 // Y_w -= U_wK X_K upwards.
-constexpr int solve_smem(int warps) { return (warps * kRingDoubles + 64 * TS + 32 * US) * 8; }
+
+struct Strip {  // what the inner loops do not need, in shared memory
+  View v;
+  const double* B;
+  double* X;  // column c0 of row 0
+  int ldx, c0, width, inverse;
+};
 
 template <int NI, bool VEC>
-__device__ __forceinline__ void solve_strip(const SysArgs& sa, const View& v, bool inverse, int c0, int width,
-                                            double* sm) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double2* ring = reinterpret_cast<double2*>(sm + warp * kRingDoubles);
-  double* Tb = sm + (blockDim.x >> 5) * kRingDoubles;
-  double* Li = Tb + 32 * TS;
-  double* Ut = Li + 32 * TS;
+__device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, double* sm) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* Tb = sm + kTb;
+  double* Li = sm + kLi;
+  double* Ut = sm + kUt;
   const int g = lane >> 2, t = lane & 3;
-  const int n = v.n, nb = sys_blocks(n);
-  const int ldx = inverse ? n : v.nrhs;
-  double* X = inverse ? sa.inv + v.inv_off : sa.X + v.b_off;
-  const double* B = sa.B + v.b_off;
+  const unsigned ring = smem(sm + kWarp + warp * kPerWarp) + 16 * lane;
+  const unsigned ulane = smem(Ut + g * US + 2 * t);
+  const double* const W = s.v.W;
+  const int n = s.v.n, nb = sys_blocks(n);
   Acc<NI> acc;
   Rows r;
+  r.live = n - 32 * warp - g;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int p = 32 * warp + 8 * i + g;
-    r.ok[i] = p < n;
-    const int row = r.ok[i] ? v.perm[p] : 0;
-    r.off[i] = (sa.w_by_position ? (r.ok[i] ? p : 0) : row) * v.ldw;
+    const bool ok = p < n;
+    const int row = ok ? s.v.perm[p] : 0;
+    r.off[i] = (unsigned)(sa.w_by_position ? (ok ? p : 0) : row) * s.v.ldw * 8;
 #pragma unroll
     for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int col = 8 * ni + 2 * t + e;
         double x = 0.0;
-        if (r.ok[i] && col < width) x = inverse ? (row == c0 + col ? 1.0 : 0.0) : B[(int64_t)row * ldx + c0 + col];
+        if (ok && col < s.width) x = s.inverse ? (row == s.c0 + col ? 1.0 : 0.0) : s.B[(int64_t)row * s.ldx + col];
         acc.v[i >> 1][ni][2 * (i & 1) + e] = x;
       }
   }
-  auto no_store = [](int, int, double, double) {};
-  fetch_inverse(Li, v.dinv);
-  ring_start<VEC, false>(ring, v.W, r, 0, n, warp > 0 && warp < nb);
+  // a block's inverse is fetched by the warps that have nothing to update
+  fetch_inverse(Li, s.v.dinv, blockDim.x);
+  ring_start<VEC, false>(ring, W, r, 0, n, warp > 0 && warp < nb);
   for (int K = 0; K < nb; ++K) {
     if (warp == K) store_tile<NI>(Tb, acc);
-    cp_wait<3>();  // the inverse; at most three operand stages stay in flight
+    cp_wait<2>();  // the inverse; at most two operand stages stay in flight
     __syncthreads();
-    tile_product<NI, false>(Li, Tb, Ut, no_store);
+    tile_product<NI, false>(Li, Tb, Ut);
     __syncthreads();
-    // the next block's L_KK^-1, after the last one the first U_KK^-1 (same block)
-    fetch_inverse(Li, v.dinv + (K + 1 < nb ? (K + 1) * 2048 : K * 2048 + 1024));
     if (warp > K && warp < nb) {
-      update<NI, VEC, false>(acc, ring, v.W, r, Ut, K, K + 1, warp > K + 1, n);
+      update<NI, VEC, false>(acc, ring, W, r, ulane, K, K + 1, warp > K + 1, n);
     } else {
+      // the next L_KK^-1, after the last one the first U_KK^-1 (same block)
+      if (warp <= K) fetch_inverse(Li, s.v.dinv + (K + 1 < nb ? (K + 1) * 2048 : K * 2048 + 1024), 32 * (K + 1));
       if (warp == K) {  // Y_K back into its owner's registers for the way up
 #pragma unroll
         for (int m = 0; m < 2; ++m)
@@ -684,24 +795,21 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const View& v, bo
       for (int q = 0; q < 4; ++q) cp_commit();  // the waits count groups
     }
   }
-  ring_start<VEC, true>(ring, v.W, r, nb - 1, n, warp < nb - 1);
+  ring_start<VEC, true>(ring, W, r, nb - 1, n, warp < nb - 1);
   for (int K = nb - 1; K >= 0; --K) {
     if (warp == K) store_tile<NI>(Tb, acc);
-    cp_wait<3>();
+    cp_wait<2>();
     __syncthreads();
-    tile_product<NI, true>(Li, Tb, Ut, [&](int row, int col, double v0, double v1) {
-      if (32 * K + row < n) {
-        double* o = X + (int64_t)(32 * K + row) * ldx + c0 + col;
-        if (col < width) o[0] = v0;
-        if (col + 1 < width) o[1] = v1;
-      }
-    });
+    tile_product<NI, true>(Li, Tb, Ut);
     __syncthreads();
-    if (K > 0) fetch_inverse(Li, v.dinv + (K - 1) * 2048 + 1024);
-    else cp_commit();
     if (warp < K) {
-      update<NI, VEC, true>(acc, ring, v.W, r, Ut, K, K - 1, warp < K - 1, n);
+      update<NI, VEC, true>(acc, ring, W, r, ulane, K, K - 1, warp < K - 1, n);
     } else {
+      const int free = (int)(blockDim.x >> 5) - K;
+      if (K > 0) fetch_inverse(Li, s.v.dinv + (K - 1) * 2048 + 1024, 32 * free, 32 * K);
+      product_out<NI, false>(Ut, s.width, K, free, [&](int row) {
+        return 32 * K + row < n ? s.X + (int64_t)(32 * K + row) * s.ldx : nullptr;
+      });
 #pragma unroll
       for (int q = 0; q < 4; ++q) cp_commit();
     }
@@ -711,29 +819,42 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const View& v, bo
 __global__ void __launch_bounds__(kSysMaxN, 1)
 k_sys_solve(SysArgs sa, const SysItem* __restrict__ items) {
   extern __shared__ __align__(16) double sm[];
-  SysItem it;
-  if (items) {
-    it = items[blockIdx.x];
-  } else {
-    const int nr = (sa.unrhs + 31) / 32, ni = sa.uinv ? (sa.un + 31) / 32 : 0;
-    it.sys = blockIdx.x / (nr + ni);
-    const int k = blockIdx.x - it.sys * (nr + ni);
-    it.inverse = k >= nr;
-    it.c0 = 32 * (k >= nr ? k - nr : k);
-    it.width = (int16_t)min(32, (it.inverse ? sa.un : sa.unrhs) - it.c0);
+  __shared__ Strip s_s;
+  __shared__ int s_skip;
+  if (threadIdx.x == 0) {
+    SysItem it;
+    if (items) {
+      it = items[blockIdx.x];
+    } else {
+      const int nr = (sa.unrhs + 31) / 32, ni = sa.uinv ? (sa.un + 31) / 32 : 0;
+      it.sys = blockIdx.x / (nr + ni);
+      const int k = blockIdx.x - it.sys * (nr + ni);
+      it.inverse = k >= nr;
+      it.c0 = 32 * (k >= nr ? k - nr : k);
+      it.width = (int16_t)min(32, (it.inverse ? sa.un : sa.unrhs) - it.c0);
+    }
+    const View v = view(sa, it.sys);
+    s_s.v = v;
+    s_s.inverse = it.inverse;
+    s_s.c0 = it.c0;
+    s_s.width = it.width;
+    s_s.ldx = it.inverse ? v.n : v.nrhs;
+    s_s.B = sa.B + v.b_off + it.c0;
+    s_s.X = (it.inverse ? sa.inv + v.inv_off : sa.X + v.b_off) + it.c0;
+    s_skip = sa.state && sa.state[v.slot];  // singular: nothing to solve with
   }
-  const View v = view(sa, it.sys);
-  if (sa.state && sa.state[v.slot]) return;  // singular: nothing to solve with
-  const bool vec = v.ldw % 2 == 0 && (reinterpret_cast<uintptr_t>(v.W) & 15) == 0;
-  if (it.width <= 8) {
-    if (vec) solve_strip<1, true>(sa, v, it.inverse, it.c0, it.width, sm);
-    else solve_strip<1, false>(sa, v, it.inverse, it.c0, it.width, sm);
-  } else if (it.width <= 16) {
-    if (vec) solve_strip<2, true>(sa, v, it.inverse, it.c0, it.width, sm);
-    else solve_strip<2, false>(sa, v, it.inverse, it.c0, it.width, sm);
+  __syncthreads();
+  if (s_skip) return;
+  const bool vec = s_s.v.ldw % 2 == 0 && (reinterpret_cast<uintptr_t>(s_s.v.W) & 15) == 0;
+  if (s_s.width <= 8) {
+    if (vec) solve_strip<1, true>(sa, s_s, sm);
+    else solve_strip<1, false>(sa, s_s, sm);
+  } else if (s_s.width <= 16) {
+    if (vec) solve_strip<2, true>(sa, s_s, sm);
+    else solve_strip<2, false>(sa, s_s, sm);
   } else {
-    if (vec) solve_strip<4, true>(sa, v, it.inverse, it.c0, it.width, sm);
-    else solve_strip<4, false>(sa, v, it.inverse, it.c0, it.width, sm);
+    if (vec) solve_strip<4, true>(sa, s_s, sm);
+    else solve_strip<4, false>(sa, s_s, sm);
   }
 }
 
@@ -744,7 +865,7 @@ k_sys_solve(SysArgs sa, const SysItem* __restrict__ items) {
 __global__ void __launch_bounds__(64)
 k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __restrict__ list) {
   __shared__ double D[32 * PS];
-  __shared__ __align__(16) double X[2][32 * TS];
+  __shared__ double X[32 * TS];
   const int s = list ? list[blockIdx.x] : blockIdx.x;
   const View v = view(sa, s);
   const int n = v.n, b = (int)blockIdx.y - 1;
@@ -780,8 +901,8 @@ k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __res
   }
   __syncthreads();
   double* di = v.dinv + (int64_t)b * 2048;
-  if (threadIdx.x < 32) tri_inverse<false>(D, X[0], di, kb);
-  else tri_inverse<true>(D, X[1], di + 1024, kb);
+  if (threadIdx.x < 32) tri_inverse<false>(D, X, di, kb);
+  else tri_inverse<true>(D, X, di + 1024, kb);
 }
 
 }  // namespace
@@ -790,7 +911,7 @@ cudaError_t launch_sys_lu(const SysArgs& sa, const int32_t* list, int nsys, int 
   if (nsys <= 0) return cudaSuccess;
   if (nmax > kSysMaxN) return cudaErrorInvalidValue;
   const int nw = sys_blocks(nmax);
-  k_sys_lu<<<nsys, 32 * nw, sizeof(double) * lu_layout(nw).total, st>>>(sa, list);
+  k_sys_lu<<<nsys, 32 * nw, sys_smem(nw), st>>>(sa, list);
   return cudaGetLastError();
 }
 
@@ -800,7 +921,7 @@ cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t ni
   if (nitems <= 0) return cudaSuccess;
   if (nmax > kSysMaxN || nitems > INT_MAX) return cudaErrorInvalidValue;
   const int nw = sys_blocks(nmax);
-  k_sys_solve<<<(unsigned)nitems, 32 * nw, solve_smem(nw), st>>>(sa, items);
+  k_sys_solve<<<(unsigned)nitems, 32 * nw, sys_smem(nw), st>>>(sa, items);
   return cudaGetLastError();
 }
 
@@ -814,9 +935,9 @@ cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int
 
 cudaError_t sys_prepare_kernels() {
   cudaError_t e = cudaFuncSetAttribute(k_sys_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sizeof(double) * lu_layout(kMaxWarps).total);
+                                       sys_smem(kMaxWarps));
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sys_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, solve_smem(kMaxWarps));
+    e = cudaFuncSetAttribute(k_sys_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, sys_smem(kMaxWarps));
   return e;
 }
 

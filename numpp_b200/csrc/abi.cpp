@@ -121,7 +121,7 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
     sa.unrhs = (flags & NPPB_WANT_SOLVE) ? nrhs : 0;
     sa.uinv = (flags & NPPB_WANT_INV) ? 1 : 0;
     NPPB_CUDA(launch_sys_lu(sa, nullptr, (int)count, n, st), "batched LU launch");
-    NPPB_CUDA(launch_sys_solve(sa, nullptr, 0, (int)count, n, st), "batched substitution launch");
+    NPPB_CUDA(launch_sys_solve_uniform(sa, (int)count, st), "batched substitution launch");
     return NPPB_OK;
   }
   if (n > 32 && !(flags & NPPB_WANT_LU)) {
@@ -215,7 +215,7 @@ int d_getrs(int64_t count, int32_t n, int32_t nrhs, const double* dLU, const int
     sa.un = n;
     sa.unrhs = nrhs;
     NPPB_CUDA(launch_sys_prepare(sa, dipiv, nullptr, (int)count, n, st), "getrs preparation launch");
-    NPPB_CUDA(launch_sys_solve(sa, nullptr, 0, (int)count, n, st), "getrs launch");
+    NPPB_CUDA(launch_sys_solve_uniform(sa, (int)count, st), "getrs launch");
     return NPPB_OK;
   }
   if (n > 32) {

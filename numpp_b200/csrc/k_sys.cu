@@ -816,8 +816,12 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
   }
 }
 
+// A kernel per strip width: narrow strips need fewer registers, so more of their
+// CTAs share an SM. items == nullptr: strips `first` .. `first` + `per` - 1 of the
+// right-hand sides (inverse: of the inverse) of every system of a uniform batch.
+template <int NI, bool VEC>
 __global__ void __launch_bounds__(kSysMaxN, 1)
-k_sys_solve(SysArgs sa, const SysItem* __restrict__ items) {
+k_sys_solve(SysArgs sa, const SysItem* __restrict__ items, int inverse, int first, int per) {
   extern __shared__ __align__(16) double sm[];
   __shared__ Strip s_s;
   __shared__ int s_skip;
@@ -826,12 +830,10 @@ k_sys_solve(SysArgs sa, const SysItem* __restrict__ items) {
     if (items) {
       it = items[blockIdx.x];
     } else {
-      const int nr = (sa.unrhs + 31) / 32, ni = sa.uinv ? (sa.un + 31) / 32 : 0;
-      it.sys = blockIdx.x / (nr + ni);
-      const int k = blockIdx.x - it.sys * (nr + ni);
-      it.inverse = k >= nr;
-      it.c0 = 32 * (k >= nr ? k - nr : k);
-      it.width = (int16_t)min(32, (it.inverse ? sa.un : sa.unrhs) - it.c0);
+      it.sys = blockIdx.x / per;
+      it.inverse = (int16_t)inverse;
+      it.c0 = 32 * (first + (int)blockIdx.x - it.sys * per);
+      it.width = (int16_t)min(32, (inverse ? sa.un : sa.unrhs) - it.c0);
     }
     const View v = view(sa, it.sys);
     s_s.v = v;
@@ -844,18 +846,7 @@ k_sys_solve(SysArgs sa, const SysItem* __restrict__ items) {
     s_skip = sa.state && sa.state[v.slot];  // singular: nothing to solve with
   }
   __syncthreads();
-  if (s_skip) return;
-  const bool vec = s_s.v.ldw % 2 == 0 && (reinterpret_cast<uintptr_t>(s_s.v.W) & 15) == 0;
-  if (s_s.width <= 8) {
-    if (vec) solve_strip<1, true>(sa, s_s, sm);
-    else solve_strip<1, false>(sa, s_s, sm);
-  } else if (s_s.width <= 16) {
-    if (vec) solve_strip<2, true>(sa, s_s, sm);
-    else solve_strip<2, false>(sa, s_s, sm);
-  } else {
-    if (vec) solve_strip<4, true>(sa, s_s, sm);
-    else solve_strip<4, false>(sa, s_s, sm);
-  }
+  if (!s_skip) solve_strip<NI, VEC>(sa, s_s, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -915,14 +906,52 @@ cudaError_t launch_sys_lu(const SysArgs& sa, const int32_t* list, int nsys, int 
   return cudaGetLastError();
 }
 
-cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t nitems, int nsys, int nmax,
-                             cudaStream_t st) {
-  if (!items) nitems = (int64_t)nsys * ((sa.unrhs + 31) / 32 + (sa.uinv ? (sa.un + 31) / 32 : 0));
+namespace {
+
+template <int NI>
+cudaError_t launch_strips(const SysArgs& sa, const SysItem* items, int64_t nitems, int nmax, int inverse, int first,
+                          int per, cudaStream_t st) {
   if (nitems <= 0) return cudaSuccess;
   if (nmax > kSysMaxN || nitems > INT_MAX) return cudaErrorInvalidValue;
   const int nw = sys_blocks(nmax);
-  k_sys_solve<<<(unsigned)nitems, 32 * nw, sys_smem(nw), st>>>(sa, items);
+  // 16-byte operand loads: workspaces always, kept factors (uniform batches) of even order
+  const bool vec = !sa.w_by_position || (sa.un % 2 == 0 && (reinterpret_cast<uintptr_t>(sa.W) & 15) == 0);
+  if (vec) k_sys_solve<NI, true><<<(unsigned)nitems, 32 * nw, sys_smem(nw), st>>>(sa, items, inverse, first, per);
+  else k_sys_solve<NI, false><<<(unsigned)nitems, 32 * nw, sys_smem(nw), st>>>(sa, items, inverse, first, per);
   return cudaGetLastError();
+}
+
+cudaError_t launch_strips(const SysArgs& sa, const SysItem* items, int64_t nitems, int nmax, int width, int inverse,
+                          int first, int per, cudaStream_t st) {
+  switch (sys_width_class(width)) {
+    case 0: return launch_strips<1>(sa, items, nitems, nmax, inverse, first, per, st);
+    case 1: return launch_strips<2>(sa, items, nitems, nmax, inverse, first, per, st);
+    default: return launch_strips<4>(sa, items, nitems, nmax, inverse, first, per, st);
+  }
+}
+
+template <int NI>
+cudaError_t prepare_strips() {
+  cudaError_t e = cudaFuncSetAttribute(k_sys_solve<NI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       sys_smem(kMaxWarps));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_sys_solve<NI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sys_smem(kMaxWarps));
+  return e;
+}
+
+}  // namespace
+
+cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t nitems, int width, int nmax,
+                             cudaStream_t st) {
+  return launch_strips(sa, items, nitems, nmax, width, 0, 0, 1, st);
+}
+
+cudaError_t launch_sys_solve_uniform(const SysArgs& sa, int nsys, cudaStream_t st) {
+  const int full = sa.unrhs / 32, rest = sa.unrhs % 32, ni = sa.uinv ? sys_blocks(sa.un) : 0;
+  cudaError_t e = launch_strips(sa, nullptr, (int64_t)nsys * full, sa.un, 32, 0, 0, full, st);
+  if (e == cudaSuccess && rest) e = launch_strips(sa, nullptr, nsys, sa.un, rest, 0, full, 1, st);
+  if (e == cudaSuccess && ni) e = launch_strips(sa, nullptr, (int64_t)nsys * ni, sa.un, 32, 1, 0, ni, st);
+  return e;
 }
 
 cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int32_t* list, int nsys, int nmax,
@@ -936,8 +965,9 @@ cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int
 cudaError_t sys_prepare_kernels() {
   cudaError_t e = cudaFuncSetAttribute(k_sys_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        sys_smem(kMaxWarps));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sys_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, sys_smem(kMaxWarps));
+  if (e == cudaSuccess) e = prepare_strips<1>();
+  if (e == cudaSuccess) e = prepare_strips<2>();
+  if (e == cudaSuccess) e = prepare_strips<4>();
   return e;
 }
 

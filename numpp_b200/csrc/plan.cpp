@@ -213,7 +213,7 @@ int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_
     SysClass sc;
     sc.first = r;
     sc.nmax = desc[sys_members[r]].n;
-    sc.item_first = (int64_t)sys_items.size();
+    std::vector<SysItem> by_width[3];
     for (; r < nsys && sys_blocks(desc[sys_members[r]].n) == sys_blocks(sc.nmax); ++r) {
       SysDesc& s = desc[sys_members[r]];
       s.pad_ = (int32_t)r;
@@ -222,16 +222,20 @@ int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_
       kind_flops[kKindUpdate] += 2.0 / 3.0 * nd * nd * nd;
       kind_flops[kKindBack] += 2.0 * nd * nd * cols;
       auto strips = [&](int16_t inverse, int columns) {
-        for (int c = 0; c < columns; c += 32)
-          sys_items.push_back(SysItem{sys_members[r], inverse, (int16_t)std::min(32, columns - c), c, 0});
+        for (int c = 0; c < columns; c += 32) {
+          const int w = std::min(32, columns - c);
+          by_width[sys_width_class(w)].push_back(SysItem{sys_members[r], inverse, (int16_t)w, c, 0});
+        }
       };
       if (s.inv_off >= 0) strips(1, s.n);
       if (solve) strips(0, s.nrhs);
     }
     sc.num = r - sc.first;
-    sc.item_count = (int64_t)sys_items.size() - sc.item_first;
-    std::stable_sort(sys_items.begin() + sc.item_first, sys_items.end(),
-                     [](const SysItem& x, const SysItem& y) { return x.width > y.width; });
+    for (int w = 0; w < 3; ++w) {
+      sc.item_first[w] = (int64_t)sys_items.size();
+      sc.item_count[w] = (int64_t)by_width[w].size();
+      sys_items.insert(sys_items.end(), by_width[w].begin(), by_width[w].end());
+    }
     sys_classes.push_back(sc);
   }
 
@@ -439,8 +443,16 @@ cudaError_t Plan::launch_sys(const Ptrs& p, int cls, cudaStream_t st) const {
   const SysClass& c = sys_classes[cls];
   const SysArgs sa = sys_args(p);
   const cudaError_t e = launch_sys_lu(sa, d_sys_list + c.first, (int)c.num, c.nmax, st);
-  if (e != cudaSuccess || !c.item_count) return e;
-  return launch_sys_solve(sa, d_sys_items + c.item_first, c.item_count, 0, c.nmax, st);
+  return e == cudaSuccess ? solve_sys(sa, c, st) : e;
+}
+
+cudaError_t Plan::solve_sys(const SysArgs& sa, const SysClass& c, cudaStream_t st) const {
+  static constexpr int kWidth[3] = {8, 16, 32};
+  for (int w = 2; w >= 0; --w) {
+    const cudaError_t e = launch_sys_solve(sa, d_sys_items + c.item_first[w], c.item_count[w], kWidth[w], c.nmax, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t Plan::launch_warp(const Ptrs& p, int cls, cudaStream_t st) const {
@@ -545,8 +557,7 @@ int Plan::time_kernels(const Ptrs& p, cudaStream_t st, double* ms) const {
   for (const SysClass& c : sys_classes) {
     const SysArgs sa = sys_args(p);
     timed(kKindUpdate, [&] { return launch_sys_lu(sa, d_sys_list + c.first, (int)c.num, c.nmax, st); });
-    if (c.item_count)
-      timed(kKindBack, [&] { return launch_sys_solve(sa, d_sys_items + c.item_first, c.item_count, 0, c.nmax, st); });
+    if (c.launches() > 1) timed(kKindBack, [&] { return solve_sys(sa, c, st); });
   }
   const StepArgs sa = step_args(p);
   for (const Chain& ch : chains) {
@@ -661,7 +672,7 @@ int Plan::launches_per_execute() const {
   };
   // wide strips: the chain's largest order bounds the passes
   int l = (int)warp_classes.size();
-  for (const SysClass& c : sys_classes) l += 1 + (c.item_count ? 1 : 0);
+  for (const SysClass& c : sys_classes) l += c.launches();
   for (const Chain& ch : chains) {
     const int nn = (int)ch.narrow_count, nw = (int)(ch.back_count - ch.narrow_count);
     for (int fwd = solve_only ? 1 : 0; fwd >= 0; --fwd) {

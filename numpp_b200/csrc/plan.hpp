@@ -40,7 +40,8 @@ class Plan {
   struct SysClass {
     int nmax;
     int64_t first, num;            // in d_sys_list
-    int64_t item_first, item_count;  // in d_sys_items
+    int64_t item_first[3], item_count[3];  // in d_sys_items, by sys_width_class
+    int launches() const { return 1 + (item_count[0] > 0) + (item_count[1] > 0) + (item_count[2] > 0); }
   };
   struct PanelRange {
     int64_t first, num;
@@ -81,6 +82,7 @@ class Plan {
   cudaError_t launch_warp(const Ptrs& p, int cls, cudaStream_t st) const;
   cudaError_t launch_chain(const Ptrs& p, int chain, cudaStream_t st) const;
   cudaError_t launch_sys(const Ptrs& p, int cls, cudaStream_t st) const;
+  cudaError_t solve_sys(const SysArgs& sa, const SysClass& c, cudaStream_t st) const;
   // Every launch of one execution in order, each between two CUDA events on
   // `st`; ms[kind] accumulates the durations per kernel kind (KernelKind).
   int time_kernels(const Ptrs& p, cudaStream_t st, double* ms) const;

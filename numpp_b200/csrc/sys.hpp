@@ -49,10 +49,12 @@ struct SysArgs {
 // LU with partial pivoting of `nsys` systems with (maximum order) nmax <= 512,
 // one CTA of sys_blocks(nmax) warps each.
 cudaError_t launch_sys_lu(const SysArgs& sa, const int32_t* list, int nsys, int nmax, cudaStream_t st);
-// Forward and back substitution of `nitems` strips (items == nullptr: every
-// strip of a uniform batch of nsys systems).
-cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t nitems, int nsys, int nmax,
+// Forward and back substitution: `nitems` strips of one width class (8, 16 or 32
+// columns at most; `width` = the widest), or every strip of a uniform batch.
+inline int sys_width_class(int width) { return width <= 8 ? 0 : width <= 16 ? 1 : 2; }
+cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t nitems, int width, int nmax,
                              cudaStream_t st);
+cudaError_t launch_sys_solve_uniform(const SysArgs& sa, int nsys, cudaStream_t st);
 // Permutations and diagonal inverses of kept factors (swap lists ipiv at
 // piv_off): fills sa.perm and sa.dinv.
 cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int32_t* list, int nsys, int nmax,

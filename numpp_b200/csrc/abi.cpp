@@ -112,6 +112,7 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
     sa.perm = perm_m.as<int32_t>();
     sa.dinv = dinv_m.as<double>();
     sa.state = state_m.as<int32_t>();
+    sa.state_stride = sizeof(int32_t);
     sa.B = dB; sa.X = dX; sa.inv = dInv;
     sa.det = (flags & NPPB_WANT_DET) ? dDet : nullptr;
     sa.sign = (flags & NPPB_WANT_SLOGDET) ? dSign : nullptr;
@@ -153,7 +154,26 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
     sa.un = n;
     sa.unrhs = (flags & NPPB_WANT_SOLVE) ? nrhs : 0;
     sa.uinv = (flags & NPPB_WANT_INV) ? 1 : 0;
-    NPPB_CUDA(run_step_uniform(sa, (int)count, st), "batched LU launch");
+    // the back substitution of the solutions and inverses that the steps carried along
+    DevMem dinv_m;
+    NPPB_RC(scratch<double>(dinv_m, (size_t)count * sys_dinv(n), st));
+    NPPB_CUDA(run_step_uniform(sa, (int)count, st, false), "batched LU launch");
+    SysArgs su{};
+    su.W = LU;
+    su.w_by_position = 1;
+    su.upper_only = 1;
+    su.dinv = dinv_m.as<double>();
+    su.state = &sa.scratch->info;
+    su.state_stride = sizeof(StepScratch);
+    su.X = dX;
+    su.inv = sa.inv;
+    su.un = n;
+    su.unrhs = sa.unrhs;
+    su.uinv = sa.uinv;
+    if (su.unrhs || su.uinv) {
+      NPPB_CUDA(launch_sys_prepare(su, nullptr, nullptr, (int)count, n, st), "substitution preparation launch");
+      NPPB_CUDA(launch_sys_solve_uniform(su, (int)count, st), "batched substitution launch");
+    }
     return NPPB_OK;
   }
   if (n > 32) {
@@ -202,7 +222,10 @@ int d_getrs(int64_t count, int32_t n, int32_t nrhs, const double* dLU, const int
   if (count == 0 || n == 0 || nrhs == 0) return NPPB_OK;
   if (!dLU || !dipiv || !dB || !dX) return arg_error("getrs needs LU, ipiv, B and X");
   if (!device()) return NPPB_E_NODEV;
-  if (n > 32 && n <= kSysMaxN) {
+  if (n > 32) {
+    // the permutation and the diagonal blocks' inverses, then both
+    // substitutions in one launch (every strip is read before it is written, so
+    // X may be B)
     DevMem perm_m, dinv_m;
     NPPB_RC(scratch<int32_t>(perm_m, (size_t)count * n, st));
     NPPB_RC(scratch<double>(dinv_m, (size_t)count * sys_dinv(n), st));
@@ -216,26 +239,6 @@ int d_getrs(int64_t count, int32_t n, int32_t nrhs, const double* dLU, const int
     sa.unrhs = nrhs;
     NPPB_CUDA(launch_sys_prepare(sa, dipiv, nullptr, (int)count, n, st), "getrs preparation launch");
     NPPB_CUDA(launch_sys_solve_uniform(sa, (int)count, st), "getrs launch");
-    return NPPB_OK;
-  }
-  if (n > 32) {
-    int rc = NPPB_OK;
-    auto pl = uniform_plan(count, n, nrhs, NPPB_WANT_SOLVE, true, false, &rc);
-    if (!pl) return rc;
-    DevMem tmp;
-    double* X = dX;
-    if (dX == dB) {  // the row gather needs a separate output
-      NPPB_RC(scratch<double>(tmp, (size_t)count * n * nrhs, st));
-      X = tmp.as<double>();
-    }
-    Plan::Ptrs p{};
-    p.B = dB; p.X = X;
-    p.LU = const_cast<double*>(dLU);
-    p.ipiv = const_cast<int32_t*>(dipiv);
-    NPPB_RC(pl->execute(p, st));
-    if (X != dX)
-      NPPB_CUDA(cudaMemcpyAsync(dX, X, sizeof(double) * count * n * nrhs, cudaMemcpyDeviceToDevice, st),
-                "device copy");
     return NPPB_OK;
   }
   Batch bt{};

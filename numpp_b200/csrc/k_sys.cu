@@ -25,6 +25,9 @@
 //
 // What bounds it: FP64 tensor throughput in 2 (mma.m16n8k8, 64 FMA per cycle
 // and SM), the dependent pivot steps in 3.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <climits>
 #include <cmath>
 
@@ -40,6 +43,7 @@ constexpr int TS = 36;   // row stride of the inversions' scratch tile
 constexpr int PS = 34;   // row stride of the panel staging tiles (16-byte reads, one row per thread)
 constexpr int GS = 10;   // row stride of the transposed 8-row U tile of a panel group
 constexpr int kMaxWarps = kSysMaxN / 32;
+namespace cg = cooperative_groups;
 constexpr unsigned kAll = 0xffffffffu;
 
 // D(16x8) += A(16x8) B(8x8), FP64, one warp. Lane 4g + t holds A[g][t],
@@ -91,6 +95,10 @@ __device__ __forceinline__ View view(const SysArgs& sa, int s) {
   }
   v.ldw = sa.w_by_position ? v.n : sys_ld(v.n);
   return v;
+}
+
+__device__ __forceinline__ int32_t* state_of(const SysArgs& sa, int slot) {
+  return reinterpret_cast<int32_t*>(reinterpret_cast<char*>(sa.state) + (int64_t)slot * sa.state_stride);
 }
 
 __device__ __forceinline__ void cp16(void* smem, const void* gmem) {
@@ -234,11 +242,20 @@ __device__ __forceinline__ void store_tile(double* Tb, const Acc<NI>& acc) {
 // triangular: half of the steps for half of its rows) with the block's rows.
 // Warps 0..3, one on each scheduler, take eight columns each (with one group of
 // eight: eight rows each); the others go on to the next barrier.
-template <int NI, bool UPPER>
+// CS > 1: into every CTA of the cluster.
+template <int NI, bool UPPER, int CS>
 __device__ __forceinline__ void tile_product(const double* Li, const double* Tb, double* Ut) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, warp = threadIdx.x >> 5;
   if (warp >= 4) return;
   const int step = min(4, (int)(blockDim.x >> 5));
+  auto put = [&](int col, int row, double v) {
+    if constexpr (CS == 1) {
+      Ut[col * US + row] = v;
+    } else {
+#pragma unroll
+      for (int c = 0; c < CS; ++c) cg::this_cluster().map_shared_rank(Ut, c)[col * US + row] = v;
+    }
+  };
   auto left = [&](int row, int q) { return *reinterpret_cast<const double2*>(Li + row * US + 8 * q + 2 * t); };
   auto right = [&](int col, int q) {
     const double* b = Tb + (8 * q + 2 * t) * BS + col;
@@ -264,7 +281,7 @@ __device__ __forceinline__ void tile_product(const double* Li, const double* Tb,
       for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-          Ut[(8 * ni + 2 * t + (e & 1)) * US + 16 * m + g + 8 * (e >> 1)] = -d[m][e];
+          put(8 * ni + 2 * t + (e & 1), 16 * m + g + 8 * (e >> 1), -d[m][e]);
     }
   } else {
     for (int mi = warp; mi < 4; mi += step) {
@@ -276,7 +293,7 @@ __device__ __forceinline__ void tile_product(const double* Li, const double* Tb,
         dmma884(d[1], x.y, y.y);
       }
 #pragma unroll
-      for (int e = 0; e < 2; ++e) Ut[(2 * t + e) * US + 8 * mi + g] = -(d[0][e] + d[1][e]);
+      for (int e = 0; e < 2; ++e) put(2 * t + e, 8 * mi + g, -(d[0][e] + d[1][e]));
     }
   }
 }
@@ -557,6 +574,8 @@ __device__ __forceinline__ int panel(PanelShared& sh, Acc<4>& acc, int& pos, boo
 constexpr int kTb = 0, kLi = 32 * US, kUt = 64 * US, kWarp = 96 * US, kPerWarp = 32 * PS;
 static_assert(kPerWarp >= kRingDoubles && PS <= US && TS <= US);
 constexpr int sys_smem(int warps) { return 8 * (kWarp + warps * kPerWarp); }
+// of a cluster's CTA: U twice, behind the per-warp regions
+constexpr int sys_cluster_smem(int warps) { return sys_smem(warps) + 8 * 32 * US; }
 
 __global__ void __launch_bounds__(kSysMaxN, 1)
 k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
@@ -631,7 +650,7 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
         if (warp == K) store_tile<4>(Tb, acc);
         cp_wait<2>();  // the inverse; at most two operand stages stay in flight
         __syncthreads();
-        tile_product<4, false>(Li, Tb, Ut);
+        tile_product<4, false, 1>(Li, Tb, Ut);
         __syncthreads();
         if (warp > K && warp < nb) {
           update<4, true, false>(acc, ring, W, r, ulane, K, K + 1, K + 1 < J && warp > K + 1, n);
@@ -683,7 +702,7 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
     __syncthreads();
     if (ps.info) {
       if (tid == 0) {
-        if (sa.state) sa.state[s_v.slot] = ps.info;
+        if (sa.state) *state_of(sa, s_v.slot) = ps.info;
         if (sa.det) sa.det[s_v.idx] = 0.0;
         if (sa.sign) sa.sign[s_v.idx] = 0.0;
         if (sa.logabs) sa.logabs[s_v.idx] = -INFINITY;
@@ -721,7 +740,7 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
   }
   for (int i = tid; i < n; i += blockDim.x) s_v.perm[i] = s_perm[i];
   if (tid == 0) {
-    if (sa.state) sa.state[s_v.slot] = 0;
+    if (sa.state) *state_of(sa, s_v.slot) = 0;
     if (sa.info) sa.info[s_v.idx] = 0;
   }
 }
@@ -738,25 +757,32 @@ struct Strip {  // what the inner loops do not need, in shared memory
   int ldx, c0, width, inverse;
 };
 
-template <int NI, bool VEC>
+// In a cluster of CS CTAs (orders above 512, or few strips) block b belongs to warp
+// b / CS of CTA b % CS. The owner of block K pushes the solved rows into every
+// CTA; U alternates between two tiles, so that one cluster barrier per block
+// suffices: a tile is rewritten two blocks later, after the barrier in between
+// that every CTA passes with its update done.
+template <int NI, bool VEC, int CS>
 __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, double* sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int rank = CS > 1 ? (int)blockIdx.x % CS : 0;
+  const int blk = warp * CS + rank;  // the warp's block
   double* Tb = sm + kTb;
   double* Li = sm + kLi;
-  double* Ut = sm + kUt;
+  double* U0 = sm + kUt;
+  double* U1 = CS > 1 ? sm + kWarp + nw * kPerWarp : U0;
   const int g = lane >> 2, t = lane & 3;
   const unsigned ring = smem(sm + kWarp + warp * kPerWarp) + 16 * lane;
-  const unsigned ulane = smem(Ut + g * US + 2 * t);
   const double* const W = s.v.W;
   const int n = s.v.n, nb = sys_blocks(n);
   Acc<NI> acc;
   Rows r;
-  r.live = n - 32 * warp - g;
+  r.live = n - 32 * blk - g;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int p = 32 * warp + 8 * i + g;
+    const int p = 32 * blk + 8 * i + g;
     const bool ok = p < n;
-    const int row = ok ? s.v.perm[p] : 0;
+    const int row = !ok ? 0 : sa.upper_only ? p : s.v.perm[p];
     r.off[i] = (unsigned)(sa.w_by_position ? (ok ? p : 0) : row) * s.v.ldw * 8;
 #pragma unroll
     for (int ni = 0; ni < NI; ++ni)
@@ -764,75 +790,100 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
       for (int e = 0; e < 2; ++e) {
         const int col = 8 * ni + 2 * t + e;
         double x = 0.0;
-        if (ok && col < s.width) x = s.inverse ? (row == s.c0 + col ? 1.0 : 0.0) : s.B[(int64_t)row * s.ldx + col];
+        if (ok && col < s.width) {
+          if (sa.upper_only) x = s.X[(int64_t)p * s.ldx + col];
+          else x = s.inverse ? (row == s.c0 + col ? 1.0 : 0.0) : s.B[(int64_t)row * s.ldx + col];
+        }
         acc.v[i >> 1][ni][2 * (i & 1) + e] = x;
       }
   }
-  // a block's inverse is fetched by the warps that have nothing to update
-  fetch_inverse(Li, s.v.dinv, blockDim.x);
-  ring_start<VEC, false>(ring, W, r, 0, n, warp > 0 && warp < nb);
-  for (int K = 0; K < nb; ++K) {
-    if (warp == K) store_tile<NI>(Tb, acc);
-    cp_wait<2>();  // the inverse; at most two operand stages stay in flight
-    __syncthreads();
-    tile_product<NI, false>(Li, Tb, Ut);
-    __syncthreads();
-    if (warp > K && warp < nb) {
-      update<NI, VEC, false>(acc, ring, W, r, ulane, K, K + 1, warp > K + 1, n);
-    } else {
-      // the next L_KK^-1, after the last one the first U_KK^-1 (same block)
-      if (warp <= K) fetch_inverse(Li, s.v.dinv + (K + 1 < nb ? (K + 1) * 2048 : K * 2048 + 1024), 32 * (K + 1));
-      if (warp == K) {  // Y_K back into its owner's registers for the way up
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-          for (int ni = 0; ni < NI; ++ni)
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              acc.v[m][ni][e] = -Ut[(8 * ni + 2 * t + (e & 1)) * US + 16 * m + g + 8 * (e >> 1)];
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) cp_commit();  // the waits count groups
+  // One block: the owner's rows times the inverse, to every CTA of the cluster.
+  auto solve_block = [&](int K, double* Ut, auto upper) {
+    if (CS == 1 || K % CS == rank) {
+      if (blk == K) store_tile<NI>(Tb, acc);
+      cp_wait<2>();  // the inverse; at most two operand stages stay in flight
+      __syncthreads();
+      tile_product<NI, decltype(upper)::value, CS>(Li, Tb, Ut);
     }
+    if constexpr (CS > 1) cg::this_cluster().sync();
+    else __syncthreads();
+  };
+  // A CTA fetches the inverse of its own next block, by the warps that have
+  // nothing to update.
+  if (!sa.upper_only) {
+    if (rank < nb) fetch_inverse(Li, s.v.dinv + rank * 2048, blockDim.x);
+    else cp_commit();
+    ring_start<VEC, false>(ring, W, r, 0, n, blk > 0 && blk < nb);
+    for (int K = 0; K < nb; ++K) {
+      double* Ut = K & 1 ? U1 : U0;
+      solve_block(K, Ut, std::false_type{});
+      if (blk > K && blk < nb) {
+        update<NI, VEC, false>(acc, ring, W, r, smem(Ut + g * US + 2 * t), K, K + 1, blk > K + 1, n);
+      } else {
+        if (K % CS == rank && blk <= K) {
+          // the next L_KK^-1; after the CTA's last one its first U_KK^-1 (same block)
+          const int free = K / CS + 1;
+          fetch_inverse(Li, s.v.dinv + (K + CS < nb ? (K + CS) * 2048 : K * 2048 + 1024), 32 * free);
+        }
+        if (blk == K) {  // Y_K back into its owner's registers for the way up
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int ni = 0; ni < NI; ++ni)
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                acc.v[m][ni][e] = -Ut[(8 * ni + 2 * t + (e & 1)) * US + 16 * m + g + 8 * (e >> 1)];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cp_commit();  // the waits count groups
+      }
+    }
+  } else {
+    // the CTA's last block
+    const int last = rank < nb ? (nb - 1 - rank) / CS * CS + rank : -1;
+    if (last >= 0) fetch_inverse(Li, s.v.dinv + last * 2048 + 1024, blockDim.x);
+    else cp_commit();
   }
-  ring_start<VEC, true>(ring, W, r, nb - 1, n, warp < nb - 1);
+  ring_start<VEC, true>(ring, W, r, nb - 1, n, blk < nb - 1);
   for (int K = nb - 1; K >= 0; --K) {
-    if (warp == K) store_tile<NI>(Tb, acc);
-    cp_wait<2>();
-    __syncthreads();
-    tile_product<NI, true>(Li, Tb, Ut);
-    __syncthreads();
-    if (warp < K) {
-      update<NI, VEC, true>(acc, ring, W, r, ulane, K, K - 1, warp < K - 1, n);
+    // the tiles go on alternating: the last block of the way down used tile (nb - 1) & 1
+    double* Ut = (nb - 1 - K) & 1 ? (nb & 1 ? U0 : U1) : (nb & 1 ? U1 : U0);
+    solve_block(K, Ut, std::true_type{});
+    if (blk < K) {
+      update<NI, VEC, true>(acc, ring, W, r, smem(Ut + g * US + 2 * t), K, K - 1, blk < K - 1, n);
     } else {
-      const int free = (int)(blockDim.x >> 5) - K;
-      if (K > 0) fetch_inverse(Li, s.v.dinv + (K - 1) * 2048 + 1024, 32 * free, 32 * K);
-      product_out<NI, false>(Ut, s.width, K, free, [&](int row) {
-        return 32 * K + row < n ? s.X + (int64_t)(32 * K + row) * s.ldx : nullptr;
-      });
+      if (K % CS == rank) {
+        const int first = K / CS, free = nw - first;
+        if (K >= CS) fetch_inverse(Li, s.v.dinv + (K - CS) * 2048 + 1024, 32 * free, 32 * first);
+        product_out<NI, false>(Ut, s.width, first, free, [&](int row) {
+          return 32 * K + row < n ? s.X + (int64_t)(32 * K + row) * s.ldx : nullptr;
+        });
+      }
 #pragma unroll
       for (int q = 0; q < 4; ++q) cp_commit();
     }
   }
+  if constexpr (CS > 1) cg::this_cluster().sync();  // no CTA leaves while another may still write to it
 }
 
 // A kernel per strip width: narrow strips need fewer registers, so more of their
 // CTAs share an SM. items == nullptr: strips `first` .. `first` + `per` - 1 of the
 // right-hand sides (inverse: of the inverse) of every system of a uniform batch.
-template <int NI, bool VEC>
+template <int NI, bool VEC, int CS>
 __global__ void __launch_bounds__(kSysMaxN, 1)
 k_sys_solve(SysArgs sa, const SysItem* __restrict__ items, int inverse, int first, int per) {
   extern __shared__ __align__(16) double sm[];
   __shared__ Strip s_s;
   __shared__ int s_skip;
   if (threadIdx.x == 0) {
+    const int b = (int)blockIdx.x / CS;
     SysItem it;
     if (items) {
-      it = items[blockIdx.x];
+      it = items[b];
     } else {
-      it.sys = blockIdx.x / per;
+      it.sys = b / per;
       it.inverse = (int16_t)inverse;
-      it.c0 = 32 * (first + (int)blockIdx.x - it.sys * per);
+      it.c0 = 32 * (first + b - it.sys * per);
       it.width = (int16_t)min(32, (inverse ? sa.un : sa.unrhs) - it.c0);
     }
     const View v = view(sa, it.sys);
@@ -843,10 +894,10 @@ k_sys_solve(SysArgs sa, const SysItem* __restrict__ items, int inverse, int firs
     s_s.ldx = it.inverse ? v.n : v.nrhs;
     s_s.B = sa.B + v.b_off + it.c0;
     s_s.X = (it.inverse ? sa.inv + v.inv_off : sa.X + v.b_off) + it.c0;
-    s_skip = sa.state && sa.state[v.slot];  // singular: nothing to solve with
+    s_skip = sa.state && *state_of(sa, v.slot);  // singular: nothing to solve with
   }
   __syncthreads();
-  if (!s_skip) solve_strip<NI, VEC>(sa, s_s, sm);
+  if (!s_skip) solve_strip<NI, VEC, CS>(sa, s_s, sm);  // the same for every CTA of a cluster
 }
 
 // ---------------------------------------------------------------------------
@@ -862,6 +913,7 @@ k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __res
   const int n = v.n, b = (int)blockIdx.y - 1;
   if (b >= sys_blocks(n)) return;
   if (b < 0) {
+    if (!ipiv) return;  // upper factors only
     extern __shared__ int piv[];
     const int32_t* src = ipiv + (sa.desc ? sa.desc[s].piv_off : (int64_t)s * n);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -892,8 +944,8 @@ k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __res
   }
   __syncthreads();
   double* di = v.dinv + (int64_t)b * 2048;
-  if (threadIdx.x < 32) tri_inverse<false>(D, X, di, kb);
-  else tri_inverse<true>(D, X, di + 1024, kb);
+  if (threadIdx.x >= 32) tri_inverse<true>(D, X, di + 1024, kb);
+  else if (ipiv) tri_inverse<false>(D, X, di, kb);
 }
 
 }  // namespace
@@ -908,17 +960,59 @@ cudaError_t launch_sys_lu(const SysArgs& sa, const int32_t* list, int nsys, int 
 
 namespace {
 
+template <int NI, bool VEC, int CS>
+cudaError_t launch_strips3(const SysArgs& sa, const SysItem* items, int64_t nitems, int nmax, int inverse, int first,
+                           int per, cudaStream_t st) {
+  const int nw = (sys_blocks(nmax) + CS - 1) / CS;
+  if constexpr (CS == 1) {
+    k_sys_solve<NI, VEC, 1><<<(unsigned)nitems, 32 * nw, sys_smem(nw), st>>>(sa, items, inverse, first, per);
+    return cudaGetLastError();
+  } else {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)nitems * CS);
+    cfg.blockDim = dim3(32 * nw);
+    cfg.dynamicSmemBytes = sys_cluster_smem(nw);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CS;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_sys_solve<NI, VEC, CS>, sa, items, inverse, first, per);
+  }
+}
+
+// CTAs per strip: what the order needs (16 blocks of 32 rows each), more while
+// the strips leave SMs idle and a CTA keeps at least four blocks (a warp for each
+// scheduler).
+int strip_cluster(int nmax, int64_t nitems) {
+  const int nb = sys_blocks(nmax);
+  int cs = 1;
+  while (nb > kMaxWarps * cs) cs *= 2;
+  while (cs < 8 && nitems * cs * 2 <= 148 && nb >= 8 * cs) cs *= 2;
+  return cs;
+}
+
 template <int NI>
 cudaError_t launch_strips(const SysArgs& sa, const SysItem* items, int64_t nitems, int nmax, int inverse, int first,
                           int per, cudaStream_t st) {
   if (nitems <= 0) return cudaSuccess;
-  if (nmax > kSysMaxN || nitems > INT_MAX) return cudaErrorInvalidValue;
-  const int nw = sys_blocks(nmax);
+  const int cs = strip_cluster(nmax, nitems);
+  if (cs > 8 || nitems * cs > INT_MAX) return cudaErrorInvalidValue;
   // 16-byte operand loads: workspaces always, kept factors (uniform batches) of even order
   const bool vec = !sa.w_by_position || (sa.un % 2 == 0 && (reinterpret_cast<uintptr_t>(sa.W) & 15) == 0);
-  if (vec) k_sys_solve<NI, true><<<(unsigned)nitems, 32 * nw, sys_smem(nw), st>>>(sa, items, inverse, first, per);
-  else k_sys_solve<NI, false><<<(unsigned)nitems, 32 * nw, sys_smem(nw), st>>>(sa, items, inverse, first, per);
-  return cudaGetLastError();
+#define NPPB_STRIPS(CS)                                                                              \
+  return vec ? launch_strips3<NI, true, CS>(sa, items, nitems, nmax, inverse, first, per, st)        \
+             : launch_strips3<NI, false, CS>(sa, items, nitems, nmax, inverse, first, per, st)
+  switch (cs) {
+    case 1: NPPB_STRIPS(1);
+    case 2: NPPB_STRIPS(2);
+    case 4: NPPB_STRIPS(4);
+    default: NPPB_STRIPS(8);
+  }
+#undef NPPB_STRIPS
 }
 
 cudaError_t launch_strips(const SysArgs& sa, const SysItem* items, int64_t nitems, int nmax, int width, int inverse,
@@ -930,12 +1024,21 @@ cudaError_t launch_strips(const SysArgs& sa, const SysItem* items, int64_t nitem
   }
 }
 
+template <int NI, int CS>
+cudaError_t prepare_strips1() {
+  const int smem = CS == 1 ? sys_smem(kMaxWarps) : sys_cluster_smem(kMaxWarps);
+  cudaError_t e = cudaFuncSetAttribute(k_sys_solve<NI, true, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_sys_solve<NI, false, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  return e;
+}
+
 template <int NI>
 cudaError_t prepare_strips() {
-  cudaError_t e = cudaFuncSetAttribute(k_sys_solve<NI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       sys_smem(kMaxWarps));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_sys_solve<NI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sys_smem(kMaxWarps));
+  cudaError_t e = prepare_strips1<NI, 1>();
+  if (e == cudaSuccess) e = prepare_strips1<NI, 2>();
+  if (e == cudaSuccess) e = prepare_strips1<NI, 4>();
+  if (e == cudaSuccess) e = prepare_strips1<NI, 8>();
   return e;
 }
 

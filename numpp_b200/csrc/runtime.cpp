@@ -174,7 +174,7 @@ Lookahead* lookahead_for_device() {
 // order: its out-of-place update reads the panel's row-move lists, which the
 // next panel overwrites.
 template <class T>
-cudaError_t run_step_blocked(const StepArgsT<T>& sa0, int count, cudaStream_t st);
+cudaError_t run_step_blocked(const StepArgsT<T>& sa0, int count, cudaStream_t st, bool substitute);
 
 int blocked_min_n() {
   static const int v = [] {
@@ -185,10 +185,10 @@ int blocked_min_n() {
 }
 
 template <class T>
-cudaError_t run_step_uniform(const StepArgsT<T>& sa, int count, cudaStream_t st) {
+cudaError_t run_step_uniform(const StepArgsT<T>& sa, int count, cudaStream_t st, bool substitute) {
   const int n = sa.un;
   if (n <= 32 || n > kStepMaxN || count <= 0) return cudaErrorInvalidValue;
-  if (sa.hist) return run_step_blocked(sa, count, st);
+  if (sa.hist) return run_step_blocked(sa, count, st, substitute);
   Lookahead* la = lookahead_for_device();
   cudaError_t e = launch_panel(sa, nullptr, count, n, 0, st);
   for (int k0 = 0; k0 < n && e == cudaSuccess; k0 += kStepNB) {
@@ -214,7 +214,7 @@ cudaError_t run_step_uniform(const StepArgsT<T>& sa, int count, cudaStream_t st)
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, la->next, 0);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, la->rest, 0);
   }
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || !substitute) return e;
   const int64_t back = (int64_t)count * uniform_back_strips(n, sa.unrhs, sa.uinv);
   if (back > INT32_MAX) return cudaErrorInvalidValue;
   return launch_back(sa, nullptr, (int)back, sa.un, sa.uinv ? 64 : std::min(64, sa.unrhs), st);
@@ -234,7 +234,7 @@ cudaError_t run_step_uniform(const StepArgsT<T>& sa, int count, cudaStream_t st)
 // trailing pass waits for it. Every element sees the same operations in the
 // same order either way.
 template <class T>
-cudaError_t run_step_blocked(const StepArgsT<T>& sa0, int count, cudaStream_t st) {
+cudaError_t run_step_blocked(const StepArgsT<T>& sa0, int count, cudaStream_t st, bool substitute) {
   StepArgsT<T> sa = sa0;
   const int n = sa.un;
   cudaError_t e = cudaSuccess;
@@ -296,7 +296,7 @@ cudaError_t run_step_blocked(const StepArgsT<T>& sa0, int count, cudaStream_t st
   sa.ubbeg = sa.ubend = 0;
   const int64_t back = (int64_t)count * uniform_back_strips(n, sa.unrhs, sa.uinv);
   if (back > INT32_MAX) return cudaErrorInvalidValue;
-  e = launch_back(sa, nullptr, (int)back, sa.un, sa.uinv ? 64 : std::min(64, sa.unrhs), cs);
+  if (substitute) e = launch_back(sa, nullptr, (int)back, sa.un, sa.uinv ? 64 : std::min(64, sa.unrhs), cs);
   if (e == cudaSuccess && cs != st) {
     e = cudaEventRecord(la->first, cs);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, la->first, 0);
@@ -304,8 +304,8 @@ cudaError_t run_step_blocked(const StepArgsT<T>& sa0, int count, cudaStream_t st
   return e;
 }
 
-template cudaError_t run_step_uniform<double>(const StepArgsT<double>&, int, cudaStream_t);
-template cudaError_t run_step_uniform<float>(const StepArgsT<float>&, int, cudaStream_t);
+template cudaError_t run_step_uniform<double>(const StepArgsT<double>&, int, cudaStream_t, bool);
+template cudaError_t run_step_uniform<float>(const StepArgsT<float>&, int, cudaStream_t, bool);
 
 template <class T>
 cudaError_t run_step_solve_uniform(const StepArgsT<T>& sa, int count, cudaStream_t st, bool prepermuted) {

@@ -41,9 +41,11 @@ struct SysArgs {
   double* sign;
   double* logabs;
   int32_t* info;        // per-system output (may be null)
-  int32_t* state;       // first zero pivot + 1 or 0, by slot (null: every system is solved)
+  int32_t* state;       // first zero pivot + 1 or 0, by slot (null: every system is solved),
+  int state_stride;     //   so many bytes apart
   int un, unrhs, uinv;  // uniform batch
   int w_by_position;    // W holds rows in pivoted order with leading dimension n (kept factors)
+  int upper_only;       // X and the inverse hold L^-1 P B already: back substitution in place
 };
 
 // LU with partial pivoting of `nsys` systems with (maximum order) nmax <= 512,
@@ -56,7 +58,7 @@ cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t ni
                              cudaStream_t st);
 cudaError_t launch_sys_solve_uniform(const SysArgs& sa, int nsys, cudaStream_t st);
 // Permutations and diagonal inverses of kept factors (swap lists ipiv at
-// piv_off): fills sa.perm and sa.dinv.
+// piv_off): fills sa.perm and sa.dinv. Null ipiv: the upper factors' inverses only.
 cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int32_t* list, int nsys, int nmax,
                                cudaStream_t st);
 cudaError_t sys_prepare_kernels();

@@ -1,0 +1,403 @@
+// Batched Cholesky factor of (count, n, n) FP64 stacks. C++20.
+//
+// The reference factors one matrix at a time, column by column, reading only
+// the lower triangle and stopping with "Matrix is not positive definite" at a
+// diagonal <= 0 (src/linalg/linalg.cpp:117-136; stacks batched.cpp:77). Here one
+// CTA, or a cluster of up to eight, keeps one matrix for the whole factorisation,
+// left-looking by 32-column blocks like the LU of k_sys.cu: block b of 32 rows
+// belongs to warp b / CS of CTA b % CS. For block column J
+//  1. the warps at or below it read their rows of A, negated, into the FP64
+//     tensor core's accumulators (the lower triangle once),
+//  2. add L_wK L_JK^T for every earlier block K: their own rows of L_wK through
+//     their operand rings, L_JK shared through two alternating tiles,
+//  3. the owner of block J factors its 32 x 32 block (a lane per row, groups of
+//     eight columns, the rest of the block by the tensor core) and inverts it,
+//  4. the warps below multiply by that inverse and write their rows of L.
+// L serves as the working storage: no workspace, and A is read before the same
+// columns of L are written, so L may be A.
+//
+// Half the operations of an LU and none of its pivot searches; the diagonal
+// blocks, 32 dependent reciprocal square roots each, bound it while few systems
+// share an SM. 512 x 256, one B200: CHOL_TIMES.
+#include <algorithm>
+#include <cmath>
+#include <new>
+
+#include "../../include/numpp_b200.h"
+#include "runtime.hpp"
+#include "sys_device.cuh"
+
+namespace nppb {
+namespace {
+
+#define NPPB_CUDA(call, what)                            \
+  do {                                                   \
+    cudaError_t e_ = (call);                             \
+    if (e_ != cudaSuccess) return cuda_status(e_, what); \
+  } while (0)
+
+template <class F>
+int guarded(F&& f) {
+  try {
+    clear_error();
+    return f();
+  } catch (const std::bad_alloc&) {
+    set_error("host allocation failed");
+    return NPPB_E_NOMEM;
+  }
+}
+
+// Shared memory, in doubles: the inversion's scratch tile, a region per warp
+// (ring / staging tile), and with more than one block the inverse and two tiles
+// of L_JK.
+constexpr int kScratch = 32 * TS;
+constexpr int chol_smem(int warps, int blocks) {
+  return 8 * (kScratch + warps * kPerWarp + (blocks > 1 ? 3 * 32 * US : 0));
+}
+
+// The 32 x 32 diagonal block by one warp: acc holds minus the block, tile (stride
+// PS) ends with its factor, zeros above the diagonal. Returns 0 or the first
+// column whose diagonal is not positive, + 1.
+__device__ __forceinline__ int factor_block(Acc<4>& acc, double* tile, int kb) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll 1
+  for (int j0 = 0; j0 < kb; j0 += 8) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      double* o = tile + (16 * m + g) * PS + j0 + 2 * t;
+      *reinterpret_cast<double2*>(o) = make_double2(-acc.v[m][0][0], -acc.v[m][0][1]);
+      *reinterpret_cast<double2*>(o + 8 * PS) = make_double2(-acc.v[m][0][2], -acc.v[m][0][3]);
+    }
+    __syncwarp();
+    double a[8];
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double2 x = *reinterpret_cast<const double2*>(tile + lane * PS + j0 + c);
+      a[c] = x.x;
+      a[c + 1] = x.y;
+    }
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const int j = j0 + s;
+      if (j < kb) {
+        const double d = __shfl_sync(kAll, a[s], j);
+        if (!(d > 0.0)) return j + 1;  // a NaN included; the same in every lane
+        const double r = rsqrt(d);
+        const double l = lane > j ? a[s] * r : lane == j ? d * r : 0.0;
+        a[s] = l;
+#pragma unroll
+        for (int c = s + 1; c < 8; ++c) {
+          const double lc = __shfl_sync(kAll, l, j0 + c);
+          a[c] = fma(-l, lc, a[c]);
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c += 2)
+      *reinterpret_cast<double2*>(tile + lane * PS + j0 + c) =
+          make_double2(j0 + c <= lane ? a[c] : 0.0, j0 + c + 1 <= lane ? a[c + 1] : 0.0);
+    __syncwarp();
+    double2 l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) l[i] = *reinterpret_cast<const double2*>(tile + (8 * i + g) * PS + j0 + 2 * t);
+#pragma unroll
+    for (int ni = 1; ni < 4; ++ni) {
+      if (j0 + 8 * ni < 32) {  // column group j0 / 8 + ni of the block: its rows are the operand
+        const double2 b = *reinterpret_cast<const double2*>(tile + (j0 + 8 * ni + g) * PS + j0 + 2 * t);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          dmma1688(acc.v[m][ni], l[2 * m], l[2 * m + 1], b);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc.v[m][ni - 1][e] = acc.v[m][ni][e];
+        }
+      }
+    }
+  }
+  // columns past kb stay what they were written as: the block's padding
+  if (kb < 32) {
+    __syncwarp();
+    for (int c = kb; c < 32; ++c) tile[lane * PS + c] = 0.0;
+  }
+  __syncwarp();
+  return 0;
+}
+
+template <bool VEC, int CS>
+__global__ void __launch_bounds__(kSysMaxN, 1)
+k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int s_fail;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int g = lane >> 2, t = lane & 3, nb = sys_blocks(n);
+  const int rank = CS > 1 ? (int)blockIdx.x % CS : 0;
+  const int64_t z = (int)blockIdx.x / CS;
+  const int blk = warp * CS + rank;
+  double* scratch = sm;
+  double* tile = sm + kScratch + warp * kPerWarp;
+  double* Li = sm + kScratch + nw * kPerWarp;
+  double* Bt = Li + 32 * US;
+  const unsigned ring = smem(tile) + 16 * lane;
+  A += z * n * n;
+  L += z * n * n;
+  const bool avec = n % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+  auto sync = [] {
+    if constexpr (CS > 1) cg::this_cluster().sync();
+    else __syncthreads();
+  };
+  // rows 32J .. 32J + 31 of L, columns of block K, into tile K & 1
+  auto fetch_rows = [&](int J, int K) {
+    double* b = Bt + (K & 1) * 32 * US;
+    for (int i = threadIdx.x; i < 512; i += blockDim.x) {
+      const int r = i >> 4, c = (i & 15) * 2, p = 32 * J + r;
+      const double* src = L + (int64_t)min(p, n - 1) * n + 32 * K + c;
+      const unsigned d = smem(b + r * US + c);
+      if constexpr (VEC) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(p < n ? 16 : 0));
+      } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(p < n ? 8 : 0));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d + 8), "l"(src + 1), "r"(p < n ? 8 : 0));
+      }
+    }
+    cp_commit();
+  };
+  if (threadIdx.x == 0) s_fail = 0;
+  sync();
+
+  Rows r;
+  r.live = n - 32 * blk - g;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int p = 32 * blk + 8 * i + g;
+    r.off[i] = (unsigned)(p < n ? p : 0) * n * 8;
+  }
+  for (int J = 0; J < nb; ++J) {
+    const int kb = min(32, n - 32 * J);
+    const bool active = blk >= J && blk < nb;
+    Acc<4> acc;
+    if (active) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int p = 32 * blk + 8 * i + g;
+        const double* src = A + (int64_t)min(p, n - 1) * n;
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          const int col = 32 * J + 8 * ni + 2 * t;
+          double x = 0.0, y = 0.0;
+          if (p < n && col <= p) {  // the lower triangle
+            if (avec && col < p) {
+              const double2 v = __ldcs(reinterpret_cast<const double2*>(src + col));
+              x = -v.x;
+              y = -v.y;
+            } else {
+              x = -__ldcs(src + col);
+              if (col < p) y = -__ldcs(src + col + 1);
+            }
+          }
+          acc.v[i >> 1][ni][2 * (i & 1)] = x;
+          acc.v[i >> 1][ni][2 * (i & 1) + 1] = y;
+        }
+      }
+    }
+    if (J > 0) {
+      fetch_rows(J, 0);
+      ring_start<VEC, false>(ring, L, r, 0, n, active);
+      for (int K = 0; K < J; ++K) {
+        cp_wait<2>();     // L_JK; at most two operand stages stay in flight
+        __syncthreads();  // and every warp is done with the other tile
+        if (K + 1 < J) fetch_rows(J, K + 1);
+        else cp_commit();
+        if (active) {
+          update<4, VEC, false>(acc, ring, L, r, smem(Bt + (K & 1) * 32 * US + g * US + 2 * t), K, K + 1, K + 1 < J, n);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) cp_commit();  // the waits count groups
+        }
+      }
+      cp_wait<0>();
+      __syncwarp();  // the ring becomes the staging tile
+    }
+    if (blk == J) {
+      const int bad = factor_block(acc, tile, kb);
+      if (bad) {
+        if (lane == 0) {
+          info[z] = 32 * J + bad;
+#pragma unroll
+          for (int c = 0; c < CS; ++c) *(CS > 1 ? cg::this_cluster().map_shared_rank(&s_fail, c) : &s_fail) = 1;
+        }
+      } else if (J + 1 < nb) {
+        tri_inverse<kLower>(tile, scratch, kb, [&](int row, int col, double v) {
+#pragma unroll
+          for (int c = 0; c < CS; ++c)
+            (CS > 1 ? cg::this_cluster().map_shared_rank(Li, c) : Li)[row * US + col] = v;
+        });
+      }
+    } else if (active) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          double* o = tile + (16 * m + g) * PS + 8 * ni + 2 * t;
+          *reinterpret_cast<double2*>(o) = make_double2(-acc.v[m][ni][0], -acc.v[m][ni][1]);
+          *reinterpret_cast<double2*>(o + 8 * PS) = make_double2(-acc.v[m][ni][2], -acc.v[m][ni][3]);
+        }
+      __syncwarp();
+    }
+    sync();  // the inverse is everywhere
+    if (s_fail) return;  // the same in every CTA of the cluster
+    if (active && blk > J) {
+      // rows times the inverse's transpose: L_JJ^-1 [n][k] = 0 for k > n
+      Acc<4> out;
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) out.v[m][ni][e] = 0.0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        double2 a[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const double2*>(tile + (8 * i + g) * PS + 8 * q + 2 * t);
+#pragma unroll
+        for (int ni = q; ni < 4; ++ni) {
+          const double2 b = *reinterpret_cast<const double2*>(Li + (8 * ni + g) * US + 8 * q + 2 * t);
+#pragma unroll
+          for (int m = 0; m < 2; ++m) dmma1688(out.v[m][ni], a[2 * m], a[2 * m + 1], b);
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          double* o = tile + (16 * m + g) * PS + 8 * ni + 2 * t;
+          *reinterpret_cast<double2*>(o) = make_double2(out.v[m][ni][0], out.v[m][ni][1]);
+          *reinterpret_cast<double2*>(o + 8 * PS) = make_double2(out.v[m][ni][2], out.v[m][ni][3]);
+        }
+      __syncwarp();
+    }
+    if (blk < nb) {
+      // the factor's rows, zeros above the diagonal
+      double* o = L + (int64_t)32 * blk * n + 32 * J + lane;
+      const int rows = lane < kb ? min(32, n - 32 * blk) : 0;
+#pragma unroll 8
+      for (int rr = 0; rr < rows; ++rr) o[(int64_t)rr * n] = blk >= J ? tile[rr * PS + lane] : 0.0;
+    }
+    if (J + 1 < nb) sync();  // this column of L before the next one reads it
+  }
+  if (threadIdx.x == 0 && rank == 0) info[z] = 0;
+}
+
+template <bool VEC, int CS>
+cudaError_t chol_prepare1() {
+  return cudaFuncSetAttribute(k_sys_chol<VEC, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              chol_smem(kMaxWarps, 2));
+}
+
+template <bool VEC, int CS>
+cudaError_t launch_chol(const double* A, double* L, int32_t* info, int64_t count, int n, cudaStream_t st) {
+  const int nb = sys_blocks(n), nw = (nb + CS - 1) / CS;
+  cudaError_t e = chol_prepare1<VEC, CS>();
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(count * CS));
+  cfg.blockDim = dim3(32 * nw);
+  cfg.dynamicSmemBytes = chol_smem(nw, nb);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CS;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = CS > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k_sys_chol<VEC, CS>, A, L, info, n);
+}
+
+int cholesky_device(int64_t count, int32_t n, const double* dA, double* dL, int32_t* dinfo, cudaStream_t st) {
+  const int cs = sys_cluster(n, count);
+  if (count * cs > INT32_MAX) {
+    set_error("batch count above 2^31-1");
+    return NPPB_E_RANGE;
+  }
+  const bool vec = n % 2 == 0 && (reinterpret_cast<uintptr_t>(dL) & 15) == 0;
+#define NPPB_CHOL(CS)                                                        \
+  NPPB_CUDA((vec ? launch_chol<true, CS>(dA, dL, dinfo, count, n, st)        \
+                 : launch_chol<false, CS>(dA, dL, dinfo, count, n, st)),     \
+            "factorisation");                                                \
+  return NPPB_OK
+  switch (cs) {
+    case 1: NPPB_CHOL(1);
+    case 2: NPPB_CHOL(2);
+    case 4: NPPB_CHOL(4);
+    default: NPPB_CHOL(8);
+  }
+#undef NPPB_CHOL
+}
+
+int check_args(int64_t count, int32_t n) {
+  if (count < 0 || n < 0) {
+    set_error("negative count or order");
+    return NPPB_E_ARG;
+  }
+  if (count > INT32_MAX) {
+    set_error("batch count above 2^31-1");
+    return NPPB_E_RANGE;
+  }
+  if (n > kStepMaxN) {
+    set_error("order above 4096 is not served by the batched path");
+    return NPPB_E_RANGE;
+  }
+  return NPPB_OK;
+}
+
+}  // namespace
+}  // namespace nppb
+
+using namespace nppb;
+
+extern "C" {
+
+int nppb_d_cholesky_batched(int64_t count, int32_t n, const double* dA, double* dL, int32_t* dinfo,
+                            void* stream) {
+  return guarded([&]() -> int {
+    const int rc = check_args(count, n);
+    if (rc != NPPB_OK) return rc;
+    if (!count || !n) return NPPB_OK;
+    if (!dA || !dL || !dinfo) {
+      set_error("cholesky needs A, L and info");
+      return NPPB_E_ARG;
+    }
+    if (!device()) return NPPB_E_NODEV;
+    return cholesky_device(count, n, dA, dL, dinfo, static_cast<cudaStream_t>(stream));
+  });
+}
+
+int nppb_cholesky_batched(int64_t count, int32_t n, const double* A, double* L, int32_t* info) {
+  return guarded([&]() -> int {
+    const int rc = check_args(count, n);
+    if (rc != NPPB_OK) return rc;
+    if (!count || !n) return NPPB_OK;
+    if (!A || !L || !info) {
+      set_error("cholesky needs A, L and info");
+      return NPPB_E_ARG;
+    }
+    if (!device()) return NPPB_E_NODEV;
+    cudaStream_t st = thread_stream();
+    const size_t nn = (size_t)count * n * n;
+    DevMem dA, dL, dI;
+    NPPB_CUDA(dA.alloc(sizeof(double) * nn, st), "allocation");
+    NPPB_CUDA(dL.alloc(sizeof(double) * nn, st), "allocation");
+    NPPB_CUDA(dI.alloc(sizeof(int32_t) * count, st), "allocation");
+    NPPB_CUDA(cudaMemcpyAsync(dA.as<double>(), A, sizeof(double) * nn, cudaMemcpyHostToDevice, st), "copy");
+    const int r = cholesky_device(count, n, dA.as<double>(), dL.as<double>(), dI.as<int32_t>(), st);
+    if (r != NPPB_OK) return r;
+    NPPB_CUDA(cudaMemcpyAsync(L, dL.as<double>(), sizeof(double) * nn, cudaMemcpyDeviceToHost, st), "copy");
+    NPPB_CUDA(cudaMemcpyAsync(info, dI.as<int32_t>(), sizeof(int32_t) * count, cudaMemcpyDeviceToHost, st), "copy");
+    NPPB_CUDA(cudaStreamSynchronize(st), "synchronize");
+    NPPB_CUDA(cudaGetLastError(), "kernel");
+    return NPPB_OK;
+  });
+}
+
+}  // extern "C"

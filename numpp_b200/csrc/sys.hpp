@@ -17,6 +17,17 @@ __host__ __device__ inline int sys_blocks(int n) { return (n + 31) / 32; }
 // Doubles of the diagonal blocks' inverses: per 32-column block L11^-1, then U11^-1.
 __host__ __device__ inline int64_t sys_dinv(int n) { return (int64_t)sys_blocks(n) * 2048; }
 
+// CTAs per work item (a strip, a Cholesky factor): what the order needs (16 blocks
+// of 32 rows each), more while the items leave SMs idle and every CTA keeps at
+// least four blocks (a warp for each scheduler).
+inline int sys_cluster(int n, int64_t items) {
+  const int nb = sys_blocks(n);
+  int cs = 1;
+  while (nb > 16 * cs) cs *= 2;
+  while (cs < 8 && items * cs * 2 <= 148 && nb >= 8 * cs) cs *= 2;
+  return cs;
+}
+
 // A strip of at most 32 columns of one system's right-hand sides or inverse.
 struct SysItem {
   int32_t sys;

@@ -1,0 +1,203 @@
+// Device pieces of the system-resident kernels (k_sys.cu, k_chol.cu): operand
+// rings, block updates and triangular inverses on the FP64 tensor core.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "dmma.cuh"
+#include "sys.hpp"
+
+namespace nppb {
+namespace {
+
+constexpr int US = 40;   // row stride of the 32 x 32 operand tiles (16-byte reads: banks 4g + t)
+constexpr int BS = 34;   // row stride of the tile read down its columns (banks 4t + g)
+constexpr int TS = 36;   // row stride of the inversions' scratch tile
+constexpr int PS = 34;   // row stride of the panel staging tiles (16-byte reads, one row per thread)
+constexpr int kMaxWarps = kSysMaxN / 32;
+namespace cg = cooperative_groups;
+constexpr unsigned kAll = 0xffffffffu;
+
+// D(16x8) += A(16x8) B(8x8), FP64, one warp. Lane 4g + t holds A[g][t],
+// A[g+8][t], A[g][t+4], A[g+8][t+4]; B[t][g], B[t+4][g]; D[g][2t], D[g][2t+1],
+// D[g+8][2t], D[g+8][2t+1]. The k index may be permuted alike on both sides:
+// the callers take k = 2t for slot t and 2t + 1 for slot t + 4, so that a lane's
+// two values lie side by side.
+__device__ __forceinline__ void dmma1688(double (&d)[4], double2 lo, double2 hi, double2 b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(lo.x), "d"(hi.x), "d"(lo.y), "d"(hi.y), "d"(b.x), "d"(b.y));
+}
+
+__device__ __forceinline__ void cp16(void* smem, const void* gmem) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// The rows of a warp's operand tile: lane 4g + t serves rows g, g+8, g+16, g+24.
+struct Rows {
+  unsigned off[4];  // byte offset of the row in W
+  int live;         // rows from row g of the tile on: row group i exists when 8i < live
+};
+
+// A warp's operand ring: stages of eight columns of its 32 rows, 2 KB each. A
+// lane fetches exactly what it will feed to the tensor core itself (columns
+// 2t, 2t+1 of rows 8i + g), so the ring is a lane-private prefetch buffer
+// (conflict-free, no barrier) that costs no registers. Three stages are in
+// flight: 24 tensor instructions, 1500 cycles, cover the latency of L2.
+constexpr int kRing = 4;
+constexpr int kRingDoubles = kRing * 256;  // of one warp
+
+// One row group of a stage: columns col, col + 1 of row 8i + g. EDGE: the columns
+// may end inside the block (zeros past them).
+template <bool VEC, bool EDGE>
+__device__ __forceinline__ void ring_load1(unsigned ring, int stage, int i, const double* W, const Rows& r, int col,
+                                           int n) {
+  const unsigned d = ring + (stage * 4 + i) * 512;
+  int size = 8 * i < r.live ? 16 : 0;
+  if (EDGE) {
+    size = min(size, 8 * max(0, n - col));
+    col = min(col, (n - 1) & ~1);  // the address stays inside the row
+  }
+  const char* p = reinterpret_cast<const char*>(W + col) + r.off[i];
+  if constexpr (VEC) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(p), "r"(size));
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(p), "r"(min(size, 8)));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d + 8), "l"(size > 8 ? p + 8 : p),
+                 "r"(max(size - 8, 0)));
+  }
+}
+
+// The first three stages of block K.
+template <bool VEC, bool EDGE>
+__device__ __forceinline__ void ring_start(unsigned ring, const double* W, const Rows& r, int K, int n, bool live) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (live) ring_load1<VEC, EDGE>(ring, q, i, W, r, 32 * K + 8 * q + 2 * (threadIdx.x & 3), n);
+    cp_commit();
+  }
+}
+
+// Everything a block step shares. NI: 8-column groups of the strip.
+template <int NI>
+struct Acc {
+  double v[2][NI][4];  // rows 16m + g, 16m + g + 8; columns 8i + 2t, + 1
+};
+
+__device__ __forceinline__ unsigned smem(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ double2 lds2(unsigned p) {  // stays where it is written
+  double2 v;
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "r"(p));
+  return v;
+}
+
+// acc -= (warp's rows of W, columns 32K..32K+31) * U, with u the lane's place in
+// -U^T (column c of U at c * US; the lane reads column g + 8i, rows 2t, 2t + 1).
+// The ring holds the first three stages; those of block Knext follow when `more`. A tensor instruction holds the pipe for 64 cycles, so every
+// register is reloaded for the next stage right behind its last use and the
+// prefetches are spread between the instructions.
+template <int NI, bool VEC, bool EDGE>
+__device__ __forceinline__ void update(Acc<NI>& acc, unsigned ring, const double* W, const Rows& r,
+                                       unsigned u, int K, int Knext, bool more, int n) {
+  const int t2 = 2 * (threadIdx.x & 3);
+  double2 a[4], b[NI];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) a[i] = lds2(ring + i * 512);
+#pragma unroll
+  for (int i = 0; i < NI; ++i) b[i] = lds2(u + i * (8 * US * 8));
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int stage = (q + 3) % 4, col = q == 0 ? 32 * K + 24 + t2 : 32 * Knext + 8 * (q - 1) + t2;
+    const bool live = q == 0 || more;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i < NI) dmma1688(acc.v[0][i], a[0], a[1], b[i]);
+      if (live) ring_load1<VEC, EDGE>(ring, stage, i, W, r, col, n);
+    }
+    cp_commit();
+    cp_wait<2>();  // the next stage has landed
+    const unsigned next = ring + (q + 1) * 2048;
+    if (q < 3) {
+      a[0] = lds2(next);
+      a[1] = lds2(next + 512);
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      dmma1688(acc.v[1][i], a[2], a[3], b[i]);
+      if (q < 3) b[i] = lds2(u + i * (8 * US * 8) + 64 * (q + 1));
+    }
+    if (q < 3) {
+      a[2] = lds2(next + 1024);
+      a[3] = lds2(next + 1536);
+    }
+  }
+}
+
+// Inverse of a 32 x 32 triangle by one warp; put(row, column, value) gets all of
+// it, zeros included, lane = column. D (stride PS, shared) holds kb live rows and
+// columns (identity past them): kUnitLower takes what lies below its diagonal,
+// kUpper and kLower that half with the diagonal. The upper triangle is inverted
+// as the lower triangle U^T. First the four 8 x 8 diagonal
+// blocks, a lane per column, then the blocks below them:
+// X_ij = -X_ii (T_ij X_jj + ... + T_i,i-1 X_i-1,j). X is a scratch tile of
+// stride TS; kUnitLower and kUpper may share it: one lives below its diagonal, the
+// other (transposed back) on and above it.
+enum TriKind { kUnitLower, kUpper, kLower };
+template <TriKind KIND, class Put>
+__device__ __forceinline__ void tri_inverse(const double* D, double* X, int kb, Put put) {
+  constexpr bool UPPER = KIND == kUpper, DIAG = KIND != kUnitLower;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  auto T = [&](int i, int k) {
+    const bool in = i < kb && k < kb;
+    return in ? (UPPER ? D[k * PS + i] : D[i * PS + k]) : (i == k ? 1.0 : 0.0);
+  };
+  auto at = [&](int i, int j) -> double& { return UPPER ? X[j * TS + i] : X[i * TS + j]; };
+  auto get = [&](int i, int j) { return i > j || (DIAG && i == j) ? at(i, j) : (i == j ? 1.0 : 0.0); };
+  {
+    const int b = lane & ~7, c = lane & 7;
+    const double rd = DIAG ? 1.0 / T(b + c, b + c) : 1.0;
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      double s = i == c ? 1.0 : 0.0;
+#pragma unroll
+      for (int q = 0; q < i; ++q) s = fma(-T(b + i, b + q), x[q], s);
+      if constexpr (DIAG) s *= __shfl_sync(kAll, rd, b + i);
+      x[i] = i >= c ? s : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (i > c || (DIAG && i == c)) at(b + i, b + c) = x[i];
+  }
+  __syncwarp();
+  for (int i = 1; i < 4; ++i)
+    for (int j = 0; j < i; ++j) {
+      double s[2] = {0.0, 0.0}, x[2] = {0.0, 0.0};
+      for (int k = 8 * j; k < 8 * i; k += 4) dmma884(s, T(8 * i + g, k + t), get(k + t, 8 * j + g));
+      // the sum's place is X_ij's until the product with X_ii replaces it
+      at(8 * i + g, 8 * j + 2 * t) = s[0];
+      at(8 * i + g, 8 * j + 2 * t + 1) = s[1];
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 8; k += 4) dmma884(x, get(8 * i + g, 8 * i + k + t), at(8 * i + k + t, 8 * j + g));
+      __syncwarp();
+      at(8 * i + g, 8 * j + 2 * t) = -x[0];
+      at(8 * i + g, 8 * j + 2 * t + 1) = -x[1];
+      __syncwarp();
+    }
+#pragma unroll 8
+  for (int r = 0; r < 32; ++r) put(r, lane, UPPER ? (lane >= r ? X[r * TS + lane] : 0.0) : get(r, lane));
+}
+
+constexpr int kPerWarp = 32 * PS;  // doubles of a warp's region: its ring, or its staging tile
+static_assert(kPerWarp >= kRingDoubles);
+
+}  // namespace
+}  // namespace nppb

@@ -47,6 +47,42 @@ int guarded(F&& f) {
   }
 }
 
+// Minus the warp's rows of a 32-column block, columns up to the diagonal, into
+// accumulators: two columns per load, all loads in flight at once (addresses are
+// clamped into the matrix, values past the triangle become zero).
+__device__ __forceinline__ void load_block(Acc<4>& acc, const double* A, bool vec, int blk, int col0, int n) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const double* src[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) src[i] = A + (int64_t)min(32 * blk + 8 * i + g, n - 1) * n;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) {
+      const int col = col0 + 8 * ni + 2 * t;
+      double2 x;
+      if (vec) {  // uniform; n is even
+        x = __ldcs(reinterpret_cast<const double2*>(src[i] + min(col, n - 2)));
+      } else {
+        x.x = __ldcs(src[i] + min(col, n - 1));
+        x.y = __ldcs(src[i] + min(col + 1, n - 1));
+      }
+      acc.v[i >> 1][ni][2 * (i & 1)] = x.x;
+      acc.v[i >> 1][ni][2 * (i & 1) + 1] = x.y;
+    }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int p = 32 * blk + 8 * i + g, end = p >= n ? 0 : p + 1;
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        double& v = acc.v[i >> 1][ni][2 * (i & 1) + e];
+        v = col0 + 8 * ni + 2 * t + e < end ? -v : 0.0;
+      }
+  }
+}
+
 // Shared memory, in doubles: the inversion's scratch tile, a region per warp
 // (ring / staging tile), and with more than one block the inverse and two tiles
 // of L_JK.
@@ -55,43 +91,47 @@ constexpr int chol_smem(int warps, int blocks) {
   return 8 * (kScratch + warps * kPerWarp + (blocks > 1 ? 3 * 32 * US : 0));
 }
 
-// The 32 x 32 diagonal block by one warp: acc holds minus the block, tile (stride
-// PS) ends with its factor, zeros above the diagonal. Returns 0 or the first
-// column whose diagonal is not positive, + 1.
-__device__ __forceinline__ int factor_block(Acc<4>& acc, double* tile, int kb) {
+// The 32 x 32 diagonal block by one warp, in its tile (stride PS), zeros above the
+// diagonal. Eight columns at a time: every lane factors the 8 x 8 block on the
+// diagonal for itself (no exchange between the dependent steps), solves its own
+// row with it, and the tensor core updates the columns right of the group.
+// Returns 0 or the first column whose diagonal is not positive, + 1.
+__device__ __forceinline__ int factor_block(double* tile, int kb) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll 1
   for (int j0 = 0; j0 < kb; j0 += 8) {
+    double a[8], d[8][8], r[8];
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      double* o = tile + (16 * m + g) * PS + j0 + 2 * t;
-      *reinterpret_cast<double2*>(o) = make_double2(-acc.v[m][0][0], -acc.v[m][0][1]);
-      *reinterpret_cast<double2*>(o + 8 * PS) = make_double2(-acc.v[m][0][2], -acc.v[m][0][3]);
-    }
-    __syncwarp();
-    double a[8];
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int c = 0; c <= i; c += 2) {
+        const double2 x = *reinterpret_cast<const double2*>(tile + (j0 + i) * PS + j0 + c);
+        d[i][c] = x.x;
+        if (c < i) d[i][c + 1] = x.y;
+      }
 #pragma unroll
     for (int c = 0; c < 8; c += 2) {
       const double2 x = *reinterpret_cast<const double2*>(tile + lane * PS + j0 + c);
       a[c] = x.x;
       a[c + 1] = x.y;
     }
+    int bad = 0;
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
-      const int j = j0 + s;
-      if (j < kb) {
-        const double d = __shfl_sync(kAll, a[s], j);
-        if (!(d > 0.0)) return j + 1;  // a NaN included; the same in every lane
-        const double r = rsqrt(d);
-        const double l = lane > j ? a[s] * r : lane == j ? d * r : 0.0;
-        a[s] = l;
+      if (j0 + s < kb && !bad && !(d[s][s] > 0.0)) bad = j0 + s + 1;  // a NaN included
+      r[s] = j0 + s < kb ? rsqrt(d[s][s]) : 1.0;
+      a[s] *= r[s];
 #pragma unroll
-        for (int c = s + 1; c < 8; ++c) {
-          const double lc = __shfl_sync(kAll, l, j0 + c);
-          a[c] = fma(-l, lc, a[c]);
-        }
+      for (int i = s + 1; i < 8; ++i) d[i][s] *= r[s];
+#pragma unroll
+      for (int k = s + 1; k < 8; ++k) {
+        a[k] = fma(-a[s], d[k][s], a[k]);
+#pragma unroll
+        for (int i = k; i < 8; ++i) d[i][k] = fma(-d[i][s], d[k][s], d[i][k]);
       }
     }
+    if (bad) return bad;  // the same in every lane
+    __syncwarp();
 #pragma unroll
     for (int c = 0; c < 8; c += 2)
       *reinterpret_cast<double2*>(tile + lane * PS + j0 + c) =
@@ -99,25 +139,26 @@ __device__ __forceinline__ int factor_block(Acc<4>& acc, double* tile, int kb) {
     __syncwarp();
     double2 l[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) l[i] = *reinterpret_cast<const double2*>(tile + (8 * i + g) * PS + j0 + 2 * t);
+    for (int i = 0; i < 4; ++i) {
+      l[i] = *reinterpret_cast<const double2*>(tile + (8 * i + g) * PS + j0 + 2 * t);
+      l[i].x = -l[i].x;
+      l[i].y = -l[i].y;
+    }
+    for (int c0 = j0 + 8; c0 < 32; c0 += 8) {  // columns c0 .. c0 + 7: their rows are the operand
+      const double2 b = *reinterpret_cast<const double2*>(tile + (c0 + g) * PS + j0 + 2 * t);
 #pragma unroll
-    for (int ni = 1; ni < 4; ++ni) {
-      if (j0 + 8 * ni < 32) {  // column group j0 / 8 + ni of the block: its rows are the operand
-        const double2 b = *reinterpret_cast<const double2*>(tile + (j0 + 8 * ni + g) * PS + j0 + 2 * t);
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-          dmma1688(acc.v[m][ni], l[2 * m], l[2 * m + 1], b);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) acc.v[m][ni - 1][e] = acc.v[m][ni][e];
-        }
+      for (int m = 0; m < 2; ++m) {
+        double* o = tile + (16 * m + g) * PS + c0 + 2 * t;
+        const double2 lo = *reinterpret_cast<const double2*>(o), hi = *reinterpret_cast<const double2*>(o + 8 * PS);
+        double v[4] = {lo.x, lo.y, hi.x, hi.y};
+        dmma1688(v, l[2 * m], l[2 * m + 1], b);
+        *reinterpret_cast<double2*>(o) = make_double2(v[0], v[1]);
+        *reinterpret_cast<double2*>(o + 8 * PS) = make_double2(v[2], v[3]);
       }
     }
-  }
-  // columns past kb stay what they were written as: the block's padding
-  if (kb < 32) {
     __syncwarp();
-    for (int c = kb; c < 32; ++c) tile[lane * PS + c] = 0.0;
   }
+  for (int c = (kb + 7) & ~7; c < 32; ++c) tile[lane * PS + c] = 0.0;  // past the last group
   __syncwarp();
   return 0;
 }
@@ -174,29 +215,13 @@ k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
     const int kb = min(32, n - 32 * J);
     const bool active = blk >= J && blk < nb;
     Acc<4> acc;
-    if (active) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int p = 32 * blk + 8 * i + g;
-        const double* src = A + (int64_t)min(p, n - 1) * n;
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-          const int col = 32 * J + 8 * ni + 2 * t;
-          double x = 0.0, y = 0.0;
-          if (p < n && col <= p) {  // the lower triangle
-            if (avec && col < p) {
-              const double2 v = __ldcs(reinterpret_cast<const double2*>(src + col));
-              x = -v.x;
-              y = -v.y;
-            } else {
-              x = -__ldcs(src + col);
-              if (col < p) y = -__ldcs(src + col + 1);
-            }
-          }
-          acc.v[i >> 1][ni][2 * (i & 1)] = x;
-          acc.v[i >> 1][ni][2 * (i & 1) + 1] = y;
-        }
-      }
+    if (active) load_block(acc, A, avec, blk, 32 * J, n);
+    if (blk > J && J + 1 < nb && 32 * blk + lane < n) {  // the next column block on its way into L2
+      const double* nx = A + (int64_t)(32 * blk + lane) * n + 32 * (J + 1);
+      const int left = min(32 * blk + lane, n - 1) - 32 * (J + 1);  // up to the diagonal
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx));
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx + min(16, left)));
+      asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx + min(31, left)));
     }
     if (J > 0) {
       fetch_rows(J, 0);
@@ -216,8 +241,19 @@ k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
       cp_wait<0>();
       __syncwarp();  // the ring becomes the staging tile
     }
+    if (active) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) {
+          double* o = tile + (16 * m + g) * PS + 8 * ni + 2 * t;
+          *reinterpret_cast<double2*>(o) = make_double2(-acc.v[m][ni][0], -acc.v[m][ni][1]);
+          *reinterpret_cast<double2*>(o + 8 * PS) = make_double2(-acc.v[m][ni][2], -acc.v[m][ni][3]);
+        }
+      __syncwarp();
+    }
     if (blk == J) {
-      const int bad = factor_block(acc, tile, kb);
+      const int bad = factor_block(tile, kb);
       if (bad) {
         if (lane == 0) {
           info[z] = 32 * J + bad;
@@ -231,16 +267,6 @@ k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
             (CS > 1 ? cg::this_cluster().map_shared_rank(Li, c) : Li)[row * US + col] = v;
         });
       }
-    } else if (active) {
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
-          double* o = tile + (16 * m + g) * PS + 8 * ni + 2 * t;
-          *reinterpret_cast<double2*>(o) = make_double2(-acc.v[m][ni][0], -acc.v[m][ni][1]);
-          *reinterpret_cast<double2*>(o + 8 * PS) = make_double2(-acc.v[m][ni][2], -acc.v[m][ni][3]);
-        }
-      __syncwarp();
     }
     sync();  // the inverse is everywhere
     if (s_fail) return;  // the same in every CTA of the cluster
@@ -280,8 +306,9 @@ k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
       // the factor's rows, zeros above the diagonal
       double* o = L + (int64_t)32 * blk * n + 32 * J + lane;
       const int rows = lane < kb ? min(32, n - 32 * blk) : 0;
-#pragma unroll 8
-      for (int rr = 0; rr < rows; ++rr) o[(int64_t)rr * n] = blk >= J ? tile[rr * PS + lane] : 0.0;
+#pragma unroll 16
+      for (int rr = 0; rr < 32; ++rr)
+        if (rr < rows) o[(int64_t)rr * n] = blk >= J ? tile[rr * PS + lane] : 0.0;
     }
     if (J + 1 < nb) sync();  // this column of L before the next one reads it
   }

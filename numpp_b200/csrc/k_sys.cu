@@ -391,10 +391,10 @@ __device__ __forceinline__ int panel(PanelShared& sh, Acc<4>& acc, int& pos, boo
 }
 
 // Shared memory, in doubles: the tiles, then a region per warp that is its operand
-// ring and, in the panel, its staging tile. The diagonal block that the
-// inversions read takes U's place, their scratch tile Tb's.
+// ring, in the panel its staging tile and in an inversion its scratch tile. The
+// diagonal block that the inversions read takes U's place.
 constexpr int kTb = 0, kLi = 32 * US, kUt = 64 * US, kWarp = 96 * US;
-static_assert(PS <= US && TS <= US);
+static_assert(PS <= US && 32 * TS <= kPerWarp);
 constexpr int sys_smem(int warps) { return 8 * (kWarp + warps * kPerWarp); }
 // of a cluster's CTA: U twice, behind the per-warp regions
 constexpr int sys_cluster_smem(int warps) { return sys_smem(warps) + 8 * 32 * US; }
@@ -467,7 +467,6 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
       if (J == 1) __syncthreads();  // the first block's inverse has been written
       fetch_inverse(Li, s_v.dinv, blockDim.x);
       ring_start<true, false>(ring, W, r, 0, n, below);
-      if (J > 1) __syncthreads();  // Tb is no longer the inversions' scratch tile
       for (int K = 0; K < J; ++K) {
         if (warp == K) store_tile<4>(Tb, acc);
         cp_wait<2>();  // the inverse; at most two operand stages stay in flight
@@ -535,8 +534,8 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
     // the diagonal block's inverses and the pivots' part of det / slogdet, each by
     // one warp, beside the other warps' loads of the next column block
     double* di = s_v.dinv + (int64_t)J * 2048;
-    if (warp == 0) tri_inverse<kUnitLower>(D11, Tb, kb, into(di));
-    if (warp == 1 % nw) tri_inverse<kUpper>(D11, Tb, kb, into(di + 1024));
+    if (warp == 0) tri_inverse<kUnitLower>(D11, stage, kb, into(di));
+    if (warp == 1 % nw) tri_inverse<kUpper>(D11, stage, kb, into(di + 1024));
     if (warp == 2 % nw && (sa.det || sa.sign || sa.logabs)) {
       // folded in the reference's order (linalg.cpp:400-403, 425-431)
       const double pv = lane < kb ? D11[lane * PS + lane] : 1.0;
@@ -729,7 +728,7 @@ k_sys_solve(SysArgs sa, const SysItem* __restrict__ items, int inverse, int firs
 __global__ void __launch_bounds__(64)
 k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __restrict__ list) {
   __shared__ double D[32 * PS];
-  __shared__ double X[32 * TS];
+  __shared__ double X[2][32 * TS];
   const int s = list ? list[blockIdx.x] : blockIdx.x;
   const View v = view(sa, s);
   const int n = v.n, b = (int)blockIdx.y - 1;
@@ -766,8 +765,8 @@ k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __res
   }
   __syncthreads();
   double* di = v.dinv + (int64_t)b * 2048;
-  if (threadIdx.x >= 32) tri_inverse<kUpper>(D, X, kb, into(di + 1024));
-  else if (ipiv) tri_inverse<kUnitLower>(D, X, kb, into(di));
+  if (threadIdx.x >= 32) tri_inverse<kUpper>(D, X[1], kb, into(di + 1024));
+  else if (ipiv) tri_inverse<kUnitLower>(D, X[0], kb, into(di));
 }
 
 }  // namespace

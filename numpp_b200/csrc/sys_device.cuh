@@ -12,7 +12,7 @@ namespace {
 
 constexpr int US = 40;   // row stride of the 32 x 32 operand tiles (16-byte reads: banks 4g + t)
 constexpr int BS = 34;   // row stride of the tile read down its columns (banks 4t + g)
-constexpr int TS = 36;   // row stride of the inversions' scratch tile
+constexpr int TS = 34;   // row stride of the inversions' scratch tile
 constexpr int PS = 34;   // row stride of the panel staging tiles (16-byte reads, one row per thread)
 constexpr int kMaxWarps = kSysMaxN / 32;
 namespace cg = cooperative_groups;
@@ -141,59 +141,117 @@ __device__ __forceinline__ void update(Acc<NI>& acc, unsigned ring, const double
 }
 
 // Inverse of a 32 x 32 triangle by one warp; put(row, column, value) gets all of
-// it, zeros included, lane = column. D (stride PS, shared) holds kb live rows and
-// columns (identity past them): kUnitLower takes what lies below its diagonal,
-// kUpper and kLower that half with the diagonal. The upper triangle is inverted
-// as the lower triangle U^T. First the four 8 x 8 diagonal
-// blocks, a lane per column, then the blocks below them:
-// X_ij = -X_ii (T_ij X_jj + ... + T_i,i-1 X_i-1,j). X is a scratch tile of
-// stride TS; kUnitLower and kUpper may share it: one lives below its diagonal, the
-// other (transposed back) on and above it.
+// it, zeros included, lane = column. D (stride PS, shared) holds it: kUnitLower
+// takes what lies below the diagonal, kUpper and kLower that half with the
+// diagonal; rows and columns from kb on become the identity's. The upper triangle
+// is inverted as the lower triangle U^T. X is a scratch tile of stride TS.
+//
+// First the four 8 x 8 diagonal blocks, a lane per column; then, twice, the
+// square below two neighbouring triangles T11, T22 of 8 and of 16 rows:
+// X21 = -X22 (T21 X11). One warp alone issues an instruction every four or five
+// cycles, so what counts is how few there are: whole tiles, no element tests.
 enum TriKind { kUnitLower, kUpper, kLower };
 template <TriKind KIND, class Put>
-__device__ __forceinline__ void tri_inverse(const double* D, double* X, int kb, Put put) {
+__device__ __forceinline__ void tri_inverse(double* D, double* X, int kb, Put put) {
   constexpr bool UPPER = KIND == kUpper, DIAG = KIND != kUnitLower;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  auto T = [&](int i, int k) {
-    const bool in = i < kb && k < kb;
-    return in ? (UPPER ? D[k * PS + i] : D[i * PS + k]) : (i == k ? 1.0 : 0.0);
-  };
+  if (kb < 32) {
+    for (int r = 0; r < 32; ++r)
+      if (r >= kb || lane >= kb) D[r * PS + lane] = r == lane ? 1.0 : 0.0;
+    __syncwarp();
+  }
+  // element (i, j) of the lower triangle that is inverted, and of its inverse
+  auto T = [&](int i, int j) { return UPPER ? D[j * PS + i] : D[i * PS + j]; };
   auto at = [&](int i, int j) -> double& { return UPPER ? X[j * TS + i] : X[i * TS + j]; };
-  auto get = [&](int i, int j) { return i > j || (DIAG && i == j) ? at(i, j) : (i == j ? 1.0 : 0.0); };
   {
     const int b = lane & ~7, c = lane & 7;
-    const double rd = DIAG ? 1.0 / T(b + c, b + c) : 1.0;
+    const double rd = DIAG ? 1.0 / D[lane * PS + lane] : 1.0;
     double x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      double s = i == c ? 1.0 : 0.0;
+    for (int i = 0; i < 8; ++i) x[i] = i == c ? 1.0 : 0.0;
 #pragma unroll
-      for (int q = 0; q < i; ++q) s = fma(-T(b + i, b + q), x[q], s);
-      if constexpr (DIAG) s *= __shfl_sync(kAll, rd, b + i);
-      x[i] = i >= c ? s : 0.0;
+    for (int q = 0; q < 8; ++q) {
+      if constexpr (DIAG) x[q] *= __shfl_sync(kAll, rd, b + q);
+#pragma unroll
+      for (int i = q + 1; i < 8; ++i) x[i] = fma(-T(b + i, b + q), x[q], x[i]);
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (i > c || (DIAG && i == c)) at(b + i, b + c) = x[i];
+    for (int i = 0; i < 8; ++i) at(b + i, b + c) = x[i];  // zeros above the diagonal among them
   }
   __syncwarp();
-  for (int i = 1; i < 4; ++i)
-    for (int j = 0; j < i; ++j) {
-      double s[2] = {0.0, 0.0}, x[2] = {0.0, 0.0};
-      for (int k = 8 * j; k < 8 * i; k += 4) dmma884(s, T(8 * i + g, k + t), get(k + t, 8 * j + g));
-      // the sum's place is X_ij's until the product with X_ii replaces it
-      at(8 * i + g, 8 * j + 2 * t) = s[0];
-      at(8 * i + g, 8 * j + 2 * t + 1) = s[1];
-      __syncwarp();
+  {  // the 8 x 8 squares at (8, 0) and (24, 16)
+    double s[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, x[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
-      for (int k = 0; k < 8; k += 4) dmma884(x, get(8 * i + g, 8 * i + k + t), at(8 * i + k + t, 8 * j + g));
-      __syncwarp();
-      at(8 * i + g, 8 * j + 2 * t) = -x[0];
-      at(8 * i + g, 8 * j + 2 * t + 1) = -x[1];
-      __syncwarp();
+    for (int k = 0; k < 8; k += 4)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) dmma884(s[h], T(16 * h + 8 + g, 16 * h + k + t), at(16 * h + k + t, 16 * h + g));
+#pragma unroll
+    for (int h = 0; h < 2; ++h)  // the sum's place is the result's
+#pragma unroll
+      for (int e = 0; e < 2; ++e) at(16 * h + 8 + g, 16 * h + 2 * t + e) = s[h][e];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; k += 4)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        dmma884(x[h], at(16 * h + 8 + g, 16 * h + 8 + k + t), at(16 * h + 8 + k + t, 16 * h + g));
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        at(16 * h + 8 + g, 16 * h + 2 * t + e) = -x[h][e];
+        at(16 * h + g, 16 * h + 8 + 2 * t + e) = 0.0;
+      }
+  }
+  __syncwarp();
+  {  // the 16 x 16 square at (16, 0)
+    double s[2][2][2], x[2][2][2];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int ni = 0; ni < 2; ++ni) s[m][ni][0] = s[m][ni][1] = x[m][ni][0] = x[m][ni][1] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) {
+      const double b[2] = {at(k + t, g), at(k + t, 8 + g)};
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const double a = T(16 + 8 * m + g, k + t);
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) dmma884(s[m][ni], a, b[ni]);
+      }
     }
-#pragma unroll 8
-  for (int r = 0; r < 32; ++r) put(r, lane, UPPER ? (lane >= r ? X[r * TS + lane] : 0.0) : get(r, lane));
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) at(16 + 8 * m + g, 8 * ni + 2 * t + e) = s[m][ni][e];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) {
+      const double b[2] = {at(16 + k + t, g), at(16 + k + t, 8 + g)};
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const double a = at(16 + 8 * m + g, 16 + k + t);
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) dmma884(x[m][ni], a, b[ni]);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) at(16 + 8 * m + g, 8 * ni + 2 * t + e) = -x[m][ni][e];
+  }
+  __syncwarp();
+#pragma unroll 4
+  for (int r = 0; r < 32; ++r) {
+    const bool zero = UPPER ? (lane < 16 && r >= 16) : (lane >= 16 && r < 16);
+    put(r, lane, zero ? 0.0 : X[r * TS + lane]);
+  }
 }
 
 constexpr int kPerWarp = 32 * PS;  // doubles of a warp's region: its ring, or its staging tile

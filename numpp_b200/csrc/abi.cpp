@@ -99,8 +99,9 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
   if ((flags & NPPB_WANT_SLOGDET) && (!dSign || !dLogabs)) return arg_error("slogdet needs Sign and Logabs");
   if ((flags & NPPB_WANT_LU) && nn && (!dLU || !dipiv)) return arg_error("keeping factors needs LU and ipiv");
   if (!device()) return NPPB_E_NODEV;
-  if (n > 32 && n <= kSysMaxN && !(flags & NPPB_WANT_LU)) {
-    // one CTA per system for the whole factorisation, one per strip for the solves
+  if (n > 32 && !(flags & NPPB_WANT_LU)) {
+    // up to order 512 one CTA per system for the whole factorisation, above it outer
+    // blocks; then one CTA or cluster per strip for the solves
     DevMem w_m, perm_m, dinv_m, state_m;
     NPPB_RC(scratch<double>(w_m, (size_t)count * n * sys_ld(n), st));
     NPPB_RC(scratch<int32_t>(perm_m, (size_t)count * n, st));
@@ -121,59 +122,15 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
     sa.un = n;
     sa.unrhs = (flags & NPPB_WANT_SOLVE) ? nrhs : 0;
     sa.uinv = (flags & NPPB_WANT_INV) ? 1 : 0;
-    NPPB_CUDA(launch_sys_lu(sa, nullptr, (int)count, n, st), "batched LU launch");
+    DevMem other_m, run_m;
+    if (n <= kSysMaxN) {
+      NPPB_CUDA(launch_sys_lu(sa, nullptr, (int)count, n, st), "batched LU launch");
+    } else {
+      NPPB_RC(scratch<int32_t>(other_m, (size_t)count * n, st));
+      NPPB_RC(scratch<double>(run_m, (size_t)count * 3, st));
+      NPPB_CUDA(run_sys_outer(sa, other_m.as<int32_t>(), run_m.as<double>(), (int)count, st), "batched LU launch");
+    }
     NPPB_CUDA(launch_sys_solve_uniform(sa, (int)count, st), "batched substitution launch");
-    return NPPB_OK;
-  }
-  if (n > 32 && !(flags & NPPB_WANT_LU)) {
-    // step-wise kernels in uniform mode: workspace and per-system scratch only
-    DevMem lu_m, sc_m;
-    double* LU = dLU;
-    if (!LU) {
-      NPPB_RC(scratch<double>(lu_m, (size_t)count * nn, st));
-      LU = lu_m.as<double>();
-    }
-    NPPB_RC(scratch<StepScratch>(sc_m, (size_t)count, st));
-    StepArgs sa{};
-    sa.scratch = sc_m.as<StepScratch>();
-    DevMem hist_m;
-    const int bmin = blocked_min_n();
-    if (bmin > 0 && n >= bmin) {  // two-level factorisation: per-system record of a block's panels
-      NPPB_RC(scratch<StepHist>(hist_m, (size_t)count, st));
-      sa.hist = hist_m.as<StepHist>();
-    }
-    sa.A = (dA == LU) ? nullptr : dA;
-    sa.LU = LU;
-    sa.ipiv = dipiv;
-    sa.B = dB; sa.X = dX;
-    sa.inv = (flags & NPPB_WANT_INV) ? dInv : nullptr;
-    sa.det = (flags & NPPB_WANT_DET) ? dDet : nullptr;
-    sa.sign = (flags & NPPB_WANT_SLOGDET) ? dSign : nullptr;
-    sa.logabs = (flags & NPPB_WANT_SLOGDET) ? dLogabs : nullptr;
-    sa.info = dinfo;
-    sa.un = n;
-    sa.unrhs = (flags & NPPB_WANT_SOLVE) ? nrhs : 0;
-    sa.uinv = (flags & NPPB_WANT_INV) ? 1 : 0;
-    // the back substitution of the solutions and inverses that the steps carried along
-    DevMem dinv_m;
-    NPPB_RC(scratch<double>(dinv_m, (size_t)count * sys_dinv(n), st));
-    NPPB_CUDA(run_step_uniform(sa, (int)count, st, false), "batched LU launch");
-    SysArgs su{};
-    su.W = LU;
-    su.w_by_position = 1;
-    su.upper_only = 1;
-    su.dinv = dinv_m.as<double>();
-    su.state = &sa.scratch->info;
-    su.state_stride = sizeof(StepScratch);
-    su.X = dX;
-    su.inv = sa.inv;
-    su.un = n;
-    su.unrhs = sa.unrhs;
-    su.uinv = sa.uinv;
-    if (su.unrhs || su.uinv) {
-      NPPB_CUDA(launch_sys_prepare(su, nullptr, nullptr, (int)count, n, st), "substitution preparation launch");
-      NPPB_CUDA(launch_sys_solve_uniform(su, (int)count, st), "batched substitution launch");
-    }
     return NPPB_OK;
   }
   if (n > 32) {

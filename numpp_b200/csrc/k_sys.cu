@@ -567,6 +567,596 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
 }
 
 // ---------------------------------------------------------------------------
+// Orders above 512: outer blocks of 128 columns. Rows keep their place in W, a copy
+// of A; what moves is the permutation.
+//  k_sys_outer   a cluster of CS CTAs per system factors the outer block's columns
+//                over all rows that are left, left-looking inside the block like
+//                k_sys_lu;
+//  k_sys_rows    U12 = L11^-1 A12, a CTA per 32-column strip right of the block;
+//  k_sys_gemm    A22 -= L21 U12, K = 128, 128 x 64 tiles, rows through the
+//                permutation.
+// The next outer block's columns are updated first and its panel then runs beside
+// the rest of the update (run_sys_outer). The step-wise kernels this replaces
+// updated the trailing matrix with K = 32 and so at the speed of memory, moved rows
+// and took 2.4 us per column of a 1024-row panel.
+//
+// In the cluster block b of 32 positions (counted from the outer block's first)
+// belongs to warp b / CS of CTA b % CS, so that every CTA keeps its share of the
+// rows that are left. Per column each warp's candidate (with its row) goes straight
+// into every CTA's table, one cluster barrier, and every warp finds the winner in
+// its own CTA's copy; the solved rows of a block step are pushed the same way (as
+// in the substitution), the pivot rows of a panel group, the new positions and the
+// diagonal block too. All warps take part in all cluster barriers.
+struct __align__(16) Record {  // a warp's candidate
+  Cand c;
+  double rp, pad;
+  double row[8];
+};
+
+struct __align__(16) ClusterShared {
+  Record own[kMaxWarps];
+  double raw[8][24];
+  double l8[8][8];
+  double u[24 * GS];
+  double pv[32];  // the panel's pivots
+};
+
+constexpr int outer_smem(int warps, int blocks) {
+  return sys_cluster_smem(warps) + 2 * blocks * (int)sizeof(Record);
+}
+
+// As panel(), over the clusters' warps: slot = the warp's block relative to the
+// panel's first (active), na = their number.
+template <int CS, int NC>  // NC: candidates per lane, 32 NC >= na
+__device__ __forceinline__ int cluster_panel(ClusterShared& sh, Record* table, Acc<4>& acc, int& pos, bool valid,
+                                             bool active, int kb, int slot, int na, double* tile, int& nswap) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  cg::cluster_group cl = cg::this_cluster();
+  Record* own = &sh.own[warp];
+  unsigned live = valid ? 0x7fffffffu : 0u;
+#pragma unroll 1
+  for (int j0 = 0; j0 < kb; j0 += 8) {
+    double a[8];
+    if (active) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        double* o = tile + (16 * m + g) * PS + j0 + 2 * t;
+        *reinterpret_cast<double2*>(o) = make_double2(acc.v[m][0][0], acc.v[m][0][1]);
+        *reinterpret_cast<double2*>(o + 8 * PS) = make_double2(acc.v[m][0][2], acc.v[m][0][3]);
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      const double2 x = active ? *reinterpret_cast<const double2*>(tile + lane * PS + j0 + c) : make_double2(0.0, 0.0);
+      a[c] = x.x;
+      a[c + 1] = x.y;
+    }
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const int j = j0 + s;
+      if (j < kb) {  // uniform
+        Record* tab = table + (s & 1) * na;
+        if (active) {  // uniform in the warp
+          const unsigned hi = (unsigned)__double2hiint(a[s]) & live;
+          const unsigned mh = __reduce_max_sync(kAll, hi);
+          const double rp = 1.0 / (hi ? a[s] : 1.0);
+          const bool me = hi == mh;
+          const unsigned top = __ballot_sync(kAll, me);
+          auto publish = [&](unsigned h, unsigned l, double r) {
+            own->c = Cand{h, l, pos, 0};
+            own->rp = r;
+#pragma unroll
+            for (int c = s & ~1; c < 8; c += 2)
+              *reinterpret_cast<double2*>(&own->row[c]) = make_double2(a[c], a[c + 1]);
+          };
+          if (me) publish(hi, (unsigned)__double2loint(a[s]), rp);
+          if ((top & (top - 1)) != 0 || mh >= kInf) {
+            unsigned h = (unsigned)__double2hiint(a[s]) & 0x7fffffffu, l = (unsigned)__double2loint(a[s]);
+            if (!live || h > kInf || (h == kInf && l)) h = l = 0;
+            bool any;
+            const bool win = exact_winner(h, l, pos, any);
+            __syncwarp();
+            if (win) publish(h, l, 1.0 / a[s]);
+            else if (!any && lane == 0) own->c = Cand{0u, 0u, INT_MAX, 0};
+          }
+          __syncwarp();
+          // 16-byte pieces of the record to every CTA
+          for (int i = lane; i < 6 * CS; i += 32) {
+            const int to = i / 6, piece = i - 6 * to;
+            reinterpret_cast<double2*>(cl.map_shared_rank(tab + slot, to))[piece] =
+                reinterpret_cast<const double2*>(own)[piece];
+          }
+        }
+        cl.sync();
+        // candidate 32 q + lane in key q: the high word without its last seven bits, then the index
+        constexpr unsigned kIdx = 127u;
+        unsigned key[NC], mine = 0;
+#pragma unroll
+        for (int q = 0; q < NC; ++q) {
+          const int i = 32 * q + lane;
+          key[q] = i < na ? (tab[i].c.hi & ~kIdx) | (kIdx - i) : 0u;
+          mine = max(mine, key[q]);
+        }
+        const unsigned mk = __reduce_max_sync(kAll, mine);
+        int same = 0;
+#pragma unroll
+        for (int q = 0; q < NC; ++q) same += 32 * q + lane < na && (key[q] ^ mk) <= kIdx;
+        const unsigned amb = __ballot_sync(kAll, same > 0), two = __ballot_sync(kAll, same > 1);
+        int gw = (int)(kIdx - (mk & kIdx));
+        if ((amb & (amb - 1)) != 0 || two != 0 || mk <= kIdx) {
+          Cand cd{0u, 0u, INT_MAX, 0};
+          int at = 0;
+#pragma unroll
+          for (int q = 0; q < NC; ++q) {
+            const int i = 32 * q + lane;
+            if (i < na) {
+              const Cand o = tab[i].c;
+              if (o.hi > cd.hi || (o.hi == cd.hi && (o.lo > cd.lo || (o.lo == cd.lo && o.pos < cd.pos)))) {
+                cd = o;
+                at = i;
+              }
+            }
+          }
+          bool any;
+          const bool best = exact_winner(cd.hi, cd.lo, cd.pos, any);
+          if (!any) return j + 1;  // the same in every warp of the cluster
+          const unsigned who = __ballot_sync(kAll, best);
+          gw = __shfl_sync(kAll, at, 31 - __clz(who));
+        }
+        const double r = tab[gw].rp;
+        const int gk = tab[gw].c.pos;
+        const double* prow = tab[gw].row;
+        if (threadIdx.x == 0) sh.pv[j] = prow[s];
+        const bool chosen = valid && pos == gk;
+        if (pos == j) pos = gk;
+        if (chosen) {
+          pos = j;
+          live = 0;
+        }
+        nswap += gk != j;
+        const double f = live ? a[s] * r : 0.0;
+        if (live) a[s] = f;
+#pragma unroll
+        for (int c = s + 1; c < 8; ++c) a[c] = fma(-f, prow[c], a[c]);
+      }
+    }
+    if (active) {
+#pragma unroll
+      for (int c = 0; c < 8; c += 2)
+        *reinterpret_cast<double2*>(tile + lane * PS + j0 + c) = make_double2(a[c], a[c + 1]);
+    }
+    if (j0 + 8 >= kb) break;
+    // the row's step in the group; 8: still below, -1: done before (or no row)
+    const bool in_group = valid && !live && pos >= j0 && pos < j0 + 8;
+    const int mine = live ? 8 : in_group ? pos - j0 : -1;
+    double2 l[4];
+    if (active) {
+      if (in_group) {
+        for (int to = 0; to < CS; ++to) {
+          double2* o = reinterpret_cast<double2*>(cl.map_shared_rank(&sh.l8[pos - j0][0], to));
+#pragma unroll
+          for (int c = 0; c < 4; ++c) o[c] = make_double2(a[2 * c], a[2 * c + 1]);
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int lim = __shfl_sync(kAll, mine, 8 * i + g);
+        if (lim >= 0 && lim < 8) {
+          for (int to = 0; to < CS; ++to) {
+            double* o = cl.map_shared_rank(&sh.raw[lim][2 * t], to);
+#pragma unroll
+            for (int ni = 1; ni < 4; ++ni)
+              *reinterpret_cast<double2*>(o + 8 * (ni - 1)) =
+                  make_double2(acc.v[i >> 1][ni][2 * (i & 1)], acc.v[i >> 1][ni][2 * (i & 1) + 1]);
+          }
+        }
+        l[i] = *reinterpret_cast<const double2*>(tile + (8 * i + g) * PS + j0 + 2 * t);
+        if (2 * t >= lim) l[i].x = 0.0;
+        if (2 * t + 1 >= lim) l[i].y = 0.0;
+      }
+    }
+    cl.sync();
+    if (warp == 0) {
+      const int c = min(lane, 23);
+      double x[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) x[s] = sh.raw[s][c];
+#pragma unroll
+      for (int q = 0; q < 7; ++q)
+#pragma unroll
+        for (int s = q + 1; s < 8; ++s) x[s] = fma(-sh.l8[s][q], x[q], x[s]);
+      if (lane < 24) {
+#pragma unroll
+        for (int s = 0; s < 8; s += 2)
+          *reinterpret_cast<double2*>(&sh.u[lane * GS + s]) = make_double2(-x[s], -x[s + 1]);
+      }
+    }
+    __syncthreads();
+    if (active) {
+#pragma unroll
+      for (int ni = 1; ni < 4; ++ni) {
+        const double2 b = *reinterpret_cast<const double2*>(&sh.u[(8 * (ni - 1) + g) * GS + 2 * t]);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          dmma1688(acc.v[m][ni], l[2 * m], l[2 * m + 1], b);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc.v[m][ni - 1][e] = acc.v[m][ni][e];
+        }
+      }
+    }
+  }
+  return 0;
+}
+
+// The outer block of blocks [jb, je). perm_in: the positions so far, perm_out: with
+// this block's pivots (the update beside it reads the former). running: det,
+// log|det| and sign by slot.
+template <int CS, int NC>
+__global__ void __launch_bounds__(kSysMaxN, 1)
+k_sys_outer(SysArgs sa, const int32_t* __restrict__ perm_in, int32_t* __restrict__ perm_out,
+            double* __restrict__ running, int jb, int je) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ ClusterShared sh;
+  __shared__ int s_perm[kSysMaxN];  // the rows at this CTA's positions
+  __shared__ double s_det[3];       // det, log|det|, sign (CTA 0)
+  __shared__ View s_v;
+  __shared__ int s_skip;
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int rank = (int)blockIdx.x % CS;
+  double* Tb = sm + kTb;
+  double* Li = sm + kLi;
+  double* U0 = sm + kUt;
+  double* U1 = sm + kWarp + nw * kPerWarp;
+  Record* table = reinterpret_cast<Record*>(U1 + 32 * US);
+  double* D11 = Tb;
+  double* stage = sm + kWarp + warp * kPerWarp;
+  const unsigned ring = smem(stage) + 16 * lane;
+  const int sys = (int)blockIdx.x / CS;
+  if (tid == 0) {
+    s_v = view(sa, sys);
+    s_skip = jb > 0 && *state_of(sa, s_v.slot);
+    const double* run = running + 3 * (int64_t)s_v.slot;
+    s_det[0] = jb ? run[0] : 1.0;
+    s_det[1] = jb ? run[1] : 0.0;
+    s_det[2] = jb ? run[2] : 1.0;
+  }
+  __syncthreads();
+  if (s_skip) return;  // the same for every CTA of the cluster
+  double* const W = s_v.W;
+  const int n = s_v.n, nb = sys_blocks(n), ldw = s_v.ldw;
+  const int blk = jb + warp * CS + rank;  // the warp's block
+  const int32_t* pin = perm_in + (int64_t)sys * n;
+  int32_t* pout = perm_out + (int64_t)sys * n;
+  for (int i = tid; i < 32 * nw; i += blockDim.x) {
+    const int p = 32 * (jb + (i >> 5) * CS + rank) + (i & 31);
+    s_perm[i] = p >= n ? 0 : jb ? pin[p] : p;
+  }
+  for (int p = rank * blockDim.x + tid; p < 32 * jb; p += CS * blockDim.x) pout[p] = pin[p];
+  cl.sync();
+
+  for (int J = jb; J < je; ++J) {
+    const int kb = min(32, n - 32 * J);
+    // the warp's rows of the column block
+    Acc<4> acc;
+    Rows r;
+    r.live = n - 32 * blk - g;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const bool ok = 8 * i < r.live;
+      const int row = ok ? s_perm[32 * warp + 8 * i + g] : 0;
+      r.off[i] = (unsigned)row * ldw * 8;
+      const double* src = W + (int64_t)row * ldw;
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni) {
+        const int col = 32 * J + 8 * ni + 2 * t;
+        double2 x = make_double2(0.0, 0.0);
+        if (ok && col < n) {
+          x = __ldcg(reinterpret_cast<const double2*>(src + col));  // the pair ends inside the row's padding
+          if (col + 1 >= n) x.y = 0.0;
+        }
+        acc.v[i >> 1][ni][2 * (i & 1)] = x.x;
+        acc.v[i >> 1][ni][2 * (i & 1) + 1] = x.y;
+      }
+    }
+    // the block's earlier columns
+    if (J > jb) {
+      const int first = jb + rank;                   // this CTA's first block
+      if (J - 1 == first) __syncthreads();           // its inverse has just been written
+      if (first < J) fetch_inverse(Li, s_v.dinv + (int64_t)first * 2048, blockDim.x);
+      else cp_commit();
+      ring_start<true, false>(ring, W, r, jb, n, blk > jb && blk < nb);
+      for (int K = jb; K < J; ++K) {
+        double* Ut = K & 1 ? U1 : U0;
+        const bool mine = (K - jb) % CS == rank;
+        if (mine) {
+          if (K == first) __syncthreads();  // the inversions are done with the diagonal block in Tb
+          if (blk == K) store_tile<4>(Tb, acc);
+          cp_wait<2>();  // the inverse; at most two operand stages stay in flight
+          __syncthreads();
+          tile_product<4, false, CS>(Li, Tb, Ut);
+        }
+        cl.sync();
+        if (blk > K && blk < nb) {
+          update<4, true, false>(acc, ring, W, r, smem(Ut + g * US + 2 * t), K, K + 1, K + 1 < J && blk > K + 1, n);
+        } else {
+          if (mine && blk <= K) {  // the owner's warps that are done: U out, its next inverse in
+            const int free = (K - jb) / CS + 1;
+            if (K + CS < J) fetch_inverse(Li, s_v.dinv + (int64_t)(K + CS) * 2048, 32 * free);
+            product_out<4, true>(Ut, ldw - 32 * J, 0, free,
+                                 [&](int row) { return W + (int64_t)s_perm[(K - jb) / CS * 32 + row] * ldw + 32 * J; });
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) cp_commit();  // the waits count groups
+        }
+      }
+      cp_wait<0>();
+      __syncwarp();  // the ring becomes the staging tile
+    }
+    // the panel
+    const bool active = blk >= J && blk < nb, valid = active && lane < n - 32 * blk;
+    const int phys = valid ? s_perm[32 * warp + lane] : 0;
+    int pos = 32 * (blk - J) + lane, nswap = 0;
+    const int info = cluster_panel<CS, NC>(sh, table, acc, pos, valid, active, kb, blk - J, nb - J, stage, nswap);
+    if (info) {  // the same in every thread of the cluster; nothing is on its way to another CTA
+      if (tid == 0 && rank == 0) {
+        *state_of(sa, s_v.slot) = 32 * J + info;
+        if (sa.det) sa.det[s_v.idx] = 0.0;
+        if (sa.sign) sa.sign[s_v.idx] = 0.0;
+        if (sa.logabs) sa.logabs[s_v.idx] = -INFINITY;
+        if (sa.info) sa.info[s_v.idx] = 32 * J + info;
+      }
+      return;
+    }
+    if (active) {
+      if (valid) {
+        const int b = J - jb + (pos >> 5);
+        cl.map_shared_rank(s_perm, b % CS)[b / CS * 32 + (pos & 31)] = phys;
+      }
+      __syncwarp();
+      double* d11 = cl.map_shared_rank(D11, (J - jb) % CS);
+      const int off = phys * ldw, at = valid ? pos : n;
+#pragma unroll 8
+      for (int rr = 0; rr < 32; ++rr) {
+        const int o = __shfl_sync(kAll, off, rr), p2 = __shfl_sync(kAll, at, rr);
+        const double x = stage[rr * PS + lane];
+        if (p2 < n && lane < kb) W[o + 32 * J + lane] = x;
+        if (p2 < kb) d11[p2 * PS + lane] = x;
+      }
+    }
+    cl.sync();  // rows, positions and the diagonal block are everywhere
+    double* di = s_v.dinv + (int64_t)J * 2048;
+    if ((J - jb) % CS == rank) {
+      if (warp == 0) tri_inverse<kUnitLower>(D11, stage, kb, into(di));
+      if (warp == 1 % nw) tri_inverse<kUpper>(D11, stage, kb, into(di + 1024));
+    }
+    if (rank == 0 && warp == 2 % nw) {
+      // folded in the reference's order (linalg.cpp:400-403, 425-431)
+      const double pv = lane < kb ? sh.pv[lane] : 1.0;
+      const double lg = log(fabs(pv)), sgn = pv / fabs(pv);
+      double det = s_det[0], la = s_det[1], sg = s_det[2];
+      if (nswap & 1) {
+        det = -det;
+        sg = -sg;
+      }
+      for (int j = 0; j < kb; ++j) {
+        det *= __shfl_sync(kAll, pv, j);
+        la += __shfl_sync(kAll, lg, j);
+        sg *= __shfl_sync(kAll, sgn, j);
+      }
+      __syncwarp();
+      if (lane == 0) {
+        s_det[0] = det;
+        s_det[1] = la;
+        s_det[2] = sg;
+        if (J + 1 == je) {
+          double* run = running + 3 * (int64_t)s_v.slot;
+          run[0] = det;
+          run[1] = la;
+          run[2] = sg;
+        }
+        if (J + 1 == nb) {
+          if (sa.det) sa.det[s_v.idx] = det;
+          if (sa.sign) sa.sign[s_v.idx] = sg;
+          if (sa.logabs) sa.logabs[s_v.idx] = la;
+        }
+      }
+    }
+  }
+  for (int i = tid; i < 32 * nw; i += blockDim.x) {
+    const int p = 32 * (jb + (i >> 5) * CS + rank) + (i & 31);
+    if (p < n) pout[p] = s_perm[i];
+  }
+  if (tid == 0 && rank == 0) {
+    *state_of(sa, s_v.slot) = 0;
+    if (sa.info && je == nb) sa.info[s_v.idx] = 0;
+  }
+}
+
+// U12 on columns [c0 + 32 blockIdx.x, +32) of system blockIdx.y: the outer block's
+// rows (four blocks, a warp each), forward substitution as in solve_strip.
+__global__ void __launch_bounds__(128, 4)
+k_sys_rows(SysArgs sa, const int32_t* __restrict__ perm, int jb, int je, int c0, int c1) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ View s_v;
+  __shared__ int s_perm[128], s_skip;
+  double* Tb = sm + kTb;
+  double* Li = sm + kLi;
+  double* Ut = sm + kUt;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const unsigned ring = smem(sm + kWarp + warp * kPerWarp) + 16 * lane;
+  if (threadIdx.x == 0) {
+    s_v = view(sa, blockIdx.y);
+    s_skip = *state_of(sa, s_v.slot);
+  }
+  __syncthreads();
+  if (s_skip) return;
+  const int n = s_v.n, ldw = s_v.ldw, cols = je - jb;
+  double* const W = s_v.W;
+  // an outer block that something lies right of is full
+  s_perm[threadIdx.x] = (int)threadIdx.x < 32 * cols ? perm[(int64_t)blockIdx.y * n + 32 * jb + threadIdx.x] : 0;
+  __syncthreads();
+  const int col0 = c0 + 32 * (int)blockIdx.x;
+  Acc<4> acc;
+  Rows r;
+  r.live = 32;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = s_perm[32 * warp + 8 * i + g];
+    r.off[i] = (unsigned)row * ldw * 8;
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni) {
+      const int col = col0 + 8 * ni + 2 * t;
+      double2 x = make_double2(0.0, 0.0);
+      if (col < c1) x = *reinterpret_cast<const double2*>(W + (int64_t)row * ldw + col);
+      acc.v[i >> 1][ni][2 * (i & 1)] = x.x;
+      acc.v[i >> 1][ni][2 * (i & 1) + 1] = x.y;
+    }
+  }
+  fetch_inverse(Li, s_v.dinv + (int64_t)jb * 2048, blockDim.x);
+  ring_start<true, false>(ring, W, r, jb, n, warp > 0 && warp < cols);
+  for (int K = 0; K < cols; ++K) {
+    if (warp == K) store_tile<4>(Tb, acc);
+    cp_wait<2>();
+    __syncthreads();
+    tile_product<4, false, 1>(Li, Tb, Ut);
+    __syncthreads();
+    if (warp > K && warp < cols) {
+      update<4, true, false>(acc, ring, W, r, smem(Ut + g * US + 2 * t), jb + K, jb + K + 1, warp > K + 1, n);
+    } else {
+      if (warp <= K) {
+        if (K + 1 < cols) fetch_inverse(Li, s_v.dinv + (int64_t)(jb + K + 1) * 2048, 32 * (K + 1));
+        product_out<4, true>(Ut, c1 - col0, 0, K + 1,
+                             [&](int row) { return W + (int64_t)s_perm[32 * K + row] * ldw + col0; });
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) cp_commit();
+    }
+  }
+}
+
+// A22 -= L21 U12 on columns [c0, c1): one CTA per 128 x 64 tile (grid.z = system).
+// Positions p0 + 128 y .. of the permutation give the rows; K = the outer block's
+// 128 columns in eight slabs of 16 through a ring of three (cp.async, 16 bytes).
+// Eight warps of 32 x 32 accumulators; the C tile is read while the first slabs
+// arrive. Bounds: FP64 tensor throughput (a tile is 8.4 us of an SM's pipe against
+// 128 KB of C read and written), two CTAs per SM to cover the ends of a tile.
+constexpr int GM = 128, GN = 64, GK = 16, GSTAGES = 3;
+constexpr int GBS = GN + 2;  // row stride of a U slab (8-byte reads down a column: banks 4t + g)
+constexpr int kGemmSlab = GM * GK + GK * GBS;
+constexpr int kGemmSmem = 8 * GSTAGES * kGemmSlab;
+
+__global__ void __launch_bounds__(256, 2)
+k_sys_gemm(SysArgs sa, const int32_t* __restrict__ perm, int jb, int je, int c0, int c1) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int s_up[128], s_row[GM], s_skip;
+  __shared__ View s_v;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  if (tid == 0) {
+    s_v = view(sa, blockIdx.z);
+    s_skip = *state_of(sa, s_v.slot);
+  }
+  __syncthreads();
+  if (s_skip) return;
+  const int n = s_v.n, ldw = s_v.ldw;
+  double* const W = s_v.W;
+  const int p0 = 32 * je + GM * (int)blockIdx.y, col0 = c0 + GN * (int)blockIdx.x;
+  const int32_t* pm = perm + (int64_t)blockIdx.z * n;
+  if (tid < 128) s_row[tid] = p0 + tid < n ? pm[p0 + tid] : -1;
+  else s_up[tid - 128] = pm[32 * jb + tid - 128];
+  __syncthreads();
+  // rows of a slab: 16-byte piece c of row r at piece c ^ 4 (r & 1): two neighbouring
+  // rows fall into the two halves of the banks
+  auto load = [&](int slab) {
+    double* a = sm + slab % GSTAGES * kGemmSlab;
+    double* b = a + GM * GK;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int idx = tid + 256 * i, r = idx >> 3, c = idx & 7, row = s_row[r];
+      const double* src = W + (int64_t)max(row, 0) * ldw + 32 * jb + GK * slab + 2 * c;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem(a + r * GK + 2 * (c ^ 4 * (r & 1)))),
+                   "l"(src), "r"(row >= 0 ? 16 : 0));
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int idx = tid + 256 * i, r = idx >> 5, c = (idx & 31) * 2;
+      const int col = min(col0 + c, ldw - 2);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem(b + r * GBS + c)),
+                   "l"(W + (int64_t)s_up[GK * slab + r] * ldw + col));
+    }
+    cp_commit();
+  };
+  constexpr int kSlabs = 128 / GK;
+  load(0);
+  load(1);
+  const int wm = 32 * (warp >> 1), wn = 32 * (warp & 1);
+  double acc[2][4][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int row = s_row[wm + 16 * m + 8 * h + g];
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni) {
+        const int col = col0 + wn + 8 * ni + 2 * t;
+        double2 x = make_double2(0.0, 0.0);
+        if (row >= 0 && col < c1) x = *reinterpret_cast<const double2*>(W + (int64_t)row * ldw + col);
+        acc[m][ni][2 * h] = -x.x;  // the tile accumulates L U - A and is negated on the way out
+        acc[m][ni][2 * h + 1] = -x.y;
+      }
+    }
+  for (int k = 0; k < kSlabs; ++k) {
+    cp_wait<1>();
+    __syncthreads();  // slab k is here, and slab k - 1 has been read
+    if (k + 2 < kSlabs) load(k + 2);
+    else cp_commit();
+    const double* a = sm + k % GSTAGES * kGemmSlab;
+    const double* b = a + GM * GK;
+#pragma unroll
+    for (int q = 0; q < GK / 8; ++q) {
+      double2 av[4], bv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = wm + 8 * i + g;
+        av[i] = *reinterpret_cast<const double2*>(a + r * GK + 2 * ((4 * q + t) ^ 4 * (r & 1)));
+      }
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni) {
+        const double* p = b + (8 * q + 2 * t) * GBS + wn + 8 * ni + g;
+        bv[ni] = make_double2(p[0], p[GBS]);
+      }
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) dmma1688(acc[m][ni], av[2 * m], av[2 * m + 1], bv[ni]);
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int row = s_row[wm + 16 * m + 8 * h + g];
+#pragma unroll
+      for (int ni = 0; ni < 4; ++ni) {
+        const int col = col0 + wn + 8 * ni + 2 * t;
+        if (row >= 0 && col < c1)
+          *reinterpret_cast<double2*>(W + (int64_t)row * ldw + col) =
+              make_double2(-acc[m][ni][2 * h], -acc[m][ni][2 * h + 1]);
+      }
+    }
+}
+
+// W <- A, rows padded to the workspace's leading dimension (zeros).
+__global__ void __launch_bounds__(256)
+k_sys_copy(const double* __restrict__ A, double* __restrict__ W, int64_t rows, int n, int ldw) {
+  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (int64_t)gridDim.x * 8)
+    for (int c = threadIdx.x & 31; c < ldw; c += 32) W[r * ldw + c] = c < n ? __ldcs(A + r * n + c) : 0.0;
+}
+
+// ---------------------------------------------------------------------------
 // Substitution of one strip: C = P B (or P times columns of the identity), then
 // Y_K = L_KK^-1 C_K and C_w -= L_wK Y_K downwards, X_K = U_KK^-1 Y_K and
 // Y_w -= U_wK X_K upwards.
@@ -781,6 +1371,65 @@ cudaError_t launch_sys_lu(const SysArgs& sa, const int32_t* list, int nsys, int 
 
 namespace {
 
+template <int CS, int NC>
+cudaError_t launch_outer1(const SysArgs& sa, const int32_t* pin, int32_t* pout, double* running, int nsys, int jb,
+                          int je, cudaStream_t st) {
+  const int blocks = sys_blocks(sa.un) - jb, nw = std::max(1, (blocks + CS - 1) / CS);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)nsys * CS);
+  cfg.blockDim = dim3(32 * nw);
+  cfg.dynamicSmemBytes = outer_smem(nw, blocks);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CS;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_sys_outer<CS, NC>, sa, pin, pout, running, jb, je);
+}
+
+template <int CS, int NC>
+cudaError_t prepare_outer() {
+  return cudaFuncSetAttribute(k_sys_outer<CS, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              outer_smem(kMaxWarps, kMaxWarps * CS));
+}
+
+}  // namespace
+
+cudaError_t launch_sys_outer(const SysArgs& sa, const int32_t* pin, int32_t* pout, double* running, int nsys, int jb,
+                             int je, cudaStream_t st) {
+  const int cs = sys_outer_cluster(32 * (sys_blocks(sa.un) - jb), nsys);
+  switch (cs) {
+    case 2: return launch_outer1<2, 1>(sa, pin, pout, running, nsys, jb, je, st);
+    case 4: return launch_outer1<4, 2>(sa, pin, pout, running, nsys, jb, je, st);
+    case 8: return launch_outer1<8, 4>(sa, pin, pout, running, nsys, jb, je, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_sys_update(const SysArgs& sa, const int32_t* perm, int nsys, int jb, int je, int c0, int c1,
+                              cudaStream_t st) {
+  if (c0 >= c1) return cudaSuccess;
+  if (nsys > 65535) return cudaErrorInvalidValue;
+  k_sys_rows<<<dim3((unsigned)(c1 - c0 + 31) / 32, (unsigned)nsys), 128, sys_smem(4), st>>>(sa, perm, jb, je, c0, c1);
+  const int rows = sa.un - 32 * je;
+  if (rows > 0)
+    k_sys_gemm<<<dim3((unsigned)(c1 - c0 + GN - 1) / GN, (unsigned)(rows + GM - 1) / GM, (unsigned)nsys), 256,
+                 kGemmSmem, st>>>(sa, perm, jb, je, c0, c1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_sys_copy(const SysArgs& sa, int nsys, cudaStream_t st) {
+  const int64_t rows = (int64_t)nsys * sa.un;
+  k_sys_copy<<<(unsigned)std::min<int64_t>((rows + 7) / 8, 148 * 16), 256, 0, st>>>(sa.A, sa.W, rows, sa.un,
+                                                                                    sys_ld(sa.un));
+  return cudaGetLastError();
+}
+
+namespace {
+
 template <int NI, bool VEC, int CS>
 cudaError_t launch_strips3(const SysArgs& sa, const SysItem* items, int64_t nitems, int nmax, int inverse, int first,
                            int per, cudaStream_t st) {
@@ -878,6 +1527,13 @@ cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int
 cudaError_t sys_prepare_kernels() {
   cudaError_t e = cudaFuncSetAttribute(k_sys_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        sys_smem(kMaxWarps));
+  if (e == cudaSuccess) e = prepare_outer<2, 1>();
+  if (e == cudaSuccess) e = prepare_outer<4, 2>();
+  if (e == cudaSuccess) e = prepare_outer<8, 4>();
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_sys_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, sys_smem(4));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_sys_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
   if (e == cudaSuccess) e = prepare_strips<1>();
   if (e == cudaSuccess) e = prepare_strips<2>();
   if (e == cudaSuccess) e = prepare_strips<4>();

@@ -219,6 +219,45 @@ cudaError_t run_step_uniform(const StepArgsT<T>& sa, int count, cudaStream_t st,
   if (back > INT32_MAX) return cudaErrorInvalidValue;
   return launch_back(sa, nullptr, (int)back, sa.un, sa.uinv ? 64 : std::min(64, sa.unrhs), st);
 }
+// Outer blocks of a uniform batch above order 512: once a block's panel is done, its
+// update of the next block's columns and that block's panel follow on a
+// high-priority stream, while the rest of the update runs on a side stream; the
+// next block's updates wait for both. The permutation alternates between two
+// buffers, so that the update beside a panel reads the one before it.
+cudaError_t run_sys_outer(const SysArgs& sa, int32_t* other, double* running, int nsys, cudaStream_t st) {
+  const int n = sa.un, nb = sys_blocks(n), steps = (nb + kSysOuter - 1) / kSysOuter;
+  int32_t* perm[2];  // panel k reads perm[k & 1] and writes the other: the last one writes sa.perm
+  perm[steps & 1] = sa.perm;
+  perm[(steps + 1) & 1] = other;
+  Lookahead* la = lookahead_for_device();
+  if (!la) return cudaErrorUnknown;
+  cudaError_t e = launch_sys_copy(sa, nsys, st);
+  if (e == cudaSuccess) e = cudaEventRecord(la->first, st);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(la->panel, la->first, 0);
+  bool rest = false;  // an update on the side stream
+  for (int k = 0; k < steps && e == cudaSuccess; ++k) {
+    const int jb = k * kSysOuter, je = std::min(nb, jb + kSysOuter);
+    const int c0 = std::min(n, 32 * je), c1 = std::min(n, c0 + 32 * kSysOuter);
+    int32_t* now = perm[(k + 1) & 1];
+    e = launch_sys_outer(sa, perm[k & 1], now, running, nsys, jb, je, la->panel);
+    if (e != cudaSuccess || c0 >= n) break;
+    if (rest) e = cudaStreamWaitEvent(la->panel, la->rest, 0);  // the previous update covers these columns
+    rest = false;
+    if (e == cudaSuccess && c1 < n) {
+      e = cudaEventRecord(la->next, la->panel);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(la->side, la->next, 0);
+      if (e == cudaSuccess) e = launch_sys_update(sa, now, nsys, jb, je, c1, n, la->side);
+      if (e == cudaSuccess) e = cudaEventRecord(la->rest, la->side);
+      rest = true;
+    }
+    if (e == cudaSuccess) e = launch_sys_update(sa, now, nsys, jb, je, c0, c1, la->panel);
+  }
+  if (e == cudaSuccess && rest) e = cudaStreamWaitEvent(la->panel, la->rest, 0);
+  if (e == cudaSuccess) e = cudaEventRecord(la->first, la->panel);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(st, la->first, 0);
+  return e;
+}
+
 // Two-level factorisation (sa.hist set): outer blocks of kStepNBO columns.
 // The panels of a block update only the block's columns (all rows below),
 // the right-hand sides and the inverse, and carry their row moves left of the

@@ -10,6 +10,7 @@
 namespace nppb {
 
 constexpr int kSysMaxN = 512;  // one CTA per system: 16 warps of 32 rows
+constexpr int kSysOuter = 4;   // blocks of an outer block (orders above 512)
 
 // Leading dimension of a factor workspace: rows start on 32-byte sectors.
 __host__ __device__ inline int sys_ld(int n) { return (n + 3) & ~3; }
@@ -25,6 +26,16 @@ inline int sys_cluster(int n, int64_t items) {
   int cs = 1;
   while (nb > 16 * cs) cs *= 2;
   while (cs < 8 && items * cs * 2 <= 148 && nb >= 8 * cs) cs *= 2;
+  return cs;
+}
+
+// CTAs per system of an outer block's panel over `rows` rows: 16 blocks each at
+// most, more while the clusters leave SMs idle (columns are faster with fewer
+// warps per CTA).
+inline int sys_outer_cluster(int rows, int64_t systems) {
+  int cs = 2;
+  while (sys_blocks(rows) > 16 * cs) cs *= 2;
+  while (cs < 8 && systems * cs * 2 <= 120 && sys_blocks(rows) >= 8 * cs) cs *= 2;
   return cs;
 }
 
@@ -59,9 +70,21 @@ struct SysArgs {
   int upper_only;       // X and the inverse hold L^-1 P B already: back substitution in place
 };
 
-// LU with partial pivoting of `nsys` systems with (maximum order) nmax <= 512,
-// one CTA of sys_blocks(nmax) warps each.
+// LU with partial pivoting of `nsys` systems with (maximum order) nmax <= 512, a
+// CTA each.
 cudaError_t launch_sys_lu(const SysArgs& sa, const int32_t* list, int nsys, int nmax, cudaStream_t st);
+// Uniform batches above order 512, in outer blocks [jb, je) of 32-column blocks:
+// W <- A; the block's panel (pin: permutation so far, pout: with its pivots;
+// running: three doubles per system); U12 and the trailing update on columns
+// [c0, c1) with pout.
+cudaError_t launch_sys_copy(const SysArgs& sa, int nsys, cudaStream_t st);
+cudaError_t launch_sys_outer(const SysArgs& sa, const int32_t* pin, int32_t* pout, double* running, int nsys, int jb,
+                             int je, cudaStream_t st);
+cudaError_t launch_sys_update(const SysArgs& sa, const int32_t* perm, int nsys, int jb, int je, int c0, int c1,
+                              cudaStream_t st);
+// All of it, the next panel beside the update: sa.perm gets the final permutation;
+// other: a second one, running: the panels' state.
+cudaError_t run_sys_outer(const SysArgs& sa, int32_t* other, double* running, int nsys, cudaStream_t st);
 // Forward and back substitution: `nitems` strips of one width class (8, 16 or 32
 // columns at most; `width` = the widest), or every strip of a uniform batch.
 inline int sys_width_class(int width) { return width <= 8 ? 0 : width <= 16 ? 1 : 2; }

@@ -13,6 +13,18 @@ __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
+// D(16x8) += A(16x8) B(8x8), FP64, one warp. Lane 4g + t holds A[g][t],
+// A[g+8][t], A[g][t+4], A[g+8][t+4]; B[t][g], B[t+4][g]; D[g][2t], D[g][2t+1],
+// D[g+8][2t], D[g+8][2t+1]. The k index may be permuted alike on both sides:
+// the callers take k = 2t for slot t and 2t + 1 for slot t + 4, so that a lane's
+// two values lie side by side.
+__device__ __forceinline__ void dmma1688(double (&d)[4], double2 lo, double2 hi, double2 b) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(lo.x), "d"(hi.x), "d"(lo.y), "d"(hi.y), "d"(b.x), "d"(b.y));
+}
+
 // Warp-wide argmax of (v, i): the largest v wins, ties go to the smaller i.
 // Every lane ends with the same pair.
 __device__ __forceinline__ void warp_argmax(double& v, int& i) {

@@ -101,6 +101,8 @@ cudaError_t launch_lu_warp(const Batch& bt, const int32_t* order, int nsys, int 
                            cudaStream_t st);
 
 // Row-major C[m,n] = A[m,k] B[k,n] in FP64 on DMMA (device pointers).
+// Shared-memory limits of the FP64 GEMM kernels (once per device).
+cudaError_t gemm_prepare();
 cudaError_t launch_gemm_f64(int64_t m, int64_t n, int64_t k, const double* A, int64_t lda,
                             const double* B, int64_t ldb, double* C, int64_t ldc,
                             cudaStream_t st);

@@ -118,6 +118,7 @@ void DevMem::release() {
 cudaError_t prepare_kernels() {
   cudaError_t e = step_prepare();
   if (e == cudaSuccess) e = sys_prepare_kernels();
+  if (e == cudaSuccess) e = gemm_prepare();
   return e == cudaSuccess ? mx_prepare() : e;
 }
 

@@ -17,6 +17,7 @@
 #include <cfloat>
 #include <cmath>
 
+#include "dmma.cuh"
 #include "mixed.hpp"
 
 namespace nppb {
@@ -250,6 +251,108 @@ k_residual(const double* __restrict__ A, const double* __restrict__ B, const dou
   }
 }
 
+// The same with 3 or more right-hand sides, on the FP64 tensor cores: eight of
+// them are one m16n8k8 operand. Per-thread products read every staged X value
+// once per row of A, and shared memory bounded them (430 us a pass over 5
+// systems of order 3001 with 8 right-hand sides, 137 us so; with 1 or 2 the
+// pass over A itself is the bound). Eight warps: 2 tiles of 16 rows x 4 shares
+// of each staged block's columns, whose sums meet in shared memory. A lane
+// loads its entries of A itself, four of a row's neighbours making 32 bytes, 8
+// columns at a time and four steps ahead of the products.
+constexpr int XB = 512;  // rows of X staged per block
+
+__global__ void __launch_bounds__(MT)
+k_residual_mma(const double* __restrict__ A, const double* __restrict__ B, const double* __restrict__ X,
+               int n, int nrhs, const double* __restrict__ rs, float* __restrict__ R32,
+               const int32_t* __restrict__ rpos, double* __restrict__ R64, RefineState* __restrict__ st,
+               int only_active, int stats) {
+  __shared__ __align__(16) double xs[XB * 8];  // [row][8]; the shares' sums [4][32][8] after the last block
+  __shared__ double red[MT / 32];
+  const int s = blockIdx.x, r0 = blockIdx.y * kMixedRows;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  if (only_active && st[s].status != kRefineActive) return;
+  const int64_t nb = (int64_t)n * nrhs;
+  const double* b = B ? B + (int64_t)s * nb : nullptr;  // null: R = -A X (the product alone)
+  const double* x = X + (int64_t)s * nb;
+  const bool first = stats && blockIdx.y == 0;
+  const int tile = warp & 1, share = warp >> 1;
+  // rows past the order read the last row; their sums go nowhere
+  const double* a0 = A + (int64_t)s * n * n + (int64_t)min(r0 + 16 * tile + g, n - 1) * n;
+  const double* a1 = A + (int64_t)s * n * n + (int64_t)min(r0 + 16 * tile + g + 8, n - 1) * n;
+  double rmax = 0.0, xmax = 0.0;
+  for (int k0 = 0; k0 < nrhs; k0 += 8) {
+    const int kc = min(8, nrhs - k0);
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int j0 = 0; j0 < n; j0 += XB) {
+      const int jn = min(XB, n - j0), j8 = (jn + 7) & ~7;
+      __syncthreads();
+      for (int idx = tid; idx < j8 * 8; idx += MT) {
+        const int j = idx >> 3, k = idx & 7;
+        const double v = j < jn && k < kc ? x[(int64_t)(j0 + j) * nrhs + k0 + k] : 0.0;
+        xs[idx] = v;
+        if (first) xmax = fmax(xmax, fabs(v));
+      }
+      __syncthreads();
+      const int per = ((j8 >> 3) + 3) >> 2, lo = 8 * share * per, hi = min(jn, lo + 8 * per);
+      int j = lo;
+#pragma unroll 1
+      for (; j + 32 <= hi; j += 32) {
+        double a[4][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = j0 + j + 8 * u + t;
+          a[u][0] = a0[c];
+          a[u][1] = a1[c];
+          a[u][2] = a0[c + 4];
+          a[u][3] = a1[c + 4];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double* xr = xs + (j + 8 * u + t) * 8 + g;
+          dmma1688(acc, make_double2(a[u][0], a[u][2]), make_double2(a[u][1], a[u][3]), make_double2(xr[0], xr[32]));
+        }
+      }
+#pragma unroll 1
+      for (; j < hi; j += 8) {  // columns past the order count as zero on both sides
+        const int c = j0 + j + t;
+        const bool in0 = j + t < jn, in1 = j + t + 4 < jn;
+        const double a[4] = {in0 ? a0[c] : 0.0, in0 ? a1[c] : 0.0, in1 ? a0[c + 4] : 0.0, in1 ? a1[c + 4] : 0.0};
+        const double* xr = xs + (j + t) * 8 + g;
+        dmma1688(acc, make_double2(a[0], a[2]), make_double2(a[1], a[3]), make_double2(xr[0], xr[32]));
+      }
+    }
+    __syncthreads();
+    {
+      double* p = xs + (share * 32 + 16 * tile) * 8;
+      p[g * 8 + 2 * t] = acc[0];
+      p[g * 8 + 2 * t + 1] = acc[1];
+      p[(g + 8) * 8 + 2 * t] = acc[2];
+      p[(g + 8) * 8 + 2 * t + 1] = acc[3];
+    }
+    __syncthreads();
+    {  // thread = (row, right-hand side)
+      const int q = tid >> 3, k = tid & 7, i = r0 + q;
+      if (i < n && k < kc) {
+        const double ax = (xs[tid] + xs[256 + tid]) + (xs[512 + tid] + xs[768 + tid]);
+        const double r = (b ? b[(int64_t)i * nrhs + k0 + k] : 0.0) - ax;
+        rmax = fmax(rmax, fabs(r));
+        if (R32) {
+          const int p = rpos ? rpos[(int64_t)s * n + i] : i;
+          R32[(int64_t)s * nb + (int64_t)p * nrhs + k0 + k] = (float)(rs[(int64_t)s * n + i] * r);
+        }
+        if (R64) R64[(int64_t)s * nb + (int64_t)i * nrhs + k0 + k] = rs[(int64_t)s * n + i] * r;
+      }
+    }
+  }
+  if (!stats) return;
+  rmax = block_max(rmax, red);
+  if (tid == 0) atomic_max_nonneg(&st[s].rmax_bits, rmax);
+  if (first) {
+    xmax = block_max(xmax, red);
+    if (tid == 0) atomic_max_nonneg(&st[s].xmax_bits, xmax);
+  }
+}
+
 // eta = max|R| / (||A||_inf max|X| + max|B|) per system; with decide, the
 // convergence / stall decision and the count of systems still refining.
 // A system is stalled when eta stops decreasing (or is NaN), or when the
@@ -365,8 +468,7 @@ cudaError_t launch_residual(const double* A, const double* B, const double* X, i
   const dim3 grid((unsigned)count, (unsigned)((n + kMixedRows - 1) / kMixedRows));
   if (nrhs == 1) k_residual<1><<<grid, MT, 0, s>>>(A, B, X, n, nrhs, rs, R32, rpos, R64, st, only_active, stats);
   else if (nrhs == 2) k_residual<2><<<grid, MT, 0, s>>>(A, B, X, n, nrhs, rs, R32, rpos, R64, st, only_active, stats);
-  else if (nrhs <= 4) k_residual<4><<<grid, MT, 0, s>>>(A, B, X, n, nrhs, rs, R32, rpos, R64, st, only_active, stats);
-  else k_residual<8><<<grid, MT, 0, s>>>(A, B, X, n, nrhs, rs, R32, rpos, R64, st, only_active, stats);
+  else k_residual_mma<<<grid, MT, 0, s>>>(A, B, X, n, nrhs, rs, R32, rpos, R64, st, only_active, stats);
   return cudaGetLastError();
 }
 }  // namespace

@@ -133,15 +133,15 @@ k_scale_rhs(const double* __restrict__ B, int n, int nrhs, const double* __restr
   __shared__ double red[MT / 32];
   const int s = blockIdx.x, tid = threadIdx.x;
   const int64_t nb = (int64_t)n * nrhs;
-  const double* b = B ? B + (int64_t)s * nb : nullptr;  // null: R = -A X (the product alone)
+  const double* b = B + (int64_t)s * nb;
   double m = 0.0;
-  for (int64_t idx = tid; idx < nb; idx += MT) {
+  for (int64_t idx = blockIdx.y * MT + tid; idx < nb; idx += (int64_t)gridDim.y * MT) {
     const double v = b[idx];
     m = fmax(m, fabs(v));
     B32[(int64_t)s * nb + idx] = (float)(rs[(int64_t)s * n + idx / nrhs] * v);
   }
   m = block_max(m, red);
-  if (tid == 0) st[s].bnorm = m;
+  if (tid == 0) atomic_max_nonneg(reinterpret_cast<unsigned long long*>(&st[s].bnorm), m);  // zero on entry
 }
 
 __global__ void __launch_bounds__(MT)
@@ -453,7 +453,9 @@ cudaError_t mixed_equil_scan(const double* A, int count, int n, int equil, doubl
 }
 cudaError_t mixed_scale_rhs(const double* B, int count, int n, int nrhs, const double* rs, float* B32,
                             RefineState* st, cudaStream_t s) {
-  k_scale_rhs<<<count, MT, 0, s>>>(B, n, nrhs, rs, B32, st);
+  // a few values per thread: a CTA a system left all but a few SMs idle (59 us at 5 systems of 3001 x 8)
+  const int64_t each = ((int64_t)n * nrhs + 4 * MT - 1) / (4 * MT);
+  k_scale_rhs<<<dim3((unsigned)count, (unsigned)(each < 64 ? each : 64)), MT, 0, s>>>(B, n, nrhs, rs, B32, st);
   return cudaGetLastError();
 }
 cudaError_t mixed_apply(double* X, const float* Y, const double* cs, int count, int n, int nrhs,

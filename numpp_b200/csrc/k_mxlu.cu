@@ -871,67 +871,74 @@ k_mx_gemm(const __grid_constant__ CUtensorMap mA1, const __grid_constant__ CUten
 // right-hand sides), C = 1, 2, 4 or 8. CTA r owns the 128-row blocks b with
 // b % C == r and keeps their right-hand sides in its shared memory. Block
 // step k: the owner computes y_k = D_k c_k (D_k the stored inverse of the
-// diagonal block), writes y_k into every CTA's shared memory (distributed
-// shared memory), and one cluster barrier publishes it; each CTA then
-// updates its own blocks, c_j -= M[block j][block k] y_k. y is
-// double-buffered: a CTA reaches step k's barrier only after finishing step
-// k-1's updates, so step k+1's owner may overwrite step k-1's buffer after it.
+// diagonal block) and writes y_k into every CTA's shared memory (distributed
+// shared memory); one cluster barrier publishes it; each CTA then updates its
+// own blocks, c_j -= M[block j][block k] y_k. The chain of steps bounds it, so
+// the owner of the next block updates that block first, solves it and arrives
+// at the barrier before its other updates; the rest of a step's updates run
+// between arrival and wait, beside the next owner's work. y has three buffers:
+// y_k's is written again with y_{k+3}, by an owner past the barrier of y_{k+2},
+// at which every CTA arrives with its updates by y_k done.
 constexpr int TS = 512;  // threads per CTA: 16 warps
 constexpr size_t kTrsv64Smem = 160 * 1024;  // shared-memory cap of the FP64-vector substitution
 
-// tmp[i][w] = sum_m D[i][m] y[m][w] for the block's 128 rows, 16 warps
-template <int W, class VT>
-__device__ __forceinline__ void block_apply16(const float* __restrict__ D, const VT* y, VT* tmp, int warp,
-                                              int lane) {
-  VT yv[4][W];
+// Sums v[0..NV) over the warp (NV a power of two, at most 32) by halving: at
+// every level a lane passes on the half it will not own, so NV sums take
+// NV - 1 + log2(32 / NV) shuffles instead of 5 NV. Lane l ends with the sum of
+// v[l / (32 / NV)].
+template <int NV, class VT>
+__device__ __forceinline__ VT warp_sums(VT (&v)[NV], int lane) {
+  int o = 16;
 #pragma unroll
-  for (int e = 0; e < 4; ++e)
+  for (int h = NV / 2; h >= 1; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int w = 0; w < W; ++w) yv[e][w] = y[(4 * lane + e) * W + w];
-#pragma unroll
-  for (int rr = 0; rr < 8; ++rr) {
-    const int i = warp + 16 * rr;
-    const float4 d = *reinterpret_cast<const float4*>(D + i * kMxNB + 4 * lane);
-    VT sum[W];
-#pragma unroll
-    for (int w = 0; w < W; ++w) sum[w] = d.x * yv[0][w] + d.y * yv[1][w] + d.z * yv[2][w] + d.w * yv[3][w];
-#pragma unroll
-    for (int o = 16; o; o >>= 1)
-#pragma unroll
-      for (int w = 0; w < W; ++w) sum[w] += __shfl_xor_sync(0xffffffffu, sum[w], o);
-    if (lane == 0)
-#pragma unroll
-      for (int w = 0; w < W; ++w) tmp[i * W + w] = sum[w];
+    for (int i = 0; i < h; ++i) {
+      const VT give = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
   }
+#pragma unroll
+  for (; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
 }
 
-// c[i] -= M[J + i][K:K+128] . y for the 128 rows of block J (local copy c), 16 warps
-template <int W, class VT>
-__device__ __forceinline__ void block_update16(const float* __restrict__ Ms, int N, int J, int K, const VT* y,
-                                               VT* c, int warp, int lane) {
+// One 128 x 128 block D (rows ld floats apart) times y (W columns of 128), 16 warps:
+// c = D y (SUB 0) or c -= D y (SUB 1). A warp takes the rows warp + 16 u, all
+// eight loads in flight before the sums, and sums G rows' W products at a time.
+// The sums over the lanes are what bounds it: one shuffle tree per row and
+// right-hand side (40 W shuffles a row group of eight) kept a substitution of 5
+// systems of order 3001 with 8 right-hand sides at 880 us; 401 us so, 201 us with the chain below.
+template <int W, int SUB, class VT>
+__device__ __forceinline__ void block_times16(const float* __restrict__ D, int64_t ld, const VT* y, VT* c, int warp,
+                                              int lane) {
+  constexpr int most = sizeof(VT) == 4 ? 32 : 8;  // sums held at a time, for the registers
+  constexpr int G = 8 * W <= most ? 8 : most / W;
   VT yv[4][W];
 #pragma unroll
   for (int e = 0; e < 4; ++e)
 #pragma unroll
-    for (int w = 0; w < W; ++w) yv[e][w] = y[(4 * lane + e) * W + w];
-  float4 m[8];  // rows warp + 16 u: all eight loads in flight before the sums
-#pragma unroll
-  for (int u = 0; u < 8; ++u)
-    m[u] = __ldcs(reinterpret_cast<const float4*>(Ms + (int64_t)(J + warp + 16 * u) * N + K + 4 * lane));
+    for (int w = 0; w < W; ++w) yv[e][w] = y[w * kMxNB + 4 * lane + e];
+  float4 m[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
-    const int i = warp + 16 * u;
-    VT sum[W];
+    const float4* p = reinterpret_cast<const float4*>(D + (int64_t)(warp + 16 * u) * ld + 4 * lane);
+    m[u] = SUB ? __ldcs(p) : *p;
+  }
 #pragma unroll
-    for (int w = 0; w < W; ++w)
-      sum[w] = m[u].x * yv[0][w] + m[u].y * yv[1][w] + m[u].z * yv[2][w] + m[u].w * yv[3][w];
+  for (int u0 = 0; u0 < 8; u0 += G) {
+    VT v[G * W];
 #pragma unroll
-    for (int o = 16; o; o >>= 1)
+    for (int u = 0; u < G; ++u)
 #pragma unroll
-      for (int w = 0; w < W; ++w) sum[w] += __shfl_xor_sync(0xffffffffu, sum[w], o);
-    if (lane == 0)
-#pragma unroll
-      for (int w = 0; w < W; ++w) c[i * W + w] -= sum[w];
+      for (int w = 0; w < W; ++w)
+        v[u * W + w] = m[u0 + u].x * yv[0][w] + m[u0 + u].y * yv[1][w] + m[u0 + u].z * yv[2][w] + m[u0 + u].w * yv[3][w];
+    const VT sum = warp_sums(v, lane);
+    constexpr int each = 32 / (G * W);  // lanes that hold the same sum
+    if (lane % each == 0) {
+      const int q = lane / each, at = (q % W) * kMxNB + warp + 16 * (u0 + q / W);
+      c[at] = SUB ? c[at] - sum : sum;
+    }
   }
 }
 
@@ -948,56 +955,66 @@ k_mx_trsv_c(const float* __restrict__ M, const float* __restrict__ Linv, const f
   if (only_active && st[s].status != kRefineActive) return;  // every CTA of the cluster: same system, same answer
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nb = N / kMxNB, nbl = (nb - rank + C - 1) / C;  // blocks this CTA owns
-  VT* cl = tsm;                                  // [nbl][128][W] owned right-hand sides
-  VT* yb = cl + (size_t)((nb + C - 1) / C) * kMxNB * W;  // [2][128][W] broadcast block solutions
-  VT* tmp = yb + 2 * kMxNB * W;                  // [128][W]
+  VT* cl = tsm;                                  // [nbl][W][128] owned right-hand sides
+  VT* yb = cl + (size_t)((nb + C - 1) / C) * kMxNB * W;  // [3][W][128] broadcast block solutions
+  VT* tmp = yb + 3 * kMxNB * W;                  // [W][128]
   const float* Ms = M + (int64_t)s * N * N;
   VT* Ys = Y + (int64_t)s * N * nrhs;
   for (int idx = tid; idx < nbl * kMxNB * W; idx += TS) {
-    const int lb = idx / (kMxNB * W), rem = idx % (kMxNB * W), i = (lb * C + rank) * kMxNB + rem / W, w = rem % W;
+    const int lb = idx / (kMxNB * W), rem = idx % (kMxNB * W), i = (lb * C + rank) * kMxNB + rem % kMxNB, w = rem / kMxNB;
     cl[idx] = c0 + w < nrhs ? Ys[(int64_t)i * nrhs + c0 + w] : VT(0);
   }
   const float* Ls = Linv + (int64_t)s * N * kMxNB;
   const float* Us = Uinv + (int64_t)s * N * kMxNB;
-  for (int pass = 0; pass < 2; ++pass) {  // L y = P c, then U x = y
-    for (int t = 0; t < nb; ++t) {
-      const int k = pass == 0 ? t : nb - 1 - t, K = k * kMxNB, buf = (pass * nb + t) & 1;
-      VT* yk = yb + buf * kMxNB * W;
-      __syncthreads();  // this CTA's updates of the previous step are in
-      if (k % C == rank) {
-        VT* ck = cl + (k / C) * kMxNB * W;
-        block_apply16<W, VT>((pass == 0 ? Ls : Us) + (int64_t)K * kMxNB, ck, tmp, warp, lane);
-        __syncthreads();
-        for (int q = 0; q < C; ++q) {
-          VT* dst = cluster.map_shared_rank(yk, q);
-          for (int idx = tid; idx < kMxNB * W; idx += TS) dst[idx] = tmp[idx];
-        }
-        for (int idx = tid; idx < kMxNB * W; idx += TS) ck[idx] = tmp[idx];
+  // steps 0 .. nb-1: L y = P c downwards; steps nb .. 2 nb - 1: U x = y upwards
+  auto block_of = [&](int q) { return q < nb ? q : 2 * nb - 1 - q; };
+  for (int q = -1; q + 1 < 2 * nb; ++q) {  // y of step q is in every CTA (q >= 0); step q + 1 is next
+    const bool up = q >= nb, next_up = q + 1 >= nb;
+    const int k = block_of(max(q, 0)), K = k * kMxNB, kn = block_of(q + 1);
+    const VT* yk = yb + (q + 3) % 3 * kMxNB * W;
+    if (kn % C == rank) {
+      VT* ck = cl + (kn / C) * kMxNB * W;
+      if (kn != k) block_times16<W, 1>(Ms + (int64_t)kn * kMxNB * N + K, N, yk, ck, warp, lane);
+      __syncthreads();
+      block_times16<W, 0>((next_up ? Us : Ls) + (int64_t)kn * kMxNB * kMxNB, kMxNB, ck, tmp, warp, lane);
+      __syncthreads();
+      VT* yn = yb + (q + 1) % 3 * kMxNB * W;
+      for (int p = 0; p < C; ++p) {
+        VT* dst = cluster.map_shared_rank(yn, p);
+        for (int idx = tid; idx < kMxNB * W; idx += TS) dst[idx] = tmp[idx];
       }
-      cluster.sync();  // y_k in every CTA
-      if (t + 1 < nb) {  // the next step's panel rows of this CTA's blocks into L2, behind this step's loads
-        const int kn = pass == 0 ? k + 1 : k - 1;
-        for (int idx = tid; idx < nbl * kMxNB * 4; idx += TS) {
-          const int lb = idx / (kMxNB * 4), j = lb * C + rank;
-          if (pass == 0 ? j > kn : j < kn) {
-            const int row = j * kMxNB + (idx / 4) % kMxNB;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(Ms + (int64_t)row * N + kn * kMxNB + 32 * (idx & 3)));
-          }
+      for (int idx = tid; idx < kMxNB * W; idx += TS) ck[idx] = tmp[idx];
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    if (q + 2 < 2 * nb) {  // into L2: the panel rows that step q + 1 reads, and the inverse behind it
+      for (int idx = tid; idx < nbl * kMxNB * 4; idx += TS) {
+        const int lb = idx / (kMxNB * 4), j = lb * C + rank;
+        if (next_up ? j < kn : j > kn) {
+          const int row = j * kMxNB + (idx / 4) % kMxNB;
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(Ms + (int64_t)row * N + kn * kMxNB + 32 * (idx & 3)));
         }
       }
+      const int k2 = block_of(q + 2);
+      if (k2 % C == rank)
+        for (int idx = tid; idx < kMxNB * 4; idx += TS)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"((q + 2 >= nb ? Us : Ls) + (int64_t)k2 * kMxNB * kMxNB + 32 * idx));
+    }
+    if (q >= 0) {
       for (int lb = 0; lb < nbl; ++lb) {
         const int j = lb * C + rank;
-        if (pass == 0 ? j > k : j < k)
-          block_update16<W, VT>(Ms, N, j * kMxNB, K, yk, cl + lb * kMxNB * W, warp, lane);
+        if (j != kn && (up ? j < k : j > k))
+          block_times16<W, 1>(Ms + (int64_t)j * kMxNB * N + K, N, yk, cl + lb * kMxNB * W, warp, lane);
       }
     }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   }
   __syncthreads();
   for (int idx = tid; idx < nbl * kMxNB * W; idx += TS) {
-    const int lb = idx / (kMxNB * W), rem = idx % (kMxNB * W), i = (lb * C + rank) * kMxNB + rem / W, w = rem % W;
+    const int lb = idx / (kMxNB * W), rem = idx % (kMxNB * W), i = (lb * C + rank) * kMxNB + rem % kMxNB, w = rem / kMxNB;
     if (c0 + w < nrhs) Ys[(int64_t)i * nrhs + c0 + w] = cl[idx];
   }
-  cluster.sync();  // no CTA leaves while a peer may still write into its shared memory
 }
 
 // Window k's row order applied to the rest of its rows (the row interchanges
@@ -1196,7 +1213,7 @@ cudaError_t mx_prepare() {
     e = cudaFuncSetAttribute(k_mx_permute, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPermSmem);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_mx_diag_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem);
-  const int csm = (int)(sizeof(float) * ((size_t)4096 * 8 + 3 * kMxNB * 8));
+  const int csm = (int)(sizeof(float) * ((size_t)4096 * 8 + 4 * kMxNB * 8));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mx_trsv_c<1, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, csm);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mx_trsv_c<2, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, csm);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mx_trsv_c<4, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, csm);
@@ -1411,7 +1428,7 @@ template <int W, class VT>
 cudaError_t launch_trsv_c(VT* Y, int nrhs, const RefineState* st, int only_active, const MxBufs& b, int C,
                           cudaStream_t s) {
   const int nb = b.N / kMxNB;
-  const size_t sm = sizeof(VT) * ((size_t)((nb + C - 1) / C) * kMxNB * W + 3 * kMxNB * W);
+  const size_t sm = sizeof(VT) * ((size_t)((nb + C - 1) / C) * kMxNB * W + 4 * kMxNB * W);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(b.count * C), (unsigned)((nrhs + W - 1) / W));
   cfg.blockDim = dim3(TS);
@@ -1429,8 +1446,14 @@ cudaError_t launch_trsv_c(VT* Y, int nrhs, const RefineState* st, int only_activ
 }
 
 cudaError_t mx_solve(float* Y, int nrhs, const RefineState* st, int only_active, const MxBufs& b, cudaStream_t s) {
-  const int W = nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : nrhs <= 4 ? 4 : 8;
+  int W = nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : nrhs <= 4 ? 4 : 8;
   const int C = trsv_cluster(b.count, (nrhs + W - 1) / W, b.N / kMxNB);
+  // SMs left over: smaller chunks, whose blocks' products are shorter (the factors
+  // are then read once per chunk, from L2 mostly)
+  int sms = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaGetLastError();
+  while (W > 1 && (int64_t)b.count * C * ((nrhs + W / 2 - 1) / (W / 2)) <= sms) W /= 2;
   switch (W) {
     case 1: return launch_trsv_c<1, float>(Y, nrhs, st, only_active, b, C, s);
     case 2: return launch_trsv_c<2, float>(Y, nrhs, st, only_active, b, C, s);
@@ -1446,7 +1469,7 @@ cudaError_t mx_solve64(double* Y, int nrhs, const RefineState* st, int only_acti
   const int nb = b.N / kMxNB;
   int W = nrhs <= 1 ? 1 : nrhs <= 2 ? 2 : 4;
   int C = trsv_cluster(b.count, (nrhs + W - 1) / W, nb);
-  while (W > 1 && sizeof(double) * ((size_t)((nb + C - 1) / C) * kMxNB * W + 3 * kMxNB * W) > kTrsv64Smem) {
+  while (W > 1 && sizeof(double) * ((size_t)((nb + C - 1) / C) * kMxNB * W + 4 * kMxNB * W) > kTrsv64Smem) {
     W >>= 1;
     C = trsv_cluster(b.count, (nrhs + W - 1) / W, nb);
   }

@@ -510,69 +510,68 @@ k_mx_diag(float* __restrict__ M, int32_t* __restrict__ perm, int32_t* __restrict
 // [U00 U01; 0 U11]^-1 = [U00^-1 -U00^-1 U01 U11^-1; 0 U11^-1], as 32^3 and
 // 64^3 shared-memory GEMMs (temporaries in the quadrants the results leave
 // zero, and at the last level in the factors' diagonal quadrants).
-constexpr size_t kInvSmem = sizeof(float) * 3 * kMxNB * DLD;
+// One CTA for L^-1 and one for U^-1 and U^-T (blockIdx.y): FP32 products of
+// one SM bound the pair (23 us a block with both in one CTA, 17 so).
+constexpr size_t kInvSmem = sizeof(float) * 2 * kMxNB * DLD;
 __global__ void __launch_bounds__(DT, 1)
 k_mx_diag_inv(const float* __restrict__ M, float* __restrict__ Linv, float* __restrict__ Uinv,
               float* __restrict__ UinvT, int N, int k) {
   extern __shared__ __align__(16) float ism[];
   float* LU = ism;                  // [128][DLD] the packed factors (position order)
-  float* Li = LU + kMxNB * DLD;     // [128][DLD] L^-1
-  float* Ui = Li + kMxNB * DLD;     // [128][DLD] U^-1
+  float* X = LU + kMxNB * DLD;      // [128][DLD] the inverse
   const int s = blockIdx.x, K = k * kMxNB, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool isL = blockIdx.y == 0;
   const float* Mb = M + (int64_t)s * N * N + (int64_t)K * N + K;
-#pragma unroll 4
+#pragma unroll 8
   for (int idx = tid; idx < kMxNB * 32; idx += DT) {
     const int r = idx >> 5, c = (idx & 31) * 4;
     *reinterpret_cast<float4*>(LU + r * DLD + c) = *reinterpret_cast<const float4*>(Mb + (int64_t)r * N + c);
   }
-  for (int idx = tid; idx < kMxNB * DLD; idx += DT) {
-    Li[idx] = 0.f;
-    Ui[idx] = 0.f;
+  for (int idx = tid; idx < kMxNB * DLD; idx += DT) X[idx] = 0.f;
+  __syncthreads();
+  // level 1: the four 32 x 32 diagonal blocks
+  if (warp < 4) {
+    if (isL) inv_lower32(LU, X, 32 * warp, lane);
+    else inv_upper32(LU, X, 32 * warp, lane);
   }
   __syncthreads();
-  // level 1: the eight 32 x 32 diagonal blocks
-  if (warp < 4) inv_lower32(LU, Li, 32 * warp, lane);
-  else inv_upper32(LU, Ui, 32 * (warp - 4), lane);
-  __syncthreads();
-  // level 2: 64 x 64 diagonal quadrants; four chains of 64 threads (one call
+  // level 2: 64 x 64 diagonal quadrants; two chains of 128 threads (one call
   // site per level in a rolled loop over the two products: compact code)
   {
-    const int ch = tid >> 6, t = tid & 63, p = ch & 1, o = 64 * p;
-    const bool isL = ch < 2;
-    float* tmp = isL ? Li + (32 * p) * DLD + 64   // temporaries in Li's upper-right quadrant
-                     : Ui + (64 + 32 * p) * DLD;  //   ... and Ui's lower-left quadrant
+    const int p = tid >> 7, t = tid & 127, o = 64 * p;
+    float* tmp = isL ? X + (32 * p) * DLD + 64   // temporaries in L^-1's upper-right quadrant
+                     : X + (64 + 32 * p) * DLD;  //   ... or U^-1's lower-left quadrant
 #pragma unroll 1
     for (int ph = 0; ph < 2; ++ph) {
       const float* A = ph == 0 ? (isL ? LU + (o + 32) * DLD + o : LU + o * DLD + o + 32)
-                               : (isL ? Li + (o + 32) * DLD + o + 32 : Ui + o * DLD + o);
-      const float* B = ph == 0 ? (isL ? Li + o * DLD + o : Ui + (o + 32) * DLD + o + 32) : tmp;
-      float* C = ph == 0 ? tmp : (isL ? Li + (o + 32) * DLD + o : Ui + o * DLD + o + 32);
-      sgemm<32, 4>(A, B, C, ph == 0 ? 1.f : -1.f, t);
+                               : (isL ? X + (o + 32) * DLD + o + 32 : X + o * DLD + o);
+      const float* B = ph == 0 ? (isL ? X + o * DLD + o : X + (o + 32) * DLD + o + 32) : tmp;
+      float* C = ph == 0 ? tmp : (isL ? X + (o + 32) * DLD + o : X + o * DLD + o + 32);
+      sgemm<32, 2>(A, B, C, ph == 0 ? 1.f : -1.f, t);
       __syncthreads();
     }
   }
-  // level 3: the off-diagonal quadrants; two chains of 128 threads, temporaries in LU's diagonal quadrants
-  {
-    const int ch = tid >> 7, t = tid & 127;
-    const bool isL = ch == 0;
-    float* tmp = isL ? LU : LU + 64 * DLD + 64;
+  // level 3: the off-diagonal quadrant, its temporary in LU's first diagonal quadrant
 #pragma unroll 1
-    for (int ph = 0; ph < 2; ++ph) {
-      const float* A = ph == 0 ? (isL ? LU + 64 * DLD : LU + 64) : (isL ? Li + 64 * DLD + 64 : Ui);
-      const float* B = ph == 0 ? (isL ? Li : Ui + 64 * DLD + 64) : tmp;
-      float* C = ph == 0 ? tmp : (isL ? Li + 64 * DLD : Ui + 64);
-      sgemm<64, 8>(A, B, C, ph == 0 ? 1.f : -1.f, t);
-      __syncthreads();
-    }
+  for (int ph = 0; ph < 2; ++ph) {
+    const float* A = ph == 0 ? (isL ? LU + 64 * DLD : LU + 64) : (isL ? X + 64 * DLD + 64 : X);
+    const float* B = ph == 0 ? (isL ? X : X + 64 * DLD + 64) : LU;
+    float* C = ph == 0 ? LU : (isL ? X + 64 * DLD : X + 64);
+    sgemm<64, 4>(A, B, C, ph == 0 ? 1.f : -1.f, tid);
+    __syncthreads();
   }
-  float* Lb = Linv + (int64_t)s * N * kMxNB + (int64_t)K * kMxNB;
-  float* Ub = Uinv + (int64_t)s * N * kMxNB + (int64_t)K * kMxNB;
-  float* UTb = UinvT + (int64_t)s * N * kMxNB + (int64_t)K * kMxNB;
-  for (int idx = tid; idx < kMxNB * kMxNB; idx += DT) {
-    const int r = idx >> 7, c = idx & 127;
-    Lb[idx] = c <= r ? Li[r * DLD + c] : 0.f;        // L^-1[r][c]
-    Ub[idx] = c >= r ? Ui[r * DLD + c] : 0.f;        // U^-1[r][c]
-    UTb[idx] = r >= c ? Ui[c * DLD + r] : 0.f;       // U^-T[r][c]
+  const int64_t at = (int64_t)s * N * kMxNB + (int64_t)K * kMxNB;
+  if (isL) {
+    for (int idx = tid; idx < kMxNB * kMxNB; idx += DT) {
+      const int r = idx >> 7, c = idx & 127;
+      Linv[at + idx] = c <= r ? X[r * DLD + c] : 0.f;  // L^-1[r][c]
+    }
+  } else {
+    for (int idx = tid; idx < kMxNB * kMxNB; idx += DT) {
+      const int r = idx >> 7, c = idx & 127;
+      Uinv[at + idx] = c >= r ? X[r * DLD + c] : 0.f;   // U^-1[r][c]
+      UinvT[at + idx] = r >= c ? X[c * DLD + r] : 0.f;  // U^-T[r][c]
+    }
   }
 }
 
@@ -1326,7 +1325,7 @@ cudaError_t mx_factor(const MxBufs& b, cudaStream_t s) {
       if ((e = cudaEventRecord(ms->ev[4], ps)) != cudaSuccess) return e;
       if ((e = cudaStreamWaitEvent(is, ms->ev[4], 0)) != cudaSuccess) return e;
     }
-    k_mx_diag_inv<<<count, DT, kInvSmem, is>>>(b.M, b.Linv, b.Uinv, b.UinvT, N, k);
+    k_mx_diag_inv<<<dim3((unsigned)count, 2), DT, kInvSmem, is>>>(b.M, b.Linv, b.Uinv, b.UinvT, N, k);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     k_mx_permute<<<dim3((unsigned)(N / PC), (unsigned)count), 256, kPermSmem, ps>>>(b.M, b.T, b.perm, N, k, count,
                                                                                    buf);

@@ -8,8 +8,8 @@
 //                  one quad of M.
 //  k_mx_diag       LU of the 256 x 128 window panel (the diagonal block's
 //                  rows and the next block's) with partial pivoting (one CTA,
-//                  the window in shared memory, 32-column panels with the
-//                  rows in registers, two per thread), then L^-1, U^-1 and U^-T of the block by
+//                  the window in shared memory, 32-column panels with a
+//                  row per thread in registers), then L^-1, U^-1 and U^-T of the block by
 //                  blocked inversion in shared memory, and the window's order.
 //  k_mx_permute    that order applied to the rest of the window's rows; the
 //                  new panel row transposed (A12^T).
@@ -164,10 +164,9 @@ k_mx_build(const double* __restrict__ A, const double* __restrict__ rs, const do
 // LU, in shared memory, blocked by 32-column panels. Rows never move: each
 // physical row of the block gets its position when it is chosen as a pivot
 // (pos_of / phys_of), so the multipliers left of a panel stay with their row
-// as in LAPACK's getrf. Panel p (columns 32p .. 32p+31) is factored by one
-// warp with the panel in registers (diag_panel: no block-wide barrier inside
-// a panel). After the panel: U12 = L11^-1 A12 over the panel's pivot rows
-// (thread = column), and A22 -= L21 U12 over the rows not yet chosen (4 x 4
+// as in LAPACK's getrf. Panel p (columns 32p .. 32p+31) is factored
+// with a row per thread in registers (diag_panel). After the panel: U12 = L11^-1 A12 over the panel's pivot rows
+// (thread = column), and A22 -= L21 U12 over the rows not yet chosen (8 x 4
 // register tiles).
 // The packed factors are then gathered into position order.
 // Inverses, from the packed factors: the eight 32 x 32 diagonal blocks of L
@@ -190,8 +189,10 @@ struct DiagAux {
   int phys_of[kMxWin];   // physical row of each position
   int act[kMxWin];       // rows not yet chosen, after a panel
   uint32_t keys[2][8];   // per warp: the key of its winner; two buffers (alternating steps)
-  float crow[2][8][32];  // per warp: its winner's panel values
-  float lcol[32][32];    // the panel's L11 columns below the diagonal (shifted to index 0)
+  float crow[2][8][8];   // per warp: its winner's values in the group's columns
+  float prow[8][32];     // the group's pivot rows when chosen, from the group's first column
+  float ug[8][24];       // their U values right of the group
+  float lcol[32][32];    // the panel's L11 columns (zeros above and on the diagonal)
   int fail;  // 1 + first position whose pivot failed, INT_MAX if none
 };
 constexpr size_t kDiagSmem = sizeof(float) * (kMxWin * DLD) + sizeof(DiagAux);
@@ -263,21 +264,20 @@ __device__ __forceinline__ void sgemm(const float* A, const float* B, float* C, 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ void st_shared_u32_if(bool c, uint32_t addr, uint32_t x) {
+// Predicated stores to shared memory: a divergent branch of one lane around
+// them costs several times their latency.
+__device__ __forceinline__ void publish_if(bool c, uint32_t addr, uint32_t x) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p st.shared.u32 [%1], %2;\n}\n" ::"r"((uint32_t)c),
       "r"(addr), "r"(x)
       : "memory");
 }
-// the 32 values v[0..31] to 128 bytes of shared memory at addr (16-byte aligned), if c
-__device__ __forceinline__ void st_shared_row_if(bool c, uint32_t addr, const float (&v)[32]) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q)
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p st.shared.v4.f32 [%1], {%2, %3, %4, %5};\n}\n" ::"r"(
-            (uint32_t)c),
-        "r"(addr + 16u * q), "f"(v[4 * q]), "f"(v[4 * q + 1]), "f"(v[4 * q + 2]), "f"(v[4 * q + 3])
-        : "memory");
+__device__ __forceinline__ void publish_row_if(bool c, uint32_t addr, const float* v) {  // 4 values
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p st.shared.v4.f32 [%1], {%2, %3, %4, %5};\n}\n" ::"r"(
+          (uint32_t)c),
+      "r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+      : "memory");
 }
 // 1 / x to about an ulp (the hardware approximation; subnormal x flushes to zero)
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -286,105 +286,133 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-// Panel of the LU (columns c0 .. c0+31) on warps 0-3: thread t owns the
-// physical rows t and t + 128 of the window (R rows), in a rolled loop over
-// the steps (the code stays small). At step j a row's 32 registers hold its
-// values in columns c0 + j .. c0 + j + 31 (shifted left by one every step
-// while the row is not chosen, so register indices are static). Step j: each
-// warp's largest key (magnitude with its 8 low mantissa bits dropped, plus
-// one) << 8 | (255 - row) over its rows not yet chosen by one warp reduction;
-// lane 0 publishes it and the owner of the warp's winner that row's values
-// (predicated stores); one barrier over the four warps; the overall winner
-// (the largest |a[j]| up to a relative 2^-15, the lowest row among those)
-// takes position c0 + j, and every row not yet chosen stores l = a[j] / pivot
-// and updates its values right of j. Keys and rows sit in two alternating
-// buffers, so one barrier per step suffices.
+// Panel of the LU (columns c0 .. c0+31) in groups of 8 columns: thread t owns
+// the physical row t of the window (R rows), its values from the group's first
+// column on in registers (shifted left by 8 after a group, in a rolled loop over
+// the groups, so the code stays small and register indices static). Step j of
+// a group: each warp's largest key (magnitude with its 8 low mantissa bits
+// dropped, plus one) << 8 | (255 - row) over its rows not yet chosen by one warp
+// reduction; lane 0 publishes it and the owner of the warp's winner that row's
+// values in the group (predicated stores); one barrier; the overall winner (the
+// largest |a[j]| up to a relative 2^-15, the lowest row among those) takes
+// position c0 + 8 gr + j, and every row not yet chosen takes l = a[j] / pivot
+// and updates its values of the group right of j. Keys and rows sit in two
+// alternating buffers, so one barrier per step suffices. After the group one warp
+// solves for its pivot rows' U right of it (lane = column) and every row not
+// yet chosen takes the group's rank-8 update: the same products in the same
+// order as step by step. What bounds a step is its chain of latencies and, with
+// all 32 columns in it, the eight broadcast reads of the pivot row by every
+// warp and some 130 instructions: 684 cycles a column so, 415 in groups (a window of
+// 256 x 128: 74 us before, 53 us).
 __device__ __forceinline__ void diag_panel(float* LU, DiagAux& ax, int c0, int t, int R) {
   constexpr unsigned FULL = 0xffffffffu;
   const int w = t >> 5, lane = t & 31;
-  bool was[2], done[2];
-  int jd[2] = {0, 0};  // step at which each row was chosen
-  int bad = INT_MAX;   // 1 + position of a row of this thread whose pivot failed
-  float v[2][32];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int r = t + 128 * h;
-    was[h] = r >= R || ax.pos_of[r] >= 0;  // rows past the window never compete
-    done[h] = was[h];
-    const float4* src = reinterpret_cast<const float4*>(LU + r * DLD + c0);
+  bool done = t >= R || ax.pos_of[t] >= 0;  // rows past the window never compete
+  float v[32];
+  {
+    const float4* src = reinterpret_cast<const float4*>(LU + t * DLD + c0);
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const float4 x = src[q];
-      v[h][4 * q] = x.x;
-      v[h][4 * q + 1] = x.y;
-      v[h][4 * q + 2] = x.z;
-      v[h][4 * q + 3] = x.w;
+      v[4 * q] = x.x;
+      v[4 * q + 1] = x.y;
+      v[4 * q + 2] = x.z;
+      v[4 * q + 3] = x.w;
     }
   }
+  const uint32_t row_key = 256u + 255u - (uint32_t)t;
 #pragma unroll 1
-  for (int j = 0; j < 32; ++j) {
-    const int b = j & 1;
-    uint32_t key = 0u;
+  for (int cg = c0; cg < c0 + 32; cg += 8) {
+    const bool was = done;
+    int jd = 0;  // step at which the row was chosen
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t kh =
-          done[h] ? 0u : ((((__float_as_uint(fabsf(v[h][0])) >> 8) + 1u) << 8) | (uint32_t)(255 - (t + 128 * h)));
-      key = max(key, kh);
-    }
-    const uint32_t wkey = __reduce_max_sync(FULL, key);
-    const int wrow = 255 - (int)(wkey & 255u);
-    // predicated stores, not a divergent branch (a one-lane branch around
-    // these stores costs several times their latency)
-    st_shared_u32_if(lane == 0, smem_addr(&ax.keys[b][w]), wkey);
-    st_shared_row_if(wkey != 0u && wrow == t, smem_addr(ax.crow[b][w]), v[0]);
-    st_shared_row_if(wkey != 0u && wrow == t + 128, smem_addr(ax.crow[b][w]), v[1]);
-    asm volatile("bar.sync 1, 128;\n" ::: "memory");
-    const uint4 kk = *reinterpret_cast<const uint4*>(ax.keys[b]);
-    const uint32_t best = max(max(kk.x, kk.y), max(kk.z, kk.w));
-    const int prow = 255 - (int)(best & 255u);
-    const float* pr = ax.crow[b][(prow & 127) >> 5];
-    // the winner's bookkeeping without a branch
+    for (int j = 0; j < 8; ++j) {
+      const int b = j & 1;
+      const uint32_t key = done ? 0u : (__float_as_uint(v[j]) & 0x7fffff00u) + row_key;
+      const uint32_t wkey = __reduce_max_sync(FULL, key);
+      // (a warp without rows left writes its slot too; its key of 0 never wins)
+      publish_if(lane == 0, smem_addr(&ax.keys[b][w]), wkey);
+      if (j < 4) publish_row_if(key == wkey, smem_addr(&ax.crow[b][w][0]), v);
+      publish_row_if(key == wkey, smem_addr(&ax.crow[b][w][4]), v + 4);
+      __syncthreads();
+      const uint4 ka = reinterpret_cast<const uint4*>(ax.keys[b])[0], kb = reinterpret_cast<const uint4*>(ax.keys[b])[1];
+      const uint32_t best = max(max(max(ka.x, ka.y), max(ka.z, ka.w)), max(max(kb.x, kb.y), max(kb.z, kb.w)));
+      // the winner's warp, as a byte offset: 32 (row / 32), row = 255 - (best & 255)
+      const float4* pr = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(ax.crow[b]) + (~best & 0xe0u));
+      float u[8];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const bool win = t + 128 * h == prow;
-      st_shared_u32_if(win, smem_addr(&ax.pos_of[t + 128 * h]), (uint32_t)(c0 + j));
-      st_shared_u32_if(win, smem_addr(&ax.phys_of[c0 + j]), (uint32_t)(t + 128 * h));
-      // the approximate reciprocal below flushes subnormals: such a pivot fails too
-      if (win && !(fabsf(v[h][0]) >= FLT_MIN && isfinite(v[h][0]))) bad = min(bad, c0 + j + 1);
-      jd[h] = win ? j : jd[h];
-      done[h] = done[h] || win;
-    }
-    if (!(done[0] && done[1])) {
-      const float rp = rcp_approx(pr[0]);
-      float u[32];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 x = reinterpret_cast<const float4*>(pr)[q];
+      for (int q = j / 4; q < 2; ++q) {
+        const float4 x = pr[q];
         u[4 * q] = x.x;
         u[4 * q + 1] = x.y;
         u[4 * q + 2] = x.z;
         u[4 * q + 3] = x.w;
       }
+      const bool win = key == best;
+      jd = win ? j : jd;
+      done = done || win;
+      // rows chosen take 0 times the pivot row: no branch, no selects
+      const float l = done ? 0.f : v[j] * rcp_approx(u[j]);
+      v[j] = done ? v[j] : l;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (!done[h]) {
-          const float l = v[h][0] * rp;
-          LU[(t + 128 * h) * DLD + c0 + j] = l;
+      for (int c = j + 1; c < 8; ++c) v[c] = fmaf(-l, u[c], v[c]);
+    }
+    if (!was) {  // the group's multipliers, or the packed row of a pivot
+      float4* dst = reinterpret_cast<float4*>(LU + t * DLD + cg);
+      dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+      dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+      if (done) {
+        ax.pos_of[t] = cg + jd;
+        ax.phys_of[cg + jd] = t;
+        float4* pd = reinterpret_cast<float4*>(ax.prow[jd]);
 #pragma unroll
-          for (int c = 0; c < 31; ++c) v[h][c] = fmaf(-l, u[c + 1], v[h][c + 1]);
-          v[h][31] = 0.f;
+        for (int q = 0; q < 8; ++q) pd[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      }
+    }
+    __syncthreads();
+    if (t < 8) {  // the approximate reciprocal flushes subnormals: such a pivot fails too
+      const float x = ax.prow[t][t];
+      if (!(fabsf(x) >= FLT_MIN && isfinite(x))) atomicMin(&ax.fail, cg + t + 1);
+    }
+    const int rest = c0 + 24 - cg;  // columns of the panel right of the group
+    if (rest == 0) break;
+    if (t < rest) {
+      float a[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] = ax.prow[j][8 + t];
+#pragma unroll
+      for (int j = 1; j < 8; ++j)
+#pragma unroll
+        for (int i = 0; i < j; ++i) a[j] = fmaf(-ax.prow[j][i], a[i], a[j]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        ax.ug[j][t] = a[j];
+        LU[ax.phys_of[cg + j] * DLD + cg + 8 + t] = a[j];
+      }
+    }
+    __syncthreads();
+    if (!done) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        if (8 * q < rest) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float4 x = *reinterpret_cast<const float4*>(&ax.ug[j][8 * q]);
+            const float4 y = *reinterpret_cast<const float4*>(&ax.ug[j][8 * q + 4]);
+            v[8 + 8 * q] = fmaf(-v[j], x.x, v[8 + 8 * q]);
+            v[9 + 8 * q] = fmaf(-v[j], x.y, v[9 + 8 * q]);
+            v[10 + 8 * q] = fmaf(-v[j], x.z, v[10 + 8 * q]);
+            v[11 + 8 * q] = fmaf(-v[j], x.w, v[11 + 8 * q]);
+            v[12 + 8 * q] = fmaf(-v[j], y.x, v[12 + 8 * q]);
+            v[13 + 8 * q] = fmaf(-v[j], y.y, v[13 + 8 * q]);
+            v[14 + 8 * q] = fmaf(-v[j], y.z, v[14 + 8 * q]);
+            v[15 + 8 * q] = fmaf(-v[j], y.w, v[15 + 8 * q]);
+          }
         }
       }
     }
-  }
-  if (bad != INT_MAX) atomicMin(&ax.fail, bad);
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    if (done[h] && !was[h]) {  // the row's U values, columns c0 + jd .. c0 + 31
-#pragma unroll
-      for (int c = 0; c < 32; ++c)
-        if (c < 32 - jd[h]) LU[(t + 128 * h) * DLD + c0 + jd[h] + c] = v[h][c];
-    }
+    for (int c = 0; c < 24; ++c) v[c] = v[c + 8];
   }
 }
 
@@ -408,41 +436,35 @@ k_mx_diag(float* __restrict__ M, int32_t* __restrict__ perm, int32_t* __restrict
 #pragma unroll 1
   for (int p = 0; p < 4; ++p) {
     const int c0 = 32 * p;
-    if (warp < 4) diag_panel(W0, ax, c0, tid, R);
+    diag_panel(W0, ax, c0, tid, R);
     __syncthreads();
     const int W = kMxNB - c0 - 32;  // trailing columns of the block
     const int Rn = R - c0 - 32;     // rows not yet chosen
     if (tid < W) {
-      // U12 = L11^-1 A12 on the panel's pivot rows, thread = column, in a
-      // rolled loop: v[i] holds position c0 + j + i at step j (shifted like
-      // the panel); the columns of L11 below the diagonal are staged first,
-      // shifted: lcol[j][i] = L(c0 + j + 1 + i, c0 + j)
+      // U12 = L11^-1 A12 on the panel's pivot rows, thread = column; the columns
+      // of L11 are staged first
       for (int idx = tid; idx < 32 * 32; idx += W) {
         const int j = idx >> 5, i = idx & 31;
-        ax.lcol[j][i] = i < 31 - j ? W0[ax.phys_of[c0 + j + 1 + i] * DLD + c0 + j] : 0.f;
+        ax.lcol[j][i] = i > j ? W0[ax.phys_of[c0 + i] * DLD + c0 + j] : 0.f;
       }
       asm volatile("bar.sync 2, %0;\n" ::"r"(W) : "memory");
       const int c = c0 + 32 + tid;
       float v[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = W0[ax.phys_of[c0 + j] * DLD + c];
-#pragma unroll 1
+#pragma unroll
       for (int j = 0; j < 31; ++j) {
-        const float x = v[0];
-        W0[ax.phys_of[c0 + j] * DLD + c] = x;
-        float lc[32];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 y = reinterpret_cast<const float4*>(ax.lcol[j])[q];
-          lc[4 * q] = y.x;
-          lc[4 * q + 1] = y.y;
-          lc[4 * q + 2] = y.z;
-          lc[4 * q + 3] = y.w;
+        for (int q = (j + 1) / 4; q < 8; ++q) {  // entries up to j are zero
+          const float4 y = *reinterpret_cast<const float4*>(&ax.lcol[j][4 * q]);
+          if (4 * q > j) v[4 * q] = fmaf(-y.x, v[j], v[4 * q]);
+          if (4 * q + 1 > j) v[4 * q + 1] = fmaf(-y.y, v[j], v[4 * q + 1]);
+          if (4 * q + 2 > j) v[4 * q + 2] = fmaf(-y.z, v[j], v[4 * q + 2]);
+          if (4 * q + 3 > j) v[4 * q + 3] = fmaf(-y.w, v[j], v[4 * q + 3]);
         }
-#pragma unroll
-        for (int i = 0; i < 31; ++i) v[i] = fmaf(-lc[i], x, v[i + 1]);
       }
-      W0[ax.phys_of[c0 + 31] * DLD + c] = v[0];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) W0[ax.phys_of[c0 + j] * DLD + c] = v[j];
     } else if (warp == 4) {
       // the rows not yet chosen, in physical order (also after the last panel:
       // the window's rows that stay below the block)
@@ -458,32 +480,39 @@ k_mx_diag(float* __restrict__ M, int32_t* __restrict__ perm, int32_t* __restrict
     }
     __syncthreads();
     if (p == 3) break;
-    // A22 -= L21 U12: 4 rows (of act) x 4 columns per task
+    // A22 -= L21 U12: 8 rows (of act) x 4 columns per task (R - c0 is a multiple
+    // of 32); 4 rows x 4 columns read 1.3 times as many operands per product
     {
-      const int ngc = W >> 2, ntask = (Rn >> 2) * ngc;
+      const int ngc = W >> 2, ntask = (Rn >> 3) * ngc;
       for (int task = tid; task < ntask; task += DT) {
         const int rg = task / ngc, cc = c0 + 32 + 4 * (task - rg * ngc);
-        float* rp[4];
-        float4 acc[4];
+        float* rp[8];
+        float4 acc[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          rp[i] = W0 + ax.act[4 * rg + i] * DLD;
+        for (int i = 0; i < 8; ++i) {
+          rp[i] = W0 + ax.act[8 * rg + i] * DLD;
           acc[i] = *reinterpret_cast<const float4*>(rp[i] + cc);
         }
-#pragma unroll 8
-        for (int m = 0; m < 32; ++m) {
-          const float4 u = *reinterpret_cast<const float4*>(W0 + ax.phys_of[c0 + m] * DLD + cc);
+#pragma unroll 2
+        for (int m = 0; m < 32; m += 4) {
+          float4 u[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float l = rp[i][c0 + m];
-            acc[i].x = fmaf(-l, u.x, acc[i].x);
-            acc[i].y = fmaf(-l, u.y, acc[i].y);
-            acc[i].z = fmaf(-l, u.z, acc[i].z);
-            acc[i].w = fmaf(-l, u.w, acc[i].w);
+          for (int q = 0; q < 4; ++q) u[q] = *reinterpret_cast<const float4*>(W0 + ax.phys_of[c0 + m + q] * DLD + cc);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 l4 = *reinterpret_cast<const float4*>(rp[i] + c0 + m);
+            const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              acc[i].x = fmaf(-l[q], u[q].x, acc[i].x);
+              acc[i].y = fmaf(-l[q], u[q].y, acc[i].y);
+              acc[i].z = fmaf(-l[q], u[q].z, acc[i].z);
+              acc[i].w = fmaf(-l[q], u[q].w, acc[i].w);
+            }
           }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(rp[i] + cc) = acc[i];
+        for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(rp[i] + cc) = acc[i];
       }
     }
     __syncthreads();

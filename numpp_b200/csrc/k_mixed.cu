@@ -429,6 +429,14 @@ k_row_positions(const int32_t* __restrict__ ipiv, int n, int32_t* __restrict__ r
   for (int q = threadIdx.x; q < n; q += MT) rpos[(int64_t)s * n + prm[q]] = q;
 }
 
+__global__ void k_export(const RefineState* __restrict__ st, int count, int refined, double* __restrict__ berr,
+                         int32_t* __restrict__ iters) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= count) return;
+  if (berr) berr[s] = st[s].eta;
+  if (iters) iters[s] = refined ? st[s].iters : 0;
+}
+
 __global__ void k_mark_fp32_failures(const int32_t* __restrict__ info32, RefineState* __restrict__ st, int count) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < count && info32[s]) st[s].status = kRefineStalled;
@@ -494,6 +502,12 @@ cudaError_t mixed_ferr(const double* X, const double* Xt, int count, int n, int 
 }
 cudaError_t mixed_row_positions(const int32_t* ipiv, int count, int n, int32_t* rpos, cudaStream_t s) {
   k_row_positions<<<count, MT, 2 * sizeof(int) * (size_t)n, s>>>(ipiv, n, rpos);
+  return cudaGetLastError();
+}
+cudaError_t mixed_export(const RefineState* st, int count, int refined, double* berr, int32_t* iters,
+                         cudaStream_t s) {
+  if (!berr && !iters) return cudaSuccess;
+  k_export<<<(count + 255) / 256, 256, 0, s>>>(st, count, refined, berr, iters);
   return cudaGetLastError();
 }
 cudaError_t mixed_mark_fp32_failures(const int32_t* info32, RefineState* st, int count, cudaStream_t s) {

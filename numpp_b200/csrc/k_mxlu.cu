@@ -1278,6 +1278,10 @@ cudaError_t mx_prepare() {
   return e;
 }
 
+cudaError_t mx_timeouts_read(int* d, cudaStream_t s) {
+  return cudaMemcpyFromSymbolAsync(d, g_mx_timeouts, sizeof(int), 0, cudaMemcpyDeviceToDevice, s);
+}
+
 int mx_timeouts_take() {
   int v = 0;
   if (cudaMemcpyFromSymbol(&v, g_mx_timeouts, sizeof(int)) != cudaSuccess) return -1;

@@ -105,7 +105,7 @@ int mixed(int64_t count64, int32_t n, int32_t nrhs, const double* dA, const doub
   NPPB_CUDA(cudaMemsetAsync(cmx.as<void>(), 0, sizeof(double) * c * n, st), "memset");
   NPPB_CUDA(cudaMemsetAsync(stm.as<void>(), 0, sizeof(RefineState) * c, st), "memset");
   NPPB_CUDA(info32.alloc(sizeof(int32_t) * c, st), "workspace");
-  NPPB_CUDA(act.alloc(sizeof(int), st), "workspace");
+  NPPB_CUDA(act.alloc(2 * sizeof(int), st), "workspace");
   RefineState* S = stm.as<RefineState>();
   const bool equil = !(flags & NPPB_MIXED_NO_EQUILIBRATE);
   if (blocked) {
@@ -127,17 +127,25 @@ int mixed(int64_t count64, int32_t n, int32_t nrhs, const double* dA, const doub
     NPPB_CUDA(mx_build(dA, rsm.as<double>(), cmx.as<double>(), equil ? 1 : 0, csm.as<double>(), S, mb, st),
               "butterfly transform");
     NPPB_CUDA(mx_factor(mb, st), "FP32 block factorisation");
-    NPPB_CUDA(cudaStreamSynchronize(st), "synchronize");
-    if (mx_timeouts_take() != 0) {
-      set_error("tensor-core block factorisation: a completion wait ran out");
-      return NPPB_E_CUDA;
-    }
+    NPPB_CUDA(mx_timeouts_read(act.as<int>() + 1, st), "readback");
     NPPB_CUDA(mixed_mark_fp32_failures(mb.info, S, count, st), "mark");
     float* Y = y32.as<float>();
     NPPB_CUDA(mx_rhs_in(b32.as<float>(), Y, nrhs, S, 0, mb, st), "transform rhs");
     NPPB_CUDA(mx_solve(Y, nrhs, S, 0, mb, st), "FP32 solve");
     NPPB_CUDA(mx_apply(Y, dX, csm.as<double>(), nrhs, S, 1, mb, st), "apply");
-    int h_act = 0;
+    int h_act[2] = {0, 0};  // systems still refining; waits of the factorisation that ran out
+    // both counts in one readback: the factorisation's is looked at behind the first residual,
+    // so that the host does not wait for the factorisation by itself
+    auto read_active = [&](int it) -> int {
+      NPPB_CUDA(cudaMemcpyAsync(h_act, act.as<int>(), sizeof(h_act), cudaMemcpyDeviceToHost, st), "readback");
+      NPPB_CUDA(cudaStreamSynchronize(st), "synchronize");
+      if (it == 0 && h_act[1] != 0) {
+        mx_timeouts_take();
+        set_error("tensor-core block factorisation: a completion wait ran out");
+        return NPPB_E_CUDA;
+      }
+      return NPPB_OK;
+    };
     if (!gmres) {
       for (int it = 0;; ++it) {
         NPPB_CUDA(cudaMemsetAsync(act.as<int>(), 0, sizeof(int), st), "memset");
@@ -145,9 +153,8 @@ int mixed(int64_t count64, int32_t n, int32_t nrhs, const double* dA, const doub
         NPPB_CUDA(mixed_residual(dA, dB, dX, count, n, nrhs, rsm.as<double>(), b32.as<float>(), nullptr, S, tol,
                                  it, max_iter, 1, act.as<int>(), st),
                   "residual");
-        NPPB_CUDA(cudaMemcpyAsync(&h_act, act.as<int>(), sizeof(int), cudaMemcpyDeviceToHost, st), "readback");
-        NPPB_CUDA(cudaStreamSynchronize(st), "synchronize");
-        if (h_act == 0 || it >= max_iter) break;
+        NPPB_RC(read_active(it));
+        if (h_act[0] == 0 || it >= max_iter) break;
         NPPB_CUDA(mx_rhs_in(b32.as<float>(), Y, nrhs, S, 1, mb, st), "transform residual");
         NPPB_CUDA(mx_solve(Y, nrhs, S, 1, mb, st), "FP32 correction solve");
         NPPB_CUDA(mx_apply(Y, dX, csm.as<double>(), nrhs, S, 0, mb, st), "apply");
@@ -175,9 +182,8 @@ int mixed(int64_t count64, int32_t n, int32_t nrhs, const double* dA, const doub
         NPPB_CUDA(mixed_residual(dA, dB, dX, count, n, nrhs, rsm.as<double>(), nullptr, nullptr, S, tol, it,
                                  max_iter, 1, act.as<int>(), st, gR.as<double>()),
                   "residual");
-        NPPB_CUDA(cudaMemcpyAsync(&h_act, act.as<int>(), sizeof(int), cudaMemcpyDeviceToHost, st), "readback");
-        NPPB_CUDA(cudaStreamSynchronize(st), "synchronize");
-        if (h_act == 0 || it >= max_iter) break;
+        NPPB_RC(read_active(it));
+        if (h_act[0] == 0 || it >= max_iter) break;
         NPPB_RC(precond(gR.as<double>(), gW.as<double>()));
         NPPB_CUDA(gm_start(gW.as<double>(), V, gS.as<GmState>(), S, count, n, nrhs, st), "GMRES start");
         for (int k = 0; k < kGmM; ++k) {
@@ -301,19 +307,15 @@ int mixed(int64_t count64, int32_t n, int32_t nrhs, const double* dA, const doub
                              0, act.as<int>(), st),
               "residual");
   if (dFerr && dXtrue) NPPB_CUDA(mixed_ferr(dX, dXtrue, count, n, nrhs, dFerr, st), "forward error");
-  NPPB_CUDA(cudaMemcpyAsync(hs.data(), S, sizeof(RefineState) * c, cudaMemcpyDeviceToHost, st), "readback");
-  NPPB_CUDA(cudaStreamSynchronize(st), "synchronize");
-  std::vector<double> berr(c);
-  std::vector<int32_t> iters(c);
-  for (size_t s = 0; s < c; ++s) {
-    berr[s] = hs[s].eta;
-    iters[s] = n > 32 ? hs[s].iters : 0;
+  NPPB_CUDA(mixed_export(S, count, n > 32 ? 1 : 0, dBerr, dIters, st), "write");
+  if (any_fallback) {
+    if (dFallback)
+      NPPB_CUDA(cudaMemcpyAsync(dFallback, fallback.data(), sizeof(int32_t) * c, cudaMemcpyHostToDevice, st), "write");
+    if (dinfo) NPPB_CUDA(cudaMemcpyAsync(dinfo, hinfo.data(), sizeof(int32_t) * c, cudaMemcpyHostToDevice, st), "write");
+  } else {
+    if (dFallback) NPPB_CUDA(cudaMemsetAsync(dFallback, 0, sizeof(int32_t) * c, st), "write");
+    if (dinfo) NPPB_CUDA(cudaMemsetAsync(dinfo, 0, sizeof(int32_t) * c, st), "write");
   }
-  if (dBerr) NPPB_CUDA(cudaMemcpyAsync(dBerr, berr.data(), sizeof(double) * c, cudaMemcpyHostToDevice, st), "write");
-  if (dIters) NPPB_CUDA(cudaMemcpyAsync(dIters, iters.data(), sizeof(int32_t) * c, cudaMemcpyHostToDevice, st), "write");
-  if (dFallback)
-    NPPB_CUDA(cudaMemcpyAsync(dFallback, fallback.data(), sizeof(int32_t) * c, cudaMemcpyHostToDevice, st), "write");
-  if (dinfo) NPPB_CUDA(cudaMemcpyAsync(dinfo, hinfo.data(), sizeof(int32_t) * c, cudaMemcpyHostToDevice, st), "write");
   NPPB_CUDA(cudaStreamSynchronize(st), "synchronize");
   return NPPB_OK;
 }

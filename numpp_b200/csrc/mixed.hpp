@@ -52,6 +52,9 @@ cudaError_t mixed_matvec(const double* A, const double* X, int count, int n, int
 cudaError_t mixed_row_positions(const int32_t* ipiv, int count, int n, int32_t* rpos, cudaStream_t s);
 cudaError_t mixed_ferr(const double* X, const double* Xt, int count, int n, int nrhs, double* ferr,
                        cudaStream_t s);
+// berr / iters (either may be null) of every system from its state; refined = 0: no corrections to report.
+cudaError_t mixed_export(const RefineState* st, int count, int refined, double* berr, int32_t* iters,
+                         cudaStream_t s);
 cudaError_t mixed_mark_fp32_failures(const int32_t* info32, RefineState* st, int count, cudaStream_t s);
 
 }  // namespace nppb

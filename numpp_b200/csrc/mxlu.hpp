@@ -90,6 +90,8 @@ cudaError_t mx_apply64(const double* Y, double* X, const double* cs, int nrhs, c
 // Bounded waits of the GEMM kernel that ran out since the last call (each
 // such CTA skipped its stores); the counter is reset. -1: unreadable.
 int mx_timeouts_take();
+// The same count to *d (device) in stream order, without a reset.
+cudaError_t mx_timeouts_read(int* d, cudaStream_t s);
 // One-time kernel attribute setup (dynamic shared memory opt-in).
 cudaError_t mx_prepare();
 

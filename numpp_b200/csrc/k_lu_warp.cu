@@ -17,7 +17,8 @@
 // The same launch finishes the requested outputs:
 //  * det  = permsign * prod U[i,i] in order i = 0..n-1   (linalg.cpp:393-407)
 //  * slogdet sign / sum log|U[i,i]| in order               (linalg.cpp:408-439)
-//  * X = A^-1 B: X[pos(r)] starts as B[r]; forward (unit L) and back (U)
+//  * X = A^-1 B: X[pos(r)] starts as B[r]; forward (unit L; the first RC columns
+//    during the elimination) and back (U)
 //    substitution run across lanes, up to RC columns at a time (linalg.cpp:73-90)
 //  * inverse = the same solve against I                    (linalg.cpp:105-115)
 //  * LU + ipiv (LAPACK-style swap list, 0-based) for getrf.
@@ -70,50 +71,85 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
   // Original row index held by each position, for getrs from stored factors.
   int orig = lane;
 
+  // the first right-hand sides ride along with the elimination (their forward substitution)
+  const bool ride = (flags & kWantSolve) && !(flags & kSolveOnly);
+  double x0[RC];
+#pragma unroll
+  for (int c = 0; c < RC; ++c)
+    x0[c] = ride && live && c < v.nrhs ? v.B[(int64_t)lane * v.nrhs + c] : 0.0;
+
   if (!(flags & kSolveOnly)) {
-    const bool nopiv = flags & kNoPivot;
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
-      const bool cand = live && (nopiv ? pos == k : pos >= k);
+      const bool cand = live && pos >= k;
       const double akk = live ? row[k] : 0.0;
-      // without pivoting the diagonal is the only candidate; <= 0 counts as a zero pivot
-      const double mag = cand ? (nopiv ? (akk > 0.0 ? akk : 0.0) : fabs(akk)) : 0.0;
-      const unsigned long long bits = (mag == mag) ? (unsigned long long)__double_as_longlong(mag) : 0ull;
-      const uint32_t hi = (uint32_t)(bits >> 32), lo = (uint32_t)bits;
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(akk) & 0x7fffffffffffffffull;
+      const bool number = cand && bits <= 0x7ff0000000000000ull;  // NaN entries are no candidates
+      const uint32_t hi = number ? (uint32_t)(bits >> 32) : 0u, lo = number ? (uint32_t)bits : 0u;
       const uint32_t mhi = __reduce_max_sync(kFull, hi);
-      const uint32_t mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
-      if ((mhi | mlo) == 0u) {  // no nonzero candidate: singular
-        info = k + 1;
-        break;
+      unsigned tops = __ballot_sync(kFull, number && hi == mhi);
+      int pl = __ffs(tops) - 1, key;
+      if (mhi != 0u && (tops & (tops - 1u)) == 0u) {  // one lane holds the largest high word
+        key = __shfl_sync(kFull, pos, pl);
+      } else {
+        const uint32_t mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
+        if ((mhi | mlo) == 0u) {  // no nonzero candidate: singular
+          info = k + 1;
+          break;
+        }
+        const bool top = number && hi == mhi && lo == mlo;
+        key = (int)__reduce_min_sync(kFull, top ? (uint32_t)pos : 0xffffffffu);
+        pl = __ffs(__ballot_sync(kFull, live && pos == key)) - 1;
       }
-      const bool top = cand && hi == mhi && lo == mlo;
-      const int key = (int)__reduce_min_sync(kFull, top ? (uint32_t)pos : 0xffffffffu);
-      const int pl = __ffs(__ballot_sync(kFull, live && pos == key)) - 1;
-      const int kl = __ffs(__ballot_sync(kFull, live && pos == k)) - 1;
       if (key != k) {
-        if (lane == pl) pos = k;
-        else if (lane == kl) pos = key;
+        pos = lane == pl ? k : live && pos == k ? key : pos;
         ++nswap;
+      } else if (lane == pl) {
+        pos = k;
       }
       if ((flags & kWantLU) && lane == 0) v.ipiv[k] = key;
       const double* prow = R + pl * kLd;
       const double pk = prow[k];
       if (lane == pl) dg = pk;
-      if (live && pos > k) {
-        const double f = row[k] / pk;
+      const bool below = live && pos > k;
+      const double f = below ? akk / pk : 0.0;
+      if (ride) {
+#pragma unroll
+        for (int c = 0; c < RC; ++c)
+          if (c < v.nrhs) {
+            const double xk = __shfl_sync(kFull, x0[c], pl);
+            const double t = fma(-f, xk, x0[c]);
+            x0[c] = below ? t : x0[c];
+          }
+      }
+      if (below) {
         row[k] = f;
-        // 16-byte pieces (rows start 16-byte aligned); the piece holding column k
-        // keeps it, columns past n are padding
+        // eight columns at a time, both rows' pieces loaded before the first store (a
+        // store to the tile holds back every later load of it: 78 cycles a 16-byte
+        // piece one by one, of 1500 for a step); columns up to k keep their multipliers,
+        // columns past n are padding
         double2* r2 = reinterpret_cast<double2*>(row);
         const double2* p2 = reinterpret_cast<const double2*>(prow);
-#pragma unroll 4
-        for (int q = (k + 1) >> 1; q < (n + 1) >> 1; ++q) {
-          const double2 pv = p2[q];
-          double2 rv = r2[q];
-          if (2 * q > k) rv.x = fma(-f, pv.x, rv.x);
-          rv.y = fma(-f, pv.y, rv.y);
-          r2[q] = rv;
-        }
+        auto piece = [&](int q, bool edge) {
+          double2 pv[4], rv[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            pv[i] = p2[q + i];
+            rv[i] = r2[q + i];
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const double tx = fma(-f, pv[i].x, rv[i].x), ty = fma(-f, pv[i].y, rv[i].y);
+            rv[i].x = !edge || 2 * (q + i) > k ? tx : rv[i].x;
+            rv[i].y = !edge || 2 * (q + i) + 1 > k ? ty : rv[i].y;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) r2[q + i] = rv[i];
+        };
+        int q = (k + 1) >> 3 << 2;
+        if (2 * q < n) piece(q, true);
+#pragma unroll 1
+        for (q += 4; 2 * q < n; q += 4) piece(q, false);
       }
       __syncwarp();
     }
@@ -152,19 +188,20 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
     double* dgs = R + 32;  // column 32 of the tile: rows 0..n-1 hold the pivot of position r
     if (live) {
       dgs[pos * kLd] = dg;
-      dgs[pos * kLd + 1] = log(fabs(dg));  // column 33
+      if (flags & kWantSlogdet) dgs[pos * kLd + 1] = log(fabs(dg));  // column 33
     }
     __syncwarp();
     double det = (nswap & 1) ? -1.0 : 1.0;
-    double sgn = det;
     double logabs = 0.0;
+    // d / |d| is exactly +-1 for finite nonzero d, NaN otherwise
+    const unsigned minus = __ballot_sync(kFull, live && dg < 0.0);
+    const bool finite = __all_sync(kFull, !live || isfinite(dg));
+    const double sgn = !finite ? (double)NAN : (__popc(minus) & 1) ? -det : det;
     if (info == 0 && lane == 0) {
+#pragma unroll 8
       for (int i = 0; i < n; ++i) {
-        const double di = dgs[i * kLd], li = dgs[i * kLd + 1];
-        det *= di;
-        logabs += li;
-        // d / |d| is exactly +-1 for finite nonzero d, NaN otherwise
-        sgn = isfinite(di) ? (di < 0.0 ? -sgn : sgn) : NAN;
+        det *= dgs[i * kLd];
+        if (flags & kWantSlogdet) logabs += dgs[i * kLd + 1];
       }
     }
     if (lane == 0) {
@@ -188,49 +225,56 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
     for (int c0 = 0; c0 < ncols; c0 += RC) {
       const int nc = min(RC, ncols - c0);  // columns of this chunk (warp-uniform)
       double x[RC];
+      if (ride && !is_inv && c0 == 0) {
 #pragma unroll
-      for (int c = 0; c < RC; ++c) {
-        const int col = c0 + c;
-        double b = 0.0;
-        if (live && c < nc) {
-          if (is_inv) b = (orig == col) ? 1.0 : 0.0;
-          else b = v.B[(int64_t)orig * ncols + col];
-        }
-        x[c] = b;
-      }
-      __syncwarp();  // every lane has read its right-hand side before any lane writes X (getrs in place)
-      // forward: unit lower, position order
-#pragma unroll 1
-      for (int k = 0; k < n; ++k) {
-        const int l = lop[k];
-        const bool below = live && pos > k;
-        const double lk = below ? row[k] : 0.0;
+        for (int c = 0; c < RC; ++c) x[c] = x0[c];
+        __syncwarp();  // every lane has read its right-hand side before any lane writes X
+      } else {
 #pragma unroll
         for (int c = 0; c < RC; ++c) {
-          if (c < nc) {
-            const double xk = __shfl_sync(kFull, x[c], l);
-            if (below) x[c] = fma(-lk, xk, x[c]);
+          const int col = c0 + c;
+          double b = 0.0;
+          if (live && c < nc) {
+            if (is_inv) b = (orig == col) ? 1.0 : 0.0;
+            else b = v.B[(int64_t)orig * ncols + col];
+          }
+          x[c] = b;
+        }
+        __syncwarp();  // every lane has read its right-hand side before any lane writes X (getrs in place)
+        // forward: unit lower, position order
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+          const int l = lop[k];
+          const bool below = live && pos > k;
+          const double lk = below ? row[k] : 0.0;
+#pragma unroll
+          for (int c = 0; c < RC; ++c) {
+            if (c < nc) {
+              const double xk = __shfl_sync(kFull, x[c], l);
+              const double t = fma(-lk, xk, x[c]);
+              x[c] = below ? t : x[c];
+            }
           }
         }
       }
-      // back: upper, multiply by the diagonal's reciprocal when the row is final
-#pragma unroll 1
+      // back: upper; a row is multiplied by the diagonal's reciprocal when it is final
+      // (every lane forms the product, the final row's is passed on: no branch)
+#pragma unroll 4
       for (int k = n - 1; k >= 0; --k) {
         const int l = lop[k];
-        if (lane == l) {
-#pragma unroll
-          for (int c = 0; c < RC; ++c) x[c] *= rdg;
-        }
         const bool above = live && pos < k;
         const double uk = above ? row[k] : 0.0;
 #pragma unroll
         for (int c = 0; c < RC; ++c) {
           if (c < nc) {
-            const double xk = __shfl_sync(kFull, x[c], l);
-            if (above) x[c] = fma(-uk, xk, x[c]);
+            const double xk = __shfl_sync(kFull, x[c] * rdg, l);
+            const double t = fma(-uk, xk, x[c]);
+            x[c] = above ? t : x[c];
           }
         }
       }
+#pragma unroll
+      for (int c = 0; c < RC; ++c) x[c] *= rdg;
       if (live) {
         double* out = is_inv ? v.inv : v.X;
 #pragma unroll

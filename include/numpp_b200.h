@@ -174,7 +174,7 @@ int nppb_d_getrs_batched(int64_t count, int32_t n, int32_t nrhs, const double* d
  * looks up the array's device address, so make that first call before any
  * stream capture. Every call shares the array: calls that overlap on the GPU
  * (other streams, other threads) race and must be ordered by the caller.
- * Always the single-level step schedule (NPPB_BLOCKED_MIN_N is ignored).
+ * Always the single-level step schedule.
  * info as for the other solves; dX must not alias dB. */
 int nppb_d_solve_batched_noalloc(int64_t count, int32_t n, int32_t nrhs, const double* dA,
                                  const double* dB, double* dX, int32_t* dinfo, void* stream);
@@ -340,8 +340,9 @@ int nppb_plan_time_classes(nppb_plan* plan, const double* dA, const double* dB, 
 /* Every launch of one execution, one after another on `stream`, each between
  * two CUDA events: ms_out[k] = summed milliseconds and flops_out[k] = the
  * arithmetic done, per kernel kind k: 0 warp-per-system LU (orders <= 32),
- * 1 panel factorisation, 2 strip update (row moves, U12, trailing update on
- * DMMA), 3 back substitution (and, for getrs plans, forward substitution). */
+ * 1 panel factorisation (orders above 512), 2 factorisation of the orders 33..512
+ * and strip update above (row moves, U12, trailing update on DMMA), 3 substitution
+ * (above 512: back substitution; for getrs plans forward substitution too). */
 int nppb_plan_time_kernels(nppb_plan* plan, const double* dA, const double* dB, double* dX,
                            double* dInv, double* dDet, double* dSign, double* dLogabs,
                            int32_t* dinfo, void* stream, double* ms_out, double* flops_out);

@@ -1,4 +1,5 @@
-// System-resident LU and substitution: orders 33..512, one CTA per system.
+// System-resident LU and substitution: orders 33..512 on one CTA per system, larger
+// ones by outer blocks of 128 columns (k_sys_outer, k_sys_rows, k_sys_gemm).
 //
 // The reference factors one matrix by an unblocked right-looking elimination
 // (src/linalg/linalg.cpp:48-71) and then substitutes (:73-90). Here one CTA keeps
@@ -211,7 +212,7 @@ __device__ __forceinline__ void product_out(const double* Ut, int cols, int firs
 // candidate with the largest high word, which is nearly always unique) and
 // repeated exactly otherwise. The group loop is rolled (the accumulators rotate),
 // which keeps the code in the instruction cache.
-// Cycles per column with 1 / 16 warps: PANEL_CYCLES.
+// Cycles per column with 1 / 16 warps: 535 / 1120 (the step-wise panel: 2500).
 struct __align__(16) Cand {
   unsigned hi, lo;  // |a| as two words; 0, 0: no candidate
   int pos, pad;
@@ -1193,7 +1194,7 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
   for (int i = 0; i < 4; ++i) {
     const int p = 32 * blk + 8 * i + g;
     const bool ok = p < n;
-    const int row = !ok ? 0 : sa.upper_only ? p : s.v.perm[p];
+    const int row = ok ? s.v.perm[p] : 0;
     r.off[i] = (unsigned)(sa.w_by_position ? (ok ? p : 0) : row) * s.v.ldw * 8;
 #pragma unroll
     for (int ni = 0; ni < NI; ++ni)
@@ -1201,10 +1202,8 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
       for (int e = 0; e < 2; ++e) {
         const int col = 8 * ni + 2 * t + e;
         double x = 0.0;
-        if (ok && col < s.width) {
-          if (sa.upper_only) x = s.X[(int64_t)p * s.ldx + col];
-          else x = s.inverse ? (row == s.c0 + col ? 1.0 : 0.0) : s.B[(int64_t)row * s.ldx + col];
-        }
+        if (ok && col < s.width)
+          x = s.inverse ? (row == s.c0 + col ? 1.0 : 0.0) : s.B[(int64_t)row * s.ldx + col];
         acc.v[i >> 1][ni][2 * (i & 1) + e] = x;
       }
   }
@@ -1221,39 +1220,32 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
   };
   // A CTA fetches the inverse of its own next block, by the warps that have
   // nothing to update.
-  if (!sa.upper_only) {
-    if (rank < nb) fetch_inverse(Li, s.v.dinv + rank * 2048, blockDim.x);
-    else cp_commit();
-    ring_start<VEC, false>(ring, W, r, 0, n, blk > 0 && blk < nb);
-    for (int K = 0; K < nb; ++K) {
-      double* Ut = K & 1 ? U1 : U0;
-      solve_block(K, Ut, std::false_type{});
-      if (blk > K && blk < nb) {
-        update<NI, VEC, false>(acc, ring, W, r, smem(Ut + g * US + 2 * t), K, K + 1, blk > K + 1, n);
-      } else {
-        if (K % CS == rank && blk <= K) {
-          // the next L_KK^-1; after the CTA's last one its first U_KK^-1 (same block)
-          const int free = K / CS + 1;
-          fetch_inverse(Li, s.v.dinv + (K + CS < nb ? (K + CS) * 2048 : K * 2048 + 1024), 32 * free);
-        }
-        if (blk == K) {  // Y_K back into its owner's registers for the way up
-#pragma unroll
-          for (int m = 0; m < 2; ++m)
-#pragma unroll
-            for (int ni = 0; ni < NI; ++ni)
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                acc.v[m][ni][e] = -Ut[(8 * ni + 2 * t + (e & 1)) * US + 16 * m + g + 8 * (e >> 1)];
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) cp_commit();  // the waits count groups
+  if (rank < nb) fetch_inverse(Li, s.v.dinv + rank * 2048, blockDim.x);
+  else cp_commit();
+  ring_start<VEC, false>(ring, W, r, 0, n, blk > 0 && blk < nb);
+  for (int K = 0; K < nb; ++K) {
+    double* Ut = K & 1 ? U1 : U0;
+    solve_block(K, Ut, std::false_type{});
+    if (blk > K && blk < nb) {
+      update<NI, VEC, false>(acc, ring, W, r, smem(Ut + g * US + 2 * t), K, K + 1, blk > K + 1, n);
+    } else {
+      if (K % CS == rank && blk <= K) {
+        // the next L_KK^-1; after the CTA's last one its first U_KK^-1 (same block)
+        const int free = K / CS + 1;
+        fetch_inverse(Li, s.v.dinv + (K + CS < nb ? (K + CS) * 2048 : K * 2048 + 1024), 32 * free);
       }
+      if (blk == K) {  // Y_K back into its owner's registers for the way up
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int ni = 0; ni < NI; ++ni)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              acc.v[m][ni][e] = -Ut[(8 * ni + 2 * t + (e & 1)) * US + 16 * m + g + 8 * (e >> 1)];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) cp_commit();  // the waits count groups
     }
-  } else {
-    // the CTA's last block
-    const int last = rank < nb ? (nb - 1 - rank) / CS * CS + rank : -1;
-    if (last >= 0) fetch_inverse(Li, s.v.dinv + last * 2048 + 1024, blockDim.x);
-    else cp_commit();
   }
   ring_start<VEC, true>(ring, W, r, nb - 1, n, blk < nb - 1);
   for (int K = nb - 1; K >= 0; --K) {
@@ -1324,7 +1316,6 @@ k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __res
   const int n = v.n, b = (int)blockIdx.y - 1;
   if (b >= sys_blocks(n)) return;
   if (b < 0) {
-    if (!ipiv) return;  // upper factors only
     extern __shared__ int piv[];
     const int32_t* src = ipiv + (sa.desc ? sa.desc[s].piv_off : (int64_t)s * n);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -1356,7 +1347,7 @@ k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __res
   __syncthreads();
   double* di = v.dinv + (int64_t)b * 2048;
   if (threadIdx.x >= 32) tri_inverse<kUpper>(D, X[1], kb, into(di + 1024));
-  else if (ipiv) tri_inverse<kUnitLower>(D, X[0], kb, into(di));
+  else tri_inverse<kUnitLower>(D, X[0], kb, into(di));
 }
 
 }  // namespace

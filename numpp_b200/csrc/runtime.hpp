@@ -60,9 +60,8 @@ cudaError_t run_warp_uniform(const Batch& bt, int64_t count, int n, cudaStream_t
 // Uniform batch of orders 33..4096 on the step-wise kernels (descriptors and
 // work items derived from block indices, no plan). sa carries the pointers,
 // the LU workspace, the per-system scratch and un / unrhs / uinv.
-// substitute = false: X and the inverse are left as L^-1 P B.
 template <class T>
-cudaError_t run_step_uniform(const StepArgsT<T>& sa, int count, cudaStream_t st, bool substitute = true);
+cudaError_t run_step_uniform(const StepArgsT<T>& sa, int count, cudaStream_t st);
 // getrs on a uniform batch from factors (LU, ipiv) a uleft=1 factorisation left: B -> X;
 // prepermuted: X already holds P B (B is not read).
 template <class T>

@@ -1,4 +1,4 @@
-// System-resident LU and substitution (orders 33..512): launch interface.
+// System-resident LU and substitution (orders above 32): launch interface.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -67,7 +67,6 @@ struct SysArgs {
   int state_stride;     //   so many bytes apart
   int un, unrhs, uinv;  // uniform batch
   int w_by_position;    // W holds rows in pivoted order with leading dimension n (kept factors)
-  int upper_only;       // X and the inverse hold L^-1 P B already: back substitution in place
 };
 
 // LU with partial pivoting of `nsys` systems with (maximum order) nmax <= 512, a

@@ -583,7 +583,7 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
 //
 // In the cluster block b of 32 positions (counted from the outer block's first)
 // belongs to warp b / CS of CTA b % CS, so that every CTA keeps its share of the
-// rows that are left. Per column each warp's candidate (with its row) goes straight
+// rows that are left. Per column the candidates (with their rows) go straight
 // into every CTA's table, one cluster barrier, and every warp finds the winner in
 // its own CTA's copy; the solved rows of a block step are pushed the same way (as
 // in the substitution), the pivot rows of a panel group, the new positions and the
@@ -596,24 +596,69 @@ struct __align__(16) Record {  // a warp's candidate
 
 struct __align__(16) ClusterShared {
   Record own[kMaxWarps];
+  Record none;  // no candidate
   double raw[8][24];
   double l8[8][8];
   double u[24 * GS];
   double pv[32];  // the panel's pivots
 };
 
-constexpr int outer_smem(int warps, int blocks) {
-  return sys_cluster_smem(warps) + 2 * blocks * (int)sizeof(Record);
+// Whether the warps' candidates go into every CTA's table directly (a pair of
+// CTAs), or the CTAs' best ones do: with more CTAs the fewer remote stores outweigh
+// the extra stage. First outer block, us: 64 x 1024 on pairs 262 directly, 269 by
+// CTA; 16 x 1024 on four 230 / 220; 8 x 4096 on eight 410 / 303.
+__host__ __device__ constexpr bool outer_direct(int cs) { return cs == 2; }
+constexpr int outer_smem(int warps, int cs) {
+  return sys_cluster_smem(warps) + 2 * (outer_direct(cs) ? warps * cs : cs) * (int)sizeof(Record);
 }
 
-// As panel(), over the clusters' warps: slot = the warp's block relative to the
-// panel's first (active), na = their number.
-template <int CS, int NC>  // NC: candidates per lane, 32 NC >= na
+// The best candidate of a warp's lanes (a lane without one has in = false): its
+// lane, or -1 if there is none. Decided on the high words without their last
+// seven bits, which hold the lane, and exactly where that leaves a choice.
+template <class Load>
+__device__ __forceinline__ int best_lane(bool in, Load load) {
+  constexpr unsigned kIdx = 127u;
+  const int lane = threadIdx.x & 31;
+  const unsigned key = in ? (load().hi & ~kIdx) | (kIdx - lane) : 0u;
+  const unsigned mk = __reduce_max_sync(kAll, key);
+  const unsigned amb = __ballot_sync(kAll, in && (key ^ mk) <= kIdx);
+  if ((amb & (amb - 1)) == 0 && mk > kIdx) return (int)(kIdx - (mk & kIdx));
+  Cand c{0u, 0u, INT_MAX, 0};
+  if (in) c = load();
+  bool any;
+  const bool best = exact_winner(c.hi, c.lo, c.pos, any);
+  const unsigned who = __ballot_sync(kAll, best);
+  return any ? 31 - __clz(who) : -1;
+}
+
+// As panel(), over the cluster. Every warp's candidate (direct), or the best of the
+// CTA's, which its first warp finds, is pushed into every CTA's table; one cluster
+// barrier, and every warp finds the winner in its own CTA's copy. slot: the warp's
+// block relative to the panel's first, na: their number; [w0, w1): the CTA's
+// active warps.
+template <int CS>
 __device__ __forceinline__ int cluster_panel(ClusterShared& sh, Record* table, Acc<4>& acc, int& pos, bool valid,
-                                             bool active, int kb, int slot, int na, double* tile, int& nswap) {
+                                             bool active, int kb, int slot, int na, int w0, int w1, double* tile,
+                                             int& nswap) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   cg::cluster_group cl = cg::this_cluster();
   Record* own = &sh.own[warp];
+  constexpr bool kDirect = outer_direct(CS);
+  const int rank = (int)cl.block_rank(), threads = blockDim.x, entries = kDirect ? na : CS;
+  const int mine_at = kDirect ? slot : rank;  // this record's place in the tables
+  // 16-byte piece lane % 6 of the record to CTA lane / 6, and to CTA lane / 6 + 5
+  const int to = lane / 6, piece = lane - 6 * to;
+  double2* dst0 = nullptr;
+  double2* dst1 = nullptr;
+  if (kDirect ? active : warp == 0) {
+    if (lane < 30 && to < CS) dst0 = reinterpret_cast<double2*>(cl.map_shared_rank(table + mine_at, to)) + piece;
+    if (lane < 30 && to + 5 < CS)
+      dst1 = reinterpret_cast<double2*>(cl.map_shared_rank(table + mine_at, to + 5)) + piece;
+  }
+  if (!kDirect && warp == 0) {
+    if (lane == 0) sh.none.c = Cand{0u, 0u, INT_MAX, 0};
+    __syncwarp();
+  }
   unsigned live = valid ? 0x7fffffffu : 0u;
 #pragma unroll 1
   for (int j0 = 0; j0 < kb; j0 += 8) {
@@ -637,16 +682,17 @@ __device__ __forceinline__ int cluster_panel(ClusterShared& sh, Record* table, A
     for (int s = 0; s < 8; ++s) {
       const int j = j0 + s;
       if (j < kb) {  // uniform
-        Record* tab = table + (s & 1) * na;
+        Record* tab = table + (s & 1) * entries;
+        const int at = (s & 1) * entries * (int)(sizeof(Record) / 16);
         if (active) {  // uniform in the warp
           const unsigned hi = (unsigned)__double2hiint(a[s]) & live;
           const unsigned mh = __reduce_max_sync(kAll, hi);
-          const double rp = 1.0 / (hi ? a[s] : 1.0);
+          const double rp = kDirect ? 1.0 / (hi ? a[s] : 1.0) : 0.0;  // every candidate's, beside the reduction
           const bool me = hi == mh;
           const unsigned top = __ballot_sync(kAll, me);
           auto publish = [&](unsigned h, unsigned l, double r) {
             own->c = Cand{h, l, pos, 0};
-            own->rp = r;
+            if (kDirect) own->rp = r;
 #pragma unroll
             for (int c = s & ~1; c < 8; c += 2)
               *reinterpret_cast<double2*>(&own->row[c]) = make_double2(a[c], a[c + 1]);
@@ -658,53 +704,32 @@ __device__ __forceinline__ int cluster_panel(ClusterShared& sh, Record* table, A
             bool any;
             const bool win = exact_winner(h, l, pos, any);
             __syncwarp();
-            if (win) publish(h, l, 1.0 / a[s]);
+            if (win) publish(h, l, kDirect ? 1.0 / a[s] : 0.0);
             else if (!any && lane == 0) own->c = Cand{0u, 0u, INT_MAX, 0};
           }
-          __syncwarp();
-          // 16-byte pieces of the record to every CTA
-          for (int i = lane; i < 6 * CS; i += 32) {
-            const int to = i / 6, piece = i - 6 * to;
-            reinterpret_cast<double2*>(cl.map_shared_rank(tab + slot, to))[piece] =
-                reinterpret_cast<const double2*>(own)[piece];
+          if (kDirect) {
+            __syncwarp();
+            if (dst0) dst0[at] = reinterpret_cast<const double2*>(own)[piece];
+          }
+        }
+        if constexpr (!kDirect) {  // the CTA's best candidate: its first warp waits for the others
+          if (warp == 0) {
+            asm volatile("bar.sync 1, %0;\n" ::"r"(threads) : "memory");
+            const int w = best_lane(lane < w1 - w0, [&] { return sh.own[w0 + lane].c; });
+            const Record* best = w < 0 ? &sh.none : &sh.own[w0 + w];
+            double2 x = reinterpret_cast<const double2*>(best)[piece];
+            if (piece == 1) x.x = 1.0 / best->row[s];  // one reciprocal a CTA, not one a warp
+            if (dst0) dst0[at] = x;
+            if (dst1) dst1[at] = x;
+            __syncwarp();
+          } else {
+            __syncwarp();
+            asm volatile("bar.arrive 1, %0;\n" ::"r"(threads) : "memory");
           }
         }
         cl.sync();
-        // candidate 32 q + lane in key q: the high word without its last seven bits, then the index
-        constexpr unsigned kIdx = 127u;
-        unsigned key[NC], mine = 0;
-#pragma unroll
-        for (int q = 0; q < NC; ++q) {
-          const int i = 32 * q + lane;
-          key[q] = i < na ? (tab[i].c.hi & ~kIdx) | (kIdx - i) : 0u;
-          mine = max(mine, key[q]);
-        }
-        const unsigned mk = __reduce_max_sync(kAll, mine);
-        int same = 0;
-#pragma unroll
-        for (int q = 0; q < NC; ++q) same += 32 * q + lane < na && (key[q] ^ mk) <= kIdx;
-        const unsigned amb = __ballot_sync(kAll, same > 0), two = __ballot_sync(kAll, same > 1);
-        int gw = (int)(kIdx - (mk & kIdx));
-        if ((amb & (amb - 1)) != 0 || two != 0 || mk <= kIdx) {
-          Cand cd{0u, 0u, INT_MAX, 0};
-          int at = 0;
-#pragma unroll
-          for (int q = 0; q < NC; ++q) {
-            const int i = 32 * q + lane;
-            if (i < na) {
-              const Cand o = tab[i].c;
-              if (o.hi > cd.hi || (o.hi == cd.hi && (o.lo > cd.lo || (o.lo == cd.lo && o.pos < cd.pos)))) {
-                cd = o;
-                at = i;
-              }
-            }
-          }
-          bool any;
-          const bool best = exact_winner(cd.hi, cd.lo, cd.pos, any);
-          if (!any) return j + 1;  // the same in every warp of the cluster
-          const unsigned who = __ballot_sync(kAll, best);
-          gw = __shfl_sync(kAll, at, 31 - __clz(who));
-        }
+        const int gw = best_lane(lane < entries, [&] { return tab[lane].c; });
+        if (gw < 0) return j + 1;  // the same in every warp of the cluster
         const double r = tab[gw].rp;
         const int gk = tab[gw].c.pos;
         const double* prow = tab[gw].row;
@@ -794,7 +819,7 @@ __device__ __forceinline__ int cluster_panel(ClusterShared& sh, Record* table, A
 // The outer block of blocks [jb, je). perm_in: the positions so far, perm_out: with
 // this block's pivots (the update beside it reads the former). running: det,
 // log|det| and sign by slot.
-template <int CS, int NC>
+template <int CS>
 __global__ void __launch_bounds__(kSysMaxN, 1)
 k_sys_outer(SysArgs sa, const int32_t* __restrict__ perm_in, int32_t* __restrict__ perm_out,
             double* __restrict__ running, int jb, int je) {
@@ -901,7 +926,9 @@ k_sys_outer(SysArgs sa, const int32_t* __restrict__ perm_in, int32_t* __restrict
     const bool active = blk >= J && blk < nb, valid = active && lane < n - 32 * blk;
     const int phys = valid ? s_perm[32 * warp + lane] : 0;
     int pos = 32 * (blk - J) + lane, nswap = 0;
-    const int info = cluster_panel<CS, NC>(sh, table, acc, pos, valid, active, kb, blk - J, nb - J, stage, nswap);
+    // the CTA's warps whose blocks lie in [J, nb)
+    const int w0 = max(0, (J - jb - rank + CS - 1) / CS), w1 = min(nw, max(w0, (nb - jb - rank + CS - 1) / CS));
+    const int info = cluster_panel<CS>(sh, table, acc, pos, valid, active, kb, blk - J, nb - J, w0, w1, stage, nswap);
     if (info) {  // the same in every thread of the cluster; nothing is on its way to another CTA
       if (tid == 0 && rank == 0) {
         *state_of(sa, s_v.slot) = 32 * J + info;
@@ -1362,14 +1389,14 @@ cudaError_t launch_sys_lu(const SysArgs& sa, const int32_t* list, int nsys, int 
 
 namespace {
 
-template <int CS, int NC>
+template <int CS>
 cudaError_t launch_outer1(const SysArgs& sa, const int32_t* pin, int32_t* pout, double* running, int nsys, int jb,
                           int je, cudaStream_t st) {
   const int blocks = sys_blocks(sa.un) - jb, nw = std::max(1, (blocks + CS - 1) / CS);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)nsys * CS);
   cfg.blockDim = dim3(32 * nw);
-  cfg.dynamicSmemBytes = outer_smem(nw, blocks);
+  cfg.dynamicSmemBytes = outer_smem(nw, CS);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1378,13 +1405,13 @@ cudaError_t launch_outer1(const SysArgs& sa, const int32_t* pin, int32_t* pout, 
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_sys_outer<CS, NC>, sa, pin, pout, running, jb, je);
+  return cudaLaunchKernelEx(&cfg, k_sys_outer<CS>, sa, pin, pout, running, jb, je);
 }
 
-template <int CS, int NC>
+template <int CS>
 cudaError_t prepare_outer() {
-  return cudaFuncSetAttribute(k_sys_outer<CS, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              outer_smem(kMaxWarps, kMaxWarps * CS));
+  return cudaFuncSetAttribute(k_sys_outer<CS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              outer_smem(kMaxWarps, CS));
 }
 
 }  // namespace
@@ -1393,9 +1420,9 @@ cudaError_t launch_sys_outer(const SysArgs& sa, const int32_t* pin, int32_t* pou
                              int je, cudaStream_t st) {
   const int cs = sys_outer_cluster(32 * (sys_blocks(sa.un) - jb), nsys);
   switch (cs) {
-    case 2: return launch_outer1<2, 1>(sa, pin, pout, running, nsys, jb, je, st);
-    case 4: return launch_outer1<4, 2>(sa, pin, pout, running, nsys, jb, je, st);
-    case 8: return launch_outer1<8, 4>(sa, pin, pout, running, nsys, jb, je, st);
+    case 2: return launch_outer1<2>(sa, pin, pout, running, nsys, jb, je, st);
+    case 4: return launch_outer1<4>(sa, pin, pout, running, nsys, jb, je, st);
+    case 8: return launch_outer1<8>(sa, pin, pout, running, nsys, jb, je, st);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -1518,9 +1545,9 @@ cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int
 cudaError_t sys_prepare_kernels() {
   cudaError_t e = cudaFuncSetAttribute(k_sys_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        sys_smem(kMaxWarps));
-  if (e == cudaSuccess) e = prepare_outer<2, 1>();
-  if (e == cudaSuccess) e = prepare_outer<4, 2>();
-  if (e == cudaSuccess) e = prepare_outer<8, 4>();
+  if (e == cudaSuccess) e = prepare_outer<2>();
+  if (e == cudaSuccess) e = prepare_outer<4>();
+  if (e == cudaSuccess) e = prepare_outer<8>();
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_sys_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, sys_smem(4));
   if (e == cudaSuccess)

@@ -91,7 +91,7 @@ cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t ni
                              cudaStream_t st);
 cudaError_t launch_sys_solve_uniform(const SysArgs& sa, int nsys, cudaStream_t st);
 // Permutations and diagonal inverses of kept factors (swap lists ipiv at
-// piv_off): fills sa.perm and sa.dinv. Null ipiv: the upper factors' inverses only.
+// piv_off): fills sa.perm and sa.dinv.
 cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int32_t* list, int nsys, int nmax,
                                cudaStream_t st);
 cudaError_t sys_prepare_kernels();

@@ -1325,7 +1325,7 @@ namespace {
 struct MxStreams {
   cudaStream_t panel = nullptr;  // the next block's diagonal factor and triangular solves, highest priority
   cudaStream_t side = nullptr;   // the bulk of the trailing update
-  cudaStream_t inv = nullptr;    // the diagonal block's inverses, beside the window permute
+  cudaStream_t rows = nullptr;    // the window permute, beside the diagonal block's inverses
   cudaEvent_t ev[6] = {};
 };
 
@@ -1334,7 +1334,7 @@ MxStreams* mx_streams() {
     std::vector<MxStreams> per_dev;
     ~Holder() {
       for (auto& m : per_dev) {
-        for (cudaStream_t t : {m.panel, m.side, m.inv})
+        for (cudaStream_t t : {m.panel, m.side, m.rows})
           if (t) cudaStreamDestroy(t);
         for (cudaEvent_t e : m.ev)
           if (e) cudaEventDestroy(e);
@@ -1350,7 +1350,7 @@ MxStreams* mx_streams() {
     int least = 0, greatest = 0;
     cudaDeviceGetStreamPriorityRange(&least, &greatest);
     bool ok = cudaStreamCreateWithPriority(&m.panel, cudaStreamNonBlocking, greatest) == cudaSuccess &&
-              cudaStreamCreateWithPriority(&m.inv, cudaStreamNonBlocking, greatest) == cudaSuccess &&
+              cudaStreamCreateWithPriority(&m.rows, cudaStreamNonBlocking, greatest) == cudaSuccess &&
               cudaStreamCreateWithFlags(&m.side, cudaStreamNonBlocking) == cudaSuccess;
     for (cudaEvent_t& e : m.ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
@@ -1393,15 +1393,17 @@ cudaError_t mx_factor(const MxBufs& b, cudaStream_t s) {
     // block k's window was last written by block k-1's cross update, earlier on ps
     k_mx_diag<<<count, DT, kDiagSmem, ps>>>(b.M, b.perm, b.info, N, k);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // the inverses beside the permute (they read the diagonal tile, which the permute leaves alone)
-    cudaStream_t is = ms ? ms->inv : ps;
+    // the permute beside the inverses (they read the diagonal tile, which the permute
+    // leaves alone); the inverses go first, on the diagonal kernel's own stream: behind
+    // the permute's many CTAs they ended 20 us after it at 64 systems of order 1024
+    cudaStream_t is = ms ? ms->rows : ps;
     if (ms) {
       if ((e = cudaEventRecord(ms->ev[4], ps)) != cudaSuccess) return e;
       if ((e = cudaStreamWaitEvent(is, ms->ev[4], 0)) != cudaSuccess) return e;
     }
-    k_mx_diag_inv<<<dim3((unsigned)count, 2), DT, kInvSmem, is>>>(b.M, b.Linv, b.Uinv, b.UinvT, N, k);
+    k_mx_diag_inv<<<dim3((unsigned)count, 2), DT, kInvSmem, ps>>>(b.M, b.Linv, b.Uinv, b.UinvT, N, k);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    k_mx_permute<<<dim3((unsigned)(N / PC), (unsigned)count), 256, kPermSmem, ps>>>(b.M, b.T, b.perm, N, k, count,
+    k_mx_permute<<<dim3((unsigned)(N / PC), (unsigned)count), 256, kPermSmem, is>>>(b.M, b.T, b.perm, N, k, count,
                                                                                    buf);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (ms) {

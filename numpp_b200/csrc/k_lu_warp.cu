@@ -14,11 +14,19 @@
 // the trailing update is a[i,j] -= f*a[k,j] (one FMA here). NaN entries are
 // never pivot candidates.
 //
+// A warp's chain of instructions bounds few systems (256 of order 32, solve and det:
+// 26.6 us with each 16-byte piece of the update loaded behind the store before it,
+// 22.5 us with eight columns at a time, the forward substitution of a single
+// right-hand side riding along with the elimination, and one reduction where a
+// single lane holds the largest high word). With up to eight columns a chunk (RC = 8)
+// the same changes cost more instructions than they save in latency (4000 systems
+// of order 24 with 5: 70 us without them, 78 us with), so that form keeps its branches.
+//
 // The same launch finishes the requested outputs:
 //  * det  = permsign * prod U[i,i] in order i = 0..n-1   (linalg.cpp:393-407)
 //  * slogdet sign / sum log|U[i,i]| in order               (linalg.cpp:408-439)
-//  * X = A^-1 B: X[pos(r)] starts as B[r]; forward (unit L; the first RC columns
-//    during the elimination) and back (U)
+//  * X = A^-1 B: X[pos(r)] starts as B[r]; forward (unit L; a single column during
+//    the elimination) and back (U)
 //    substitution run across lanes, up to RC columns at a time (linalg.cpp:73-90)
 //  * inverse = the same solve against I                    (linalg.cpp:105-115)
 //  * LU + ipiv (LAPACK-style swap list, 0-based) for getrf.
@@ -38,6 +46,8 @@ constexpr int kLd = 34;          // row stride of a warp's tile (doubles): colum
 template <int NP, int RC>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
+  constexpr int UF = RC == 1 ? 4 : 1;  // substitution steps per loop body (small code with several columns)
+  constexpr bool kOne = RC == 1;       // one column: no branches in its substitution either
   __shared__ int s_lane_of_pos[kWarpsPerCta][32];
   __shared__ __align__(16) double s_rows[kWarpsPerCta][32 * kLd];  // row r at r * kLd (16-byte aligned rows)
   const int lane = threadIdx.x & 31;
@@ -71,25 +81,24 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
   // Original row index held by each position, for getrs from stored factors.
   int orig = lane;
 
-  // the first right-hand sides ride along with the elimination (their forward substitution)
-  const bool ride = (flags & kWantSolve) && !(flags & kSolveOnly);
-  double x0[RC];
-#pragma unroll
-  for (int c = 0; c < RC; ++c)
-    x0[c] = ride && live && c < v.nrhs ? v.B[(int64_t)lane * v.nrhs + c] : 0.0;
+  // a single right-hand side rides along with the elimination (its forward substitution);
+  // eight of them cost there what the loop of their own does
+  const bool ride = kOne && (flags & kWantSolve) && !(flags & kSolveOnly);
+  double x0 = ride && live && v.nrhs > 0 ? v.B[(int64_t)lane * v.nrhs] : 0.0;
 
   if (!(flags & kSolveOnly)) {
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
       const bool cand = live && pos >= k;
       const double akk = live ? row[k] : 0.0;
-      const unsigned long long bits = (unsigned long long)__double_as_longlong(akk) & 0x7fffffffffffffffull;
-      const bool number = cand && bits <= 0x7ff0000000000000ull;  // NaN entries are no candidates
+      const double mag = cand ? fabs(akk) : 0.0;
+      const bool number = mag == mag;  // NaN entries are no candidates
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(mag);
       const uint32_t hi = number ? (uint32_t)(bits >> 32) : 0u, lo = number ? (uint32_t)bits : 0u;
       const uint32_t mhi = __reduce_max_sync(kFull, hi);
-      unsigned tops = __ballot_sync(kFull, number && hi == mhi);
+      const unsigned tops = kOne ? __ballot_sync(kFull, cand && hi == mhi) : 0u;
       int pl = __ffs(tops) - 1, key;
-      if (mhi != 0u && (tops & (tops - 1u)) == 0u) {  // one lane holds the largest high word
+      if (kOne && mhi != 0u && (tops & (tops - 1u)) == 0u) {  // one lane holds the largest high word
         key = __shfl_sync(kFull, pos, pl);
       } else {
         const uint32_t mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
@@ -97,32 +106,30 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
           info = k + 1;
           break;
         }
-        const bool top = number && hi == mhi && lo == mlo;
+        const bool top = cand && hi == mhi && lo == mlo;
         key = (int)__reduce_min_sync(kFull, top ? (uint32_t)pos : 0xffffffffu);
         pl = __ffs(__ballot_sync(kFull, live && pos == key)) - 1;
       }
       if (key != k) {
         pos = lane == pl ? k : live && pos == k ? key : pos;
         ++nswap;
-      } else if (lane == pl) {
-        pos = k;
       }
       if ((flags & kWantLU) && lane == 0) v.ipiv[k] = key;
       const double* prow = R + pl * kLd;
       const double pk = prow[k];
       if (lane == pl) dg = pk;
       const bool below = live && pos > k;
-      const double f = below ? akk / pk : 0.0;
-      if (ride) {
-#pragma unroll
-        for (int c = 0; c < RC; ++c)
-          if (c < v.nrhs) {
-            const double xk = __shfl_sync(kFull, x0[c], pl);
-            const double t = fma(-f, xk, x0[c]);
-            x0[c] = below ? t : x0[c];
-          }
+      double f = 0.0;
+      if constexpr (kOne) {
+        f = below ? akk / pk : 0.0;
+        if (ride) {
+          const double xk = __shfl_sync(kFull, x0, pl);
+          const double t = fma(-f, xk, x0);
+          x0 = below ? t : x0;
+        }
       }
       if (below) {
+        if constexpr (!kOne) f = row[k] / pk;
         row[k] = f;
         // eight columns at a time, both rows' pieces loaded before the first store (a
         // store to the tile holds back every later load of it: 78 cycles a 16-byte
@@ -146,10 +153,21 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) r2[q + i] = rv[i];
         };
-        int q = (k + 1) >> 3 << 2;
-        if (2 * q < n) piece(q, true);
+        if (kOne && n > 8) {
+          int q = (k + 1) >> 3 << 2;
+          if (2 * q < n) piece(q, true);
 #pragma unroll 1
-        for (q += 4; 2 * q < n; q += 4) piece(q, false);
+          for (q += 4; 2 * q < n; q += 4) piece(q, false);
+        } else {  // few columns, or many warps' worth of work: no column too many
+#pragma unroll 4
+          for (int q = (k + 1) >> 1; q < (n + 1) >> 1; ++q) {
+            const double2 pv = p2[q];
+            double2 rv = r2[q];
+            if (2 * q > k) rv.x = fma(-f, pv.x, rv.x);
+            rv.y = fma(-f, pv.y, rv.y);
+            r2[q] = rv;
+          }
+        }
       }
       __syncwarp();
     }
@@ -226,8 +244,7 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
       const int nc = min(RC, ncols - c0);  // columns of this chunk (warp-uniform)
       double x[RC];
       if (ride && !is_inv && c0 == 0) {
-#pragma unroll
-        for (int c = 0; c < RC; ++c) x[c] = x0[c];
+        x[0] = x0;
         __syncwarp();  // every lane has read its right-hand side before any lane writes X
       } else {
 #pragma unroll
@@ -242,7 +259,7 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
         }
         __syncwarp();  // every lane has read its right-hand side before any lane writes X (getrs in place)
         // forward: unit lower, position order
-#pragma unroll 4
+#pragma unroll UF
         for (int k = 0; k < n; ++k) {
           const int l = lop[k];
           const bool below = live && pos > k;
@@ -251,30 +268,41 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
           for (int c = 0; c < RC; ++c) {
             if (c < nc) {
               const double xk = __shfl_sync(kFull, x[c], l);
-              const double t = fma(-lk, xk, x[c]);
-              x[c] = below ? t : x[c];
+              if constexpr (kOne) {
+                const double t = fma(-lk, xk, x[c]);
+                x[c] = below ? t : x[c];
+              } else {
+                if (below) x[c] = fma(-lk, xk, x[c]);
+              }
             }
           }
         }
       }
       // back: upper; a row is multiplied by the diagonal's reciprocal when it is final
-      // (every lane forms the product, the final row's is passed on: no branch)
-#pragma unroll 4
+      // (with one column every lane forms the product and the final row's is passed on)
+#pragma unroll UF
       for (int k = n - 1; k >= 0; --k) {
         const int l = lop[k];
+        if (!kOne && lane == l) {
+#pragma unroll
+          for (int c = 0; c < RC; ++c) x[c] *= rdg;
+        }
         const bool above = live && pos < k;
         const double uk = above ? row[k] : 0.0;
 #pragma unroll
         for (int c = 0; c < RC; ++c) {
           if (c < nc) {
-            const double xk = __shfl_sync(kFull, x[c] * rdg, l);
-            const double t = fma(-uk, xk, x[c]);
-            x[c] = above ? t : x[c];
+            const double xk = __shfl_sync(kFull, kOne ? x[c] * rdg : x[c], l);
+            if constexpr (kOne) {
+              const double t = fma(-uk, xk, x[c]);
+              x[c] = above ? t : x[c];
+            } else {
+              if (above) x[c] = fma(-uk, xk, x[c]);
+            }
           }
         }
       }
-#pragma unroll
-      for (int c = 0; c < RC; ++c) x[c] *= rdg;
+      if (kOne) x[0] *= rdg;
       if (live) {
         double* out = is_inv ? v.inv : v.X;
 #pragma unroll

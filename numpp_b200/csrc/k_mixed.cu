@@ -9,6 +9,7 @@
 //  k_scale_rhs    r * B in FP32 (the first right-hand side), ||B||_max
 //  k_apply        X = c * Y (first solution) or X += c * Y (correction), FP64
 //  k_residual     R = B - A X in FP64 and r * R in FP32 for the next correction
+//                 (k_residual_mma: 3 or more right-hand sides, on the FP64 tensor core)
 //  k_refine_decide eta = max|R| / (||A||_inf max|X| + max|B|) (normwise
 //                 backward error) and the convergence / stall decision
 //                 (stalled: the contraction shown cannot reach tol in the
@@ -177,8 +178,7 @@ k_apply(double* __restrict__ X, const float* __restrict__ Y, const double* __res
 }
 
 // One CTA per (system, kMixedRows rows of A): R = B - A X for those rows,
-// right-hand sides in chunks of RC (1, 2, 4 or 8: the smallest power of two
-// covering nrhs, at most 8), X staged through shared memory in blocks of
+// one or two right-hand sides (RC), X staged through shared memory in blocks of
 // XS / RC rows; each warp keeps kMixedRows / 8 rows' sums in registers and
 // reads its rows of A coalesced. max |R| (and, by the first CTA, max |X|) go
 // to the system's running maxima; k_refine_decide turns them into eta. With

@@ -19,7 +19,8 @@
 //                  chunks), split into TF32 hi / lo in shared memory, one
 //                  thread issues tcgen05.mma.kind::tf32 (M = N = 128) into a
 //                  TMEM accumulator, tcgen05.ld epilogue against the C tile
-//                  (loaded by TMA behind the products), TMA store.
+//                  (loaded by TMA into the operand stages once they are
+//                  free), TMA store.
 //  k_mx_trsv_c     forward and back substitution by 128-row blocks with the
 //                  stored diagonal-block inverses: a cluster of 1..8 CTAs per
 //                  system and right-hand-side chunk, each holding its blocks'

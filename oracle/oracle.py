@@ -46,7 +46,7 @@ def build_oracle(ref_src: str | None = None) -> None:
     and present; without one the reference build is skipped."""
     subprocess.run(["make", "-s", "-C", _HERE], check=True)
     src = ref_src or os.environ.get("NUMPP_REF_SRC")
-    if src and os.path.isdir(src):
+    if src and os.path.isdir(os.path.join(src, "src", "linalg")):
         subprocess.run(["make", "-s", "-C", _HERE, "ref", "dropin", "refcuda", f"REF={src}"], check=True)
 
 

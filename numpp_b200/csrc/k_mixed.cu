@@ -274,11 +274,13 @@ k_residual(const double* __restrict__ A, const double* __restrict__ B, const dou
 // The same with 3 or more right-hand sides, on the FP64 tensor cores: eight of
 // them are one m16n8k8 operand. Per-thread products read every staged X value
 // once per row of A, and shared memory bounded them (430 us a pass over 5
-// systems of order 3001 with 8 right-hand sides, 137 us so; with 1 or 2 the
+// systems of order 3001 with 8 right-hand sides, 106 us so; with 1 or 2 the
 // pass over A itself is the bound). Eight warps: 2 tiles of 16 rows x 4 shares
 // of each staged block's columns, whose sums meet in shared memory. A lane
-// loads its entries of A itself, four of a row's neighbours making 32 bytes, 8
-// columns at a time and four steps ahead of the products.
+// loads its entries of A itself, four of a row's neighbours making 32 bytes, 32
+// columns at a time, the next ones behind the products of these (134 us with the
+// loads of a step waited for before its products; 137 us with the registers held to
+// three CTAs an SM).
 constexpr int XB = 512;  // rows of X staged per block
 
 __global__ void __launch_bounds__(MT)
@@ -315,30 +317,40 @@ k_residual_mma(const double* __restrict__ A, const double* __restrict__ B, const
       __syncthreads();
       const int per = ((j8 >> 3) + 3) >> 2, lo = 8 * share * per, hi = min(jn, lo + 8 * per);
       int j = lo;
-#pragma unroll 1
-      for (; j + 32 <= hi; j += 32) {
-        double a[4][4];
+      double a[4][4];
+      auto load = [&](int at) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const int c = j0 + j + 8 * u + t;
+          const int c = j0 + at + 8 * u + t;
           a[u][0] = a0[c];
           a[u][1] = a1[c];
           a[u][2] = a0[c + 4];
           a[u][3] = a1[c + 4];
         }
+      };
+      if (j + 32 <= hi) load(j);
+#pragma unroll 1
+      for (; j + 32 <= hi; j += 32) {
+        double2 lo2[4], hi2[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          lo2[u] = make_double2(a[u][0], a[u][2]);
+          hi2[u] = make_double2(a[u][1], a[u][3]);
+        }
+        if (j + 64 <= hi) load(j + 32);  // on their way behind these products
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const double* xr = xs + (j + 8 * u + t) * 8 + g;
-          dmma1688(acc, make_double2(a[u][0], a[u][2]), make_double2(a[u][1], a[u][3]), make_double2(xr[0], xr[32]));
+          dmma1688(acc, lo2[u], hi2[u], make_double2(xr[0], xr[32]));
         }
       }
 #pragma unroll 1
       for (; j < hi; j += 8) {  // columns past the order count as zero on both sides
         const int c = j0 + j + t;
         const bool in0 = j + t < jn, in1 = j + t + 4 < jn;
-        const double a[4] = {in0 ? a0[c] : 0.0, in0 ? a1[c] : 0.0, in1 ? a0[c + 4] : 0.0, in1 ? a1[c + 4] : 0.0};
+        const double b[4] = {in0 ? a0[c] : 0.0, in0 ? a1[c] : 0.0, in1 ? a0[c + 4] : 0.0, in1 ? a1[c + 4] : 0.0};
         const double* xr = xs + (j + t) * 8 + g;
-        dmma1688(acc, make_double2(a[0], a[2]), make_double2(a[1], a[3]), make_double2(xr[0], xr[32]));
+        dmma1688(acc, make_double2(b[0], b[2]), make_double2(b[1], b[3]), make_double2(xr[0], xr[32]));
       }
     }
     __syncthreads();

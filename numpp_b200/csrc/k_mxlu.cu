@@ -1019,6 +1019,8 @@ k_mx_trsv_c(const float* __restrict__ M, const float* __restrict__ Linv, const f
   const int rank = (int)cluster.block_rank();
   const int s = blockIdx.x / C, c0 = blockIdx.y * W;
   if (only_active && st[s].status != kRefineActive) return;  // every CTA of the cluster: same system, same answer
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nb = N / kMxNB, nbl = (nb - rank + C - 1) / C;  // blocks this CTA owns
   VT* cl = tsm;                                  // [nbl][W][128] owned right-hand sides
@@ -1032,6 +1034,8 @@ k_mx_trsv_c(const float* __restrict__ M, const float* __restrict__ Linv, const f
   }
   const float* Ls = Linv + (int64_t)s * N * kMxNB;
   const float* Us = Uinv + (int64_t)s * N * kMxNB;
+  __syncwarp();  // every CTA runs: y_0 may be pushed
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   // steps 0 .. nb-1: L y = P c downwards; steps nb .. 2 nb - 1: U x = y upwards
   auto block_of = [&](int q) { return q < nb ? q : 2 * nb - 1 - q; };
   for (int q = -1; q + 1 < 2 * nb; ++q) {  // y of step q is in every CTA (q >= 0); step q + 1 is next

@@ -208,6 +208,10 @@ k_panel(StepArgsT<T> sa, const int32_t* __restrict__ list, int k0) {
   } else if (sc->info) {
     return;  // the same for every CTA of the cluster
   }
+  if constexpr (CS > 1) {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  }
   T* dst = sa.LU + d.lu_off;
   const T* src = (k0 == 0 && sa.A) ? sa.A + d.a_off : dst;
   if (rank == 0) {
@@ -229,6 +233,8 @@ k_panel(StepArgsT<T> sa, const int32_t* __restrict__ list, int k0) {
   if (tid == 0) s_ndisp = 0;
   cp_async_wait<0>();
   __syncthreads();
+  if constexpr (CS > 1)  // every CTA runs: candidates may be pushed into its shared memory
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   T a[RPT][NB];
   int pos[RPT];
   bool valid[RPT];

@@ -1214,6 +1214,7 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
   const unsigned ring = smem(sm + kWarp + warp * kPerWarp) + 16 * lane;
   const double* const W = s.v.W;
   const int n = s.v.n, nb = sys_blocks(n);
+  if constexpr (CS > 1) cluster_arrive();
   Acc<NI> acc;
   Rows r;
   r.live = n - 32 * blk - g;
@@ -1250,6 +1251,7 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
   if (rank < nb) fetch_inverse(Li, s.v.dinv + rank * 2048, blockDim.x);
   else cp_commit();
   ring_start<VEC, false>(ring, W, r, 0, n, blk > 0 && blk < nb);
+  if constexpr (CS > 1) cluster_wait();  // every CTA runs: block 0's rows may be pushed
   for (int K = 0; K < nb; ++K) {
     double* Ut = K & 1 ? U1 : U0;
     solve_block(K, Ut, std::false_type{});

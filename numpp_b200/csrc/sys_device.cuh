@@ -79,6 +79,19 @@ struct Acc {
   double v[2][NI][4];  // rows 16m + g, 16m + g + 8; columns 8i + 2t, + 1
 };
 
+// The two halves of a cluster barrier, by whole warps. A CTA's shared memory may be
+// written by a peer only once the CTA is known to run: kernels that push before
+// their first cluster barrier arrive on entry and wait ahead of that push, so
+// that their own loads cover the wait.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
 __device__ __forceinline__ unsigned smem(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ double2 lds2(unsigned p) {  // stays where it is written
   double2 v;

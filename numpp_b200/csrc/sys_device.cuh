@@ -253,6 +253,7 @@ __device__ __forceinline__ void tri_inverse(double* D, double* X, int kb, Put pu
     const bool zero = UPPER ? (lane < 16 && r >= 16) : (lane >= 16 && r < 16);
     put(r, lane, zero ? 0.0 : X[r * TS + lane]);
   }
+  __syncwarp();  // the callers' scratch becomes an operand ring, whose copies overwrite what other lanes read here
 }
 
 constexpr int kPerWarp = 32 * PS;  // doubles of a warp's region: its ring, or its staging tile

@@ -262,7 +262,7 @@ k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
           for (int c = 0; c < CS; ++c) *(CS > 1 ? cg::this_cluster().map_shared_rank(&s_fail, c) : &s_fail) = 1;
         }
       } else if (J + 1 < nb) {
-        tri_inverse<kLower>(tile, scratch, kb, [&](int row, int col, double v) {
+        tri_inverse<kLower, false>(tile, scratch, kb, [&](int row, int col, double v) {
 #pragma unroll
           for (int c = 0; c < CS; ++c)
             (CS > 1 ? cg::this_cluster().map_shared_rank(Li, c) : Li)[row * US + col] = v;

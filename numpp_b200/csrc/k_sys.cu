@@ -22,7 +22,8 @@
 //
 // Substitution (k_sys_solve) is the same loop on a strip of at most 32
 // right-hand sides or inverse columns: forward through the blocks with
-// L_KK^-1, back with U_KK^-1, in one launch.
+// L_KK^-1, back with U_KK^-1 (with U_KK itself where that is ill-conditioned, so
+// that the solution keeps the backward error of a substitution), in one launch.
 //
 // What bounds it: FP64 tensor throughput in 2 (mma.m16n8k8, 64 FMA per cycle
 // and SM), the dependent pivot steps in 3.
@@ -170,6 +171,77 @@ __device__ __forceinline__ void tile_product(const double* Li, const double* Tb,
       }
 #pragma unroll
       for (int e = 0; e < 2; ++e) put(2 * t + e, 8 * mi + g, -(d[0][e] + d[1][e]));
+    }
+  }
+}
+
+// A block that is marked as too ill-conditioned for that: T holds the triangle itself
+// as tri_inverse leaves it, and the rows are substituted in their tile, by one warp
+// with a lane per column, eight rows in registers at a time (no division here: with
+// one, strips of 32 columns spill around it and every solve loses 1%). The loads are
+// written where they are to happen, for the registers.
+template <bool UPPER>
+__device__ __forceinline__ bool tri_marked(const double* T) { return T[UPPER ? 31 * US + 1 : 31] != 0.0; }
+
+__device__ __forceinline__ double lds1(unsigned p) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v) : "r"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts1(unsigned p, double v) {
+  asm volatile("st.shared.f64 [%0], %1;\n" ::"r"(p), "d"(v) : "memory");
+}
+
+template <int NI, bool UPPER>
+__device__ __forceinline__ void tile_substitute(const double* T, double* Tb) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x >= 32 || lane >= 8 * NI) return;
+  const unsigned c = smem(Tb + lane), tri = smem(T);
+#pragma unroll 1
+  for (int s = 0; s < 4; ++s) {
+    const int i0 = UPPER ? 24 - 8 * s : 8 * s;
+    const unsigned ci = c + i0 * (8 * BS), ti = tri + i0 * (8 * US);  // row i0 of the strip and of T
+    double x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = lds1(ci + i * (8 * BS));
+#pragma unroll 1
+    for (int p = 0; p < 8 * s; ++p) {  // the rows solved before
+      const int q = UPPER ? 31 - p : p;
+      const double y = lds1(c + q * (8 * BS));
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = fma(-lds1(ti + i * (8 * US) + 8 * q), y, x[i]);
+    }
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      const int j = UPPER ? 7 - p : p;
+      double col[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (UPPER ? i < j : i > j) col[i] = lds1(ti + i * (8 * US) + 8 * (i0 + j));
+      if constexpr (UPPER) {
+        const unsigned row = ti + j * (8 * US);
+        x[j] = x[j] * lds1(row + 8 * (i0 + j)) * lds1(i0 + j ? row : tri + 8 * (2 * US + 1));
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (UPPER ? i < j : i > j) x[i] = fma(-col[i], x[j], x[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sts1(ci + i * (8 * BS), x[i]);
+  }
+}
+
+// Ut <- -Tb^T, as tile_product leaves it.
+template <int NI, int CS>
+__device__ __forceinline__ void tile_negate(const double* Tb, double* Ut) {
+  for (int i = threadIdx.x; i < 256 * NI; i += blockDim.x) {
+    const int row = i & 31, col = i >> 5;
+    const double v = -Tb[row * BS + col];
+    if constexpr (CS == 1) {
+      Ut[col * US + row] = v;
+    } else {
+#pragma unroll
+      for (int c = 0; c < CS; ++c) cg::this_cluster().map_shared_rank(Ut, c)[col * US + row] = v;
     }
   }
 }
@@ -535,8 +607,8 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
     // the diagonal block's inverses and the pivots' part of det / slogdet, each by
     // one warp, beside the other warps' loads of the next column block
     double* di = s_v.dinv + (int64_t)J * 2048;
-    if (warp == 0) tri_inverse<kUnitLower>(D11, stage, kb, into(di));
-    if (warp == 1 % nw) tri_inverse<kUpper>(D11, stage, kb, into(di + 1024));
+    if (warp == 0) tri_inverse<kUnitLower, false>(D11, stage, kb, into(di));
+    if (warp == 1 % nw) tri_inverse<kUpper, true>(D11, stage, kb, into(di + 1024));
     if (warp == 2 % nw && (sa.det || sa.sign || sa.logabs)) {
       // folded in the reference's order (linalg.cpp:400-403, 425-431)
       const double pv = lane < kb ? D11[lane * PS + lane] : 1.0;
@@ -958,8 +1030,8 @@ k_sys_outer(SysArgs sa, const int32_t* __restrict__ perm_in, int32_t* __restrict
     cl.sync();  // rows, positions and the diagonal block are everywhere
     double* di = s_v.dinv + (int64_t)J * 2048;
     if ((J - jb) % CS == rank) {
-      if (warp == 0) tri_inverse<kUnitLower>(D11, stage, kb, into(di));
-      if (warp == 1 % nw) tri_inverse<kUpper>(D11, stage, kb, into(di + 1024));
+      if (warp == 0) tri_inverse<kUnitLower, false>(D11, stage, kb, into(di));
+      if (warp == 1 % nw) tri_inverse<kUpper, true>(D11, stage, kb, into(di + 1024));
     }
     if (rank == 0 && warp == 2 % nw) {
       // folded in the reference's order (linalg.cpp:400-403, 425-431)
@@ -1241,7 +1313,14 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
       if (blk == K) store_tile<NI>(Tb, acc);
       cp_wait<2>();  // the inverse; at most two operand stages stay in flight
       __syncthreads();
-      tile_product<NI, decltype(upper)::value, CS>(Li, Tb, Ut);
+      constexpr bool kUp = decltype(upper)::value;
+      if (!tri_marked<kUp>(Li)) {  // uniform
+        tile_product<NI, kUp, CS>(Li, Tb, Ut);
+      } else {
+        tile_substitute<NI, kUp>(Li, Tb);
+        __syncthreads();
+        tile_negate<NI, CS>(Tb, Ut);
+      }
     }
     if constexpr (CS > 1) cg::this_cluster().sync();
     else __syncthreads();
@@ -1375,8 +1454,8 @@ k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __res
   }
   __syncthreads();
   double* di = v.dinv + (int64_t)b * 2048;
-  if (threadIdx.x >= 32) tri_inverse<kUpper>(D, X[1], kb, into(di + 1024));
-  else tri_inverse<kUnitLower>(D, X[0], kb, into(di));
+  if (threadIdx.x >= 32) tri_inverse<kUpper, true>(D, X[1], kb, into(di + 1024));
+  else tri_inverse<kUnitLower, true>(D, X[0], kb, into(di));
 }
 
 }  // namespace

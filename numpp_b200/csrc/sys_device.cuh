@@ -151,10 +151,20 @@ __device__ __forceinline__ void update(Acc<NI>& acc, unsigned ring, const double
 // square below two neighbouring triangles T11, T22 of 8 and of 16 rows:
 // X21 = -X22 (T21 X11). One warp alone issues an instruction every four or five
 // cycles, so what counts is how few there are: whole tiles, no element tests.
+//
+// CHECK: a product with the inverse leaves a residual of the order of
+// eps max|T| max|T^-1| relative to the result, where substitution leaves eps. Up to
+// kTriProduct the two agree within a factor of two (6e-16 against 4e-16, the worst
+// of 4000 triangles of all scalings; 6e-15 at 1000, 6e-12 at 1e7); above it, or
+// with an infinity or a NaN, put gets T itself (its diagonal as reciprocals) and a
+// mark where a zero is otherwise, and whoever uses the block substitutes. Blocks of
+// n I + N(0,1) lie at 1, of N(0,1) at 2 to 20 but for the last.
+constexpr double kTriProduct = 32.0;
 enum TriKind { kUnitLower, kUpper, kLower };
-template <TriKind KIND, class Put>
+template <TriKind KIND, bool CHECK, class Put>
 __device__ __forceinline__ void tri_inverse(double* D, double* X, int kb, Put put) {
   constexpr bool UPPER = KIND == kUpper, DIAG = KIND != kUnitLower;
+  static_assert(!CHECK || KIND != kLower);
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   if (kb < 32) {
     for (int r = 0; r < 32; ++r)
@@ -248,6 +258,47 @@ __device__ __forceinline__ void tri_inverse(double* D, double* X, int kb, Put pu
         for (int e = 0; e < 2; ++e) at(16 + 8 * m + g, 8 * ni + 2 * t + e) = -x[m][ni][e];
   }
   __syncwarp();
+  if constexpr (CHECK) {
+    // high words of the magnitudes, of the kb x kb triangle proper
+    unsigned big_t = DIAG ? 0u : 0x3ff00000u, big_x = 0u;
+#pragma unroll 8
+    for (int r = 0; r < 32; ++r) {
+      const bool in = (UPPER ? r <= lane && lane < kb : r >= lane && r < kb);
+      const unsigned ht = (unsigned)__double2hiint(D[r * PS + lane]) & 0x7fffffffu;
+      const unsigned hx = (unsigned)__double2hiint(X[r * TS + lane]) & 0x7fffffffu;
+      if (in && (DIAG || r != lane)) big_t = max(big_t, ht);
+      if (in) big_x = max(big_x, hx);
+    }
+    big_t = __reduce_max_sync(kAll, big_t);
+    big_x = __reduce_max_sync(kAll, big_x);
+    const bool fine = big_t < 0x7ff00000u && big_x < 0x7ff00000u &&
+                      __hiloint2double((int)big_t, 0) * __hiloint2double((int)big_x, 0) <= kTriProduct;
+    if (!fine) {
+      // the diagonal as two factors of its reciprocal, both within range: a power of two
+      // in its place, the reciprocal of the rest in columns 0 and 1, zeros otherwise
+      double scale = 1.0, rest = 1.0;
+      if constexpr (UPPER) {
+        const double d = D[lane * PS + lane];
+        const unsigned h = (unsigned)__double2hiint(d) & 0x7fffffffu;
+        scale = h < 0x07b00000u ? 0x1p128 : h >= 0x78300000u ? 0x1p-128 : 1.0;  // 2^-900, 2^900
+        rest = 1.0 / (d * scale);
+      }
+#pragma unroll 1
+      for (int r = 0; r < 32; ++r) {
+        const double v = D[r * PS + lane], q = __shfl_sync(kAll, rest, r);
+        if constexpr (UPPER)
+          put(r, lane, r < lane ? v : r == lane ? scale : lane == 0 ? q : r == 31 && lane == 1 ? 1.0 : 0.0);
+        else
+          put(r, lane, r > lane ? v : r == lane || (r == 0 && lane == 31) ? 1.0 : 0.0);
+      }
+      if constexpr (UPPER) {
+        __syncwarp();
+        if (lane == 0) put(2, 1, rest);
+      }
+      __syncwarp();
+      return;
+    }
+  }
 #pragma unroll 4
   for (int r = 0; r < 32; ++r) {
     const bool zero = UPPER ? (lane < 16 && r >= 16) : (lane >= 16 && r < 16);

@@ -206,13 +206,16 @@ __device__ __forceinline__ void jacobi_round(double* J, int js, double* V, int v
   const float fc = (float)(fabs(cc) * power2(-((ea + eb) / 2)));
   worst = fmaxf(worst, fc * rsqrtf(fa * fb));
   // tan of the rotation angle, the smaller root of t^2 + 2 zeta t - 1 = 0 with
-  // zeta = (bb - aa) / (2 |cc|); both legs scaled by one power of two
-  const double p = fabs(bb - aa), s2 = 2.0 * fabs(cc);
-  const double down = power2(-max(min(max(exponent(p), exponent(s2)), 1022), -1022));
-  const float fp = (float)(p * down), fs = (float)(s2 * down);
-  float tn = fs / (fp + sqrtf(fmaf(fp, fp, fs * fs)));
-  if (bb < aa) tn = -tn;
-  const double td = tn, cs = rsqrt(fma(td, td, 1.0)), sn = cs * td;
+  // zeta = (bb - aa) / (2 |cc|); both legs halved and scaled by one power of two. An
+  // angle near or below FP32's range (columns of very different lengths) would
+  // never turn the pair: there the root is 1 / (2 zeta) to the last bit.
+  const double p = fabs(0.5 * bb - 0.5 * aa), s1 = fabs(cc);
+  const double down = power2(-max(min(max(exponent(p), exponent(s1)), 1022), -1022));
+  const float fp = (float)(p * down), fs = (float)(s1 * down);
+  double td = fs / (fp + sqrtf(fmaf(fp, fp, fs * fs)));
+  if (fs < 0x1p-60f * fp) td = 0.5 * (s1 / p);
+  if (bb < aa) td = -td;
+  const double cs = rsqrt(fma(td, td, 1.0)), sn = cs * td;
   const double sj = cc < 0.0 ? -sn : sn, cj = cc < 0.0 ? -cs : cs;
   if constexpr (R8 > 0) {
 #pragma unroll

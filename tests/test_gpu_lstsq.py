@@ -158,3 +158,22 @@ def test_nan_and_infinity_stay_where_they_are(lib):
             assert np.count_nonzero(np.isfinite(sv)) == 9
             np.testing.assert_allclose(np.sort(sv[np.isfinite(sv)])[::-1],
                                        np.linalg.svd(np.delete(A, col, 1), compute_uv=False), rtol=1e-12)
+
+
+@pytest.mark.parametrize("shift", [60, 100, 126, 140, 153, 300, 480])
+@pytest.mark.parametrize("m,n,col", [(40, 6, 0), (40, 6, 5), (100, 33, 16)])
+def test_columns_of_very_different_lengths(lib, m, n, col, shift):
+    """Scaling a column by a power of two scales its unknown by the inverse and changes nothing
+    else, also where the pair's rotation angle is far below FP32's range (rcond = 0: every column
+    counts). Bar: that of the unscaled problem (test_reduced_and_direct_sweeps)."""
+    rng = np.random.default_rng(m + col)
+    A, b = rng.standard_normal((m, n)), rng.standard_normal(m)
+    x0 = np.linalg.lstsq(A, b, rcond=None)[0]
+    s = np.linalg.svd(A, compute_uv=False)
+    As = A.copy()
+    As[:, col] *= 2.0 ** -shift
+    x, _, rank, _ = la.lstsq(As, b, rcond=0.0)
+    assert rank == n
+    x[col] *= 2.0 ** -shift
+    eps = np.finfo(float).eps
+    assert np.linalg.norm(x - x0) <= 50 * (m + n) * eps * (s[0] / s[-1]) ** 2 * np.linalg.norm(x0)

@@ -19,7 +19,7 @@
 //     rank, and the residuals.
 // Latency bounds it: N - 1 dependent rounds per sweep, each two dot-product
 // reductions deep plus a division, a square root and a reciprocal square root.
-// 1024 problems of 200 x 32 with one right-hand side, one B200: 0.67 ms, against
+// 1024 problems of 200 x 32 with one right-hand side, one B200: 0.68 ms, against
 // 18.2 ms with the whole CTA on one pair after the other on all 200 rows (1.2 ms
 // on the triangle with V accumulated and the angles in FP64).
 // Sums run in a different order than the reference's, so the results agree
@@ -41,6 +41,7 @@ constexpr int LT = 256;               // threads per problem
 constexpr int kLsqMaxN = 64;          // columns of the tall orientation
 constexpr int kLsqMaxK = 64;          // right-hand sides
 constexpr int32_t kLsqLeft = -1;      // rank of a problem that the first launch has left to the second
+constexpr double kLsqMostA = 0x1p480, kLsqMostB = 0x1p900;  // largest magnitudes that are reduced to the triangle
 constexpr size_t kLsqMaxSmem = 220 * 1024;  // dynamic shared memory of one problem
 
 #define NPPB_CUDA(call, what)                            \
@@ -289,7 +290,7 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
   double* sinv = sig + N;
   int* ord = reinterpret_cast<int*>(lsq + l.ord);
   __shared__ float s_off[LT / 32];
-  __shared__ int s_rank;
+  __shared__ int s_rank, s_leave;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NWARP = LT / 32;
@@ -302,11 +303,14 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
     const int r = idx / n, c = idx - r * n;
     const double x = Az[idx];
     W[wide ? r * l.ws + c : c * l.ws + r] = x;
-    odd |= !isfinite(x);
+    odd |= !(fabs(x) <= kLsqMostA);
   }
   // a NaN or an infinity must stay in its own column, where a reflection would
-  // spread it: such a problem is left to the launch that sweeps the matrix itself
+  // spread it, and a reflection's sums must stay within range: such a problem is
+  // left to the launch that sweeps the matrix itself (here, at a reflection of tiny
+  // length below, and at the right-hand sides)
   const bool qr = l.qr;
+  if (tid == 0) s_leave = 0;
   if (qr && __syncthreads_or(odd)) {
     if (tid == 0) rank[z] = kLsqLeft;
     return;
@@ -317,9 +321,14 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
     const int carried = wide ? 0 : l.nbuf;  // right-hand sides reflected along
     for (int idx = tid; idx < carried * M; idx += LT) {
       const int r = idx / carried, c = idx - r * carried;
-      buf[c * l.ws + r] = Bz[(int64_t)r * k + c];
+      const double x = Bz[(int64_t)r * k + c];
+      buf[c * l.ws + r] = x;
+      odd |= !(fabs(x) <= kLsqMostB);
     }
-    __syncthreads();
+    if (__syncthreads_or(odd)) {
+      if (tid == 0) rank[z] = kLsqLeft;
+      return;
+    }
     // Warp 0 takes column q + 1 first and derives reflection q + 1 from it
     // while the other columns are still being updated: one barrier per column.
     for (int q = -1; q < N; ++q) {
@@ -335,9 +344,22 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
           s2 = lane_sum<32>(s2);
           const double x0 = x[c];
           double beta = x0, tc = 0.0, hc = 1.0;
-          if (s2 != 0.0) {  // else nothing is left to annihilate
-            beta = -copysign(sqrt(fma(x0, x0, s2)), x0);
+          const double n2 = fma(x0, x0, s2);
+          if (n2 < 0x1p-960) {  // squares near or past the end of the range, or a column of zeros
+            bool some = false;
+            for (int r = c + lane; r < M; r += 32) some |= x[r] != 0.0;
+            if (__any_sync(0xffffffffu, some)) s_leave = 1;
+          } else if (s2 != 0.0) {  // else nothing is left to annihilate
+            beta = -copysign(sqrt(n2), x0);
             hc = x0 - beta;
+            // v near length 1 (an exact scaling): v^T x then stays within range with x
+            const int e = exponent(n2) >> 1;
+            if (e < -15 || e > 15) {
+              const double sc = power2(-e);
+              for (int r = c + 1 + lane; r < M; r += 32) x[r] *= sc;
+              hc *= sc;
+              s2 *= sc * sc;
+            }
             tc = 2.0 / fma(hc, hc, s2);
           }
           if (lane == 0) {
@@ -348,6 +370,10 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
         }
       }
       __syncthreads();
+    }
+    if (s_leave) {
+      if (tid == 0) rank[z] = kLsqLeft;
+      return;
     }
     // the triangle out of W: through registers, J's place may be W's
     double tri[kLsqMaxN * kLsqMaxN / LT];
@@ -448,14 +474,20 @@ again:
     if (qr && !wide && j0 > 0) {  // the first group went through the reflections with the matrix
       if (warp < jn) {
         double* x = buf + (size_t)warp * l.ws;
-        for (int r = lane; r < M; r += 32) x[r] = Bz[(int64_t)r * k + j0 + warp];
+        for (int r = lane; r < M; r += 32) {
+          x[r] = Bz[(int64_t)r * k + j0 + warp];
+          odd |= !(fabs(x[r]) <= kLsqMostB);
+        }
         __syncwarp();
         for (int q = 0; q < N; ++q) {
           reflect(W + (size_t)q * l.ws, head[q], tau[q], x, q, M);
           __syncwarp();
         }
       }
-      __syncthreads();
+      if (__syncthreads_or(odd)) {
+        if (tid == 0) rank[z] = kLsqLeft;
+        return;
+      }
     }
     if (full) {
       // R x = (Q^T b)'s first N rows (tall) or R^T y = b, x = Q y (wide): a warp

@@ -177,3 +177,55 @@ def test_columns_of_very_different_lengths(lib, m, n, col, shift):
     x[col] *= 2.0 ** -shift
     eps = np.finfo(float).eps
     assert np.linalg.norm(x - x0) <= 50 * (m + n) * eps * (s[0] / s[-1]) ** 2 * np.linalg.norm(x0)
+
+
+@pytest.mark.parametrize("m,n,k", [(200, 32, 1), (200, 32, 11), (64, 32, 3), (20, 90, 2)])
+@pytest.mark.parametrize("shift", [-600, -518, -505, -300, 300, 478, 500, 505])
+def test_entries_towards_the_ends_of_the_range(lib, m, n, k, shift):
+    """A scaled by a power of two scales S and the inverse of X; nothing else changes. Squares of
+    2^-518 are subnormal: their sums hold 2^-1074 / 2^(-1036 + 7) of a norm, and S with them;
+    those of 2^-600 are zero, and so is every singular value."""
+    rng = np.random.default_rng(m + k)
+    A, B = rng.standard_normal((m, n)), rng.standard_normal((m, k))
+    x, res, rank, s = la.lstsq(np.ldexp(A, shift), B)
+    if shift == -600:
+        assert rank == 0 and not s.any() and not x.any()
+        return
+    s0 = np.linalg.svd(A, compute_uv=False)
+    x0 = np.linalg.pinv(A) @ B
+    assert rank == min(m, n)
+    rel = 1e-9 if shift == -518 else 50 * (m + n) * np.finfo(float).eps * (s0[0] / s0[-1]) ** 2
+    np.testing.assert_allclose(np.ldexp(s, -shift), s0, rtol=rel)
+    assert np.linalg.norm(np.ldexp(x, shift) - x0) <= rel * np.linalg.norm(x0)
+    if m > n:
+        np.testing.assert_allclose(res, ((A @ x0 - B) ** 2).sum(axis=0), rtol=1e-8)
+
+
+@pytest.mark.parametrize("col", [0, 7, 31])
+@pytest.mark.parametrize("shift", [-600, -518, -480, -200, 200, 500])
+def test_one_column_towards_the_ends_of_the_range(lib, col, shift):
+    """Default tolerance: a tiny column counts as none, beside a huge one the others do."""
+    rng = np.random.default_rng(col)
+    A, B = rng.standard_normal((200, 32)), rng.standard_normal((200, 2))
+    A[:, col] = np.ldexp(A[:, col], shift)
+    x, _, rank, s = la.lstsq(A, B)
+    keep = np.arange(32) != col if shift < 0 else np.arange(32) == col
+    want = np.zeros((32, 2))
+    want[keep] = np.linalg.lstsq(A[:, keep], B, rcond=None)[0]
+    assert rank == keep.sum() and np.isfinite(s).all()
+    assert np.linalg.norm(x[keep] - want[keep]) <= 1e-10 * np.linalg.norm(want[keep])
+
+
+@pytest.mark.parametrize("j", [0, 9])
+@pytest.mark.parametrize("value", [np.nan, np.inf, 2.0 ** 1000])
+def test_right_hand_sides_out_of_range_stay_alone(lib, j, value):
+    rng = np.random.default_rng(5)
+    A, B = rng.standard_normal((100, 20)), rng.standard_normal((100, 12))
+    C = B.copy()
+    C[3, j] = value
+    x0 = la.lstsq(A, B)[0]
+    x = la.lstsq(A, C)[0]
+    others = np.arange(12) != j
+    np.testing.assert_allclose(x[:, others], x0[:, others], rtol=1e-10, atol=1e-12)
+    if np.isfinite(value):
+        np.testing.assert_allclose(x[:, j], np.linalg.pinv(A)[:, 3] * value, rtol=1e-10)

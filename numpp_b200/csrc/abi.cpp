@@ -2,6 +2,7 @@
 // C++20 host code over the sm_100a kernels; no exception crosses the ABI.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstring>
 #include <new>
@@ -84,6 +85,20 @@ int finish(cudaStream_t st) {
     if (rc_ != NPPB_OK) return rc_; \
   } while (0)
 
+// A uniform batch whole, or, while its workspace does not fit the device's memory, in
+// halves, quarters and so on one after the other: run(part) allocates for `part`
+// systems and works through the batch with that. (The inverses of the diagonal
+// blocks take 512 n bytes a system: several times a matrix of order 33.)
+template <class F>
+int in_parts(int64_t count, F&& run) {
+  for (int64_t part = count;; part = (part + 1) / 2) {
+    const int rc = run(part);
+    if (rc != NPPB_E_NOMEM || part == 1) return rc;
+    cudaGetLastError();
+    clear_error();
+  }
+}
+
 int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA, const double* dB,
              double* dX, double* dInv, double* dDet, double* dSign, double* dLogabs, double* dLU,
              int32_t* dipiv, int32_t* dinfo, cudaStream_t st) {
@@ -102,36 +117,52 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
   if (n > 32 && !(flags & NPPB_WANT_LU)) {
     // up to order 512 one CTA per system for the whole factorisation, above it outer
     // blocks; then one CTA or cluster per strip for the solves
-    DevMem w_m, perm_m, dinv_m, state_m;
-    NPPB_RC(scratch<double>(w_m, (size_t)count * n * sys_ld(n), st));
-    NPPB_RC(scratch<int32_t>(perm_m, (size_t)count * n, st));
-    NPPB_RC(scratch<double>(dinv_m, (size_t)count * sys_dinv(n), st));
-    NPPB_RC(scratch<int32_t>(state_m, (size_t)count, st));
-    SysArgs sa{};
-    sa.A = dA;
-    sa.W = w_m.as<double>();
-    sa.perm = perm_m.as<int32_t>();
-    sa.dinv = dinv_m.as<double>();
-    sa.state = state_m.as<int32_t>();
-    sa.state_stride = sizeof(int32_t);
-    sa.B = dB; sa.X = dX; sa.inv = dInv;
-    sa.det = (flags & NPPB_WANT_DET) ? dDet : nullptr;
-    sa.sign = (flags & NPPB_WANT_SLOGDET) ? dSign : nullptr;
-    sa.logabs = (flags & NPPB_WANT_SLOGDET) ? dLogabs : nullptr;
-    sa.info = dinfo;
-    sa.un = n;
-    sa.unrhs = (flags & NPPB_WANT_SOLVE) ? nrhs : 0;
-    sa.uinv = (flags & NPPB_WANT_INV) ? 1 : 0;
-    DevMem other_m, run_m;
-    if (n <= kSysMaxN) {
-      NPPB_CUDA(launch_sys_lu(sa, nullptr, (int)count, n, st), "batched LU launch");
-    } else {
-      NPPB_RC(scratch<int32_t>(other_m, (size_t)count * n, st));
-      NPPB_RC(scratch<double>(run_m, (size_t)count * 3, st));
-      NPPB_CUDA(run_sys_outer(sa, other_m.as<int32_t>(), run_m.as<double>(), (int)count, st), "batched LU launch");
-    }
-    NPPB_CUDA(launch_sys_solve_uniform(sa, (int)count, st), "batched substitution launch");
-    return NPPB_OK;
+    const int ld = sys_ld(n);
+    // a caller's workspace serves where its rows have the factors' stride and alignment
+    const bool given = dLU && ld == n && (reinterpret_cast<uintptr_t>(dLU) & 15) == 0;
+    return in_parts(count, [&](int64_t part) -> int {
+      DevMem w_m, perm_m, dinv_m, state_m, other_m, run_m;
+      if (!given) NPPB_RC(scratch<double>(w_m, (size_t)part * n * ld, st));
+      NPPB_RC(scratch<int32_t>(perm_m, (size_t)part * n, st));
+      NPPB_RC(scratch<double>(dinv_m, (size_t)part * sys_dinv(n), st));
+      NPPB_RC(scratch<int32_t>(state_m, (size_t)part, st));
+      if (n > kSysMaxN) {
+        NPPB_RC(scratch<int32_t>(other_m, (size_t)part * n, st));
+        NPPB_RC(scratch<double>(run_m, (size_t)part * 3, st));
+      }
+      for (int64_t s = 0; s < count; s += part) {
+        const int num = (int)std::min(part, count - s);
+        SysArgs sa{};
+        sa.A = dA + s * nn;
+        sa.W = given ? dLU + s * nn : w_m.as<double>();
+        sa.perm = perm_m.as<int32_t>();
+        sa.dinv = dinv_m.as<double>();
+        sa.state = state_m.as<int32_t>();
+        sa.state_stride = sizeof(int32_t);
+        if (flags & NPPB_WANT_SOLVE) {
+          sa.unrhs = nrhs;
+          if (dB) sa.B = dB + s * n * nrhs;
+          if (dX) sa.X = dX + s * n * nrhs;
+        }
+        if (flags & NPPB_WANT_INV) {
+          sa.uinv = 1;
+          sa.inv = dInv + s * nn;
+        }
+        if (flags & NPPB_WANT_DET) sa.det = dDet + s;
+        if (flags & NPPB_WANT_SLOGDET) {
+          sa.sign = dSign + s;
+          sa.logabs = dLogabs + s;
+        }
+        if (dinfo) sa.info = dinfo + s;
+        sa.un = n;
+        if (n <= kSysMaxN)
+          NPPB_CUDA(launch_sys_lu(sa, nullptr, num, n, st), "batched LU launch");
+        else
+          NPPB_CUDA(run_sys_outer(sa, other_m.as<int32_t>(), run_m.as<double>(), num, st), "batched LU launch");
+        NPPB_CUDA(launch_sys_solve_uniform(sa, num, st), "batched substitution launch");
+      }
+      return NPPB_OK;
+    });
   }
   if (n > 32) {
     // factors kept (getrf): a cached uniform plan also carries the row moves
@@ -183,20 +214,26 @@ int d_getrs(int64_t count, int32_t n, int32_t nrhs, const double* dLU, const int
     // the permutation and the diagonal blocks' inverses, then both
     // substitutions in one launch (every strip is read before it is written, so
     // X may be B)
-    DevMem perm_m, dinv_m;
-    NPPB_RC(scratch<int32_t>(perm_m, (size_t)count * n, st));
-    NPPB_RC(scratch<double>(dinv_m, (size_t)count * sys_dinv(n), st));
-    SysArgs sa{};
-    sa.W = const_cast<double*>(dLU);
-    sa.w_by_position = 1;
-    sa.perm = perm_m.as<int32_t>();
-    sa.dinv = dinv_m.as<double>();
-    sa.B = dB; sa.X = dX;
-    sa.un = n;
-    sa.unrhs = nrhs;
-    NPPB_CUDA(launch_sys_prepare(sa, dipiv, nullptr, (int)count, n, st), "getrs preparation launch");
-    NPPB_CUDA(launch_sys_solve_uniform(sa, (int)count, st), "getrs launch");
-    return NPPB_OK;
+    return in_parts(count, [&](int64_t part) -> int {
+      DevMem perm_m, dinv_m;
+      NPPB_RC(scratch<int32_t>(perm_m, (size_t)part * n, st));
+      NPPB_RC(scratch<double>(dinv_m, (size_t)part * sys_dinv(n), st));
+      for (int64_t s = 0; s < count; s += part) {
+        const int num = (int)std::min(part, count - s);
+        SysArgs sa{};
+        sa.W = const_cast<double*>(dLU) + s * n * n;
+        sa.w_by_position = 1;
+        sa.perm = perm_m.as<int32_t>();
+        sa.dinv = dinv_m.as<double>();
+        sa.B = dB + s * n * nrhs;
+        sa.X = dX + s * n * nrhs;
+        sa.un = n;
+        sa.unrhs = nrhs;
+        NPPB_CUDA(launch_sys_prepare(sa, dipiv + s * n, nullptr, num, n, st), "getrs preparation launch");
+        NPPB_CUDA(launch_sys_solve_uniform(sa, num, st), "getrs launch");
+      }
+      return NPPB_OK;
+    });
   }
   Batch bt{};
   bt.A = dLU; bt.LU = const_cast<double*>(dLU); bt.ipiv = const_cast<int32_t*>(dipiv);

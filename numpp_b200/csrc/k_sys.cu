@@ -604,11 +604,11 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
       }
       return;
     }
-    // the diagonal block's inverses and the pivots' part of det / slogdet, each by
+    // the diagonal block's inverses (U's for the substitution only) and the pivots' part of det / slogdet, each by
     // one warp, beside the other warps' loads of the next column block
     double* di = s_v.dinv + (int64_t)J * 2048;
     if (warp == 0) tri_inverse<kUnitLower, false>(D11, stage, kb, into(di));
-    if (warp == 1 % nw) tri_inverse<kUpper, true>(D11, stage, kb, into(di + 1024));
+    if ((sa.X || sa.inv) && warp == 1 % nw) tri_inverse<kUpper, true>(D11, stage, kb, into(di + 1024));
     if (warp == 2 % nw && (sa.det || sa.sign || sa.logabs)) {
       // folded in the reference's order (linalg.cpp:400-403, 425-431)
       const double pv = lane < kb ? D11[lane * PS + lane] : 1.0;
@@ -1031,7 +1031,7 @@ k_sys_outer(SysArgs sa, const int32_t* __restrict__ perm_in, int32_t* __restrict
     double* di = s_v.dinv + (int64_t)J * 2048;
     if ((J - jb) % CS == rank) {
       if (warp == 0) tri_inverse<kUnitLower, false>(D11, stage, kb, into(di));
-      if (warp == 1 % nw) tri_inverse<kUpper, true>(D11, stage, kb, into(di + 1024));
+      if ((sa.X || sa.inv) && warp == 1 % nw) tri_inverse<kUpper, true>(D11, stage, kb, into(di + 1024));
     }
     if (rank == 0 && warp == 2 % nw) {
       // folded in the reference's order (linalg.cpp:400-403, 425-431)
@@ -1521,6 +1521,7 @@ cudaError_t launch_sys_update(const SysArgs& sa, const int32_t* perm, int nsys, 
 }
 
 cudaError_t launch_sys_copy(const SysArgs& sa, int nsys, cudaStream_t st) {
+  if (sa.A == sa.W) return cudaSuccess;  // in place
   const int64_t rows = (int64_t)nsys * sa.un;
   k_sys_copy<<<(unsigned)std::min<int64_t>((rows + 7) / 8, 148 * 16), 256, 0, st>>>(sa.A, sa.W, rows, sa.un,
                                                                                     sys_ld(sa.un));

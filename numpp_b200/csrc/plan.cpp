@@ -96,21 +96,49 @@ Plan::~Plan() {
   if (fork) cudaEventDestroy(fork);
   if (done) cudaEventDestroy(done);
   if (cap) cudaStreamDestroy(cap);
-  for (void* p : {(void*)d_desc, (void*)d_order, (void*)d_lu, (void*)d_piv, (void*)d_scratch,
-                  (void*)d_step_list, (void*)d_items, (void*)d_back, (void*)d_sys_list, (void*)d_sys_items,
-                  (void*)d_perm, (void*)d_dinv, (void*)d_state})
-    if (p) {
-      if (alloc_stream) cudaFreeAsync(p, alloc_stream);
-      else cudaFree(p);
-    }
+  release();
   for (void* p : {(void*)hA, (void*)hB, (void*)hX, (void*)hInv, (void*)hDet, (void*)hSign, (void*)hLog, (void*)hInfo})
     if (p) cudaFree(p);
   if (prev >= 0) cudaSetDevice(prev);
 }
 
+// The tables, workspaces and classes of a build.
+void Plan::release() {
+  auto drop = [&](auto*& p) {
+    if (p && alloc_stream) cudaFreeAsync(p, alloc_stream);
+    else if (p) cudaFree(p);
+    p = nullptr;
+  };
+  drop(d_desc); drop(d_order); drop(d_lu); drop(d_piv); drop(d_scratch); drop(d_step_list); drop(d_items); drop(d_back);
+  drop(d_sys_list); drop(d_sys_items); drop(d_perm); drop(d_dinv); drop(d_state);
+  warp_classes.clear();
+  sys_classes.clear();
+  chains.clear();
+  a_elems = b_elems = inv_elems = lu_elems = piv_elems = 0;
+  nsys = nstep_sys = nback = 0;
+  step_nmax = 0;
+  sys_flops = sys_bytes = step_flops = step_bytes = 0.0;
+  for (double& f : kind_flops) f = 0.0;
+}
+
 int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_t* a_off,
                 const int64_t* b_off, const int64_t* inv_off, int fl, bool solve_only_, bool own_lu,
                 const int64_t* lu_off_ext, const int64_t* piv_off_ext) {
+  int rc = build_with(true, cnt, n, nrhs, a_off, b_off, inv_off, fl, solve_only_, own_lu, lu_off_ext, piv_off_ext);
+  if (rc == NPPB_E_NOMEM && nsys) {
+    // no room for the diagonal blocks' inverses (512 n bytes a system): the step
+    // kernels keep 8616 bytes a system instead
+    cudaGetLastError();
+    clear_error();
+    release();
+    rc = build_with(false, cnt, n, nrhs, a_off, b_off, inv_off, fl, solve_only_, own_lu, lu_off_ext, piv_off_ext);
+  }
+  return rc;
+}
+
+int Plan::build_with(bool sys_path, int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_t* a_off,
+                     const int64_t* b_off, const int64_t* inv_off, int fl, bool solve_only_, bool own_lu,
+                     const int64_t* lu_off_ext, const int64_t* piv_off_ext) {
   if ((lu_off_ext == nullptr) != (piv_off_ext == nullptr)) return arg_error("factor offsets come in pairs");
   ext_factors = lu_off_ext != nullptr;
   if (ext_factors) own_lu = false;
@@ -134,7 +162,7 @@ int Plan::build(int64_t cnt, const int32_t* n, const int32_t* nrhs, const int64_
   std::vector<std::vector<int32_t>> warp_members(3);
   std::vector<int32_t> sys_members, step_members;
   // orders 33..512 whose factors are not kept: one CTA per system
-  const bool resident = own_lu && !solve_only && !(fl & NPPB_WANT_LU);
+  const bool resident = sys_path && own_lu && !solve_only && !(fl & NPPB_WANT_LU);
   int64_t lu = 0, piv = 0, perm = 0, dinv = 0;
   for (int64_t i = 0; i < cnt; ++i) {
     const int ni = n[i];
@@ -429,8 +457,8 @@ SysArgs Plan::sys_args(const Ptrs& p) const {
   sa.perm = d_perm;
   sa.dinv = d_dinv;
   sa.B = p.B;
-  sa.X = p.X;
-  sa.inv = p.Inv;
+  sa.X = (flags & NPPB_WANT_SOLVE) ? p.X : nullptr;
+  sa.inv = (flags & NPPB_WANT_INV) ? p.Inv : nullptr;
   sa.det = p.Det;
   sa.sign = p.Sign;
   sa.logabs = p.Logabs;

@@ -132,6 +132,10 @@ class Plan {
   int32_t* hInfo = nullptr;
 
  private:
+  int build_with(bool sys_path, int64_t count, const int32_t* n, const int32_t* nrhs, const int64_t* a_off,
+                 const int64_t* b_off, const int64_t* inv_off, int flags, bool solve_only, bool own_lu,
+                 const int64_t* lu_off_ext, const int64_t* piv_off_ext);
+  void release();
   void add_cost(const SysDesc& s, double& fl, double& by) const;
   cudaError_t ensure_lookahead();  // a side stream and two events per chain
   // forward (getrs) or back substitution of one chain's strips

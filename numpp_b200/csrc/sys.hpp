@@ -57,7 +57,7 @@ struct SysArgs {
   int32_t* perm;        // position -> row of A (and of W, unless w_by_position)
   double* dinv;         // inverses of the diagonal blocks
   const double* B;
-  double* X;
+  double* X;            // X and inv null: nothing is solved for
   double* inv;
   double* det;
   double* sign;

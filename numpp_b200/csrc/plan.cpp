@@ -48,21 +48,54 @@ int arg_error(const std::string& m) {
     if (e_ != cudaSuccess) return nppb::cuda_status(e_, what); \
   } while (0)
 
-// Device allocation of a plan: plain, or stream-ordered on `ord` (no device
-// synchronisation; used by plans built and dropped per batch).
-cudaError_t plan_alloc(void** p, size_t bytes, cudaStream_t ord) {
-  return ord ? cudaMallocAsync(p, bytes, ord) : cudaMalloc(p, bytes);
-}
+// The tables and workspaces of a plan in one device allocation (plain, or
+// stream-ordered on `ord`: no device synchronisation, for plans built and dropped per
+// batch), the tables in front and in one upload.
+class Arena {
+ public:
+  template <class T>
+  void table(T*& d, const std::vector<T>& h) {
+    if (h.empty()) return;
+    const size_t at = reserve(sizeof(T) * h.size());
+    host_.resize(at + sizeof(T) * h.size());
+    std::memcpy(host_.data() + at, h.data(), sizeof(T) * h.size());
+    place(d, at);
+  }
+  template <class T>
+  void scratch(T*& d, int64_t count) {
+    if (count > 0) place(d, reserve(sizeof(T) * (size_t)count));
+  }
+  int make(void** base, cudaStream_t ord) {
+    if (!end_) return NPPB_OK;
+    NPPB_CUDA(ord ? cudaMallocAsync(base, end_, ord) : cudaMalloc(base, end_), "plan allocation");
+    for (const Place& p : places_) p.set(p.slot, static_cast<char*>(*base) + p.at);
+    if (host_.empty()) return NPPB_OK;
+    // from pageable memory: the call returns once the source has been staged
+    NPPB_CUDA(ord ? cudaMemcpyAsync(*base, host_.data(), host_.size(), cudaMemcpyHostToDevice, ord)
+                  : cudaMemcpy(*base, host_.data(), host_.size(), cudaMemcpyHostToDevice),
+              "plan upload");
+    return NPPB_OK;
+  }
 
-template <class T>
-int upload(T** d, const std::vector<T>& h, cudaStream_t ord) {
-  if (h.empty()) return NPPB_OK;
-  NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(d), sizeof(T) * h.size(), ord), "plan allocation");
-  // from pageable memory: the call returns once the source has been staged
-  if (ord) NPPB_CUDA(cudaMemcpyAsync(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, ord), "plan upload");
-  else NPPB_CUDA(cudaMemcpy(*d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice), "plan upload");
-  return NPPB_OK;
-}
+ private:
+  size_t reserve(size_t bytes) {
+    const size_t at = end_;
+    end_ += (bytes + 255) & ~size_t{255};
+    return at;
+  }
+  struct Place {
+    void* slot;  // a T*
+    void (*set)(void* slot, void* p);
+    size_t at;
+  };
+  template <class T>
+  void place(T*& d, size_t at) {
+    places_.push_back({&d, [](void* slot, void* p) { *static_cast<T**>(slot) = static_cast<T*>(p); }, at});
+  }
+  std::vector<char> host_;
+  std::vector<Place> places_;
+  size_t end_ = 0;
+};
 
 // one class per k_panel configuration (CTA size, rows per thread, cluster size)
 int panel_class(int m) {
@@ -104,13 +137,15 @@ Plan::~Plan() {
 
 // The tables, workspaces and classes of a build.
 void Plan::release() {
-  auto drop = [&](auto*& p) {
-    if (p && alloc_stream) cudaFreeAsync(p, alloc_stream);
-    else if (p) cudaFree(p);
-    p = nullptr;
-  };
-  drop(d_desc); drop(d_order); drop(d_lu); drop(d_piv); drop(d_scratch); drop(d_step_list); drop(d_items); drop(d_back);
-  drop(d_sys_list); drop(d_sys_items); drop(d_perm); drop(d_dinv); drop(d_state);
+  if (arena && alloc_stream) cudaFreeAsync(arena, alloc_stream);
+  else if (arena) cudaFree(arena);
+  arena = nullptr;
+  d_desc = nullptr;
+  d_order = d_step_list = d_sys_list = d_perm = d_state = d_piv = nullptr;
+  d_items = d_back = nullptr;
+  d_sys_items = nullptr;
+  d_scratch = nullptr;
+  d_dinv = d_lu = nullptr;
   warp_classes.clear();
   sys_classes.clear();
   chains.clear();
@@ -189,10 +224,11 @@ int Plan::build_with(bool sys_path, int64_t cnt, const int32_t* n, const int32_t
     s.inv_off = (want_inv && inv_off[i] >= 0) ? inv_off[i] : -1;
     s.piv_off = ext_factors ? piv_off_ext[i] : piv;
     lu += (int64_t)ni * (sys ? sys_ld(ni) : ni);
-    piv += ni;
-    if (sys) {
+    if (sys) {  // its pivots are the permutation
       perm += ni;
       dinv += sys_dinv(ni);
+    } else {
+      piv += ni;
     }
     a_elems = std::max(a_elems, a_off[i] + (int64_t)ni * ni);
     if (solve) b_elems = std::max(b_elems, b_off[i] + (int64_t)ni * ki);
@@ -371,29 +407,21 @@ int Plan::build_with(bool sys_path, int64_t cnt, const int32_t* n, const int32_t
   else lookahead = lookahead_mode != 0;
   nback = (int64_t)back.size();
 
-  int rc = upload(&d_desc, desc, alloc_stream);
-  if (rc == NPPB_OK) rc = upload(&d_order, order, alloc_stream);
-  if (rc == NPPB_OK) rc = upload(&d_step_list, step_members, alloc_stream);
-  if (rc == NPPB_OK) rc = upload(&d_items, items, alloc_stream);
-  if (rc == NPPB_OK) rc = upload(&d_back, back, alloc_stream);
-  if (rc == NPPB_OK) rc = upload(&d_sys_list, sys_members, alloc_stream);
-  if (rc == NPPB_OK) rc = upload(&d_sys_items, sys_items, alloc_stream);
-  if (rc != NPPB_OK) return rc;
-  if (nsys) {
-    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_perm), sizeof(int32_t) * perm, alloc_stream), "plan scratch");
-    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_dinv), sizeof(double) * dinv, alloc_stream), "plan scratch");
-    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_state), sizeof(int32_t) * nsys, alloc_stream), "plan scratch");
-  }
-  if (nstep_sys)
-    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_scratch), sizeof(StepScratch) * nstep_sys, alloc_stream),
-              "plan scratch");
-  if (lu_elems)
-    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_lu), sizeof(double) * lu_elems, alloc_stream),
-              "plan LU workspace");
-  if (piv_elems)
-    NPPB_CUDA(plan_alloc(reinterpret_cast<void**>(&d_piv), sizeof(int32_t) * piv_elems, alloc_stream),
-              "plan pivot workspace");
-  return NPPB_OK;
+  Arena mem;
+  mem.table(d_desc, desc);
+  mem.table(d_order, order);
+  mem.table(d_step_list, step_members);
+  mem.table(d_items, items);
+  mem.table(d_back, back);
+  mem.table(d_sys_list, sys_members);
+  mem.table(d_sys_items, sys_items);
+  mem.scratch(d_perm, perm);
+  mem.scratch(d_dinv, dinv);
+  mem.scratch(d_state, nsys);
+  mem.scratch(d_scratch, nstep_sys);
+  mem.scratch(d_lu, lu_elems);
+  mem.scratch(d_piv, piv_elems);
+  return mem.make(&arena, alloc_stream);
 }
 
 void Plan::add_cost(const SysDesc& s, double& fl, double& by) const {

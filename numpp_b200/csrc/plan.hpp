@@ -112,6 +112,7 @@ class Plan {
   int step_nmax = 0;
   double sys_flops = 0.0, sys_bytes = 0.0, step_flops = 0.0, step_bytes = 0.0;
 
+  void* arena = nullptr;  // one allocation: every table and workspace below lies in it
   SysDesc* d_desc = nullptr;
   int32_t* d_order = nullptr;
   int32_t* d_step_list = nullptr;

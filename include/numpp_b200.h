@@ -298,8 +298,9 @@ int nppb_plan_execute(nppb_plan* plan, const double* dA, const double* dB, doubl
  * the current trailing update inside a chain), on these device buffers, a
  * warm-up and two replays each, and keeps the fastest; *chains_out = the
  * chain count kept, negated when look-ahead is on; *ms_out = its time per
- * execution. The outputs are written as by nppb_plan_execute; synchronises
- * `stream`. */
+ * execution. A plan without step chains (every order at most 512) has one
+ * configuration: it is kept, and timed for *ms_out. The outputs are written
+ * as by nppb_plan_execute; synchronises `stream`. */
 int nppb_plan_autotune(nppb_plan* plan, const double* dA, const double* dB, double* dX, double* dInv,
                        double* dDet, double* dSign, double* dLogabs, int32_t* dinfo, void* stream,
                        int32_t* chains_out, float* ms_out);

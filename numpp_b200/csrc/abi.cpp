@@ -138,7 +138,6 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
         sa.perm = perm_m.as<int32_t>();
         sa.dinv = dinv_m.as<double>();
         sa.state = state_m.as<int32_t>();
-        sa.state_stride = sizeof(int32_t);
         if (flags & NPPB_WANT_SOLVE) {
           sa.unrhs = nrhs;
           if (dB) sa.B = dB + s * n * nrhs;
@@ -229,7 +228,7 @@ int d_getrs(int64_t count, int32_t n, int32_t nrhs, const double* dLU, const int
         sa.X = dX + s * n * nrhs;
         sa.un = n;
         sa.unrhs = nrhs;
-        NPPB_CUDA(launch_sys_prepare(sa, dipiv + s * n, nullptr, num, n, st), "getrs preparation launch");
+        NPPB_CUDA(launch_sys_prepare(sa, dipiv + s * n, num, st), "getrs preparation launch");
         NPPB_CUDA(launch_sys_solve_uniform(sa, num, st), "getrs launch");
       }
       return NPPB_OK;

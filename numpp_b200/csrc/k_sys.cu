@@ -83,10 +83,6 @@ __device__ __forceinline__ View view(const SysArgs& sa, int s) {
   return v;
 }
 
-__device__ __forceinline__ int32_t* state_of(const SysArgs& sa, int slot) {
-  return reinterpret_cast<int32_t*>(reinterpret_cast<char*>(sa.state) + (int64_t)slot * sa.state_stride);
-}
-
 __device__ __forceinline__ void bar_active(int threads) {  // the warps of the panel
   asm volatile("bar.sync 1, %0;\n" ::"r"(threads) : "memory");
 }
@@ -596,7 +592,7 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
     __syncthreads();
     if (ps.info) {
       if (tid == 0) {
-        if (sa.state) *state_of(sa, s_v.slot) = ps.info;
+        if (sa.state) sa.state[s_v.slot] = ps.info;
         if (sa.det) sa.det[s_v.idx] = 0.0;
         if (sa.sign) sa.sign[s_v.idx] = 0.0;
         if (sa.logabs) sa.logabs[s_v.idx] = -INFINITY;
@@ -634,7 +630,7 @@ k_sys_lu(SysArgs sa, const int32_t* __restrict__ list) {
   }
   for (int i = tid; i < n; i += blockDim.x) s_v.perm[i] = s_perm[i];
   if (tid == 0) {
-    if (sa.state) *state_of(sa, s_v.slot) = 0;
+    if (sa.state) sa.state[s_v.slot] = 0;
     if (sa.info) sa.info[s_v.idx] = 0;
   }
 }
@@ -916,7 +912,7 @@ k_sys_outer(SysArgs sa, const int32_t* __restrict__ perm_in, int32_t* __restrict
   const int sys = (int)blockIdx.x / CS;
   if (tid == 0) {
     s_v = view(sa, sys);
-    s_skip = jb > 0 && *state_of(sa, s_v.slot);
+    s_skip = jb > 0 && sa.state[s_v.slot];
     const double* run = running + 3 * (int64_t)s_v.slot;
     s_det[0] = jb ? run[0] : 1.0;
     s_det[1] = jb ? run[1] : 0.0;
@@ -1003,7 +999,7 @@ k_sys_outer(SysArgs sa, const int32_t* __restrict__ perm_in, int32_t* __restrict
     const int info = cluster_panel<CS>(sh, table, acc, pos, valid, active, kb, blk - J, nb - J, w0, w1, stage, nswap);
     if (info) {  // the same in every thread of the cluster; nothing is on its way to another CTA
       if (tid == 0 && rank == 0) {
-        *state_of(sa, s_v.slot) = 32 * J + info;
+        sa.state[s_v.slot] = 32 * J + info;
         if (sa.det) sa.det[s_v.idx] = 0.0;
         if (sa.sign) sa.sign[s_v.idx] = 0.0;
         if (sa.logabs) sa.logabs[s_v.idx] = -INFINITY;
@@ -1071,7 +1067,7 @@ k_sys_outer(SysArgs sa, const int32_t* __restrict__ perm_in, int32_t* __restrict
     if (p < n) pout[p] = s_perm[i];
   }
   if (tid == 0 && rank == 0) {
-    *state_of(sa, s_v.slot) = 0;
+    sa.state[s_v.slot] = 0;
     if (sa.info && je == nb) sa.info[s_v.idx] = 0;
   }
 }
@@ -1090,7 +1086,7 @@ k_sys_rows(SysArgs sa, const int32_t* __restrict__ perm, int jb, int je, int c0,
   const unsigned ring = smem(sm + kWarp + warp * kPerWarp) + 16 * lane;
   if (threadIdx.x == 0) {
     s_v = view(sa, blockIdx.y);
-    s_skip = *state_of(sa, s_v.slot);
+    s_skip = sa.state[s_v.slot];
   }
   __syncthreads();
   if (s_skip) return;
@@ -1157,7 +1153,7 @@ k_sys_gemm(SysArgs sa, const int32_t* __restrict__ perm, int jb, int je, int c0,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   if (tid == 0) {
     s_v = view(sa, blockIdx.z);
-    s_skip = *state_of(sa, s_v.slot);
+    s_skip = sa.state[s_v.slot];
   }
   __syncthreads();
   if (s_skip) return;
@@ -1405,7 +1401,7 @@ k_sys_solve(SysArgs sa, const SysItem* __restrict__ items, int inverse, int firs
     s_s.ldx = it.inverse ? v.n : v.nrhs;
     s_s.B = sa.B + v.b_off + it.c0;
     s_s.X = (it.inverse ? sa.inv + v.inv_off : sa.X + v.b_off) + it.c0;
-    s_skip = sa.state && *state_of(sa, v.slot);  // singular: nothing to solve with
+    s_skip = sa.state && sa.state[v.slot];  // singular: nothing to solve with
   }
   __syncthreads();
   if (!s_skip) solve_strip<NI, VEC, CS>(sa, s_s, sm);  // the same for every CTA of a cluster
@@ -1414,18 +1410,16 @@ k_sys_solve(SysArgs sa, const SysItem* __restrict__ items, int inverse, int firs
 // ---------------------------------------------------------------------------
 // Kept factors: the permutation of the swap list (every thread follows its own
 // rows through the swaps; the list is read by broadcast) in CTA (s, 0), the
-// diagonal blocks' inverses in the CTAs (s, b).
+// diagonal blocks' inverses in the CTAs (s, b + 1).
 __global__ void __launch_bounds__(64)
-k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv, const int32_t* __restrict__ list) {
+k_sys_prepare(SysArgs sa, const int32_t* __restrict__ ipiv) {
   __shared__ double D[32 * PS];
   __shared__ double X[2][32 * TS];
-  const int s = list ? list[blockIdx.x] : blockIdx.x;
-  const View v = view(sa, s);
+  const View v = view(sa, blockIdx.x);
   const int n = v.n, b = (int)blockIdx.y - 1;
-  if (b >= sys_blocks(n)) return;
   if (b < 0) {
     extern __shared__ int piv[];
-    const int32_t* src = ipiv + (sa.desc ? sa.desc[s].piv_off : (int64_t)s * n);
+    const int32_t* src = ipiv + (int64_t)blockIdx.x * n;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
       const int p = src[i];
       piv[i] = p < i || p >= n ? i : p;  // a swap list only names rows >= its own
@@ -1616,11 +1610,9 @@ cudaError_t launch_sys_solve_uniform(const SysArgs& sa, int nsys, cudaStream_t s
   return e;
 }
 
-cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int32_t* list, int nsys, int nmax,
-                               cudaStream_t st) {
-  if (nsys <= 0) return cudaSuccess;
-  const dim3 grid((unsigned)nsys, (unsigned)sys_blocks(nmax) + 1);
-  k_sys_prepare<<<grid, 64, sizeof(int) * (size_t)nmax, st>>>(sa, ipiv, list);
+cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, int nsys, cudaStream_t st) {
+  const dim3 grid((unsigned)nsys, (unsigned)sys_blocks(sa.un) + 1);
+  k_sys_prepare<<<grid, 64, sizeof(int) * (size_t)sa.un, st>>>(sa, ipiv);
   return cudaGetLastError();
 }
 

@@ -19,10 +19,9 @@
 // workspace and the step state before reading them). Calls that overlap on the
 // GPU race on it.
 //
-// This solve always takes the single-level step kernels (it ignores
-// NPPB_BLOCKED_MIN_N, whose two-level schedule needs a per-call history
-// buffer), so with that variable set its results can differ from the
-// allocating solve's in the last bits.
+// This solve always takes the step kernels, whose workspace is a matrix and 8616 bytes
+// a system; the allocating solve takes the system-resident kernels above order 32,
+// so the two can differ in the last bits.
 #include <cuda_runtime.h>
 
 #include <cstddef>

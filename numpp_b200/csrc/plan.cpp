@@ -492,7 +492,6 @@ SysArgs Plan::sys_args(const Ptrs& p) const {
   sa.logabs = p.Logabs;
   sa.info = p.info;
   sa.state = d_state;
-  sa.state_stride = sizeof(int32_t);
   return sa;
 }
 

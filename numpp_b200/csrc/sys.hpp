@@ -63,8 +63,7 @@ struct SysArgs {
   double* sign;
   double* logabs;
   int32_t* info;        // per-system output (may be null)
-  int32_t* state;       // first zero pivot + 1 or 0, by slot (null: every system is solved),
-  int state_stride;     //   so many bytes apart
+  int32_t* state;       // first zero pivot + 1 or 0, by slot (null: every system is solved)
   int un, unrhs, uinv;  // uniform batch
   int w_by_position;    // W holds rows in pivoted order with leading dimension n (kept factors)
 };
@@ -90,10 +89,9 @@ inline int sys_width_class(int width) { return width <= 8 ? 0 : width <= 16 ? 1 
 cudaError_t launch_sys_solve(const SysArgs& sa, const SysItem* items, int64_t nitems, int width, int nmax,
                              cudaStream_t st);
 cudaError_t launch_sys_solve_uniform(const SysArgs& sa, int nsys, cudaStream_t st);
-// Permutations and diagonal inverses of kept factors (swap lists ipiv at
-// piv_off): fills sa.perm and sa.dinv.
-cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, const int32_t* list, int nsys, int nmax,
-                               cudaStream_t st);
+// Permutations and diagonal inverses of a uniform batch's kept factors (swap lists
+// ipiv): fills sa.perm and sa.dinv.
+cudaError_t launch_sys_prepare(const SysArgs& sa, const int32_t* ipiv, int nsys, cudaStream_t st);
 cudaError_t sys_prepare_kernels();
 
 }  // namespace nppb

@@ -150,14 +150,13 @@ Lookahead* lookahead_for_device() {
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
   if ((int)h.per_dev.size() <= dev) h.per_dev.resize(dev + 1);
   Lookahead& l = h.per_dev[dev];
-  if (!l.side) {
+  if (!l.next) {  // the last of them: all are there, or what is missing is tried again
     int least = 0, greatest = 0;
     cudaDeviceGetStreamPriorityRange(&least, &greatest);
-    if (cudaStreamCreateWithFlags(&l.side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithPriority(&l.panel, cudaStreamNonBlocking, greatest) != cudaSuccess ||
-        cudaEventCreateWithFlags(&l.first, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&l.rest, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&l.next, cudaEventDisableTiming) != cudaSuccess) {
+    auto event = [](cudaEvent_t& e) { return e || cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess; };
+    if (!(l.side || cudaStreamCreateWithFlags(&l.side, cudaStreamNonBlocking) == cudaSuccess) ||
+        !(l.panel || cudaStreamCreateWithPriority(&l.panel, cudaStreamNonBlocking, greatest) == cudaSuccess) ||
+        !event(l.first) || !event(l.rest) || !event(l.next)) {
       cudaGetLastError();
       return nullptr;
     }
@@ -219,32 +218,43 @@ cudaError_t run_sys_outer(const SysArgs& sa, int32_t* other, double* running, in
   perm[steps & 1] = sa.perm;
   perm[(steps + 1) & 1] = other;
   Lookahead* la = lookahead_for_device();
-  if (!la) return cudaErrorUnknown;
+  const cudaStream_t ps = la ? la->panel : st, us = la ? la->side : st;  // without them: one after the other
+  // `to` goes on behind everything so far on `from`
+  auto behind = [&](cudaStream_t to, cudaStream_t from, cudaEvent_t ev) -> cudaError_t {
+    if (to == from) return cudaSuccess;
+    const cudaError_t r = cudaEventRecord(ev, from);
+    return r == cudaSuccess ? cudaStreamWaitEvent(to, ev, 0) : r;
+  };
+  const cudaEvent_t first = la ? la->first : nullptr, next = la ? la->next : nullptr, upd = la ? la->rest : nullptr;
   cudaError_t e = launch_sys_copy(sa, nsys, st);
-  if (e == cudaSuccess) e = cudaEventRecord(la->first, st);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(la->panel, la->first, 0);
+  if (e == cudaSuccess) e = behind(ps, st, first);
+  if (e != cudaSuccess) return e;
   bool rest = false;  // an update on the side stream
   for (int k = 0; k < steps && e == cudaSuccess; ++k) {
     const int jb = k * kSysOuter, je = std::min(nb, jb + kSysOuter);
     const int c0 = std::min(n, 32 * je), c1 = std::min(n, c0 + 32 * kSysOuter);
     int32_t* now = perm[(k + 1) & 1];
-    e = launch_sys_outer(sa, perm[k & 1], now, running, nsys, jb, je, la->panel);
+    e = launch_sys_outer(sa, perm[k & 1], now, running, nsys, jb, je, ps);
     if (e != cudaSuccess || c0 >= n) break;
-    if (rest) e = cudaStreamWaitEvent(la->panel, la->rest, 0);  // the previous update covers these columns
-    rest = false;
+    if (rest) {  // the previous update covers these columns
+      e = behind(ps, us, upd);
+      rest = e != cudaSuccess;
+    }
     if (e == cudaSuccess && c1 < n) {
-      e = cudaEventRecord(la->next, la->panel);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(la->side, la->next, 0);
-      if (e == cudaSuccess) e = launch_sys_update(sa, now, nsys, jb, je, c1, n, la->side);
-      if (e == cudaSuccess) e = cudaEventRecord(la->rest, la->side);
+      e = behind(us, ps, next);
+      if (e == cudaSuccess) e = launch_sys_update(sa, now, nsys, jb, je, c1, n, us);
       rest = true;
     }
-    if (e == cudaSuccess) e = launch_sys_update(sa, now, nsys, jb, je, c0, c1, la->panel);
+    if (e == cudaSuccess) e = launch_sys_update(sa, now, nsys, jb, je, c0, c1, ps);
   }
-  if (e == cudaSuccess && rest) e = cudaStreamWaitEvent(la->panel, la->rest, 0);
-  if (e == cudaSuccess) e = cudaEventRecord(la->first, la->panel);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(st, la->first, 0);
-  return e;
+  // after an error too: what has been launched ends before the workspace goes back on `st`
+  cudaError_t j = rest ? behind(ps, us, upd) : cudaSuccess;
+  if (j == cudaSuccess) j = behind(st, ps, first);
+  if (j != cudaSuccess) {
+    cudaStreamSynchronize(us);
+    cudaStreamSynchronize(ps);
+  }
+  return e == cudaSuccess ? j : e;
 }
 
 template cudaError_t run_step_uniform<double>(const StepArgsT<double>&, int, cudaStream_t);

@@ -132,6 +132,19 @@ __device__ __forceinline__ int factor_block(double* tile, int kb) {
       }
     }
     if (bad) return bad;  // the same in every lane
+    // the lane's own diagonal: d times the reciprocal root, corrected once, so that
+    // squares give their roots exactly (and an infinity stays one)
+    double dd = 1.0, rr = 1.0;
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (lane == j0 + s) {
+        dd = d[s][s];
+        rr = r[s];
+      }
+    const double q = dd * rr, root = isinf(dd) ? dd : fma(0.5 * rr, fma(-q, q, dd), q);
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (lane == j0 + s) a[s] = root;
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < 8; c += 2)

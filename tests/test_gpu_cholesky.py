@@ -83,3 +83,20 @@ def test_cholesky_device_entry(lib, oracle):
     Lo, _ = oracle.cholesky(A)
     assert _close(dL.cpu().numpy(), Lo, A)
     assert lib.nppb_d_cholesky_batched(1, 5000, None, None, None, None) == _lib.E_RANGE
+
+
+@pytest.mark.parametrize("n", [1, 7, 33, 70, 300])
+def test_roots_of_squares_and_of_infinity(lib, n):
+    """The factor of a diagonal of squares is their roots, without rounding; an infinite entry's
+    root is infinite and its column's multipliers are zero (linalg.cpp:126-133)."""
+    A = np.zeros((8, n, n))
+    roots = np.arange(1.0, 8 * n + 1).reshape(8, n)
+    A[:, range(n), range(n)] = roots ** 2
+    L = la.cholesky(A)
+    np.testing.assert_array_equal(L[:, range(n), range(n)], roots)
+    assert np.count_nonzero(L) == 8 * n
+    if n > 1:
+        A[0, 0, 0], A[0, n - 1, 0] = np.inf, 5.0
+        L = la.cholesky(A[:1])[0]
+        assert L[0, 0] == np.inf and L[n - 1, 0] == 0.0
+        np.testing.assert_array_equal(L[range(1, n), range(1, n)], roots[0, 1:])

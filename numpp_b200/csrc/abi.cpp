@@ -85,6 +85,19 @@ int finish(cudaStream_t st) {
     if (rc_ != NPPB_OK) return rc_; \
   } while (0)
 
+// Whether a call substitutes so many strips of 32 columns that clusters of 4 (orders
+// to 2048) or 8 CTAs, which read a system's whole factors once per strip, fall
+// behind the step kernels, which read them once per 64-column strip and CTA row.
+// Never up to order 1024. Inverses, ms on clusters / step kernels: 4 x 2048 (256
+// strips) 9.8 / 9.7, 16 x 1536 (768) 14.2 / 12.1, 1 x 2560 (80) 10.7 / 9.5, 8 x 4096
+// (1024) 137 / 91; 4 x 4096 with
+// 1024 right-hand sides (128) 27.7 / 27.4, 2 x 4096 with 1024 (64) 18.3 / 19.5. Re-solves: 32 x 1025 with 1025 (1056)
+// 10.0 / 11.3, 32 x 1536 with 1536 (1536) 20.4 / 17.1, 4 x 2049 with 2049 (260) 14.9 / 18.2, 8 x
+// 2049 (520) 28.4 / 21.2, 1 x 3072 with 3072 (96) 8.8 / 7.0.
+bool many_strips(int n, int64_t strips, int to2048, int to3000, int above) {
+  return n > 1024 && strips > (n <= 2048 ? to2048 : n < 3000 ? to3000 : above);
+}
+
 // A uniform batch whole, or, while its workspace does not fit the device's memory, in
 // halves, quarters and so on one after the other: run(part) allocates for `part`
 // systems and works through the batch with that. (The inverses of the diagonal
@@ -114,6 +127,39 @@ int d_linalg(int64_t count, int32_t n, int32_t nrhs, int flags, const double* dA
   if ((flags & NPPB_WANT_SLOGDET) && (!dSign || !dLogabs)) return arg_error("slogdet needs Sign and Logabs");
   if ((flags & NPPB_WANT_LU) && nn && (!dLU || !dipiv)) return arg_error("keeping factors needs LU and ipiv");
   if (!device()) return NPPB_E_NODEV;
+  const int64_t columns = ((flags & NPPB_WANT_SOLVE) ? (nrhs + 31) / 32 : 0) + ((flags & NPPB_WANT_INV) ? sys_blocks(n) : 0);
+  if (n > 32 && !(flags & NPPB_WANT_LU) && many_strips(n, count * columns, 250, 75, 75)) {
+    // the step kernels carry the columns along with the factorisation
+    DevMem lu_m, sc_m;
+    double* LU = dLU;
+    int rc = NPPB_OK;
+    if (!LU) {
+      rc = scratch<double>(lu_m, (size_t)count * nn, st);
+      LU = lu_m.as<double>();
+    }
+    if (rc == NPPB_OK) rc = scratch<StepScratch>(sc_m, (size_t)count, st);
+    if (rc == NPPB_OK) {
+      StepArgs sa{};
+      sa.scratch = sc_m.as<StepScratch>();
+      sa.A = (dA == LU) ? nullptr : dA;
+      sa.LU = LU;
+      sa.ipiv = dipiv;
+      sa.B = dB; sa.X = dX;
+      sa.inv = (flags & NPPB_WANT_INV) ? dInv : nullptr;
+      sa.det = (flags & NPPB_WANT_DET) ? dDet : nullptr;
+      sa.sign = (flags & NPPB_WANT_SLOGDET) ? dSign : nullptr;
+      sa.logabs = (flags & NPPB_WANT_SLOGDET) ? dLogabs : nullptr;
+      sa.info = dinfo;
+      sa.un = n;
+      sa.unrhs = (flags & NPPB_WANT_SOLVE) ? nrhs : 0;
+      sa.uinv = (flags & NPPB_WANT_INV) ? 1 : 0;
+      NPPB_CUDA(run_step_uniform(sa, (int)count, st), "batched LU launch");
+      return NPPB_OK;
+    }
+    if (rc != NPPB_E_NOMEM) return rc;
+    cudaGetLastError();  // no room for whole factors: in parts, below
+    clear_error();
+  }
   if (n > 32 && !(flags & NPPB_WANT_LU)) {
     // up to order 512 one CTA per system for the whole factorisation, above it outer
     // blocks; then one CTA or cluster per strip for the solves
@@ -209,6 +255,30 @@ int d_getrs(int64_t count, int32_t n, int32_t nrhs, const double* dLU, const int
   if (count == 0 || n == 0 || nrhs == 0) return NPPB_OK;
   if (!dLU || !dipiv || !dB || !dX) return arg_error("getrs needs LU, ipiv, B and X");
   if (!device()) return NPPB_E_NODEV;
+  if (n > 32 && many_strips(n, count * ((nrhs + 31) / 32), 1000, 300, 90)) {
+    int rc = NPPB_OK;
+    auto pl = uniform_plan(count, n, nrhs, NPPB_WANT_SOLVE, true, false, &rc);
+    DevMem tmp;
+    double* X = dX;
+    if (rc == NPPB_OK && dX == dB) {  // the row gather needs a separate output
+      rc = scratch<double>(tmp, (size_t)count * n * nrhs, st);
+      X = tmp.as<double>();
+    }
+    if (rc == NPPB_OK) {
+      Plan::Ptrs p{};
+      p.B = dB; p.X = X;
+      p.LU = const_cast<double*>(dLU);
+      p.ipiv = const_cast<int32_t*>(dipiv);
+      NPPB_RC(pl->execute(p, st));
+      if (X != dX)
+        NPPB_CUDA(cudaMemcpyAsync(dX, X, sizeof(double) * count * n * nrhs, cudaMemcpyDeviceToDevice, st),
+                  "device copy");
+      return NPPB_OK;
+    }
+    if (rc != NPPB_E_NOMEM) return rc;
+    cudaGetLastError();
+    clear_error();
+  }
   if (n > 32) {
     // the permutation and the diagonal blocks' inverses, then both
     // substitutions in one launch (every strip is read before it is written, so

@@ -132,3 +132,46 @@ def test_mixed_fallback(lib, n):
     X, rep = solve_mixed(A, B, tol=8 * n * EPS, max_iter=5)
     assert rep["fallback"][2] and not rep["info"].any()
     check(A, X, B, "mixed")
+
+
+@pytest.mark.parametrize("n,k,count", [(1030, 2048, 4), (1030, 1984, 4), (2080, 2400, 1), (2080, 2401, 1)])
+def test_many_right_hand_sides(torch, n, k, count):
+    """Both sides of the rule that hands calls with very many columns to the step kernels (orders
+    above 1024). The residual is taken in FP64, which adds (n + 2) eps: 10 n eps in all."""
+    from numpp_b200 import _lib, device
+    A = torch.from_numpy(matrices(n)[:count]).cuda()
+    B = torch.from_numpy(rhs(A.cpu().numpy(), k)).cuda()
+
+    def bound(X, B):
+        r = (A @ X - B).abs().amax(dim=1)
+        scale = A.abs().sum(dim=2).amax(dim=1)[:, None] * X.abs().amax(dim=1) + B.abs().amax(dim=1)
+        assert bool((r <= 10 * n * EPS * scale).all()), float((r / scale).max())
+
+    X, info = device.solve(A, B, check=False)
+    assert not info.any()
+    bound(X, B)
+    X = device.inv(A)
+    bound(X, torch.eye(n, dtype=torch.float64, device="cuda").expand_as(A))
+    P, st, L = _lib.ptr, torch.cuda.current_stream().cuda_stream, _lib.load()
+    LU, Y = torch.empty_like(A), B.clone()
+    piv, info = (torch.zeros(s, dtype=torch.int32, device="cuda") for s in ((count, n), (count,)))
+    assert L.nppb_d_linalg_batched(count, n, 0, _lib.WANT_LU, P(A), None, None, None, None, None, None, P(LU), P(piv),
+                                   P(info), st) == _lib.OK
+    assert L.nppb_d_getrs_batched(count, n, k, P(LU), P(piv), P(Y), P(Y), st) == _lib.OK  # in place
+    bound(Y, B)
+
+
+def test_many_right_hand_sides_of_kept_factors(torch):
+    from numpp_b200 import _lib
+    P, st, L = _lib.ptr, torch.cuda.current_stream().cuda_stream, _lib.load()
+    for n, k in ((3008, 2880), (3008, 2912)):
+        A = torch.from_numpy(matrices(n)[:1]).cuda()
+        B = torch.randn(1, n, k, dtype=torch.float64, device="cuda")
+        LU, X = torch.empty_like(A), torch.empty_like(B)
+        piv, info = (torch.zeros(s, dtype=torch.int32, device="cuda") for s in ((1, n), (1,)))
+        assert L.nppb_d_linalg_batched(1, n, 0, _lib.WANT_LU, P(A), None, None, None, None, None, None, P(LU), P(piv),
+                                       P(info), st) == _lib.OK
+        assert L.nppb_d_getrs_batched(1, n, k, P(LU), P(piv), P(B), P(X), st) == _lib.OK
+        r = (A @ X - B).abs().amax(dim=1)
+        scale = A.abs().sum(dim=2).amax(dim=1)[:, None] * X.abs().amax(dim=1) + B.abs().amax(dim=1)
+        assert bool((r <= 10 * n * EPS * scale).all())

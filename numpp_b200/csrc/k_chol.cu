@@ -179,14 +179,15 @@ __device__ __forceinline__ int factor_block(double* tile, int kb) {
 
 template <bool VEC, int CS>
 __global__ void __launch_bounds__(kSysMaxN, 1)
-k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
+k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n, int jb, int je) {
   extern __shared__ __align__(16) double sm[];
   __shared__ int s_fail;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3, nb = sys_blocks(n);
   const int rank = CS > 1 ? (int)blockIdx.x % CS : 0;
   const int64_t z = (int)blockIdx.x / CS;
-  const int blk = warp * CS + rank;
+  const int blk = jb + warp * CS + rank;
+  if (jb > 0 && info[z]) return;  // read ahead of the barrier that a writer has passed: the same in every CTA
   double* scratch = sm;
   double* tile = sm + kScratch + warp * kPerWarp;
   double* Li = sm + kScratch + nw * kPerWarp;
@@ -225,7 +226,7 @@ k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
     const int p = 32 * blk + 8 * i + g;
     r.off[i] = (unsigned)(p < n ? p : 0) * n * 8;
   }
-  for (int J = 0; J < nb; ++J) {
+  for (int J = jb; J < je; ++J) {
     const int kb = min(32, n - 32 * J);
     const bool active = blk >= J && blk < nb;
     Acc<4> acc;
@@ -237,10 +238,10 @@ k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
       asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx + min(16, left)));
       asm volatile("prefetch.global.L2 [%0];\n" ::"l"(nx + min(31, left)));
     }
-    if (J > 0) {
-      fetch_rows(J, 0);
-      ring_start<VEC, false>(ring, L, r, 0, n, active);
-      for (int K = 0; K < J; ++K) {
+    if (J > jb) {
+      fetch_rows(J, jb);
+      ring_start<VEC, false>(ring, L, r, jb, n, active);
+      for (int K = jb; K < J; ++K) {
         cp_wait<2>();     // L_JK; at most two operand stages stay in flight
         __syncthreads();  // and every warp is done with the other tile
         if (K + 1 < J) fetch_rows(J, K + 1);
@@ -324,9 +325,105 @@ k_sys_chol(const double* A, double* L, int32_t* __restrict__ info, int n) {
       for (int rr = 0; rr < 32; ++rr)
         if (rr < rows) o[(int64_t)rr * n] = blk >= J ? tile[rr * PS + lane] : 0.0;
     }
-    if (J + 1 < nb) sync();  // this column of L before the next one reads it
+    if (J + 1 < je) sync();  // this column of L before the next one reads it
   }
-  if (threadIdx.x == 0 && rank == 0) info[z] = 0;
+  if (jb == 0 && threadIdx.x == 0 && rank == 0) info[z] = 0;
+}
+
+// Orders above 2048: outer blocks of 128 columns. k_sys_chol factors a block's columns
+// over all rows below (left-looking inside it), k_chol_update subtracts their
+// products from the rest of the lower triangle. One cluster for the whole matrix
+// keeps 8 SMs busy: 24.5 ms for one matrix of order 4096, where the unpivoted LU on the step
+// kernels had taken 12.
+//
+// Rows 32 je .. n - 1 minus L_21 L_21^T on and below the diagonal, K = 128: a CTA per
+// 128 x 64 tile (grid.z = system), slabs of 16 columns of both row ranges through a
+// ring of three, as in k_sys_gemm. src: A for the first block, L after it.
+constexpr int CM = 128, CN = 64, CK = 16, CSTAGES = 3;
+constexpr int kCholSlab = (CM + CN) * CK;
+constexpr int kCholUpdateSmem = 8 * CSTAGES * kCholSlab;
+
+template <bool VEC>
+__global__ void __launch_bounds__(256, 2)
+k_chol_update(const double* src, double* L, const int32_t* __restrict__ info, int n, int jb, int je) {
+  extern __shared__ __align__(16) double sm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int64_t z = blockIdx.z;
+  const int row0 = 32 * je + CM * (int)blockIdx.y, col0 = 32 * je + CN * (int)blockIdx.x;
+  if (col0 >= row0 + CM || info[z]) return;  // above the diagonal; not positive definite
+  src += z * n * n;
+  L += z * n * n;
+  // 192 rows of a slab (128 of the tile's rows, then 64 of its columns); 16-byte piece
+  // c of row r at piece c ^ 4 (r & 1): neighbouring rows fall into the two halves of the banks
+  auto load = [&](int slab) {
+    double* a = sm + slab % CSTAGES * kCholSlab;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const int idx = tid + 256 * i, r = idx >> 3, c = idx & 7;
+      const int row = r < CM ? row0 + r : col0 + r - CM;
+      const double* p = L + (int64_t)min(row, n - 1) * n + 32 * jb + CK * slab + 2 * c;
+      const unsigned d = smem(a + r * CK + 2 * (c ^ 4 * (r & 1)));
+      if constexpr (VEC) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(p), "r"(row < n ? 16 : 0));
+      } else {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(p), "r"(row < n ? 8 : 0));
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d + 8), "l"(p + 1), "r"(row < n ? 8 : 0));
+      }
+    }
+    cp_commit();
+  };
+  constexpr int kSlabs = 128 / CK;
+  load(0);
+  load(1);
+  const int wm = 32 * (warp >> 1), wn = 32 * (warp & 1);
+  double acc[2][4][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = row0 + wm + 16 * m + 8 * (e >> 1) + g, col = col0 + wn + 8 * ni + 2 * t + (e & 1);
+        acc[m][ni][e] = row < n && col <= row ? -src[(int64_t)row * n + col] : 0.0;
+      }
+  for (int k = 0; k < kSlabs; ++k) {
+    cp_wait<1>();
+    __syncthreads();  // slab k is here, and slab k - 1 has been read
+    if (k + 2 < kSlabs) load(k + 2);
+    else cp_commit();
+    const double* a = sm + k % CSTAGES * kCholSlab;
+    const double* b = a + CM * CK;
+#pragma unroll
+    for (int q = 0; q < CK / 8; ++q) {
+      double2 av[4], bv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = wm + 8 * i + g, c = wn + 8 * i + g;
+        av[i] = *reinterpret_cast<const double2*>(a + r * CK + 2 * ((4 * q + t) ^ 4 * (r & 1)));
+        bv[i] = *reinterpret_cast<const double2*>(b + c * CK + 2 * ((4 * q + t) ^ 4 * (c & 1)));
+      }
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int ni = 0; ni < 4; ++ni) dmma1688(acc[m][ni], av[2 * m], av[2 * m + 1], bv[ni]);
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int row = row0 + wm + 16 * m + 8 * (e >> 1) + g, col = col0 + wn + 8 * ni + 2 * t + (e & 1);
+        if (row < n && col <= row) L[(int64_t)row * n + col] = -acc[m][ni][e];
+      }
+}
+
+// Zeros right of each row's 128-column diagonal block (the outer blocks write the rest).
+__global__ void __launch_bounds__(256) k_chol_zeros(double* L, int n) {
+  const int row = blockIdx.x, end = min(n, (row / 128 + 1) * 128);
+  double* o = L + ((int64_t)blockIdx.y * n + row) * n;
+  for (int c = end + threadIdx.x; c < n; c += 256) o[c] = 0.0;
 }
 
 template <bool VEC, int CS>
@@ -335,9 +432,11 @@ cudaError_t chol_prepare1() {
                               chol_smem(kMaxWarps, 2));
 }
 
+// Columns of the blocks [jb, je).
 template <bool VEC, int CS>
-cudaError_t launch_chol(const double* A, double* L, int32_t* info, int64_t count, int n, cudaStream_t st) {
-  const int nb = sys_blocks(n), nw = (nb + CS - 1) / CS;
+cudaError_t launch_chol(const double* A, double* L, int32_t* info, int64_t count, int n, int jb, int je,
+                        cudaStream_t st) {
+  const int nb = sys_blocks(n) - jb, nw = (nb + CS - 1) / CS;
   cudaError_t e = chol_prepare1<VEC, CS>();
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
@@ -352,28 +451,57 @@ cudaError_t launch_chol(const double* A, double* L, int32_t* info, int64_t count
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = CS > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_sys_chol<VEC, CS>, A, L, info, n);
+  return cudaLaunchKernelEx(&cfg, k_sys_chol<VEC, CS>, A, L, info, n, jb, je);
+}
+
+template <bool VEC>
+cudaError_t launch_chol(const double* A, double* L, int32_t* info, int64_t count, int n, int jb, int je,
+                        cudaStream_t st) {
+  switch (sys_cluster(n - 32 * jb, count)) {
+    case 1: return launch_chol<VEC, 1>(A, L, info, count, n, jb, je, st);
+    case 2: return launch_chol<VEC, 2>(A, L, info, count, n, jb, je, st);
+    case 4: return launch_chol<VEC, 4>(A, L, info, count, n, jb, je, st);
+    default: return launch_chol<VEC, 8>(A, L, info, count, n, jb, je, st);
+  }
+}
+
+template <bool VEC>
+cudaError_t run_chol_outer(const double* A, double* L, int32_t* info, int64_t count, int n, cudaStream_t st) {
+  constexpr int kOuter = 4;
+  const int nb = sys_blocks(n);
+  cudaError_t e = cudaFuncSetAttribute(k_chol_update<VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       kCholUpdateSmem);
+  for (int jb = 0; jb < nb && e == cudaSuccess; jb += kOuter) {
+    const int je = std::min(nb, jb + kOuter), rest = n - 32 * je;
+    const double* src = jb ? L : A;
+    e = launch_chol<VEC>(src, L, info, count, n, jb, je, st);
+    if (e != cudaSuccess || rest <= 0) break;
+    const dim3 grid((unsigned)(rest + CN - 1) / CN, (unsigned)(rest + CM - 1) / CM, (unsigned)count);
+    k_chol_update<VEC><<<grid, 256, kCholUpdateSmem, st>>>(src, L, info, n, jb, je);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess) return e;
+  // behind every reader of A, which may be L
+  k_chol_zeros<<<dim3((unsigned)n, (unsigned)count), 256, 0, st>>>(L, n);
+  return cudaGetLastError();
 }
 
 int cholesky_device(int64_t count, int32_t n, const double* dA, double* dL, int32_t* dinfo, cudaStream_t st) {
-  const int cs = sys_cluster(n, count);
-  if (count * cs > INT32_MAX) {
+  if (count * sys_cluster(n, count) > INT32_MAX) {
     set_error("batch count above 2^31-1");
     return NPPB_E_RANGE;
   }
   const bool vec = n % 2 == 0 && (reinterpret_cast<uintptr_t>(dL) & 15) == 0;
-#define NPPB_CHOL(CS)                                                        \
-  NPPB_CUDA((vec ? launch_chol<true, CS>(dA, dL, dinfo, count, n, st)        \
-                 : launch_chol<false, CS>(dA, dL, dinfo, count, n, st)),     \
-            "factorisation");                                                \
-  return NPPB_OK
-  switch (cs) {
-    case 1: NPPB_CHOL(1);
-    case 2: NPPB_CHOL(2);
-    case 4: NPPB_CHOL(4);
-    default: NPPB_CHOL(8);
-  }
-#undef NPPB_CHOL
+  const int nb = sys_blocks(n);
+  if (n > 2048 && count <= 65535)
+    NPPB_CUDA((vec ? run_chol_outer<true>(dA, dL, dinfo, count, n, st)
+                   : run_chol_outer<false>(dA, dL, dinfo, count, n, st)),
+              "factorisation");
+  else
+    NPPB_CUDA((vec ? launch_chol<true>(dA, dL, dinfo, count, n, 0, nb, st)
+                   : launch_chol<false>(dA, dL, dinfo, count, n, 0, nb, st)),
+              "factorisation");
+  return NPPB_OK;
 }
 
 int check_args(int64_t count, int32_t n) {

@@ -100,3 +100,32 @@ def test_roots_of_squares_and_of_infinity(lib, n):
         L = la.cholesky(A[:1])[0]
         assert L[0, 0] == np.inf and L[n - 1, 0] == 0.0
         np.testing.assert_array_equal(L[range(1, n), range(1, n)], roots[0, 1:])
+
+
+@pytest.mark.parametrize("n", [2048, 2049, 2050, 2176, 2300])
+@pytest.mark.parametrize("inplace", [False, True])
+def test_outer_blocks(lib, n, inplace):
+    """Orders above 2048 go by outer blocks of 128 columns: odd and even ones, partial last blocks,
+    matrices that are not positive definite in the first, a middle and the last block, with NaN
+    above the diagonal. Bar: 8 (n + 2) eps cond(A) of the factor (test_gpu_resident.py)."""
+    torch = pytest.importorskip("torch")
+    P, st = _lib.ptr, torch.cuda.current_stream().cuda_stream
+    bad = [None, 5, 1500, n - 1]
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    W = torch.randn(1, n, n, dtype=torch.float64, device="cuda", generator=g)
+    A0 = W[0] @ W[0].T
+    A0.diagonal().add_(float(n))
+    A = A0.tril().repeat(4, 1, 1)
+    A[:, torch.triu(torch.ones(n, n, device="cuda"), 1).bool()] = float("nan")
+    for s, b in enumerate(bad):
+        if b is not None:
+            A[s, b, b] = -1.0
+    L = A if inplace else torch.full_like(A, 7.0)
+    info = torch.full((4,), -1, dtype=torch.int32, device="cuda")
+    assert lib.nppb_d_cholesky_batched(4, n, P(A), P(L), P(info), st) == _lib.OK, _lib.last_error()
+    assert info.tolist() == [0 if b is None else b + 1 for b in bad]
+    want = np.linalg.cholesky(A0.cpu().numpy())
+    got = L[0].cpu().numpy()
+    assert not np.triu(got, 1).any()
+    assert np.abs(got - want).max() <= 8 * (n + 2) * 2.0 ** -53 * np.linalg.cond(A0.cpu().numpy()) * np.abs(want).max()

@@ -158,7 +158,7 @@ __device__ __forceinline__ int factor_block(double* tile, int kb) {
       l[i].x = -l[i].x;
       l[i].y = -l[i].y;
     }
-    for (int c0 = j0 + 8; c0 < 32; c0 += 8) {  // columns c0 .. c0 + 7: their rows are the operand
+    for (int c0 = j0 + 8; c0 < kb; c0 += 8) {  // columns c0 .. c0 + 7: their rows are the operand
       const double2 b = *reinterpret_cast<const double2*>(tile + (c0 + g) * PS + j0 + 2 * t);
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
@@ -175,6 +175,32 @@ __device__ __forceinline__ int factor_block(double* tile, int kb) {
   for (int c = (kb + 7) & ~7; c < 32; ++c) tile[lane * PS + c] = 0.0;  // past the last group
   __syncwarp();
   return 0;
+}
+
+// Orders up to 32: a warp per system, as many warps to a CTA (at most four) as leave
+// every SM a CTA. A CTA of k_sys_chol per system instead takes 148 us for 40000 systems
+// of order 4 and 209 of order 9.
+__global__ void __launch_bounds__(128)
+k_chol_warp(const double* A, double* L, int32_t* __restrict__ info, int count, int n) {
+  extern __shared__ __align__(16) double sm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, z = blockIdx.x * (blockDim.x >> 5) + warp;
+  if (z >= count) return;
+  double* tile = sm + warp * 32 * PS;
+  A += (int64_t)z * n * n;
+  L += (int64_t)z * n * n;
+  {
+    double x[32];
+#pragma unroll
+    for (int r = 0; r < 32; ++r) x[r] = r < n && lane <= r ? __ldcs(A + r * n + lane) : 0.0;
+#pragma unroll
+    for (int r = 0; r < 32; ++r) tile[r * PS + lane] = x[r];
+  }
+  __syncwarp();
+  const int bad = factor_block(tile, n);
+  if (lane == 0) info[z] = bad;
+  if (bad || lane >= n) return;
+#pragma unroll 8
+  for (int r = 0; r < n; ++r) L[r * n + lane] = tile[r * PS + lane];
 }
 
 template <bool VEC, int CS>
@@ -493,7 +519,12 @@ int cholesky_device(int64_t count, int32_t n, const double* dA, double* dL, int3
   }
   const bool vec = n % 2 == 0 && (reinterpret_cast<uintptr_t>(dL) & 15) == 0;
   const int nb = sys_blocks(n);
-  if (n > 2048 && count <= 65535)
+  if (n <= 32) {
+    const int w = (int)std::min<int64_t>(4, (count + 147) / 148);
+    k_chol_warp<<<(unsigned)((count + w - 1) / w), 32 * w, w * 32 * PS * (int)sizeof(double), st>>>(dA, dL, dinfo,
+                                                                                                  (int)count, n);
+    NPPB_CUDA(cudaGetLastError(), "factorisation");
+  } else if (n > 2048 && count <= 65535)
     NPPB_CUDA((vec ? run_chol_outer<true>(dA, dL, dinfo, count, n, st)
                    : run_chol_outer<false>(dA, dL, dinfo, count, n, st)),
               "factorisation");

@@ -14,13 +14,13 @@
 // the trailing update is a[i,j] -= f*a[k,j] (one FMA here). NaN entries are
 // never pivot candidates.
 //
-// A warp's chain of instructions bounds few systems (256 of order 32, solve and det:
-// 26.6 us with each 16-byte piece of the update loaded behind the store before it,
-// 22.5 us with eight columns at a time, the forward substitution of a single
-// right-hand side riding along with the elimination, and one reduction where a
-// single lane holds the largest high word). With up to eight columns a chunk (RC = 8)
-// the same changes cost more instructions than they save in latency (4000 systems
-// of order 24 with 5: 70 us without them, 78 us with), so that form keeps its branches.
+// A warp's chain of instructions bounds few systems. CHAIN (full tiles, order 32, with
+// at most one right-hand side) shortens it: eight columns of the update at a time, the
+// forward substitution riding along with the elimination, and one reduction where a
+// single lane holds the largest high word: 256 systems, solve and det, 26.9 us without
+// it, 22.5 us with it. It costs more instructions than it saves in latency below order
+// 32 (launch_np) and with up to eight columns a chunk (RC = 8; 4000 systems of order
+// 24 with 5: 70 us without, 78 us with).
 //
 // The same launch finishes the requested outputs:
 //  * det  = permsign * prod U[i,i] in order i = 0..n-1   (linalg.cpp:393-407)
@@ -43,11 +43,12 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWarpsPerCta = 2;  // small batches spread over more SMs
 constexpr int kLd = 34;          // row stride of a warp's tile (doubles): columns 32, 33 are scratch
 
-template <int NP, int RC>
+template <int NP, int RC, bool CHAIN>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
   constexpr int UF = RC == 1 ? 4 : 1;  // substitution steps per loop body (small code with several columns)
   constexpr bool kOne = RC == 1;       // one column: no branches in its substitution either
+  static_assert(!CHAIN || RC == 1);
   __shared__ int s_lane_of_pos[kWarpsPerCta][32];
   __shared__ __align__(16) double s_rows[kWarpsPerCta][32 * kLd];  // row r at r * kLd (16-byte aligned rows)
   const int lane = threadIdx.x & 31;
@@ -81,9 +82,8 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
   // Original row index held by each position, for getrs from stored factors.
   int orig = lane;
 
-  // a single right-hand side rides along with the elimination (its forward substitution);
-  // eight of them cost there what the loop of their own does
-  const bool ride = kOne && (flags & kWantSolve) && !(flags & kSolveOnly);
+  // CHAIN: a single right-hand side rides along with the elimination (its forward substitution)
+  const bool ride = CHAIN && (flags & kWantSolve) && !(flags & kSolveOnly);
   double x0 = ride && live && v.nrhs > 0 ? v.B[(int64_t)lane * v.nrhs] : 0.0;
 
   if (!(flags & kSolveOnly)) {
@@ -96,9 +96,9 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
       const unsigned long long bits = (unsigned long long)__double_as_longlong(mag);
       const uint32_t hi = number ? (uint32_t)(bits >> 32) : 0u, lo = number ? (uint32_t)bits : 0u;
       const uint32_t mhi = __reduce_max_sync(kFull, hi);
-      const unsigned tops = kOne ? __ballot_sync(kFull, cand && hi == mhi) : 0u;
+      const unsigned tops = CHAIN ? __ballot_sync(kFull, cand && hi == mhi) : 0u;
       int pl = __ffs(tops) - 1, key;
-      if (kOne && mhi != 0u && (tops & (tops - 1u)) == 0u) {  // one lane holds the largest high word
+      if (CHAIN && mhi != 0u && (tops & (tops - 1u)) == 0u) {  // one lane holds the largest high word
         key = __shfl_sync(kFull, pos, pl);
       } else {
         const uint32_t mlo = __reduce_max_sync(kFull, hi == mhi ? lo : 0u);
@@ -120,7 +120,7 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
       if (lane == pl) dg = pk;
       const bool below = live && pos > k;
       double f = 0.0;
-      if constexpr (kOne) {
+      if constexpr (CHAIN) {
         f = below ? akk / pk : 0.0;
         if (ride) {
           const double xk = __shfl_sync(kFull, x0, pl);
@@ -129,9 +129,9 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
         }
       }
       if (below) {
-        if constexpr (!kOne) f = row[k] / pk;
+        if constexpr (!CHAIN) f = row[k] / pk;
         row[k] = f;
-        // eight columns at a time, both rows' pieces loaded before the first store (a
+        // CHAIN: eight columns at a time, both rows' pieces loaded before the first store (a
         // store to the tile holds back every later load of it: 78 cycles a 16-byte
         // piece one by one, of 1500 for a step); columns up to k keep their multipliers,
         // columns past n are padding
@@ -153,12 +153,12 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) r2[q + i] = rv[i];
         };
-        if (kOne && n > 8) {
+        if constexpr (CHAIN) {
           int q = (k + 1) >> 3 << 2;
           if (2 * q < n) piece(q, true);
 #pragma unroll 1
           for (q += 4; 2 * q < n; q += 4) piece(q, false);
-        } else {  // few columns, or many warps' worth of work: no column too many
+        } else {
 #pragma unroll 4
           for (int q = (k + 1) >> 1; q < (n + 1) >> 1; ++q) {
             const double2 pv = p2[q];
@@ -316,11 +316,16 @@ k_lu_warp(Batch bt, const int32_t* __restrict__ order, int nsys) {
 template <int NP>
 cudaError_t launch_np(const Batch& bt, const int32_t* order, int nsys, cudaStream_t st) {
   const int grid = (nsys + kWarpsPerCta - 1) / kWarpsPerCta;
-  // one right-hand-side column and no inverse (a uniform batch says so): the one-column substitution
-  if (!bt.desc && bt.nrhs <= 1 && !(bt.flags & kWantInv))
-    k_lu_warp<NP, 1><<<grid, kWarpsPerCta * 32, 0, st>>>(bt, order, nsys);
+  // one right-hand-side column and no inverse (a uniform batch says so): the one-column
+  // substitution, and at order 32, whose rows are whole pieces, CHAIN. Below it the plain
+  // elimination: det of 256 systems, us plain / CHAIN: order 32 21.8 / 18.8, 31 21.0 / 23.7,
+  // 24 16.7 / 18.7, 9 8.4 / 10.0; of 4096: 32 59.5 / 60.5, 31 59.4 / 67.5, 17 27.0 / 37.3.
+  if (bt.desc || bt.nrhs > 1 || (bt.flags & kWantInv))
+    k_lu_warp<NP, 8, false><<<grid, kWarpsPerCta * 32, 0, st>>>(bt, order, nsys);
+  else if (bt.n == NP)
+    k_lu_warp<NP, 1, true><<<grid, kWarpsPerCta * 32, 0, st>>>(bt, order, nsys);
   else
-    k_lu_warp<NP, 8><<<grid, kWarpsPerCta * 32, 0, st>>>(bt, order, nsys);
+    k_lu_warp<NP, 1, false><<<grid, kWarpsPerCta * 32, 0, st>>>(bt, order, nsys);
   return cudaGetLastError();
 }
 

@@ -70,15 +70,16 @@ struct LsqLayout {
 // neighbouring columns, which then fall into the two halves of the banks.
 int lsq_stride8(int n) { return (n + 7) / 16 * 16 + 8; }
 
-LsqLayout lsq_layout(int m, int n, int k, bool want_qr) {
+// nbuf: right-hand sides carried at once (at least 1 of k > 0); negative: no reduction.
+LsqLayout lsq_layout(int m, int n, int k, int nbuf) {
   const int wide = m < n, M = wide ? n : m, N = wide ? m : n;
   LsqLayout l{};
   l.ws = M | 1;
-  l.qr = want_qr ? 1 : 0;
+  l.qr = nbuf >= 0 ? 1 : 0;
   int at = l.ws * N;
   if (l.qr) {
     l.js = l.vs = lsq_stride8(N);
-    l.nbuf = k < LT / 32 ? k : LT / 32;
+    l.nbuf = nbuf;
     l.buf = at;
     at += l.nbuf * l.ws;
     // once every right-hand side has been carried along, nothing reads the
@@ -113,18 +114,22 @@ LsqLayout lsq_layout(int m, int n, int k, bool want_qr) {
 }
 
 // Reducing to the triangle pays for M >= 2 N (a sweep then runs on N instead
-// of M rows). Its rounding is at the level of the default tolerance's factor
+// of M rows) and N >= 3 (one or two columns have no sweeps to speak of: 64 x 1 takes 6
+// us directly, 11 us with the reduction and its second launch). The right-hand sides
+// are carried in as large groups as fit. Its rounding is at the level of the default tolerance's factor
 // eps * max(m, n); a smaller rcond keeps the sweeps on the matrix itself, so
 // that exactly dependent columns still give exact zeros there, and so do
 // small problems, whose default tolerance is a few eps.
 LsqLayout lsq_plan(int m, int n, int k, double rcond) {
   const int wide = m < n, M = wide ? n : m, N = wide ? m : n;
   const bool robust = rcond < 0 || rcond >= 2.220446049250313e-16 * M;
-  if (M >= 2 * N && M >= 64 && robust) {
-    const LsqLayout l = lsq_layout(m, n, k, true);
-    if (sizeof(double) * (size_t)l.doubles <= kLsqMaxSmem) return l;
+  if (M >= 2 * N && M >= 64 && N >= 3 && robust) {
+    for (int nbuf = k < LT / 32 ? k : LT / 32; nbuf >= (k > 0 ? 1 : 0); --nbuf) {
+      const LsqLayout l = lsq_layout(m, n, k, nbuf);
+      if (sizeof(double) * (size_t)l.doubles <= kLsqMaxSmem) return l;
+    }
   }
-  return lsq_layout(m, n, k, false);
+  return lsq_layout(m, n, k, -1);
 }
 
 template <int W>
@@ -158,10 +163,11 @@ __device__ __forceinline__ int exponent(double x) { return (__double2hiint(x) >>
 // therefore taken in FP32 on values scaled into its range by powers of two. A
 // rotation then leaves 1e-7 of the dot product instead of 1e-16, and the sweeps
 // end on the same measured 1e-15.
-template <bool VECS, int R8>
+// LP lanes per pair (R8: with LP = 8 only).
+template <bool VECS, int R8, int LP>
 __device__ __forceinline__ void jacobi_round(double* J, int js, double* V, int vs, int N, int rows, int t,
                                              float& worst) {
-  const int E = N + (N & 1), pair = threadIdx.x >> 3, l8 = threadIdx.x & 7;
+  const int E = N + (N & 1), pair = threadIdx.x / LP, l8 = threadIdx.x % LP;
   int i = pair == 0 ? E - 1 : t + pair < E - 1 ? t + pair : t + pair - (E - 1);
   int j = pair == 0 ? t : t >= pair ? t - pair : t - pair + E - 1;
   if (i > j) {
@@ -189,16 +195,16 @@ __device__ __forceinline__ void jacobi_round(double* J, int js, double* V, int v
       cc = fma(xi[q], xj[q], cc);
     }
   } else {
-    for (int r = l8; r < rows; r += 8) {
+    for (int r = l8; r < rows; r += LP) {
       const double x = wi[r], y = wj[r];
       aa = fma(x, x, aa);
       bb = fma(y, y, bb);
       cc = fma(x, y, cc);
     }
   }
-  aa = lane_sum<8>(aa);
-  bb = lane_sum<8>(bb);
-  cc = lane_sum<8>(cc);
+  aa = lane_sum<LP>(aa);
+  bb = lane_sum<LP>(bb);
+  cc = lane_sum<LP>(cc);
   if (!on || !(aa > 0.0) || !(bb > 0.0) || !(fabs(cc) > 0.0)) return;  // nothing to turn (or a NaN)
   if (isinf(aa) || isinf(bb) || isinf(cc)) return;
   // |cc| / sqrt(aa bb): aa and bb scaled to [1, 4) by even powers of two
@@ -228,7 +234,7 @@ __device__ __forceinline__ void jacobi_round(double* J, int js, double* V, int v
       }
     }
   } else {
-    for (int r = l8; r < rows; r += 8) {
+    for (int r = l8; r < rows; r += LP) {
       const double x = wi[r], y = wj[r];
       wi[r] = cs * x - sj * y;
       wj[r] = sn * x + cj * y;
@@ -237,7 +243,7 @@ __device__ __forceinline__ void jacobi_round(double* J, int js, double* V, int v
   if constexpr (VECS) {
     double* vi = V + i * vs;
     double* vj = V + j * vs;
-    for (int r = l8; r < N; r += 8) {
+    for (int r = l8; r < N; r += LP) {
       const double x = vi[r], y = vj[r];
       vi[r] = cs * x - sj * y;
       vj[r] = sn * x + cj * y;
@@ -251,8 +257,9 @@ __device__ __forceinline__ void jacobi_sweeps(double* J, int js, double* V, int 
   for (int sweep = 0; sweep < 60 && N > 1; ++sweep) {
     float worst = 0.f;
     for (int t = 0; t < E - 1; ++t) {
-      if (rows <= 32) jacobi_round<VECS, 4>(J, js, V, vs, N, rows, t, worst);
-      else jacobi_round<VECS, 0>(J, js, V, vs, N, rows, t, worst);
+      if (rows <= 32) jacobi_round<VECS, 4, 8>(J, js, V, vs, N, rows, t, worst);
+      else if (E / 2 > LT / 32) jacobi_round<VECS, 0, 8>(J, js, V, vs, N, rows, t, worst);
+      else jacobi_round<VECS, 0, 32>(J, js, V, vs, N, rows, t, worst);  // a warp for each of few pairs
       __syncthreads();  // the next round pairs these columns differently
     }
 #pragma unroll
@@ -609,7 +616,7 @@ int lstsq_device(int64_t count, int32_t m, int32_t n, int32_t k, const double* d
   k_lstsq<<<(unsigned)count, LT, smem, st>>>(m, n, k, dA, dB, rcond, l, 0, dX, dS, drank, dres, dhas);
   NPPB_CUDA(cudaGetLastError(), "least squares");
   if (l.qr) {  // problems with a NaN or an infinity; the others' CTAs return at once
-    const LsqLayout d = lsq_layout(m, n, k, false);
+    const LsqLayout d = lsq_layout(m, n, k, -1);
     k_lstsq<<<(unsigned)count, LT, sizeof(double) * (size_t)d.doubles, st>>>(m, n, k, dA, dB, rcond, d, 1, dX, dS,
                                                                             drank, dres, dhas);
     NPPB_CUDA(cudaGetLastError(), "least squares");

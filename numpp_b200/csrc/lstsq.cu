@@ -43,6 +43,7 @@ constexpr int kLsqMaxK = 64;          // right-hand sides
 constexpr int32_t kLsqLeft = -1;      // rank of a problem that the first launch has left to the second
 constexpr double kLsqMostA = 0x1p480, kLsqMostB = 0x1p900;  // largest magnitudes that are reduced to the triangle
 constexpr size_t kLsqMaxSmem = 220 * 1024;  // dynamic shared memory of one problem
+constexpr size_t kLsqHalfSmem = 112 * 1024;  // of two that share an SM
 
 #define NPPB_CUDA(call, what)                            \
   do {                                                   \
@@ -113,21 +114,34 @@ LsqLayout lsq_layout(int m, int n, int k, int nbuf) {
   return l;
 }
 
+// A round of at most four pairs of long columns: a warp a pair leaves most of the CTA
+// idle, so the whole CTA takes one pair after the other (300 x 3 with rcond = 0: 32 us so, one
+// problem; 6000 x 3: 79 us, 238 us with a warp a pair).
+__host__ __device__ bool wide_pairs(int N, int rows) {
+  const int E = N + (N & 1);
+  return E <= 8 && rows > 100 * E;
+}
+
 // Reducing to the triangle pays for M >= 2 N (a sweep then runs on N instead
 // of M rows) and N >= 3 (one or two columns have no sweeps to speak of: 64 x 1 takes 6
-// us directly, 11 us with the reduction and its second launch). The right-hand sides
-// are carried in as large groups as fit. Its rounding is at the level of the default tolerance's factor
+// us directly, 11 us with the reduction and its second launch). Right-hand sides in
+// groups of fewer than four leave the CTA idle: 5000 x 4 with 20 takes 1045 us one by one,
+// 429 us directly; so do long solutions of wide problems behind the first group (2048
+// of 5 x 2000 with 20: 2110 us, 1441 us directly). Its rounding is at the level of the default tolerance's factor
 // eps * max(m, n); a smaller rcond keeps the sweeps on the matrix itself, so
 // that exactly dependent columns still give exact zeros there, and so do
 // small problems, whose default tolerance is a few eps.
 LsqLayout lsq_plan(int m, int n, int k, double rcond) {
   const int wide = m < n, M = wide ? n : m, N = wide ? m : n;
   const bool robust = rcond < 0 || rcond >= 2.220446049250313e-16 * M;
-  if (M >= 2 * N && M >= 64 && N >= 3 && robust) {
-    for (int nbuf = k < LT / 32 ? k : LT / 32; nbuf >= (k > 0 ? 1 : 0); --nbuf) {
-      const LsqLayout l = lsq_layout(m, n, k, nbuf);
-      if (sizeof(double) * (size_t)l.doubles <= kLsqMaxSmem) return l;
-    }
+  if (M >= 2 * N && M >= 64 && N >= 3 && robust && !(wide && k > LT / 32 && wide_pairs(N, M))) {
+    // the largest group of at least four that leaves room for two CTAs an SM, else that fits at all
+    const int most = k < LT / 32 ? k : LT / 32, least = k < 4 ? k : 4;
+    for (const size_t limit : {kLsqHalfSmem, kLsqMaxSmem})
+      for (int nbuf = most; nbuf >= least; --nbuf) {
+        const LsqLayout l = lsq_layout(m, n, k, nbuf);
+        if (sizeof(double) * (size_t)l.doubles <= limit) return l;
+      }
   }
   return lsq_layout(m, n, k, -1);
 }
@@ -152,18 +166,44 @@ __device__ __forceinline__ void reflect(const double* w, double head, double tau
 __device__ __forceinline__ double power2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
 __device__ __forceinline__ int exponent(double x) { return (__double2hiint(x) >> 20) - 1023; }
 
-// One-sided Jacobi on N columns of `rows` rows at J (stride js), the rotations
-// accumulated in V (stride vs) with VECS. In round t of the round-robin over an
-// even number E of players, E - 1 meets t and the others meet the one with
-// t + p = t - p (mod E - 1): E / 2 disjoint pairs, eight lanes each.
-//
 // The FP64 pipe (a warp instruction every two cycles) is what the rounds share:
 // the angle, of which only c^2 + s^2 = 1 has to hold to the last bit, and the
 // relative dot product, which is only compared with the threshold, are
 // therefore taken in FP32 on values scaled into its range by powers of two. A
 // rotation then leaves 1e-7 of the dot product instead of 1e-16, and the sweeps
 // end on the same measured 1e-15.
-// LP lanes per pair (R8: with LP = 8 only).
+// aa, bb: the columns' squared norms, cc their dot product. x_i <- cs x_i - sj x_j,
+// x_j <- sn x_i + cj x_j; false: nothing to turn.
+__device__ __forceinline__ bool jacobi_angle(double aa, double bb, double cc, float& worst, double& cs, double& sn,
+                                             double& sj, double& cj) {
+  if (!(aa > 0.0) || !(bb > 0.0) || !(fabs(cc) > 0.0)) return false;  // nothing to turn (or a NaN)
+  if (isinf(aa) || isinf(bb) || isinf(cc)) return false;
+  // |cc| / sqrt(aa bb): aa and bb scaled to [1, 4) by even powers of two
+  const int ea = max(min(exponent(aa), 1022), -1022) & ~1, eb = max(min(exponent(bb), 1022), -1022) & ~1;
+  const float fa = (float)(aa * power2(-ea)), fb = (float)(bb * power2(-eb));
+  const float fc = (float)(fabs(cc) * power2(-((ea + eb) / 2)));
+  worst = fmaxf(worst, fc * rsqrtf(fa * fb));
+  // tan of the rotation angle, the smaller root of t^2 + 2 zeta t - 1 = 0 with
+  // zeta = (bb - aa) / (2 |cc|); both legs halved and scaled by one power of two. An
+  // angle near or below FP32's range (columns of very different lengths) would
+  // never turn the pair: there the root is 1 / (2 zeta) to the last bit.
+  const double p = fabs(0.5 * bb - 0.5 * aa), s1 = fabs(cc);
+  const double down = power2(-max(min(max(exponent(p), exponent(s1)), 1022), -1022));
+  const float fp = (float)(p * down), fs = (float)(s1 * down);
+  double td = fs / (fp + sqrtf(fmaf(fp, fp, fs * fs)));
+  if (fs < 0x1p-60f * fp) td = 0.5 * (s1 / p);
+  if (bb < aa) td = -td;
+  cs = rsqrt(fma(td, td, 1.0));
+  sn = cs * td;
+  sj = cc < 0.0 ? -sn : sn;
+  cj = cc < 0.0 ? -cs : cs;
+  return true;
+}
+
+// One-sided Jacobi on N columns of `rows` rows at J (stride js), the rotations
+// accumulated in V (stride vs) with VECS. In round t of the round-robin over an
+// even number E of players, E - 1 meets t and the others meet the one with
+// t + p = t - p (mod E - 1): E / 2 disjoint pairs, LP lanes each (R8: with LP = 8 only).
 template <bool VECS, int R8, int LP>
 __device__ __forceinline__ void jacobi_round(double* J, int js, double* V, int vs, int N, int rows, int t,
                                              float& worst) {
@@ -205,25 +245,8 @@ __device__ __forceinline__ void jacobi_round(double* J, int js, double* V, int v
   aa = lane_sum<LP>(aa);
   bb = lane_sum<LP>(bb);
   cc = lane_sum<LP>(cc);
-  if (!on || !(aa > 0.0) || !(bb > 0.0) || !(fabs(cc) > 0.0)) return;  // nothing to turn (or a NaN)
-  if (isinf(aa) || isinf(bb) || isinf(cc)) return;
-  // |cc| / sqrt(aa bb): aa and bb scaled to [1, 4) by even powers of two
-  const int ea = max(min(exponent(aa), 1022), -1022) & ~1, eb = max(min(exponent(bb), 1022), -1022) & ~1;
-  const float fa = (float)(aa * power2(-ea)), fb = (float)(bb * power2(-eb));
-  const float fc = (float)(fabs(cc) * power2(-((ea + eb) / 2)));
-  worst = fmaxf(worst, fc * rsqrtf(fa * fb));
-  // tan of the rotation angle, the smaller root of t^2 + 2 zeta t - 1 = 0 with
-  // zeta = (bb - aa) / (2 |cc|); both legs halved and scaled by one power of two. An
-  // angle near or below FP32's range (columns of very different lengths) would
-  // never turn the pair: there the root is 1 / (2 zeta) to the last bit.
-  const double p = fabs(0.5 * bb - 0.5 * aa), s1 = fabs(cc);
-  const double down = power2(-max(min(max(exponent(p), exponent(s1)), 1022), -1022));
-  const float fp = (float)(p * down), fs = (float)(s1 * down);
-  double td = fs / (fp + sqrtf(fmaf(fp, fp, fs * fs)));
-  if (fs < 0x1p-60f * fp) td = 0.5 * (s1 / p);
-  if (bb < aa) td = -td;
-  const double cs = rsqrt(fma(td, td, 1.0)), sn = cs * td;
-  const double sj = cc < 0.0 ? -sn : sn, cj = cc < 0.0 ? -cs : cs;
+  double cs, sn, sj, cj;
+  if (!on || !jacobi_angle(aa, bb, cc, worst, cs, sn, sj, cj)) return;
   if constexpr (R8 > 0) {
 #pragma unroll
     for (int q = 0; q < R8; ++q) {
@@ -251,12 +274,63 @@ __device__ __forceinline__ void jacobi_round(double* J, int js, double* V, int v
   }
 }
 
+// One pair by the whole CTA: few and very long columns.
 template <bool VECS>
-__device__ __forceinline__ void jacobi_sweeps(double* J, int js, double* V, int vs, int N, int rows, float* s_off) {
+__device__ __forceinline__ void jacobi_wide(double* wi, double* wj, double* vi, double* vj, int N, int rows,
+                                            double (*red)[LT / 32], float& worst) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double aa = 0.0, bb = 0.0, cc = 0.0;
+  for (int r = threadIdx.x; r < rows; r += LT) {
+    const double x = wi[r], y = wj[r];
+    aa = fma(x, x, aa);
+    bb = fma(y, y, bb);
+    cc = fma(x, y, cc);
+  }
+  aa = lane_sum<32>(aa);
+  bb = lane_sum<32>(bb);
+  cc = lane_sum<32>(cc);
+  if (lane == 0) {
+    red[0][warp] = aa;
+    red[1][warp] = bb;
+    red[2][warp] = cc;
+  }
+  __syncthreads();
+  aa = bb = cc = 0.0;
+#pragma unroll
+  for (int w = 0; w < LT / 32; ++w) {
+    aa += red[0][w];
+    bb += red[1][w];
+    cc += red[2][w];
+  }
+  double cs, sn, sj, cj;
+  if (jacobi_angle(aa, bb, cc, worst, cs, sn, sj, cj)) {  // the same in every thread
+    for (int r = threadIdx.x; r < rows; r += LT) {
+      const double x = wi[r], y = wj[r];
+      wi[r] = cs * x - sj * y;
+      wj[r] = sn * x + cj * y;
+    }
+    if (VECS && (int)threadIdx.x < N) {
+      const double x = vi[threadIdx.x], y = vj[threadIdx.x];
+      vi[threadIdx.x] = cs * x - sj * y;
+      vj[threadIdx.x] = sn * x + cj * y;
+    }
+  }
+  __syncthreads();  // the columns are final, and red has been read
+}
+
+template <bool VECS>
+__device__ __forceinline__ void jacobi_sweeps(double* J, int js, double* V, int vs, int N, int rows, float* s_off,
+                                              double (*red)[LT / 32]) {
   const int E = N + (N & 1), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int sweep = 0; sweep < 60 && N > 1; ++sweep) {
     float worst = 0.f;
-    for (int t = 0; t < E - 1; ++t) {
+    const bool by_cta = VECS && wide_pairs(N, rows);
+    if (by_cta) {
+      for (int i = 0; i < N; ++i)
+        for (int j = i + 1; j < N; ++j)
+          jacobi_wide<VECS>(J + i * js, J + j * js, V + i * vs, V + j * vs, N, rows, red, worst);
+    }
+    for (int t = 0; t < E - 1 && !by_cta; ++t) {
       if (rows <= 32) jacobi_round<VECS, 4, 8>(J, js, V, vs, N, rows, t, worst);
       else if (E / 2 > LT / 32) jacobi_round<VECS, 0, 8>(J, js, V, vs, N, rows, t, worst);
       else jacobi_round<VECS, 0, 32>(J, js, V, vs, N, rows, t, worst);  // a warp for each of few pairs
@@ -297,6 +371,7 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
   double* sinv = sig + N;
   int* ord = reinterpret_cast<int*>(lsq + l.ord);
   __shared__ float s_off[LT / 32];
+  __shared__ double red[3][LT / 32];
   __shared__ int s_rank, s_leave;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -405,8 +480,8 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
   // A triangle of full rank gives x by substitution: V is only accumulated (in
   // sweeps of their own) for the rank-deficient ones.
   bool vecs = !qr;
-  if (vecs) jacobi_sweeps<true>(J, js, V, l.vs, N, Mj, s_off);
-  else jacobi_sweeps<false>(J, js, V, l.vs, N, Mj, s_off);
+  if (vecs) jacobi_sweeps<true>(J, js, V, l.vs, N, Mj, s_off, red);
+  else jacobi_sweeps<false>(J, js, V, l.vs, N, Mj, s_off, red);
 again:
   // singular values: the column norms; the columns normalised in place
   for (int c = warp; c < N; c += NWARP) {
@@ -465,7 +540,7 @@ again:
       J[c * js + r] = R[c * js + r];
     }
     __syncthreads();
-    jacobi_sweeps<true>(J, js, V, l.vs, N, Mj, s_off);
+    jacobi_sweeps<true>(J, js, V, l.vs, N, Mj, s_off, red);
     vecs = true;
     goto again;
   }
@@ -565,11 +640,12 @@ again:
     }
     __syncthreads();  // buf is refilled by the next group; x is complete for the residuals
     if (form) {
-      // residuals, one warp per column: (qr) the part of Q^T b that the
-      // columns of A cannot reach, else the rows of b - A x
-      for (int j = warp; j < jn; j += NWARP) {
+      // residuals: (qr) the part of Q^T b that the columns of A cannot reach, else the
+      // rows of b - A x; one warp per column, or the whole CTA where few columns are long
+      const bool all = m >= 256 && (jn < NWARP || !qr);
+      for (int j = all ? 0 : warp; j < jn; j += all ? 1 : NWARP) {
         double acc = 0.0;
-        for (int i = (qr ? n : 0) + lane; i < m; i += 32) {
+        for (int i = (qr ? n : 0) + (all ? tid : lane); i < m; i += all ? LT : 32) {
           double d;
           if (qr) {
             d = buf[(size_t)j * l.ws + i];
@@ -581,7 +657,18 @@ again:
           acc = fma(d, d, acc);
         }
         acc = lane_sum<32>(acc);
-        if (lane == 0) resid[z * k + j0 + j] = acc;
+        if (!all) {
+          if (lane == 0) resid[z * k + j0 + j] = acc;
+          continue;
+        }
+        if (lane == 0) red[j & 1][warp] = acc;
+        __syncthreads();
+        if (tid == 0) {
+          double sum = 0.0;
+#pragma unroll
+          for (int w = 0; w < NWARP; ++w) sum += red[j & 1][w];
+          resid[z * k + j0 + j] = sum;
+        }
       }
       __syncthreads();
     }

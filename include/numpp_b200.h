@@ -142,7 +142,10 @@ int nppb_solve_det_batched(int64_t count, int32_t n, int32_t nrhs, const double*
 /* `flags` selects outputs: NPPB_WANT_* below. Null output pointers are
  * allowed for outputs not selected. dLU/dipiv are the factor workspace
  * (count*n*n doubles, count*n int32); pass NULL to let the library allocate
- * it stream-ordered for the call. With NPPB_WANT_LU the factors stay there. */
+ * it stream-ordered for the call. With NPPB_WANT_LU the factors stay there;
+ * without it orders above 32 use dLU where n is a multiple of 4 and dLU 16-byte
+ * aligned (dLU may be dA), and allocate about 520 n bytes a system beside it (the whole
+ * workspace otherwise), for as many systems at a time as fit the device. */
 enum {
   NPPB_WANT_LU = 1,
   NPPB_WANT_SOLVE = 2,

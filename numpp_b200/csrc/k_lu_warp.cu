@@ -17,8 +17,8 @@
 // A warp's chain of instructions bounds few systems. CHAIN (full tiles, order 32, with
 // at most one right-hand side) shortens it: eight columns of the update at a time, the
 // forward substitution riding along with the elimination, and one reduction where a
-// single lane holds the largest high word: 256 systems, solve and det, 26.9 us without
-// it, 22.5 us with it. It costs more instructions than it saves in latency below order
+// single lane holds the largest high word: 256 systems, solve and det, 25.2 us without
+// it, 21.1 us with it. It costs more instructions than it saves in latency below order
 // 32 (launch_np) and with up to eight columns a chunk (RC = 8; 4000 systems of order
 // 24 with 5: 70 us without, 78 us with).
 //

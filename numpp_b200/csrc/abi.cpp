@@ -255,7 +255,10 @@ int d_getrs(int64_t count, int32_t n, int32_t nrhs, const double* dLU, const int
   if (count == 0 || n == 0 || nrhs == 0) return NPPB_OK;
   if (!dLU || !dipiv || !dB || !dX) return arg_error("getrs needs LU, ipiv, B and X");
   if (!device()) return NPPB_E_NODEV;
-  if (n > 32 && many_strips(n, count * ((nrhs + 31) / 32), 1000, 300, 90)) {
+  // (not under capture: a plan's executions wait for one another across streams)
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (many_strips(n, count * ((nrhs + 31) / 32), 1000, 300, 90) &&
+      cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
     int rc = NPPB_OK;
     auto pl = uniform_plan(count, n, nrhs, NPPB_WANT_SOLVE, true, false, &rc);
     DevMem tmp;

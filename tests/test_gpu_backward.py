@@ -175,3 +175,42 @@ def test_many_right_hand_sides_of_kept_factors(torch):
         r = (A @ X - B).abs().amax(dim=1)
         scale = A.abs().sum(dim=2).amax(dim=1)[:, None] * X.abs().amax(dim=1) + B.abs().amax(dim=1)
         assert bool((r <= 10 * n * EPS * scale).all())
+
+
+def test_many_right_hand_sides_under_capture(torch):
+    """Captured twice, the calls replay to what they give outside (the re-solve takes its general
+    form there, so its digits may differ)."""
+    from numpp_b200 import _lib, device
+    P, L = _lib.ptr, _lib.load()
+    n, k, count = 1030, 2048, 16
+    A = torch.from_numpy(matrices(n)[:4]).cuda().repeat(4, 1, 1)
+    A.diagonal(dim1=1, dim2=2).add_(1.0)
+    B = torch.randn(count, n, k, dtype=torch.float64, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    LU = torch.empty_like(A)
+    piv, info = (torch.zeros(s, dtype=torch.int32, device="cuda") for s in ((count, n), (count,)))
+    assert L.nppb_d_linalg_batched(count, n, 0, _lib.WANT_LU, P(A), None, None, None, None, None, None, P(LU), P(piv),
+                                   P(info), st) == _lib.OK
+    X = torch.zeros(2, count, n, k, dtype=torch.float64, device="cuda")
+
+    def calls():
+        s = torch.cuda.current_stream().cuda_stream
+        assert L.nppb_d_getrs_batched(count, n, k, P(LU), P(piv), P(B), P(X[0]), s) == _lib.OK, _lib.last_error()
+        assert L.nppb_d_linalg_batched(count, n, k, _lib.WANT_SOLVE, P(A), P(B), P(X[1]), None, None, None, None, None,
+                                       None, P(info), s) == _lib.OK, _lib.last_error()
+
+    calls()
+    torch.cuda.synchronize()
+    want = X.clone()
+    for _ in range(2):
+        X.zero_()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            calls()
+        graph.replay()
+        torch.cuda.synchronize()
+        for x, w in zip(X, want):
+            r = (A @ x - B).abs().amax()
+            scale = A.abs().sum(dim=2).amax() * x.abs().amax() + B.abs().amax()
+            assert bool(r <= 10 * n * EPS * scale)
+        assert torch.equal(X[1], want[1])

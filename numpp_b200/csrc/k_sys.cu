@@ -242,6 +242,15 @@ __device__ __forceinline__ void tile_negate(const double* Tb, double* Ut) {
   }
 }
 
+// The marks of a system's blocks, at most 16: L's in the lower half, U's in the upper. Read once
+// on entry, behind the strip's own loads, instead of from the tile after each block's barrier:
+// 229 re-solves of 201 x 64 160 us (166), 400 inverses of order 201 914 us (922). On clusters the
+// tile's form stays: 48 re-solves of 777 x 16 take 208 us with it, 223 us with this one.
+__device__ __forceinline__ unsigned tri_marks(const double* dinv, int nb) {
+  const int lane = threadIdx.x & 31, b = lane & 15;
+  return __ballot_sync(kAll, b < nb && dinv[b * 2048 + (lane < 16 ? 31 : 1024 + 31 * 32 + 1)] != 0.0);
+}
+
 // The product's rows to memory, by warps first .. first + count - 1 (those that
 // have nothing to update): row(r) is where row r goes, or null; PAIRS: 16 bytes
 // at once, else up to `cols` columns.
@@ -1283,6 +1292,7 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
   const double* const W = s.v.W;
   const int n = s.v.n, nb = sys_blocks(n);
   if constexpr (CS > 1) cluster_arrive();
+  const unsigned marks = CS == 1 ? tri_marks(s.v.dinv, nb) : 0u;
   Acc<NI> acc;
   Rows r;
   r.live = n - 32 * blk - g;
@@ -1310,7 +1320,8 @@ __device__ __forceinline__ void solve_strip(const SysArgs& sa, const Strip& s, d
       cp_wait<2>();  // the inverse; at most two operand stages stay in flight
       __syncthreads();
       constexpr bool kUp = decltype(upper)::value;
-      if (!tri_marked<kUp>(Li)) {  // uniform
+      const bool marked = CS == 1 ? marks >> (kUp ? K + 16 : K) & 1 : tri_marked<kUp>(Li);  // uniform
+      if (!marked) {
         tile_product<NI, kUp, CS>(Li, Tb, Ut);
       } else {
         tile_substitute<NI, kUp>(Li, Tb);

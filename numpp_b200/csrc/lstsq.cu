@@ -350,7 +350,10 @@ __device__ __forceinline__ void jacobi_sweeps(double* J, int js, double* V, int 
 
 // One problem per CTA. A (m x n), B (m x k) row-major in global memory; X
 // (n x k), S (min(m, n)), rank, resid (k) and has_resid out. k = 0: singular
-// values (and rank) only.
+// values (and rank) only. QR: by way of the triangle. Each way has its own kernel: in one
+// for both the direct way ran 2 to 14% longer (2000 of 5 x 2000 with 64 and rcond = 0 2587 us,
+// 2123 now; 300 of 64 x 2 11.4, 10.4).
+template <bool QR>
 __global__ void __launch_bounds__(LT, 4)
 k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restrict__ B, double rcond, LsqLayout l,
         int left_only, double* __restrict__ X, double* __restrict__ S, int32_t* __restrict__ rank,
@@ -391,15 +394,14 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
   // spread it, and a reflection's sums must stay within range: such a problem is
   // left to the launch that sweeps the matrix itself (here, at a reflection of tiny
   // length below, and at the right-hand sides)
-  const bool qr = l.qr;
-  if (tid == 0) s_leave = 0;
-  if (qr && __syncthreads_or(odd)) {
+  if (QR && tid == 0) s_leave = 0;
+  if (QR && __syncthreads_or(odd)) {
     if (tid == 0) rank[z] = kLsqLeft;
     return;
   }
   const int js = l.js;
-  const int Mj = qr ? N : M;  // rows of the Jacobi columns
-  if (qr) {
+  const int Mj = QR ? N : M;  // rows of the Jacobi columns
+  if constexpr (QR) {
     const int carried = wide ? 0 : l.nbuf;  // right-hand sides reflected along
     for (int idx = tid; idx < carried * M; idx += LT) {
       const int r = idx / carried, c = idx - r * carried;
@@ -479,9 +481,8 @@ k_lstsq(int m, int n, int k, const double* __restrict__ A, const double* __restr
 
   // A triangle of full rank gives x by substitution: V is only accumulated (in
   // sweeps of their own) for the rank-deficient ones.
-  bool vecs = !qr;
-  if (vecs) jacobi_sweeps<true>(J, js, V, l.vs, N, Mj, s_off, red);
-  else jacobi_sweeps<false>(J, js, V, l.vs, N, Mj, s_off, red);
+  bool vecs = !QR;
+  jacobi_sweeps<!QR>(J, js, V, l.vs, N, Mj, s_off, red);
 again:
   // singular values: the column norms; the columns normalised in place
   for (int c = warp; c < N; c += NWARP) {
@@ -532,8 +533,8 @@ again:
   __syncthreads();
   if (tid == 0) rank[z] = s_rank;
   if (k == 0) return;
-  const bool full = !vecs && s_rank == N;
-  if (!vecs && !full) {
+  const bool full = QR && !vecs && s_rank == N;
+  if (QR && !vecs && !full) {
     __syncthreads();  // every thread has read s_rank
     for (int idx = tid; idx < N * N; idx += LT) {
       const int c = idx / N, r = idx - c * N;
@@ -550,10 +551,10 @@ again:
   double* Xz = X + z * (int64_t)n * k;
   const bool form = m > n && s_rank == n;
   if (tid == 0) has_resid[z] = form ? 1 : 0;
-  const int step = qr ? l.nbuf : k;  // right-hand sides at a time
+  const int step = QR ? l.nbuf : k;  // right-hand sides at a time
   for (int j0 = 0; j0 < k; j0 += step) {
     const int jn = min(step, k - j0);
-    if (qr && !wide && j0 > 0) {  // the first group went through the reflections with the matrix
+    if (QR && !wide && j0 > 0) {  // the first group went through the reflections with the matrix
       if (warp < jn) {
         double* x = buf + (size_t)warp * l.ws;
         for (int r = lane; r < M; r += 32) {
@@ -603,8 +604,8 @@ again:
     for (int q = warp; !full && q < N * jn; q += NWARP) {
       const int c = q / jn, j = q - c * jn;
       const double* uc = wide ? V + (size_t)ord[c] * l.vs : J + (size_t)ord[c] * js;
-      const bool own = qr && !wide;
-      const int rows = wide || qr ? N : M;
+      const bool own = QR && !wide;
+      const int rows = QR || wide ? N : M;
       double t = 0.0;
       for (int p = lane; p < rows; p += 32)
         t = fma(uc[p], own ? buf[(size_t)j * l.ws + p] : Bz[(int64_t)p * k + j0 + j], t);
@@ -614,18 +615,18 @@ again:
     __syncthreads();
     // x = (right vectors) T1: V's columns (tall), J's (wide), or (wide, qr)
     // Q applied to J's
-    const int xr = wide && qr ? N : n;
+    const int xr = QR && wide ? N : n, stride = wide ? js : l.vs;
     for (int q = tid; !full && q < xr * jn; q += LT) {
       const int i = q / jn, j = q - i * jn;
+      const double* v = (wide ? J : V) + i;
+      const double* tc = T1 + j0 + j;
       double t = 0.0;
-      for (int c = 0; c < N; ++c) {
-        const double v = wide ? J[(size_t)ord[c] * js + i] : V[(size_t)ord[c] * l.vs + i];
-        t = fma(v, T1[(size_t)c * k + j0 + j], t);
-      }
-      if (wide && qr) buf[(size_t)j * l.ws + i] = t;
+#pragma unroll 4
+      for (int c = 0; c < N; ++c) t = fma(v[ord[c] * stride], tc[c * k], t);
+      if (QR && wide) buf[(size_t)j * l.ws + i] = t;
       else Xz[(int64_t)i * k + j0 + j] = t;
     }
-    if (wide && qr) {
+    if (QR && wide) {
       __syncthreads();
       if (warp < jn) {
         double* x = buf + (size_t)warp * l.ws;
@@ -642,12 +643,12 @@ again:
     if (form) {
       // residuals: (qr) the part of Q^T b that the columns of A cannot reach, else the
       // rows of b - A x; one warp per column, or the whole CTA where few columns are long
-      const bool all = m >= 256 && (jn < NWARP || !qr);
+      const bool all = m >= 256 && (jn < NWARP || !QR);
       for (int j = all ? 0 : warp; j < jn; j += all ? 1 : NWARP) {
         double acc = 0.0;
-        for (int i = (qr ? n : 0) + (all ? tid : lane); i < m; i += all ? LT : 32) {
+        for (int i = (QR ? n : 0) + (all ? tid : lane); i < m; i += all ? LT : 32) {
           double d;
-          if (qr) {
+          if constexpr (QR) {
             d = buf[(size_t)j * l.ws + i];
           } else {
             double ax = 0.0;
@@ -698,13 +699,17 @@ int lstsq_device(int64_t count, int32_t m, int32_t n, int32_t k, const double* d
   const LsqLayout l = lsq_plan(m, n, k, rcond);
   const size_t smem = sizeof(double) * (size_t)l.doubles;
   // one value for every shape: threads with different shapes do not disturb one another
-  NPPB_CUDA(cudaFuncSetAttribute(k_lstsq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLsqMaxSmem + 4096),
+  NPPB_CUDA(cudaFuncSetAttribute(k_lstsq<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLsqMaxSmem + 4096),
             "attribute");
-  k_lstsq<<<(unsigned)count, LT, smem, st>>>(m, n, k, dA, dB, rcond, l, 0, dX, dS, drank, dres, dhas);
+  if (l.qr)
+    NPPB_CUDA(cudaFuncSetAttribute(k_lstsq<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLsqMaxSmem + 4096),
+              "attribute");
+  const auto kernel = l.qr ? k_lstsq<true> : k_lstsq<false>;
+  kernel<<<(unsigned)count, LT, smem, st>>>(m, n, k, dA, dB, rcond, l, 0, dX, dS, drank, dres, dhas);
   NPPB_CUDA(cudaGetLastError(), "least squares");
   if (l.qr) {  // problems with a NaN or an infinity; the others' CTAs return at once
     const LsqLayout d = lsq_layout(m, n, k, -1);
-    k_lstsq<<<(unsigned)count, LT, sizeof(double) * (size_t)d.doubles, st>>>(m, n, k, dA, dB, rcond, d, 1, dX, dS,
+    k_lstsq<false><<<(unsigned)count, LT, sizeof(double) * (size_t)d.doubles, st>>>(m, n, k, dA, dB, rcond, d, 1, dX, dS,
                                                                             drank, dres, dhas);
     NPPB_CUDA(cudaGetLastError(), "least squares");
   }
